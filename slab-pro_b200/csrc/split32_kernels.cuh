@@ -1687,12 +1687,14 @@ __device__ __forceinline__ void load_grid_scn(const Shared& sh, int sid, GridScn
 // K3 + K6: computeGridVelocity (src/simulation.cpp:800-875) for the TILE^2
 // nodes owned by one grid tile. A node's P2G sum is the partials of the
 // tiles whose window covers it, added in a fixed order (own, -x, -y, -xy).
-// h_max / v_max2 are updated in the node block; the FP64 grid mass sum is
-// the conservation diagnostic.
+// h_max / v_max2 are updated in the node block; the FP64 grid mass sum and
+// the active-node count are diagnostics: every CTA adds them up over its run
+// of grid tiles and touches their two addresses once per run and scenario.
+// (Two atomics per grid tile on the same two addresses held the kernel up.)
 // Latency: the scenario's values stay in shared memory across a run of its
 // grid tiles, and thread 0 reads the grid-tile list two entries ahead.
 __device__ __forceinline__ void grid_body(const Shared& sh) {
-    __shared__ int s_gt, s_blk;
+    __shared__ int s_gt, s_blk, s_sid;
     __shared__ int s_slot[4];
     __shared__ double s_red[NCELL / 32];
     __shared__ unsigned s_act[NCELL / 32];
@@ -1704,18 +1706,49 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
     // thread 0: the current and the next entry of the flat grid-tile list
     int2 e_cur = make_int2(-1, 0), e_nxt = make_int2(-1, 0);
     if (tid == 0) {
-        Z.sid = -1;
         if (w0 < w1) e_cur = reinterpret_cast<const int2*>(sh.gflat)[w0];
         if (w0 + 1 < w1) e_nxt = reinterpret_cast<const int2*>(sh.gflat)[w0 + 1];
     }
+    // mass and active nodes of this thread over the CTA's run of one scenario
+    int csid = -1;
+    double macc = 0.0;
+    unsigned nacc = 0;
+    auto flush = [&] {
+        nacc = __reduce_add_sync(0xffffffffu, nacc);
+        for (int o = 16; o > 0; o >>= 1) macc += __shfl_xor_sync(0xffffffffu, macc, o);
+        if ((tid & 31) == 0) {
+            s_red[tid >> 5] = macc;
+            s_act[tid >> 5] = nacc;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            double sum = 0.0;
+            unsigned na = 0;
+            for (int k = 0; k < NCELL / 32; ++k) {
+                sum += s_red[k];
+                na += s_act[k];
+            }
+            if (sum != 0.0) atomicAdd(&Z.n->grid_mass, sum);
+            if (na) atomicAdd(&Z.c->node_steps, (unsigned long long)na);
+        }
+        macc = 0.0;
+        nacc = 0;
+    };
     for (int w = w0; w < w1; ++w) {
         if (tid == 0) {
-            if (e_cur.x != Z.sid) load_grid_scn(sh, e_cur.x, Z);  // a new scenario in this CTA's run
+            s_sid = e_cur.x;
             s_gt = e_cur.y;
             e_cur = e_nxt;
             if (w + 2 < w1) e_nxt = reinterpret_cast<const int2*>(sh.gflat)[w + 2];
         }
         __syncthreads();
+        if (s_sid != csid) {  // uniform: a new scenario in this CTA's run
+            if (csid >= 0) flush();
+            csid = s_sid;
+            __syncthreads();
+            if (tid == 0) load_grid_scn(sh, csid, Z);
+            __syncthreads();
+        }
         Ctl* c = Z.c;
         const int gt = s_gt;
         const int gi = gt / sh.TY, gj = gt % sh.TY;
@@ -1755,7 +1788,6 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
         const int blk = s_blk;
         // the block of this grid tile is entry k of contributor k's window (for G2P)
         if (tid < 4 && s_slot[tid] >= 0) sh.desc[s_slot[tid]].blk4[tid] = blk;
-        double mloc = 0.0;
         if (blk >= 0) {
             float q[NQ];
 #pragma unroll
@@ -1813,7 +1845,8 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
                 out = make_float4(nvx, nvy, nvx - vox, nvy - voy);
                 sh.hmax[bn] = fmaxf(hmax0, hn);
                 sh.vmax2[bn] = fmaxf(vmax0, nvx * nvx + nvy * nvy);
-                mloc = (double)mi;
+                macc += (double)mi;
+                nacc += 1u;
             }
             sh.nv[bn] = out;
             if (Z.outs) {
@@ -1824,26 +1857,11 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
                 sh.oFy[bn] = inside ? q[5] : 0.f;
             }
         }
-        // FP64 grid mass and active-node count of this tile (fixed-order block reduction)
-        const unsigned act = __popc(__ballot_sync(0xffffffffu, mloc != 0.0));
-        for (int o = 16; o > 0; o >>= 1) mloc += __shfl_xor_sync(0xffffffffu, mloc, o);
-        if ((tid & 31) == 0) {
-            s_red[tid >> 5] = mloc;
-            s_act[tid >> 5] = act;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double sum = 0.0;
-            unsigned na = 0;
-            for (int k = 0; k < NCELL / 32; ++k) {
-                sum += s_red[k];
-                na += s_act[k];
-            }
-            if (sum != 0.0) atomicAdd(&Z.n->grid_mass, sum);
-            if (na) atomicAdd(&c->node_steps, (unsigned long long)na);
-        }
-        __syncthreads();
+        // (the shared values of this item are rewritten only after the next
+        // item's barriers, which every thread passes once it has read them)
     }
+    if (csid >= 0) flush();
+    __syncthreads();  // the shared memory may serve another phase next
 }
 
 __global__ void __launch_bounds__(NCELL) k_grid(Shared sh) { grid_body(sh); }
@@ -1874,6 +1892,7 @@ struct G2PScn {
     double dx;
     float dt, dt_ood, ood, fr;
     int sid, seq, act_cap, outs, need_vz;
+    int in_i0, in_i1, in_j0, in_j1;  // tiles in this range cannot hold an extreme position of the particle box
 };
 
 __device__ __forceinline__ void load_g2p_scn(const Shared& sh, int sid, G2PScn& z) {
@@ -1899,6 +1918,18 @@ __device__ __forceinline__ void load_g2p_scn(const Shared& sh, int sid, G2PScn& 
     z.act_cap = S.act_cap;
     z.outs = n->outs != 0;
     z.need_vz = z.outs || n->vz_next;
+    // Positions of the box's extreme particles at the start of the step, in
+    // cells. A particle moves to a neighbour tile at most (farther raises
+    // ERR_MOVE), less than 2 TILE cells, so after the step the box still
+    // reaches to within that of its old faces; a tile whose particles all end
+    // up further inside cannot change it.
+    constexpr int D = 2 * TILE + 2;
+    const int i0 = (int)(__longlong_as_double((long long)c->pos[0]) * c->one_over_dx), i1 = (int)(__longlong_as_double((long long)c->pos[1]) * c->one_over_dx);
+    const int j0 = (int)(__longlong_as_double((long long)c->pos[2]) * c->one_over_dx), j1 = (int)(__longlong_as_double((long long)c->pos[3]) * c->one_over_dx);
+    z.in_i0 = (i0 + D + TILE - 1) / TILE + 1;
+    z.in_i1 = (i1 - D) / TILE - 2;
+    z.in_j0 = (j0 + D + TILE - 1) / TILE + 1;
+    z.in_j1 = (j1 - D) / TILE - 2;
 }
 
 // puts tile tt on the next step's active list, once
@@ -1908,6 +1939,16 @@ __device__ __forceinline__ void g2p_activate(const G2PScn& z, int tt) {
         if (kk < z.act_cap) z.act_list_nxt[kk] = tt;
         else atomicOr(&z.c->err, ERR_CAPACITY);
     }
+}
+
+// the largest |v|^2 of a run of tiles into the scenario's control block: one
+// atomic per warp, and only if it raises the value seen (speeds squared are
+// >= 0, so their bit patterns order like the values)
+__device__ __forceinline__ void g2p_flush_vmax2(const G2PScn& z, float vmax2) {
+    const double v = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(vmax2)));
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+    unsigned long long* acc = reinterpret_cast<unsigned long long*>(&z.c->vmax2_acc);
+    if ((threadIdx.x & 31) == 0 && bits > *reinterpret_cast<volatile unsigned long long*>(acc)) atomicMax(acc, bits);
 }
 
 #ifndef SLAB_G2P_CAP
@@ -1934,7 +1975,7 @@ struct G2PSmem {
     int dcnt[9];
     TileDesc d;
     G2PScn z;
-    double red[5][NCELL / 32];
+    double red[4][NCELL / 32];
 };
 
 // one candidate of a tile in G2P: its index, data, and whether it is in the tile
@@ -2010,6 +2051,7 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
     if (w0 < w1) load_desc(sh.desc + w0, &sm.d);
     if (tid == 0) sm.z.sid = -1;
     int pend_tt = -1;  // threads 0..8: neighbour tile the previous tile activates
+    float vmax2 = 0.f;  // largest |v|^2 of this thread's particles over the CTA's run of one scenario
     SLAB_PHASE_BEGIN;
     for (int w = w0; w < w1; ++w) {
         if (tid < 9) sm.dcnt[tid] = 0;
@@ -2020,6 +2062,8 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
         if (sm.d.sid != sm.z.sid) {  // uniform: a new scenario in this CTA's run
             if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);
             pend_tt = -1;
+            if (w > w0) g2p_flush_vmax2(sm.z, vmax2);
+            vmax2 = 0.f;
             __syncthreads();
             if (tid == 0) load_g2p_scn(sh, sm.d.sid, sm.z);
             __syncthreads();
@@ -2082,7 +2126,8 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
         const float dt = Z.dt;
         const float dt_ood = Z.dt_ood;
         const double dx = Z.dx;
-        double mnx = INFINITY, mxx = 0.0, mny = INFINITY, mxy = 0.0, vv = 0.0;
+        const bool edge = ti < Z.in_i0 || ti > Z.in_i1 || tj < Z.in_j0 || tj > Z.in_j1;  // uniform: may change the particle box
+        double mnx = INFINITY, mxx = 0.0, mny = INFINITY, mxy = 0.0;
         int front = 0, back = 0;  // stayers / movers placed so far (same in every thread)
         G2PCand nxt = pre;
         for (int k0 = 0; k0 < ncand; k0 += NCELL) {
@@ -2157,12 +2202,14 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
                     d = dir_of(ib, jb, ti, tj);
                     if (d < 0) d = 4;
                 }
-                const double px = ((double)ib + (double)fn.x) * dx, py = ((double)jb + (double)fn.y) * dx;
-                mnx = fmin(mnx, px);
-                mxx = fmax(mxx, px);
-                mny = fmin(mny, py);
-                mxy = fmax(mxy, py);
-                vv = fmax(vv, (double)(vn.x * vn.x + vn.y * vn.y));
+                if (edge) {
+                    const double px = ((double)ib + (double)fn.x) * dx, py = ((double)jb + (double)fn.y) * dx;
+                    mnx = fmin(mnx, px);
+                    mxx = fmax(mxx, px);
+                    mny = fmin(mny, py);
+                    mxy = fmax(mxy, py);
+                }
+                vmax2 = fmaxf(vmax2, vn.x * vn.x + vn.y * vn.y);
                 if (!isfinite(vn.x) || !isfinite(vn.y) || !isfinite(hn) || !isfinite(fn.x) || !isfinite(fn.y))
                     atomicOr(&c->err, ERR_NONFINITE);
             }
@@ -2226,33 +2273,30 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
             }
             if (cnt) pend_tt = (ti + dir_i(tid)) * sh.TY + (tj + dir_j(tid));
         }
-        // per-tile reductions into the scenario's control block
-        mnx = warp_min(mnx);
-        mxx = warp_max(mxx);
-        mny = warp_min(mny);
-        mxy = warp_max(mxy);
-        vv = warp_max(vv);
-        if (lane == 0) {
-            sm.red[0][warp] = mnx;
-            sm.red[1][warp] = mxx;
-            sm.red[2][warp] = mny;
-            sm.red[3][warp] = mxy;
-            sm.red[4][warp] = vv;
-        }
-        __syncthreads();
-        if (tid == 0 && total > 0) {
-            for (int k = 1; k < NCELL / 32; ++k) {
-                mnx = fmin(mnx, sm.red[0][k]);
-                mxx = fmax(mxx, sm.red[1][k]);
-                mny = fmin(mny, sm.red[2][k]);
-                mxy = fmax(mxy, sm.red[3][k]);
-                vv = fmax(vv, sm.red[4][k]);
+        if (edge) {  // the tile's particle box into the scenario's control block
+            mnx = warp_min(mnx);
+            mxx = warp_max(mxx);
+            mny = warp_min(mny);
+            mxy = warp_max(mxy);
+            if (lane == 0) {
+                sm.red[0][warp] = mnx;
+                sm.red[1][warp] = mxx;
+                sm.red[2][warp] = mny;
+                sm.red[3][warp] = mxy;
             }
-            atomicMin(reinterpret_cast<unsigned long long*>(&c->pos_acc[0]), (unsigned long long)__double_as_longlong(mnx));
-            atomicMax(reinterpret_cast<unsigned long long*>(&c->pos_acc[1]), (unsigned long long)__double_as_longlong(mxx));
-            atomicMin(reinterpret_cast<unsigned long long*>(&c->pos_acc[2]), (unsigned long long)__double_as_longlong(mny));
-            atomicMax(reinterpret_cast<unsigned long long*>(&c->pos_acc[3]), (unsigned long long)__double_as_longlong(mxy));
-            atomicMax(reinterpret_cast<unsigned long long*>(&c->vmax2_acc), (unsigned long long)__double_as_longlong(vv));
+            __syncthreads();
+            if (tid == 0 && total > 0) {
+                for (int k = 1; k < NCELL / 32; ++k) {
+                    mnx = fmin(mnx, sm.red[0][k]);
+                    mxx = fmax(mxx, sm.red[1][k]);
+                    mny = fmin(mny, sm.red[2][k]);
+                    mxy = fmax(mxy, sm.red[3][k]);
+                }
+                atomicMin(reinterpret_cast<unsigned long long*>(&c->pos_acc[0]), (unsigned long long)__double_as_longlong(mnx));
+                atomicMax(reinterpret_cast<unsigned long long*>(&c->pos_acc[1]), (unsigned long long)__double_as_longlong(mxx));
+                atomicMin(reinterpret_cast<unsigned long long*>(&c->pos_acc[2]), (unsigned long long)__double_as_longlong(mny));
+                atomicMax(reinterpret_cast<unsigned long long*>(&c->pos_acc[3]), (unsigned long long)__double_as_longlong(mxy));
+            }
         }
         __syncthreads();
         if (w + 1 < w1 && tid < DESC_WORDS) reinterpret_cast<int*>(&sm.d)[tid] = dn;
@@ -2260,6 +2304,7 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
         SLAB_PHASE_TILE_G2P();
     }
     if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);  // the last tile's
+    if (w0 < w1) g2p_flush_vmax2(sm.z, vmax2);
 }
 
 __global__ void __launch_bounds__(NCELL, G2P_MIN_BLOCKS) k_g2p(Shared sh, const double* __restrict__ z64) {
