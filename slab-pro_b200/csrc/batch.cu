@@ -22,6 +22,7 @@ void set_thread_error(const std::string& msg);
 using namespace slab;
 
 struct slab_batch {
+    MemoryUser memory;  // first: destroyed after the buffers
     Terrain terrain;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
@@ -110,7 +111,7 @@ slab_status slab_batch_create(const slab_terrain_desc* td, const double* z, int3
         b->stream = b->own_stream;
         b->max_scn = max_scenarios;
         b->d_ctl = dmalloc<Ctl>(max_scenarios);
-        SLAB_CUDA(cudaMallocHost(&b->h_ctl, max_scenarios * sizeof(Ctl)));
+        b->h_ctl = static_cast<Ctl*>(take_pinned(max_scenarios * sizeof(Ctl)));
         Terrain& t = b->terrain;
         t.Nx = td->Nx;
         t.Ny = td->Ny;
@@ -354,8 +355,8 @@ void slab_batch_destroy(slab_batch* b) {
     b->terrain.grad.reset();
     b->terrain.cos_t.reset();
     b->terrain.dem32.reset();
-    if (b->d_ctl) cudaFree(b->d_ctl);
-    if (b->h_ctl) cudaFreeHost(b->h_ctl);
+    release_device(b->d_ctl);
+    release_pinned(b->h_ctl);
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     delete b;
 }

@@ -31,6 +31,7 @@ struct FrameSlot {
 };
 
 struct slab_ctx {
+    MemoryUser memory;  // first: destroyed after the buffers
     Terrain terrain;
     slab_params params{};
     bool have_params = false;
@@ -218,7 +219,7 @@ slab_status slab_create(const slab_terrain_desc* td, const double* z, slab_ctx**
         SLAB_CUDA(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
         c->stream = c->own_stream;
         c->d_ctl = dmalloc<Ctl>(1);
-        SLAB_CUDA(cudaMallocHost(&c->h_ctl, sizeof(Ctl)));
+        c->h_ctl = static_cast<Ctl*>(take_pinned(sizeof(Ctl)));
         Terrain& t = c->terrain;
         t.Nx = td->Nx;
         t.Ny = td->Ny;
@@ -413,13 +414,11 @@ slab_status slab_frame_capture(slab_ctx* c, int32_t slot) {
         const int64_t nodes = nI > 0 && nJ > 0 ? nI * nJ : 0;
         const size_t need_f = (size_t)c->Np * 8 + (size_t)nodes * 6;
         if (need_f > F.cap) {
-            if (F.host) cudaFreeHost(F.host);
+            release_pinned(F.host);  // its copy is over
             F.host = nullptr;
             F.cap = 0;
             F.dev = dalloc<float>(need_f);
-            void* h = nullptr;
-            SLAB_CUDA(cudaMallocHost(&h, need_f * sizeof(float)));
-            F.host = static_cast<float*>(h);
+            F.host = static_cast<float*>(take_pinned(need_f * sizeof(float)));
             F.cap = need_f;
         }
         if (!F.packed) {
@@ -551,7 +550,7 @@ void slab_destroy(slab_ctx* c) {
         cudaStreamDestroy(c->copy_stream);
     }
     for (FrameSlot& F : c->frames) {
-        if (F.host) cudaFreeHost(F.host);
+        release_pinned(F.host);
         if (F.packed) cudaEventDestroy(F.packed);
         if (F.copied) cudaEventDestroy(F.copied);
         F.dev.reset();
@@ -561,8 +560,8 @@ void slab_destroy(slab_ctx* c) {
     c->terrain.grad.reset();
     c->terrain.cos_t.reset();
     c->terrain.dem32.reset();
-    if (c->d_ctl) cudaFree(c->d_ctl);
-    if (c->h_ctl) cudaFreeHost(c->h_ctl);
+    release_device(c->d_ctl);
+    release_pinned(c->h_ctl);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
 }

@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "blocks.hpp"
 #include "common.cuh"
 #include "slab_gpu.h"
 
@@ -32,19 +33,10 @@ struct Error {
                                 std::string(#call) + ": " + cudaGetErrorString(e_)};                        \
     } while (0)
 
-template <typename T> T* dmalloc(size_t n) {
-    void* p = nullptr;
-    if (n == 0) n = 1;
-    cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        throw Error{SLAB_E_OOM, "cudaMalloc of " + std::to_string(n * sizeof(T)) + " bytes failed: " + cudaGetErrorString(e)};
-    }
-    return static_cast<T*>(p);
-}
+template <typename T> T* dmalloc(size_t n) { return static_cast<T*>(take_device((n ? n : 1) * sizeof(T))); }
 
 struct DFree {
-    void operator()(void* p) const { cudaFree(p); }
+    void operator()(void* p) const { release_device(p); }
 };
 template <typename T> using dptr = std::unique_ptr<T, DFree>;
 template <typename T> dptr<T> dalloc(size_t n) { return dptr<T>(dmalloc<T>(n)); }
@@ -58,7 +50,7 @@ struct Scratch {
     size_t cap = 0;
     char* get(size_t bytes) {
         if (bytes > cap) {
-            buf.reset();  // cudaFree waits for the device: no work still uses the old buffer
+            buf.reset();  // handed out again only once no work uses it (blocks.hpp)
             buf = dalloc<char>(bytes);
             cap = bytes;
         }

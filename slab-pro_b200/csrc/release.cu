@@ -101,6 +101,38 @@ __global__ void k_release_particles(Shape S, int Np, const int* __restrict__ sel
     }
 }
 
+// h added n times to 0.0, each sum rounded to double, without n additions.
+// Within a binade [B/2, B) the sums are multiples of one ulp u, and once one
+// sum has been rounded there every further addition adds the same multiple of
+// u: h rounded to u, a tie always to the same side, since the first sum's last
+// bit is then even and an even increment keeps it so. So a binade is one
+// rounded addition and one exact product. (12 M additions took 13 ms.)
+double repeated_sum(double h, int64_t n) {
+    double s = 0.0;
+    int64_t k = 0;
+    while (k < n) {
+        const double a = s + h, b = a + h;  // two rounded additions
+        if (k + 2 > n || std::ilogb(a) != std::ilogb(b)) {
+            s = a;
+            ++k;
+            continue;
+        }
+        s = b;
+        k += 2;
+        const double B = std::ldexp(1.0, std::ilogb(b) + 1);
+        const double d = (b + h) - b;  // the binade's increment, exact while b + h < B
+        if (!(b + h < B) || !(d > 0.0)) continue;
+        // sums that stay below B with one increment to spare; the products and
+        // sums are multiples of u below B: exact
+        const int64_t m = std::min<int64_t>(n - k, (int64_t)((B - b) / d) - 2);
+        if (m > 0) {
+            s = b + (double)m * d;
+            k += m;
+        }
+    }
+    return s;
+}
+
 }  // namespace
 
 int64_t release_estimate(const slab_release& r, double dx) {
@@ -158,9 +190,7 @@ DevRelease generate_release(const Terrain& T, const slab_release& r, double rho,
     SLAB_CUDA(cudaStreamSynchronize(st));
     if (Np <= 0) throw Error{SLAB_E_ARG, "the release holds no sample"};
     // A = V / sum h with sum h accumulated in particle order (src/simulation.cpp:428-441)
-    double sum_h = 0.0;
-    for (int p = 0; p < Np; ++p) sum_h += r.h0;
-    const double A_init = volume / sum_h;
+    const double A_init = volume / repeated_sum(r.h0, Np);
     DevRelease out;
     out.Np = Np;
     out.buf = dalloc<double>((size_t)9 * Np);

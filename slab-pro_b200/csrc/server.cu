@@ -66,6 +66,7 @@ struct Request {
 }  // namespace
 
 struct slab_server {
+    MemoryUser memory;  // first: destroyed after the buffers
     Terrain terrain;
     cudaStream_t stream = nullptr;
     int max_slots = 0;
@@ -349,7 +350,7 @@ slab_status slab_server_create(const slab_terrain_desc* td, const double* z, con
         s->max_slots = cfg->max_scenarios;
         s->chunk = cfg->chunk_steps > 0 ? cfg->chunk_steps : 32;
         s->d_ctl = dmalloc<Ctl>(s->max_slots);
-        SLAB_CUDA(cudaMallocHost(&s->h_ctl, s->max_slots * sizeof(Ctl)));
+        s->h_ctl = static_cast<Ctl*>(take_pinned(s->max_slots * sizeof(Ctl)));
         Terrain& t = s->terrain;
         t.Nx = td->Nx;
         t.Ny = td->Ny;
@@ -371,7 +372,7 @@ slab_status slab_server_create(const slab_terrain_desc* td, const double* z, con
         SLAB_CUDA(cudaStreamSynchronize(s->stream));
         size_t free_b = 0, total_b = 0;
         SLAB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        s->budget = cfg->hbm_budget_bytes > 0 ? cfg->hbm_budget_bytes : (int64_t)(free_b / 2);
+        s->budget = cfg->hbm_budget_bytes > 0 ? cfg->hbm_budget_bytes : (int64_t)((free_b + kept_device_bytes()) / 2);
         s->slot_req.assign(s->max_slots, -1);
         s->worker = std::thread(worker_loop, s);
     });
@@ -588,8 +589,8 @@ void slab_server_destroy(slab_server* s) {
     s->terrain.grad.reset();
     s->terrain.cos_t.reset();
     s->terrain.dem32.reset();
-    if (s->d_ctl) cudaFree(s->d_ctl);
-    if (s->h_ctl) cudaFreeHost(s->h_ctl);
+    release_device(s->d_ctl);
+    release_pinned(s->h_ctl);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
 }
