@@ -157,6 +157,8 @@ class Engine32 {
     dptr<int32_t> d_blk_stamp, d_blk_owner, d_misc, d_work_pref, d_gflat, d_wlist, d_free_blocks;
     dptr<Scn> d_scn;
     dptr<SCnt> d_cnt;
+    dptr<SDyn> d_dyn;
+    Ctl* ctl0 = nullptr;  // control block of scenario 0 (scenario s has ctl0 + s)
     std::vector<SCnt> h_cnt;
     dptr<TileDesc> d_desc;
     dptr<float> d_part;

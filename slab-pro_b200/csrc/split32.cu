@@ -236,6 +236,7 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     d_work_pref = dalloc<int32_t>(max_scn + 1);
     d_scn = dalloc<Scn>(max_scn);
     d_cnt = dalloc<SCnt>(max_scn);
+    d_dyn = dalloc<SDyn>(max_scn);
     h_cnt.resize(max_scn);
     slots.resize(max_scn);
     spare.resize(max_scn);
@@ -322,6 +323,7 @@ Shared Engine32::shared() const {
     sh.Ny = T.Ny;
     sh.TX = TX;
     sh.TY = TY;
+    sh.dx = T.dx;
     sh.dem = T.dem32.get();
     sh.nv = d_nv.get();
     sh.hmax = d_hmax.get();
@@ -338,6 +340,8 @@ Shared Engine32::shared() const {
     sh.nscn = nscn;
     sh.scn = d_scn.get();
     sh.cnt = d_cnt.get();
+    sh.ctl = ctl0;
+    sh.dyn = d_dyn.get();
     sh.work_pref = d_work_pref.get();
     sh.wlist = d_wlist.get();
     sh.wcount = d_misc.get() + 2;
@@ -533,6 +537,11 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
         S.blk_of = dalloc<int32_t>(ntiles);
     }
     S.cnt = d_cnt.get() + sid;
+    if (!ctl0) {
+        ctl0 = ctl - sid;
+        graphs.clear();
+    }
+    if (ctl0 + sid != ctl) throw Error{SLAB_E_STATE, "control blocks of a context's scenarios must be consecutive"};
     ensure_work_cap(work_cap_total + S.act_cap);
     work_cap_total += S.act_cap;
 
@@ -615,13 +624,13 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
 }
 
 void Engine32::launch_begin(int t0) {
-    k32::k_begin<<<1, 1024, 0, st>>>(shared(), t0);
+    k32::k_begin<<<1, k32::CTL_THREADS, 0, st>>>(shared(), t0);
     SLAB_CUDA(cudaGetLastError());
 }
 
 void Engine32::launch_t0() {
     const Shared sh = shared();
-    k32::k_begin<<<1, 1024, 0, st>>>(sh, 1);
+    k32::k_begin<<<1, k32::CTL_THREADS, 0, st>>>(sh, 1);
     k32::k_prep<<<grid_prep, 256, 0, st>>>(sh);
     launch_p2g(sh);
     k32::k_grid<<<grid_grid, NCELL, 0, st>>>(sh);
@@ -662,12 +671,12 @@ void Engine32::launch_kernel(int k, const Shared& sh) {
         case 1: launch_p2g(sh); break;
         case 2: k32::k_grid<<<grid_grid, NCELL, 0, st>>>(sh); break;
         case 3: k32::k_g2p<<<grid_g2p, NCELL, 0, st>>>(sh, T.z.get()); break;
-        case 4: k32::k_end<<<1, 1024, 0, st>>>(sh); break;
+        case 4: k32::k_end<<<1, k32::CTL_THREADS, 0, st>>>(sh); break;
     }
 }
 
 void Engine32::arm(int64_t steps_left, int stop_at_frame) {
-    k32::k_arm_begin<<<1, 1024, 0, st>>>(shared(), steps_left, stop_at_frame);
+    k32::k_arm_begin<<<1, k32::CTL_THREADS, 0, st>>>(shared(), steps_left, stop_at_frame);
     SLAB_CUDA(cudaGetLastError());
     nlaunch += 1;
 }
@@ -740,7 +749,7 @@ void Engine32::launch_step_timed(const Shared& sh, cudaEvent_t* e) {
     SLAB_CUDA(cudaEventRecord(e[4], st));
     k32::k_g2p<<<grid_g2p, NCELL, 0, st>>>(sh, T.z.get());
     SLAB_CUDA(cudaEventRecord(e[5], st));
-    k32::k_end<<<1, 1024, 0, st>>>(sh);
+    k32::k_end<<<1, k32::CTL_THREADS, 0, st>>>(sh);
     SLAB_CUDA(cudaEventRecord(e[6], st));
 }
 

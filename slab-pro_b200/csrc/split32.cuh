@@ -68,6 +68,16 @@ struct SCnt {
     int32_t vz_valid;      // buffer vz / z were written by the last G2P (an output step)
 };
 
+// Values of one scenario that hold for a whole step, written at its start by
+// the control kernels (begin_scenarios): with the static descriptor (Scn) all
+// that the other kernels need to know, so that a CTA loads both in one round.
+struct alignas(16) SDyn {
+    int32_t seq, stepid, outs, need_vz;
+    float dt, dt_ood;
+    int32_t in_i0, in_i1, in_j0, in_j1;  // tiles in this range cannot hold an extreme position of the particle box
+    int32_t pad_[2];
+};
+
 // Work descriptor of one active tile t for the running step (written by
 // k_prep). Its particles are found in 9 candidate ranges of the current
 // buffer: range 4 holds the stayers of t's own segment, range d != 4 the
@@ -91,7 +101,7 @@ constexpr int GRP_STRIDE = 16;
 constexpr int GRP_STAMP = 12;
 
 // Device descriptor of one scenario.
-struct Scn {
+struct alignas(16) Scn {
     Ctl* ctl;
     SCnt* cnt;
     // physics (FP32 copies of slab_params)
@@ -114,6 +124,7 @@ struct Scn {
 // Shared by all scenarios of a context: terrain and node-block pool.
 struct Shared {
     int32_t Nx, Ny, TX, TY;
+    double dx;
     const float4* dem;  // gx, gy, cos(theta), z per node
     // node blocks, NCELL nodes each
     float4* nv;        // vx, vy, flip x, flip y
@@ -131,6 +142,8 @@ struct Shared {
     int32_t nscn;
     const Scn* scn;
     SCnt* cnt;            // [nscn] step counters (scn[s].cnt == cnt + s)
+    Ctl* ctl;             // [nscn] control blocks (scn[s].ctl == ctl + s)
+    SDyn* dyn;            // [nscn] values of the running step
     int32_t* work_pref;   // [nscn+1] prefix of active tiles (P2G / G2P work)
     int32_t* wlist;       // [2][work_cap] work items of the two P2G kernels: dense tiles, then sparse ones
     int32_t* wcount;      // [2] their counts

@@ -141,45 +141,98 @@ __device__ __forceinline__ int tile_of_cell(int32_t cell, int TY) { return (cell
 
 // ---------------------------------------------------------------- control
 
-// K5 (first half), run by one CTA: per scenario, the stop rules of the
-// running advance call and Simulation::updateDt (ctl_begin), then the
-// prefix of active tiles over scenarios (the work list of the step).
-// t0_pass: simulate()'s t=0 pass for scenarios that still need it.
-__device__ void begin_scenarios(const Shared& sh, int t0_pass) {
+// Step control of one scenario, one thread: what the step before left (its
+// end), then the stop rules of the running advance call and
+// Simulation::updateDt (ctl_begin), then the values that the step's kernels
+// read. The control block and counters are read whole in one round and written
+// back once: field by field, each branch waited for its own load (5.3 us for
+// the kernel with one scenario, the time of about 12 dependent loads).
+enum : int { CTL_BEGIN = 0, CTL_T0 = 1, CTL_ARM = 2, CTL_END = 3 };
+
+__device__ __forceinline__ int step_control(const Shared& sh, int s, int what, int64_t steps_left, int stop_at_frame) {
+    Ctl k = sh.ctl[s];
+    SCnt n = sh.cnt[s];
+    const int Np = sh.scn[s].Np;
+    const float ood = sh.scn[s].ood;
+    if (what == CTL_ARM) {  // start of an advance call: its step budget and frame-stop rule
+        k.stop = 0;
+        k.frame_hit = 0;
+        k.steps_left = steps_left;
+        k.stop_at_frame = stop_at_frame;
+    }
+    if (what == CTL_END && k.active) {
+        if (n.cursor != Np) k.err |= ERR_CAPACITY;
+        ctl_end(&k);
+        n.seq += 1;
+        n.vz_valid = n.outs;
+    }
+    if (what == CTL_T0) {  // simulate()'s t=0 pass for scenarios that still need it
+        if (n.t0_pending) {
+            ctl_begin_t0(&k, sh.Nx, sh.Ny);
+            n.t0_pending = 0;
+        } else {
+            k.active = 0;
+        }
+    } else if (n.t0_pending) {
+        k.active = 0;  // added after the last t=0 pass: waits for the next one
+    } else {
+        ctl_begin(&k, sh.Nx, sh.Ny);
+    }
+    int cnt = 0;
+    if (k.active) {
+        n.stepid += 1;
+        n.act_count[0] = (n.seq & 1) ? 0 : n.act_count[0];  // the next step's list starts empty
+        n.act_count[1] = (n.seq & 1) ? n.act_count[1] : 0;
+        n.cursor = 0;
+        n.grid_mass = 0.0;
+        n.outs = k.write_outputs;
+        const int frame_after = k.frame + (k.frame_end ? 1 : 0);
+        const double nft = __dmul_rn(k.output_dt, (double)(frame_after + 1));
+        n.vz_next = (k.keep_outputs || __dadd_rn(k.new_time, k.dt_max) > nft - 1e-12) ? 1 : 0;
+        cnt = (n.seq & 1) ? n.act_count[1] : n.act_count[0];
+        SDyn y;
+        y.seq = n.seq;
+        y.stepid = n.stepid;
+        y.outs = n.outs != 0;
+        y.need_vz = n.outs || n.vz_next;
+        y.dt = (float)k.dt;
+        y.dt_ood = y.dt * ood;
+        // Cells of the box's extreme particles at the start of the step. A
+        // particle moves to a neighbour tile at most (farther raises
+        // ERR_MOVE), less than 2 TILE cells, so after the step the box still
+        // reaches to within that of its old faces; a tile whose particles all
+        // end up further inside cannot change it.
+        constexpr int D = 2 * TILE + 2;
+        const int i0 = (int)(__longlong_as_double((long long)k.pos[0]) * k.one_over_dx);
+        const int i1 = (int)(__longlong_as_double((long long)k.pos[1]) * k.one_over_dx);
+        const int j0 = (int)(__longlong_as_double((long long)k.pos[2]) * k.one_over_dx);
+        const int j1 = (int)(__longlong_as_double((long long)k.pos[3]) * k.one_over_dx);
+        y.in_i0 = (i0 + D + TILE - 1) / TILE + 1;
+        y.in_i1 = (i1 - D) / TILE - 2;
+        y.in_j0 = (j0 + D + TILE - 1) / TILE + 1;
+        y.in_j1 = (j1 - D) / TILE - 2;
+        y.pad_[0] = y.pad_[1] = 0;
+        sh.dyn[s] = y;
+    }
+    sh.ctl[s] = k;
+    sh.cnt[s] = n;
+    return cnt;
+}
+
+// K5, run by one CTA: the control of every scenario, then the prefix of
+// active tiles over scenarios (the work list of the step).
+__device__ __forceinline__ void control_scenarios(const Shared& sh, int what, int64_t steps_left = 0, int stop_at_frame = 0) {
     __shared__ int s_warp[33];
     __shared__ int s_tot;
     const int tid = threadIdx.x;
     int total = 0;
     for (int base = 0; base < sh.nscn; base += blockDim.x) {
         const int s = base + tid;
-        int cnt = 0;
-        if (s < sh.nscn) {
-            const Scn& S = sh.scn[s];
-            Ctl* c = S.ctl;
-            SCnt* n = S.cnt;
-            if (t0_pass) {
-                if (n->t0_pending) {
-                    ctl_begin_t0(c, sh.Nx, sh.Ny);
-                    n->t0_pending = 0;
-                } else {
-                    c->active = 0;
-                }
-            } else if (n->t0_pending) {
-                c->active = 0;  // added after the last t=0 pass: waits for the next one
-            } else {
-                ctl_begin(c, sh.Nx, sh.Ny);
-            }
-            if (c->active) {
-                n->stepid += 1;
-                n->act_count[(n->seq + 1) & 1] = 0;
-                n->cursor = 0;
-                n->grid_mass = 0.0;
-                n->outs = c->write_outputs;
-                const int frame_after = c->frame + (c->frame_end ? 1 : 0);
-                const double nft = __dmul_rn(c->output_dt, (double)(frame_after + 1));
-                n->vz_next = (c->keep_outputs || __dadd_rn(c->new_time, c->dt_max) > nft - 1e-12) ? 1 : 0;
-                cnt = n->act_count[n->seq & 1];
-            }
+        const int cnt = s < sh.nscn ? step_control(sh, s, what, steps_left, stop_at_frame) : 0;
+        if (sh.nscn == 1) {
+            total = cnt;  // thread 0's, the only one that uses it
+            if (tid == 0) sh.work_pref[0] = 0;
+            break;
         }
         const int ex = block_exclusive_scan(cnt, s_warp);
         if (s < sh.nscn) sh.work_pref[s] = total + ex;
@@ -190,29 +243,44 @@ __device__ void begin_scenarios(const Shared& sh, int t0_pass) {
     }
     if (tid == 0) {
         sh.work_pref[sh.nscn] = min(total, sh.work_cap);
-        if (total > sh.work_cap) atomicOr(&sh.scn[0].ctl->err, ERR_CAPACITY);
+        if (total > sh.work_cap) atomicOr(&sh.ctl[0].err, ERR_CAPACITY);
         *sh.gcount = 0;
         sh.wcount[0] = 0;
         sh.wcount[1] = 0;
     }
 }
 
-__global__ void k_begin(Shared sh, int t0_pass) { begin_scenarios(sh, t0_pass); }
+constexpr int CTL_THREADS = 256;  // one thread per scenario; enough registers for the control block
+
+__global__ void __launch_bounds__(CTL_THREADS) k_begin(Shared sh, int t0_pass) { control_scenarios(sh, t0_pass ? CTL_T0 : CTL_BEGIN); }
 
 // Start of an advance call: every scenario gets the step budget and the
 // frame-stop rule, then the first step begins.
-__global__ void k_arm_begin(Shared sh, int64_t steps_left, int stop_at_frame) {
-    for (int s = threadIdx.x; s < sh.nscn; s += blockDim.x) {
-        Ctl* c = sh.scn[s].ctl;
-        c->stop = 0;
-        c->frame_hit = 0;
-        c->steps_left = steps_left;
-        c->stop_at_frame = stop_at_frame;
-    }
-    __syncthreads();
-    begin_scenarios(sh, 0);
+__global__ void __launch_bounds__(CTL_THREADS) k_arm_begin(Shared sh, int64_t steps_left, int stop_at_frame) {
+    control_scenarios(sh, CTL_ARM, steps_left, stop_at_frame);
 }
 
+// A scenario's static descriptor and step values in shared memory, loaded by
+// the threads of a CTA (or warp) together: one round of loads, whatever a
+// kernel reads of it afterwards. (One thread following the pointers field by
+// field took four rounds at the start of every CTA.)
+struct ScnSm {
+    Scn s;
+    SDyn y;
+    int sid;
+    __device__ __forceinline__ PBuf cur() const { return s.buf[y.seq & 1]; }
+    __device__ __forceinline__ PBuf next() const { return s.buf[(y.seq & 1) ^ 1]; }
+};
+static_assert(sizeof(Scn) % 16 == 0 && sizeof(SDyn) % 16 == 0, "loaded as 16-byte words");
+
+__device__ __forceinline__ void load_scn(const Shared& sh, int sid, ScnSm& z, int t, int nt) {
+    constexpr int A = sizeof(Scn) / 16, B = sizeof(SDyn) / 16;
+    for (int k = t; k < A + B; k += nt) {
+        if (k < A) reinterpret_cast<int4*>(&z.s)[k] = reinterpret_cast<const int4*>(sh.scn + sid)[k];
+        else reinterpret_cast<int4*>(&z.y)[k - A] = reinterpret_cast<const int4*>(sh.dyn + sid)[k - A];
+    }
+    if (t == 0) z.sid = sid;
+}
 
 // The work items of one CTA: a contiguous range of the flat work list, so
 // that consecutive items mostly belong to the same scenario.
@@ -248,29 +316,33 @@ __device__ __forceinline__ int p2g_item(const Shared& sh, int cls, int i) { retu
 // the lanes write the descriptor's words side by side.
 constexpr int PREP_LANES = 16;
 constexpr int PREP_THREADS = 256;
+constexpr int PREP_MAX_TILES = 1024 / PREP_LANES;  // tiles of one block pass (the persistent kernel runs larger blocks)
 static_assert(sizeof(TileDesc) == 28 * 4 && offsetof(TileDesc, rstart) == 4 * 4 && offsetof(TileDesc, rpref) == 13 * 4 &&
                   offsetof(TileDesc, blk4) == 23 * 4,
               "k_prep writes the descriptor word by word");
 
 __device__ __forceinline__ void prep_body(const Shared& sh) {
+    __shared__ int s_sid[PREP_MAX_TILES], s_cnt[PREP_MAX_TILES], s_ng[PREP_MAX_TILES];  // of the block's tiles
+    __shared__ int s_off[PREP_MAX_TILES], s_goff[PREP_MAX_TILES], s_cat[PREP_MAX_TILES];
     const int nwork = sh.work_pref[sh.nscn];
     const int lane = threadIdx.x & 31, r = lane & (PREP_LANES - 1);
-    const int per_block = (int)blockDim.x / PREP_LANES;
+    const int per_block = (int)blockDim.x / PREP_LANES, mine = threadIdx.x / PREP_LANES;
     const int stride = gridDim.x * per_block;
-    // whole warps run every iteration (the shuffles need both halves); a half
+    // whole blocks run every iteration (barriers and shuffles); a half warp
     // without a tile computes with valid = false
-    for (int w0 = blockIdx.x * per_block; w0 + (int)(threadIdx.x & ~31u) / PREP_LANES < nwork; w0 += stride) {
-        const int w = w0 + threadIdx.x / PREP_LANES;
+    for (int w0 = blockIdx.x * per_block; w0 < nwork; w0 += stride) {
+        const int w = w0 + mine;
         const bool valid = w < nwork;
         int sid = 0, loc = 0;
         if (valid) find_work(sh.work_pref, sh.nscn, w, sid, loc);
         const Scn& S = sh.scn[sid];
-        SCnt* n = sh.cnt + sid;  // no load of S.cnt in the chain
+        const SDyn& n = sh.dyn[sid];
         int seq = 0, stamp = 0, t = 0;
         if (valid) {
-            seq = n->seq;
-            stamp = n->stepid;
-            t = S.act_list[seq & 1][loc];
+            const int32_t *l0 = S.act_list[0], *l1 = S.act_list[1];  // loaded beside seq
+            seq = n.seq;
+            stamp = n.stepid;
+            t = ((seq & 1) ? l1 : l0)[loc];
         }
         const int cur = seq & 1;
         const int ti = t / sh.TY, tj = t % sh.TY;
@@ -310,30 +382,42 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
 #pragma unroll
         for (int o = PREP_LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o, PREP_LANES);
         const int ncand = __shfl_sync(0xffffffffu, incl, 8, PREP_LANES);
-        // lane 0: the segment cursor and the class list (one atomic per address and warp)
-        const bool leader = valid && r == 0;
-        const unsigned lmask = __ballot_sync(0xffffffffu, leader);
-        int nxt_off = 0;
-        if (leader) {
-            const WarpAdd a_cur = warp_add_issue(&n->cursor, cnt, lmask);
-            const int cls = cnt > sh.split_min ? 0 : 1;
-            WarpAdd a_cls{};
-            if (sh.split_min >= 0) a_cls = warp_add_issue(sh.wcount + cls, 1, lmask);
-            nxt_off = warp_add_finish(a_cur);
-            if (sh.split_min >= 0) {  // dense tiles to the cell-sorted P2G, sparse ones to the fixed-point P2G
-                const int at = warp_add_finish(a_cls);
-                if (at < sh.work_cap) sh.wlist[cls * sh.work_cap + at] = w;
-            }
-            S.slot_of[t] = w;
-        }
-        // the new grid tiles onto the flat grid-tile list, in lane order
+        // the segment cursor, the class lists and the flat grid-tile list: one
+        // atomic per address and block, by its first warp (one per address and
+        // warp made 3 same-address atomics per two tiles: 44 us on 47 k tiles)
         const unsigned gmask = __ballot_sync(0xffffffffu, new_gt);
         const unsigned hbits = (lane < PREP_LANES ? 0x0000ffffu : 0xffff0000u);
-        const int ng = __popc(gmask & hbits);
-        int at_g = 0;
-        if (leader) at_g = warp_atomic_add(sh.gcount, ng, lmask);
-        at_g = __shfl_sync(0xffffffffu, at_g, lane & ~(PREP_LANES - 1));
-        nxt_off = __shfl_sync(0xffffffffu, nxt_off, lane & ~(PREP_LANES - 1));
+        if (r == 0) {
+            s_sid[mine] = valid ? sid : -1;
+            s_cnt[mine] = cnt;
+            s_ng[mine] = __popc(gmask & hbits);
+            if (valid) S.slot_of[t] = w;
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            for (int q0 = 0; q0 < per_block; q0 += 32) {
+                const int q = q0 + lane;
+                const int qs = q < per_block ? s_sid[q] : -1;
+                const unsigned m = __ballot_sync(0xffffffffu, qs >= 0);
+                if (qs >= 0) {
+                    const int qc = s_cnt[q], cls = qc > sh.split_min ? 0 : 1;
+                    const WarpAdd a_cur = warp_add_issue(&sh.cnt[qs].cursor, qc, m);
+                    const WarpAdd a_gt = warp_add_issue(sh.gcount, s_ng[q], m);
+                    WarpAdd a_cls{};
+                    if (sh.split_min >= 0) a_cls = warp_add_issue(sh.wcount + cls, 1, m);
+                    s_off[q] = warp_add_finish(a_cur);
+                    s_goff[q] = warp_add_finish(a_gt);
+                    if (sh.split_min >= 0) s_cat[q] = warp_add_finish(a_cls);
+                }
+            }
+        }
+        __syncthreads();
+        const int nxt_off = s_off[mine], at_g = s_goff[mine];
+        if (valid && r == 0 && sh.split_min >= 0) {  // dense tiles to the cell-sorted P2G, sparse ones to the fixed-point P2G
+            const int at = s_cat[mine];
+            if (at < sh.work_cap) sh.wlist[(cnt > sh.split_min ? 0 : 1) * sh.work_cap + at] = w;
+        }
+        // the new grid tiles onto the flat grid-tile list, in lane order
         if (new_gt) {
             const int at = at_g + __popc(gmask & hbits & ((1u << lane) - 1u));
             if (at < sh.gcap) {
@@ -1073,14 +1157,15 @@ __device__ __forceinline__ void p2c_rows(P2CSmem& sm, bool staged, const float4*
 // the CTA's scenario values for a run of its tiles (thread 0)
 template <typename Sm> __device__ __forceinline__ void p2c_load_scenario(Sm& sm, const Shared& sh, int sid) {
     const Scn& S = sh.scn[sid];
-    const SCnt* n = S.cnt;
-    const int cur = n->seq & 1;
-    sm.B = S.buf[cur];
-    sm.nxt_cell = S.buf[cur ^ 1].cell;
+    const SDyn& n = sh.dyn[sid];
+    const int cur = n.seq & 1;
+    const PBuf b0 = S.buf[0], b1 = S.buf[1];  // loaded beside seq
+    sm.B = cur ? b1 : b0;
+    sm.nxt_cell = cur ? b0.cell : b1.cell;
     sm.ctl = S.ctl;
     sm.g = S.g;
     sm.hod = 0.5f * S.ood;
-    sm.outs = n->outs != 0;
+    sm.outs = n.outs != 0;
     sm.csid = sid;
 }
 
@@ -1499,9 +1584,10 @@ __device__ __forceinline__ void p2g_sparse_body(const Shared& sh, int cls, unsig
         if (sm.d.sid != csid) {  // uniform: a new scenario in this CTA's run
             csid = sm.d.sid;
             const Scn& S = sh.scn[csid];
-            const SCnt* n = S.cnt;
-            B = S.buf[n->seq & 1];
-            outs = n->outs != 0;
+            const SDyn& n = sh.dyn[csid];
+            const PBuf b0 = S.buf[0], b1 = S.buf[1];  // loaded beside seq
+            B = (n.seq & 1) ? b1 : b0;
+            outs = n.outs != 0;
             g = S.g;
             hod = 0.5f * S.ood;
             ctl = S.ctl;
@@ -1648,42 +1734,6 @@ __global__ void __launch_bounds__(P2S_THREADS, P2S_MIN_BLOCKS) k_p2g_sparse(Shar
 
 // ------------------------------------------------------------ grid update
 
-// Values of one scenario that the grid update reads for every grid tile.
-struct GridScn {
-    SCnt* n;
-    Ctl* c;
-    int32_t* act_stamp;
-    int32_t* slot_of;
-    int32_t* blk_of;
-    float dt, g, mu_c, mu_v, xi, mu1, mu2, I0, d, phi;
-    int sid, seq, stepid, outs, fric;
-};
-
-__device__ __forceinline__ void load_grid_scn(const Shared& sh, int sid, GridScn& z) {
-    const Scn& S = sh.scn[sid];
-    SCnt* n = S.cnt;
-    z.n = n;
-    z.c = S.ctl;
-    z.act_stamp = S.act_stamp;
-    z.slot_of = S.slot_of;
-    z.blk_of = S.blk_of;
-    z.dt = (float)S.ctl->dt;
-    z.g = S.g;
-    z.mu_c = S.mu_c;
-    z.mu_v = S.mu_v;
-    z.xi = S.xi;
-    z.mu1 = S.mu1;
-    z.mu2 = S.mu2;
-    z.I0 = S.I0;
-    z.d = S.d;
-    z.phi = S.phi;
-    z.fric = S.fric;
-    z.sid = sid;
-    z.seq = n->seq;
-    z.stepid = n->stepid;
-    z.outs = n->outs;
-}
-
 // K3 + K6: computeGridVelocity (src/simulation.cpp:800-875) for the TILE^2
 // nodes owned by one grid tile. A node's P2G sum is the partials of the
 // tiles whose window covers it, added in a fixed order (own, -x, -y, -xy).
@@ -1698,7 +1748,9 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
     __shared__ int s_slot[4];
     __shared__ double s_red[NCELL / 32];
     __shared__ unsigned s_act[NCELL / 32];
-    __shared__ GridScn Z;
+    __shared__ ScnSm zs;
+    const Scn& Z = zs.s;
+    const SDyn& Y = zs.y;
     const int tid = threadIdx.x;
     const int li = tid / TILE, lj = tid % TILE;
     int w0, w1;
@@ -1728,8 +1780,8 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
                 sum += s_red[k];
                 na += s_act[k];
             }
-            if (sum != 0.0) atomicAdd(&Z.n->grid_mass, sum);
-            if (na) atomicAdd(&Z.c->node_steps, (unsigned long long)na);
+            if (sum != 0.0) atomicAdd(&Z.cnt->grid_mass, sum);
+            if (na) atomicAdd(&Z.ctl->node_steps, (unsigned long long)na);
         }
         macc = 0.0;
         nacc = 0;
@@ -1746,10 +1798,10 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
             if (csid >= 0) flush();
             csid = s_sid;
             __syncthreads();
-            if (tid == 0) load_grid_scn(sh, csid, Z);
+            load_scn(sh, csid, zs, tid, NCELL);
             __syncthreads();
         }
-        Ctl* c = Z.c;
+        Ctl* c = Z.ctl;
         const int gt = s_gt;
         const int gi = gt / sh.TY, gj = gt % sh.TY;
         if (tid < 4) {
@@ -1759,7 +1811,7 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
             if (ti_ >= 0 && tj_ >= 0) {
                 const int tt = ti_ * sh.TY + tj_;
                 const int st_ = Z.act_stamp[tt], sl = Z.slot_of[tt];  // both loads in flight together
-                if (st_ == Z.seq) slot = sl;
+                if (st_ == Y.seq) slot = sl;
             }
             s_slot[tid] = slot;
         } else if (tid == 32) {
@@ -1778,10 +1830,10 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
                     blk = -1;
                 } else {
                     Z.blk_of[gt] = blk;
-                    sh.blk_owner[blk] = Z.sid;
+                    sh.blk_owner[blk] = zs.sid;
                 }
             }
-            if (blk >= 0) sh.blk_stamp[blk] = Z.stepid;
+            if (blk >= 0) sh.blk_stamp[blk] = Y.stepid;
             s_blk = blk;
         }
         __syncthreads();
@@ -1815,7 +1867,7 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
                 const float vox = q[1] / mi, voy = q[2] / mi;
                 vzn = q[6] / mi;
                 hn = q[3] / mi;
-                const float dt = Z.dt;
+                const float dt = Y.dt;
                 const float vtx = vox + dt * (q[4] / mi), vty = voy + dt * (q[5] / mi);
                 const float vsq = vtx * vtx + vty * vty;
                 float nvx = 0.f, nvy = 0.f;
@@ -1849,7 +1901,7 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
                 nacc += 1u;
             }
             sh.nv[bn] = out;
-            if (Z.outs) {
+            if (Y.outs) {
                 sh.oh[bn] = hn;
                 sh.om[bn] = inside ? mi : 0.f;
                 sh.ovz[bn] = vzn;
@@ -1879,75 +1931,23 @@ __device__ __forceinline__ int dir_of(int ib, int jb, int ti, int tj) {
 #endif
 constexpr int G2P_MIN_BLOCKS = SLAB_G2P_MIN_BLOCKS;  // resident G2P CTAs per SM the register budget is cut for
 
-// Values of one scenario that a G2P launch reads for every tile: loaded
-// once per run of consecutive tiles of that scenario.
-struct G2PScn {
-    SCnt* n;
-    Ctl* c;
-    PBuf B, O;                 // current and next particle buffers
-    int32_t* grp_nxt;          // segment records of the next step
-    int32_t* act_stamp;
-    int32_t* act_list_nxt;
-    int32_t* act_count_nxt;
-    double dx;
-    float dt, dt_ood, ood, fr;
-    int sid, seq, act_cap, outs, need_vz;
-    int in_i0, in_i1, in_j0, in_j1;  // tiles in this range cannot hold an extreme position of the particle box
-};
-
-__device__ __forceinline__ void load_g2p_scn(const Shared& sh, int sid, G2PScn& z) {
-    const Scn& S = sh.scn[sid];
-    SCnt* n = S.cnt;
-    Ctl* c = S.ctl;
-    const int seq = n->seq, cur = seq & 1, nxt = cur ^ 1;
-    z.n = n;
-    z.c = c;
-    z.B = S.buf[cur];
-    z.O = S.buf[nxt];
-    z.grp_nxt = S.grp[nxt];
-    z.act_stamp = S.act_stamp;
-    z.act_list_nxt = S.act_list[nxt];
-    z.act_count_nxt = &n->act_count[nxt];
-    z.dx = c->dx;
-    z.dt = (float)c->dt;
-    z.ood = S.ood;
-    z.dt_ood = z.dt * S.ood;
-    z.fr = S.fr;
-    z.sid = sid;
-    z.seq = seq;
-    z.act_cap = S.act_cap;
-    z.outs = n->outs != 0;
-    z.need_vz = z.outs || n->vz_next;
-    // Positions of the box's extreme particles at the start of the step, in
-    // cells. A particle moves to a neighbour tile at most (farther raises
-    // ERR_MOVE), less than 2 TILE cells, so after the step the box still
-    // reaches to within that of its old faces; a tile whose particles all end
-    // up further inside cannot change it.
-    constexpr int D = 2 * TILE + 2;
-    const int i0 = (int)(__longlong_as_double((long long)c->pos[0]) * c->one_over_dx), i1 = (int)(__longlong_as_double((long long)c->pos[1]) * c->one_over_dx);
-    const int j0 = (int)(__longlong_as_double((long long)c->pos[2]) * c->one_over_dx), j1 = (int)(__longlong_as_double((long long)c->pos[3]) * c->one_over_dx);
-    z.in_i0 = (i0 + D + TILE - 1) / TILE + 1;
-    z.in_i1 = (i1 - D) / TILE - 2;
-    z.in_j0 = (j0 + D + TILE - 1) / TILE + 1;
-    z.in_j1 = (j1 - D) / TILE - 2;
-}
-
 // puts tile tt on the next step's active list, once
-__device__ __forceinline__ void g2p_activate(const G2PScn& z, int tt) {
-    if (atomicMax(&z.act_stamp[tt], z.seq + 1) < z.seq + 1) {
-        const int kk = atomicAdd(z.act_count_nxt, 1);
-        if (kk < z.act_cap) z.act_list_nxt[kk] = tt;
-        else atomicOr(&z.c->err, ERR_CAPACITY);
+__device__ __forceinline__ void g2p_activate(const ScnSm& z, int tt) {
+    const int seq1 = z.y.seq + 1;
+    if (atomicMax(&z.s.act_stamp[tt], seq1) < seq1) {
+        const int kk = atomicAdd(&z.s.cnt->act_count[seq1 & 1], 1);
+        if (kk < z.s.act_cap) z.s.act_list[seq1 & 1][kk] = tt;
+        else atomicOr(&z.s.ctl->err, ERR_CAPACITY);
     }
 }
 
 // the largest |v|^2 of a run of tiles into the scenario's control block: one
 // atomic per warp, and only if it raises the value seen (speeds squared are
 // >= 0, so their bit patterns order like the values)
-__device__ __forceinline__ void g2p_flush_vmax2(const G2PScn& z, float vmax2) {
+__device__ __forceinline__ void g2p_flush_vmax2(const ScnSm& z, float vmax2) {
     const double v = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(vmax2)));
     const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-    unsigned long long* acc = reinterpret_cast<unsigned long long*>(&z.c->vmax2_acc);
+    unsigned long long* acc = reinterpret_cast<unsigned long long*>(&z.s.ctl->vmax2_acc);
     if ((threadIdx.x & 31) == 0 && bits > *reinterpret_cast<volatile unsigned long long*>(acc)) atomicMax(acc, bits);
 }
 
@@ -1974,7 +1974,7 @@ struct G2PSmem {
     int wst[2][NCELL / 32], wmv[2][NCELL / 32];  // per-warp stayer / mover counts of a chunk (double buffered)
     int dcnt[9];
     TileDesc d;
-    G2PScn z;
+    ScnSm z;
     double red[4][NCELL / 32];
 };
 
@@ -2065,15 +2065,15 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
             if (w > w0) g2p_flush_vmax2(sm.z, vmax2);
             vmax2 = 0.f;
             __syncthreads();
-            if (tid == 0) load_g2p_scn(sh, sm.d.sid, sm.z);
+            load_scn(sh, sm.d.sid, sm.z, tid, NCELL);
             __syncthreads();
         }
-        const G2PScn& Z = sm.z;
-        Ctl* c = Z.c;
+        const ScnSm& Z = sm.z;
+        Ctl* c = Z.s.ctl;
         const int t = sm.d.t;
         const int ti = t / sh.TY, tj = t % sh.TY;
-        const bool outs = Z.outs != 0;
-        const bool need_vz = Z.need_vz != 0;
+        const bool outs = Z.y.outs != 0;
+        const bool need_vz = Z.y.need_vz != 0;
         const int ncand = sm.d.rpref[9];
         const bool staged = ncand <= G2P_CAP;
         // the tile's candidates (the first chunk's, for a tile over the stage),
@@ -2081,7 +2081,7 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
         // and the windows fill by asynchronous copies
         G2PCand pre = {};
         if (staged) {
-            const PBuf& B = Z.B;
+            const PBuf& B = Z.s.buf[Z.y.seq & 1];
             for (int k = tid; k < ncand; k += NCELL) {
                 int r;
                 const int src = cand_to_index(k, sm.d, r);
@@ -2093,7 +2093,7 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
                 cpa::copy4(&sm.st.id[k], B.id + src);
             }
         } else {
-            pre = load_g2p_cand(sm.d, Z.B, tid, ncand, t, sh.TY);
+            pre = load_g2p_cand(sm.d, Z.cur(), tid, ncand, t, sh.TY);
         }
         // the node window by per-thread asynchronous copies; a part whose grid tile
         // has no block this step (or past the terrain edge) is zero. (Bulk copies
@@ -2121,12 +2121,12 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
         SLAB_PHASE_MARK(10);
         const int total = sm.d.total;
         const int base = sm.d.nxt_off;
-        const PBuf& B = Z.B;
-        const PBuf O = Z.O;
-        const float dt = Z.dt;
-        const float dt_ood = Z.dt_ood;
-        const double dx = Z.dx;
-        const bool edge = ti < Z.in_i0 || ti > Z.in_i1 || tj < Z.in_j0 || tj > Z.in_j1;  // uniform: may change the particle box
+        const PBuf& B = Z.s.buf[Z.y.seq & 1];
+        const PBuf O = Z.next();
+        const float dt = Z.y.dt;
+        const float dt_ood = Z.y.dt_ood;
+        const double dx = sh.dx;
+        const bool edge = ti < Z.y.in_i0 || ti > Z.y.in_i1 || tj < Z.y.in_j0 || tj > Z.y.in_j1;  // uniform: may change the particle box
         double mnx = INFINITY, mxx = 0.0, mny = INFINITY, mxy = 0.0;
         int front = 0, back = 0;  // stayers / movers placed so far (same in every thread)
         G2PCand nxt = pre;
@@ -2169,8 +2169,8 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
                         fly += nv.w * wgt;
                         div += (dwx[a] * wy[b]) * nv.x + (dwy[b] * wx[a]) * nv.y;
                     }
-                div *= Z.ood;
-                const float fr = Z.fr;
+                div *= Z.s.ood;
+                const float fr = Z.s.fr;
                 vn = make_float2(fr * (v.x + flx) + (1.f - fr) * picx, fr * (v.y + fly) + (1.f - fr) * picy);
                 hn = h / (1.f + dt * div);
                 if (need_vz) {
@@ -2261,14 +2261,14 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
         }
         __syncthreads();
         if (tid < 9) {
-            int32_t* G = Z.grp_nxt + (size_t)t * GRP_STRIDE;
+            int32_t* G = Z.s.grp[(Z.y.seq & 1) ^ 1] + (size_t)t * GRP_STRIDE;
             const int cnt = tid == 4 ? sm.front : sm.dcnt[tid];
             G[3 + tid] = cnt;
             if (tid == 0) {
                 G[0] = base;
                 G[1] = base + sm.front;
                 G[2] = base + sm.front + sm.back;
-                G[GRP_STAMP] = Z.seq + 1;
+                G[GRP_STAMP] = Z.y.seq + 1;
                 if (sm.front + sm.back != total) atomicOr(&c->err, ERR_CAPACITY);
             }
             if (cnt) pend_tt = (ti + dir_i(tid)) * sh.TY + (tj + dir_j(tid));
@@ -2315,22 +2315,7 @@ __global__ void __launch_bounds__(NCELL, G2P_MIN_BLOCKS) k_g2p(Shared sh, const 
 // K5: end of the step for every running scenario (the per-step reductions
 // of G2P into dt, time and the remesh box), then the next step's dt, stop
 // rules and work list. One CTA, after G2P.
-__device__ __forceinline__ void end_body(const Shared& sh) {
-    for (int s = threadIdx.x; s < sh.nscn; s += blockDim.x) {
-        const Scn& S = sh.scn[s];
-        Ctl* c = S.ctl;
-        if (!c->active) continue;
-        SCnt* n = S.cnt;
-        if (n->cursor != S.Np) atomicOr(&c->err, ERR_CAPACITY);
-        ctl_end(c);
-        n->seq += 1;
-        n->vz_valid = n->outs;
-    }
-    __syncthreads();
-    begin_scenarios(sh, 0);
-}
-
-__global__ void k_end(Shared sh) { end_body(sh); }
+__global__ void __launch_bounds__(CTL_THREADS) k_end(Shared sh) { control_scenarios(sh, CTL_END); }
 
 // ------------------------------------------------------- persistent steps
 
@@ -2411,7 +2396,7 @@ __global__ void __launch_bounds__(NCELL, P2C_MIN_BLOCKS) k_persist(Shared sh, co
         if (!grid_sync(sh, bar, limit)) return;
         g2p_body(sh, z64, *reinterpret_cast<G2PSmem*>(smem_raw));
         if (!grid_sync(sh, bar, limit)) return;
-        if (blockIdx.x == 0) end_body(sh);
+        if (blockIdx.x == 0) control_scenarios(sh, CTL_END);
         if (!grid_sync(sh, bar, limit)) return;
         if (*reinterpret_cast<volatile const int*>(sh.work_pref + sh.nscn) == 0) break;  // the same value in every CTA
     }
