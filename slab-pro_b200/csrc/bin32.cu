@@ -87,14 +87,11 @@ __global__ void k_bin_gather(int Np, const int32_t* __restrict__ order, const in
                              const double* __restrict__ m, const double* __restrict__ z, PBuf out) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < Np; k += gridDim.x * blockDim.x) {
         const int q = order[k];
-        out.cell[k] = cell[q];
-        out.f[k] = f[q];
-        out.v[k] = make_float2((float)v[2 * q], (float)v[2 * q + 1]);
-        out.h[k] = (float)h[q];
-        out.m[k] = (float)m[q];
+        const float2 fq = f[q];
+        out.a[k] = make_float4(fq.x, fq.y, (float)v[2 * q], (float)v[2 * q + 1]);
+        out.b[k] = make_float4((float)h[q], (float)m[q], __int_as_float(cell[q]), __int_as_float(q));
         out.vz[k] = (float)vz[q];
         out.z[k] = (float)z[q];
-        out.id[k] = q;
     }
 }
 

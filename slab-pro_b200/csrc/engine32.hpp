@@ -24,9 +24,9 @@ class Engine32 {
         int act_alloc = 0;  // tile list length
         Ctl* ctl = nullptr;
         Ctl* h_ctl = nullptr;
-        dptr<int32_t> cell[2], id[2], grp[2], act_list[2];
-        dptr<float2> f[2], v[2];
-        dptr<float> h[2], m[2], vz[2], z[2];
+        dptr<int32_t> grp[2], act_list[2];
+        dptr<float4> a[2], b[2];  // PBuf
+        dptr<float> vz[2], z[2];
         dptr<int32_t> act_stamp, slot_of, nxt_off, gt_stamp, blk_of;
         SCnt* cnt = nullptr;  // in the engine's counter array
     };
@@ -42,9 +42,7 @@ class Engine32 {
     void launch_step();
     void launch_kernel(int k, const Shared& sh);
     void launch_p2g(const Shared& sh);
-    void launch_p2g_cell(const Shared& sh, int cls);
-    CUtensorMap dem_map;   // the FP32 terrain as [Nx][4 Ny] floats, 9 x 9-node boxes (the cell P2G's terrain window)
-    bool p2g_tma = false;  // k_p2g_cell<true>: the next tile's loads staged by TMA bulk copies (SLAB_P2G_TMA=1)
+    CUtensorMap dem_map;   // the FP32 terrain as [Nx][4 Ny] floats, 9 x 9-node boxes (P2G's terrain window)
     // persistent steps: a chunk of steps as one cooperative launch of k_persist
     // (SLAB_PERSIST=1 or set_persistent); its grid waits give up after
     // persist_limit clock cycles (ERR_TIMEOUT)
@@ -91,8 +89,8 @@ class Engine32 {
     int64_t pending_blocks = 0;  // node blocks of scenarios added since the last t=0 pass (an estimate)
     int grid_p2g = 0, grid_p2g_cell = 0, grid_p2g_hilo = 0, grid_p2g_sparse = 0, grid_g2p = 0, grid_grid = 0, grid_prep = 0;
 
-    // Launch-shape tuner of the step's five work kernels (k_prep, k_p2g_cell,
-    // k_p2g_sparse, k_grid, k_g2p). Each CTA of these kernels takes a
+    // Launch-shape tuner of the step's work kernels (k_prep, k_p2g_tiles --
+    // shapes 1 and 2, its dense and sparse tiles, go together --, k_grid, k_g2p). Each CTA of these kernels takes a
     // contiguous slice of a device-built work list and every work item is
     // computed by one CTA alone, so the grid size changes which CTA computes a
     // tile, never a value: all candidates give bitwise the same results. The
@@ -154,7 +152,7 @@ class Engine32 {
                                     bool with_v);
     dptr<float4> d_nv;
     dptr<float> d_hmax, d_vmax2, d_oh, d_om, d_ovz, d_oFx, d_oFy;
-    dptr<int32_t> d_blk_stamp, d_blk_owner, d_misc, d_work_pref, d_gflat, d_wlist, d_free_blocks;
+    dptr<int32_t> d_blk_stamp, d_blk_owner, d_misc, d_work_pref, d_gflat, d_free_blocks;
     dptr<Scn> d_scn;
     dptr<SCnt> d_cnt;
     dptr<SDyn> d_dyn;

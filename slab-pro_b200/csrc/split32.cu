@@ -98,10 +98,11 @@ __global__ void k_max_full(const int32_t* __restrict__ blk_of, int TY, int Nx, i
 // id[k]: x y vx vy vz z h A as float32 (the PLY vertex layout), A = m / (h rho).
 __global__ void k_pack_particles(PBuf B, int Np, double dx, double rho, float* __restrict__ out) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < Np; k += gridDim.x * blockDim.x) {
-        const int32_t c = B.cell[k];
-        const float2 f = B.f[k], v = B.v[k];
-        const float h = B.h[k], m = B.m[k];
-        float* o = out + (size_t)B.id[k] * 8;
+        const float4 pa = B.a[k], pb = B.b[k];
+        const int32_t c = __float_as_int(pb.z);
+        const float2 f = make_float2(pa.x, pa.y), v = make_float2(pa.z, pa.w);
+        const float h = pb.x, m = pb.y;
+        float* o = out + (size_t)__float_as_int(pb.w) * 8;
         o[0] = (float)(((double)cell_i(c) + (double)f.x) * dx);
         o[1] = (float)(((double)cell_j(c) + (double)f.y) * dx);
         o[2] = v.x;
@@ -122,26 +123,26 @@ struct Unpack {
 };
 __global__ void k_unpack_particles(PBuf B, int Np, double dx, double rho, Unpack o, int* __restrict__ bad) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < Np; k += gridDim.x * blockDim.x) {
-        const int q = B.id[k];
+        const float4 pa = B.a[k], pb = B.b[k];
+        const int q = __float_as_int(pb.w);
         if ((unsigned)q >= (unsigned)Np) {
             atomicOr(bad, 1);
             continue;
         }
-        const int32_t c = B.cell[k];
-        const float2 f = B.f[k];
+        const int32_t c = __float_as_int(pb.z);
+        const float2 f = make_float2(pa.x, pa.y);
         if (o.x) {
             o.x[2 * q] = __dmul_rn(__dadd_rn((double)cell_i(c), (double)f.x), dx);
             o.x[2 * q + 1] = __dmul_rn(__dadd_rn((double)cell_j(c), (double)f.y), dx);
         }
         if (o.v) {
-            const float2 v = B.v[k];
-            o.v[2 * q] = v.x;
-            o.v[2 * q + 1] = v.y;
+            o.v[2 * q] = pa.z;
+            o.v[2 * q + 1] = pa.w;
         }
         if (o.vz) o.vz[q] = B.vz[k];
-        if (o.h) o.h[q] = B.h[k];
-        if (o.m) o.m[q] = B.m[k];
-        if (o.A) o.A[q] = __ddiv_rn((double)B.m[k], __dmul_rn((double)B.h[k], rho));
+        if (o.h) o.h[q] = pb.x;
+        if (o.m) o.m[q] = pb.y;
+        if (o.A) o.A[q] = __ddiv_rn((double)pb.y, __dmul_rn((double)pb.x, rho));
         if (o.z) o.z[q] = B.z[k];
     }
 }
@@ -251,9 +252,7 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g<k32::ACC_I32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GSmem)));
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g<k32::ACC_HILO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GSmem)));
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g<k32::ACC_I64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GSmem)));
-    SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g_cell<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2CSmem)));
-    SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g_cell<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2CSmemTma)));
-    if (const char* e = std::getenv("SLAB_P2G_TMA")) p2g_tma = std::atoi(e) != 0;
+    SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GTileSmem)));
     {
         // the terrain window of the cell P2G as one tensor copy per tile: the
         // float4 terrain seen as [Nx][4 Ny] floats (rows 16 Ny bytes apart), boxes
@@ -281,19 +280,14 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, k32::k_p2g_warp, k32::P2W_THREADS,
                                                             k32::P2W_WARPS * sizeof(k32::P2WWarp)));
     int occ_c = 0, occ_h = 0;
-    if (p2g_tma)
-        SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k32::k_p2g_cell<true>, k32::P2C_THREADS, sizeof(k32::P2CSmemTma)));
-    else
-        SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k32::k_p2g_cell<false>, k32::P2C_THREADS, sizeof(k32::P2CSmem)));
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k32::k_p2g_tiles, k32::P2G_T, sizeof(k32::P2GTileSmem)));
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k32::k_p2g<k32::ACC_HILO>, k32::P2G_THREADS, sizeof(k32::P2GSmem)));
-    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p, NCELL, 0));
-    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k32::k_grid, NCELL, 0));
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p, k32::G2P_T, 0));
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k32::k_grid, k32::GRID_T, 0));
     grid_p2g = sms * std::max(occ_p, 1);
     grid_p2g_cell = sms * std::max(occ_c, 1);
     grid_p2g_hilo = sms * std::max(occ_h, 1);
-    int occ_s = 0;
-    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k32::k_p2g_sparse, k32::P2S_THREADS, sizeof(k32::P2SSmem)));
-    grid_p2g_sparse = sms * std::max(occ_s, 1);
+    grid_p2g_sparse = grid_p2g_cell;  // sparse tiles run in the same kernel
     grid_g2p = sms * std::max(occ_g, 1);
     grid_grid = sms * std::max(occ_u, 1);
     int occ_d = 0;
@@ -307,7 +301,7 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     int coop = 0, occ_ps = 0;
     SLAB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k32::PERSIST_SMEM));
-    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_ps, k32::k_persist, NCELL, k32::PERSIST_SMEM));
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_ps, k32::k_persist, k32::P2G_T, k32::PERSIST_SMEM));
     grid_persist = coop ? sms * occ_ps : 0;
     if (const char* e = std::getenv("SLAB_PERSIST")) persist = std::atoi(e) != 0 && grid_persist > 0;
     timer.nk = 5;  // k_prep, P2G, grid update, G2P, k_end
@@ -343,8 +337,6 @@ Shared Engine32::shared() const {
     sh.ctl = ctl0;
     sh.dyn = d_dyn.get();
     sh.work_pref = d_work_pref.get();
-    sh.wlist = d_wlist.get();
-    sh.wcount = d_misc.get() + 2;
     sh.split_min = acc_mode == k32::ACC_MIXED ? split_min : -1;
     sh.gflat = d_gflat.get();
     sh.gcount = d_misc.get() + 6;
@@ -472,7 +464,6 @@ void Engine32::ensure_work_cap(int64_t need) {
     d_desc = dalloc<TileDesc>(cap);
     d_part = dalloc<float>((size_t)cap * PART_STRIDE);
     d_gflat = dalloc<int32_t>((size_t)8 * cap);  // up to 4 grid tiles per active tile, 2 ints each
-    d_wlist = dalloc<int32_t>((size_t)2 * cap);
     work_cap = (int)cap;
     graphs.clear();
 }
@@ -513,15 +504,10 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     const bool new_parts = S.Np_alloc < Np, new_lists = S.act_alloc < S.act_cap, new_tiles = !S.blk_of;
     for (int b = 0; b < 2; ++b) {
         if (new_parts) {
-            // padded past Np: P2G's bulk copies round a range's end up to 16 bytes
-            S.cell[b] = dalloc<int32_t>(Np + PARTICLE_PAD);
-            S.f[b] = dalloc<float2>(Np + PARTICLE_PAD);
-            S.v[b] = dalloc<float2>(Np + PARTICLE_PAD);
-            S.h[b] = dalloc<float>(Np + PARTICLE_PAD);
-            S.m[b] = dalloc<float>(Np + PARTICLE_PAD);
-            S.id[b] = dalloc<int32_t>(Np + PARTICLE_PAD);
-            S.vz[b] = dalloc<float>(Np + PARTICLE_PAD);
-            S.z[b] = dalloc<float>(Np + PARTICLE_PAD);
+            S.a[b] = dalloc<float4>(Np);
+            S.b[b] = dalloc<float4>(Np);
+            S.vz[b] = dalloc<float>(Np);
+            S.z[b] = dalloc<float>(Np);
         }
         if (new_tiles) S.grp[b] = dalloc<int32_t>((size_t)ntiles * GRP_STRIDE);
         if (new_lists) S.act_list[b] = dalloc<int32_t>(S.act_cap);
@@ -550,7 +536,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     for (int b = 0; b < 2; ++b)  // every record stale (stamp -1)
         SLAB_CUDA(cudaMemsetAsync(S.grp[b].get(), 0xff, (size_t)ntiles * GRP_STRIDE * sizeof(int32_t), st));
     SLAB_CUDA(cudaMemsetAsync(S.act_stamp.get(), 0xff, ntiles * sizeof(int32_t), st));
-    const PBuf out0{S.cell[0].get(), S.f[0].get(), S.v[0].get(), S.h[0].get(), S.m[0].get(), S.id[0].get(), S.vz[0].get(), S.z[0].get()};
+    const PBuf out0{S.a[0].get(), S.b[0].get(), S.vz[0].get(), S.z[0].get()};
     const BinResult bin = bin_particles(T, TY, ntiles, st, Np, x, v, vz, h, m, z, out0, S.grp[0].get(), S.act_list[0].get(),
                                         S.act_stamp.get(), S.act_cap, scratch);
     const std::vector<uint32_t>& alist = bin.tiles;
@@ -605,7 +591,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     D.phi = (float)p.friction.phi;
     D.Np = Np;
     for (int b = 0; b < 2; ++b) {
-        D.buf[b] = PBuf{S.cell[b].get(), S.f[b].get(), S.v[b].get(), S.h[b].get(), S.m[b].get(), S.id[b].get(), S.vz[b].get(), S.z[b].get()};
+        D.buf[b] = PBuf{S.a[b].get(), S.b[b].get(), S.vz[b].get(), S.z[b].get()};
         D.grp[b] = S.grp[b].get();
         D.act_list[b] = S.act_list[b].get();
     }
@@ -633,35 +619,24 @@ void Engine32::launch_t0() {
     k32::k_begin<<<1, k32::CTL_THREADS, 0, st>>>(sh, 1);
     k32::k_prep<<<grid_prep, 256, 0, st>>>(sh);
     launch_p2g(sh);
-    k32::k_grid<<<grid_grid, NCELL, 0, st>>>(sh);
+    k32::k_grid<<<grid_grid, k32::GRID_T, 0, st>>>(sh);
     SLAB_CUDA(cudaGetLastError());
-    nlaunch += acc_mode == k32::ACC_MIXED ? 5 : 4;
+    nlaunch += 4;
     pending_blocks = 0;  // later reads of the pool count see these blocks
 }
 
-// the cell-sorted P2G; SLAB_P2G_TMA=1 stages the next tile's loads with TMA
-// bulk copies (same sums, in the same order)
-void Engine32::launch_p2g_cell(const Shared& sh, int cls) {
-    if (p2g_tma)
-        k32::k_p2g_cell<true><<<grid_p2g_cell, k32::P2C_THREADS, sizeof(k32::P2CSmemTma), st>>>(sh, cls, dem_map);
-    else
-        k32::k_p2g_cell<false><<<grid_p2g_cell, k32::P2C_THREADS, sizeof(k32::P2CSmem), st>>>(sh, cls, dem_map);
-}
-
 void Engine32::launch_p2g(const Shared& sh) {
-    if (acc_mode == k32::ACC_MIXED) {  // dense tiles, then sparse tiles
-        launch_p2g_cell(sh, 0);
-        k32::k_p2g_sparse<<<grid_p2g_sparse, k32::P2S_THREADS, sizeof(k32::P2SSmem), st>>>(sh, 1);
+    if (acc_mode == k32::ACC_MIXED || acc_mode == k32::ACC_CELL) {  // dense and sparse tiles, or every tile as a dense one
+        const int grid = std::max(grid_p2g_cell, grid_p2g_sparse);
+        k32::k_p2g_tiles<<<grid, k32::P2G_T, sizeof(k32::P2GTileSmem), st>>>(sh, dem_map);
     } else if (acc_mode == k32::ACC_WARP) {
-        k32::k_p2g_warp<<<grid_p2g, k32::P2W_THREADS, k32::P2W_WARPS * sizeof(k32::P2WWarp), st>>>(sh, -1);
-    } else if (acc_mode == k32::ACC_CELL) {
-        launch_p2g_cell(sh, -1);
+        k32::k_p2g_warp<<<grid_p2g, k32::P2W_THREADS, k32::P2W_WARPS * sizeof(k32::P2WWarp), st>>>(sh);
     } else if (acc_mode == k32::ACC_I32) {
-        k32::k_p2g<k32::ACC_I32><<<grid_p2g_hilo, k32::P2G_THREADS, sizeof(k32::P2GSmem), st>>>(sh, -1);
+        k32::k_p2g<k32::ACC_I32><<<grid_p2g_hilo, k32::P2G_THREADS, sizeof(k32::P2GSmem), st>>>(sh);
     } else if (acc_mode == k32::ACC_I64) {
-        k32::k_p2g<k32::ACC_I64><<<grid_p2g_hilo, k32::P2G_THREADS, sizeof(k32::P2GSmem), st>>>(sh, -1);
+        k32::k_p2g<k32::ACC_I64><<<grid_p2g_hilo, k32::P2G_THREADS, sizeof(k32::P2GSmem), st>>>(sh);
     } else {
-        k32::k_p2g<k32::ACC_HILO><<<grid_p2g_hilo, k32::P2G_THREADS, sizeof(k32::P2GSmem), st>>>(sh, -1);
+        k32::k_p2g<k32::ACC_HILO><<<grid_p2g_hilo, k32::P2G_THREADS, sizeof(k32::P2GSmem), st>>>(sh);
     }
 }
 
@@ -669,8 +644,8 @@ void Engine32::launch_kernel(int k, const Shared& sh) {
     switch (k) {
         case 0: k32::k_prep<<<grid_prep, 256, 0, st>>>(sh); break;
         case 1: launch_p2g(sh); break;
-        case 2: k32::k_grid<<<grid_grid, NCELL, 0, st>>>(sh); break;
-        case 3: k32::k_g2p<<<grid_g2p, NCELL, 0, st>>>(sh, T.z.get()); break;
+        case 2: k32::k_grid<<<grid_grid, k32::GRID_T, 0, st>>>(sh); break;
+        case 3: k32::k_g2p<<<grid_g2p, k32::G2P_T, 0, st>>>(sh, T.z.get()); break;
         case 4: k32::k_end<<<1, k32::CTL_THREADS, 0, st>>>(sh); break;
     }
 }
@@ -741,13 +716,12 @@ void Engine32::launch_step_timed(const Shared& sh, cudaEvent_t* e) {
     SLAB_CUDA(cudaEventRecord(e[0], st));
     k32::k_prep<<<grid_prep, 256, 0, st>>>(sh);
     SLAB_CUDA(cudaEventRecord(e[1], st));
-    launch_p2g_cell(sh, 0);
-    SLAB_CUDA(cudaEventRecord(e[2], st));
-    k32::k_p2g_sparse<<<grid_p2g_sparse, k32::P2S_THREADS, sizeof(k32::P2SSmem), st>>>(sh, 1);
+    launch_p2g(sh);
+    SLAB_CUDA(cudaEventRecord(e[2], st));  // (shape 2, the sparse tiles', goes with shape 1: one kernel runs both)
     SLAB_CUDA(cudaEventRecord(e[3], st));
-    k32::k_grid<<<grid_grid, NCELL, 0, st>>>(sh);
+    k32::k_grid<<<grid_grid, k32::GRID_T, 0, st>>>(sh);
     SLAB_CUDA(cudaEventRecord(e[4], st));
-    k32::k_g2p<<<grid_g2p, NCELL, 0, st>>>(sh, T.z.get());
+    k32::k_g2p<<<grid_g2p, k32::G2P_T, 0, st>>>(sh, T.z.get());
     SLAB_CUDA(cudaEventRecord(e[5], st));
     k32::k_end<<<1, k32::CTL_THREADS, 0, st>>>(sh);
     SLAB_CUDA(cudaEventRecord(e[6], st));
@@ -774,6 +748,7 @@ void Engine32::tune_pick() {
             if (ms[k][c] < 0.97 * ms[k][2] && ms[k][c] < ms[k][best]) best = c;
         tune.pick[k] = best;
     }
+    tune.pick[2] = tune.pick[1];
     apply_shapes(tune.pick);
     graphs.clear();  // the step graphs carry the grid sizes
     if (!tune.key.empty()) {
@@ -813,7 +788,7 @@ void Engine32::launch_persistent(int chunk) {
     long long lim = persist_limit;
     k32::GridBar* bar = reinterpret_cast<k32::GridBar*>(d_bar.get());
     void* args[] = {&sh, &z64, &n, &lim, &bar, &dem_map};
-    SLAB_CUDA(cudaLaunchCooperativeKernel((const void*)k32::k_persist, dim3(grid_persist), dim3(NCELL), args, k32::PERSIST_SMEM, st));
+    SLAB_CUDA(cudaLaunchCooperativeKernel((const void*)k32::k_persist, dim3(grid_persist), dim3(k32::P2G_T), args, k32::PERSIST_SMEM, st));
     nlaunch += 1;
 }
 
@@ -873,7 +848,7 @@ void Engine32::enqueue_steps(int chunk) {
         }
     }
     tune.steps += chunk;
-    nlaunch += (acc_mode == k32::ACC_MIXED ? 6 : 5) * (int64_t)chunk;
+    nlaunch += 5 * (int64_t)chunk;
 }
 
 SCnt Engine32::counters(int sid) {
@@ -1118,19 +1093,17 @@ namespace {
 // position (from the split cell + offset), velocity and mass of particle p of
 // a buffer, for the moments reduction
 struct SplitParticle {
-    const int32_t* cell;
-    const float2* f;
-    const float2* v;
-    const float* m;
+    const float4* a;
+    const float4* b;
     double dx;
     __device__ void operator()(int p, double& x, double& y, double& vx, double& vy, double& mass) const {
-        const int32_t c = cell[p];
-        const float2 fp = f[p], vp = v[p];
-        x = ((double)cell_i(c) + (double)fp.x) * dx;
-        y = ((double)cell_j(c) + (double)fp.y) * dx;
-        vx = vp.x;
-        vy = vp.y;
-        mass = m[p];
+        const float4 pa = a[p], pb = b[p];
+        const int32_t c = __float_as_int(pb.z);
+        x = ((double)cell_i(c) + (double)pa.x) * dx;
+        y = ((double)cell_j(c) + (double)pa.y) * dx;
+        vx = pa.z;
+        vy = pa.w;
+        mass = pb.y;
     }
 };
 }  // namespace
@@ -1140,7 +1113,7 @@ void Engine32::moments(int sid, double out[6]) {
     const SCnt c = counters(sid);
     const int b = c.seq & 1;  // the buffer the last G2P wrote
     if (!d_mom) d_mom = dalloc<double>((size_t)MOM_BLOCKS * MOM_N + MOM_N);
-    const SplitParticle get{S.cell[b].get(), S.f[b].get(), S.v[b].get(), S.m[b].get(), T.dx};
+    const SplitParticle get{S.a[b].get(), S.b[b].get(), T.dx};
     k_moments<<<MOM_BLOCKS, MOM_THREADS, 0, st>>>(S.Np, get, d_mom.get());
     k_moments_final<<<1, MOM_THREADS, 0, st>>>(d_mom.get(), d_mom.get() + (size_t)MOM_BLOCKS * MOM_N);
     nlaunch += 2;

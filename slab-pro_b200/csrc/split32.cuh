@@ -6,8 +6,8 @@
 // particle is nodes ib..ib+2 (the reference's i_base = int(x/dx - 0.5),
 // src/simulation.cpp:741-742). Offsets stay O(1), so km-scale domains keep
 // ~1e-7 dx resolution where an absolute FP32 coordinate would keep ~1e-3 m.
-// Per particle (SoA): cell 4 B, f 8, v 8, h 4, m 4, id 4; vz and z only in
-// steps that feed an output frame.
+// Per particle two 16-byte words, {f, v} and {h, m, cell, id}; vz and z only
+// in steps that feed an output frame.
 //
 // Sparse tiles. Base cells are grouped in TILE x TILE tiles. Particles are
 // stored per tile: G2P writes tile t's particles into t's segment of the
@@ -37,23 +37,23 @@ constexpr int TN = TILE + 2;          // node window edge of a tile
 constexpr int NCELL = TILE * TILE;    // cells per tile = threads per CTA
 constexpr int NQ = 7;                 // P2G sums: m, m vx, m vy, m h, Fx, Fy, m vz
 constexpr int PART_STRIDE = NQ * TN * TN;  // floats per tile partial
-constexpr int CHUNK = 1024;           // particles staged per pass of P2G/G2P
-constexpr int PARTICLE_PAD = 16;      // elements allocated past the last particle of every particle array
 
 __host__ __device__ inline int32_t pack_cell(int ib, int jb) { return (ib << 16) | jb; }
 __host__ __device__ inline int cell_i(int32_t c) { return (int)((uint32_t)c >> 16); }
 __host__ __device__ inline int cell_j(int32_t c) { return (int)(c & 0xffff); }
 
+// A particle buffer. The state a step moves is two 16-byte words, so that a
+// particle is two loads and two stores whichever order the particles of a
+// tile lie in (as six arrays it was six of each, and the kernels are bound by
+// instruction issue).
 struct PBuf {
-    int32_t* cell;
-    float2* f;
-    float2* v;
-    float* h;
-    float* m;
-    int32_t* id;
+    float4* a;  // offset f.x, f.y; velocity v.x, v.y
+    float4* b;  // h, m, cell, id (the last two as integer bits)
     float* vz;
     float* z;
 };
+__device__ __forceinline__ int32_t p_cell(const PBuf& B, int q) { return reinterpret_cast<const int32_t*>(B.b)[4 * (size_t)q + 2]; }
+__device__ __forceinline__ int32_t p_id(const PBuf& B, int q) { return reinterpret_cast<const int32_t*>(B.b)[4 * (size_t)q + 3]; }
 
 // Per-scenario counters (device).
 struct SCnt {
@@ -145,9 +145,7 @@ struct Shared {
     Ctl* ctl;             // [nscn] control blocks (scn[s].ctl == ctl + s)
     SDyn* dyn;            // [nscn] values of the running step
     int32_t* work_pref;   // [nscn+1] prefix of active tiles (P2G / G2P work)
-    int32_t* wlist;       // [2][work_cap] work items of the two P2G kernels: dense tiles, then sparse ones
-    int32_t* wcount;      // [2] their counts
-    int32_t split_min;    // tiles with more particles go to the dense kernel; < 0: one P2G kernel for all
+    int32_t split_min;    // tiles with more particles take the cell-sorted P2G, the others the fixed-point one
     int32_t pad3_;
     int32_t* gflat;       // [gcap][2] grid tiles of the running step: (scenario, grid tile)
     int32_t* gcount;      // entries in gflat

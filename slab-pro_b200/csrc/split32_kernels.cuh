@@ -130,6 +130,24 @@ __device__ __forceinline__ int cand_to_index(int q, const TileDesc& D, int& d) {
     return D.rstart[d] + (q - D.rpref[d]);
 }
 
+// candidate index -> particle index in the current buffer (range d). Most
+// candidates are the tile's own stayers, range 4.
+__device__ __forceinline__ int cand_index(int q, const TileDesc& D, int& d) {
+    const int p4 = D.rpref[4], p5 = D.rpref[5];
+    if (q >= p4 && q < p5) {
+        d = 4;
+        return D.rstart[4] + (q - p4);
+    }
+    d = q < p4 ? 0 : 5;
+    while (d < 8 && D.rpref[d + 1] <= q) ++d;
+    return D.rstart[d] + (q - D.rpref[d]);
+}
+
+// two-wide FP32 (one instruction each on sm_100), rounded as written
+__device__ __forceinline__ float2 f2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 f2mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
 constexpr int DESC_WORDS = (int)(sizeof(TileDesc) / 4);
 
 // copy a descriptor to shared memory (threads 0..27)
@@ -245,8 +263,6 @@ __device__ __forceinline__ void control_scenarios(const Shared& sh, int what, in
         sh.work_pref[sh.nscn] = min(total, sh.work_cap);
         if (total > sh.work_cap) atomicOr(&sh.ctl[0].err, ERR_CAPACITY);
         *sh.gcount = 0;
-        sh.wcount[0] = 0;
-        sh.wcount[1] = 0;
     }
 }
 
@@ -282,26 +298,21 @@ __device__ __forceinline__ void load_scn(const Shared& sh, int sid, ScnSm& z, in
     if (t == 0) z.sid = sid;
 }
 
-// The work items of one CTA: a contiguous range of the flat work list, so
-// that consecutive items mostly belong to the same scenario.
-__device__ __forceinline__ void work_range(int nwork, int& w0, int& w1) {
-    const int per = (nwork + (int)gridDim.x - 1) / (int)gridDim.x;
-    w0 = min((int)blockIdx.x * per, nwork);
-    w1 = min(w0 + per, nwork);
-}
-
-// Scenario of the last work item looked up, with the step fields that do not
-// change during a launch (so a new item of the same scenario costs no loads).
-struct WorkCache {
-    int sid = -1, lo = 0, hi = 0, seq = 0, stepid = 0;
+// The work items w0, w0 + step, ... < w1 of one of n workers. Of several
+// scenarios a worker takes a contiguous run of the flat list, so that
+// consecutive items mostly belong to the same scenario. Of one scenario it
+// takes every n-th item: the list is roughly in the order of space, so runs of
+// it are all dense tiles for one worker and all sparse ones for the next (300 k
+// particles in a thin tongue: P2G 62 us with runs, 49 us with strides).
+struct WorkItems {
+    int w0, w1, step;
 };
-
-// Work items of a P2G kernel: class 0 (dense tiles), 1 (sparse tiles), or
-// -1 (every active tile, when the step runs one P2G kernel).
-__device__ __forceinline__ int p2g_count(const Shared& sh, int cls) {
-    return cls < 0 ? sh.work_pref[sh.nscn] : min(sh.wcount[cls], sh.work_cap);
+__device__ __forceinline__ WorkItems work_items(const Shared& sh, int nwork, int me, int n) {
+    if (sh.nscn == 1) return {me, nwork, n};
+    const int per = (nwork + n - 1) / n;
+    const int w0 = min(me * per, nwork);
+    return {w0, min(w0 + per, nwork), 1};
 }
-__device__ __forceinline__ int p2g_item(const Shared& sh, int cls, int i) { return cls < 0 ? i : sh.wlist[cls * sh.work_cap + i]; }
 
 // K1 (bookkeeping half): a tile's particles are the stayers of its own
 // segment in the current buffer plus the movers of the 8 neighbour segments
@@ -323,7 +334,7 @@ static_assert(sizeof(TileDesc) == 28 * 4 && offsetof(TileDesc, rstart) == 4 * 4 
 
 __device__ __forceinline__ void prep_body(const Shared& sh) {
     __shared__ int s_sid[PREP_MAX_TILES], s_cnt[PREP_MAX_TILES], s_ng[PREP_MAX_TILES];  // of the block's tiles
-    __shared__ int s_off[PREP_MAX_TILES], s_goff[PREP_MAX_TILES], s_cat[PREP_MAX_TILES];
+    __shared__ int s_off[PREP_MAX_TILES], s_goff[PREP_MAX_TILES];
     const int nwork = sh.work_pref[sh.nscn];
     const int lane = threadIdx.x & 31, r = lane & (PREP_LANES - 1);
     const int per_block = (int)blockDim.x / PREP_LANES, mine = threadIdx.x / PREP_LANES;
@@ -382,7 +393,7 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
 #pragma unroll
         for (int o = PREP_LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o, PREP_LANES);
         const int ncand = __shfl_sync(0xffffffffu, incl, 8, PREP_LANES);
-        // the segment cursor, the class lists and the flat grid-tile list: one
+        // the segment cursor and the flat grid-tile list: one
         // atomic per address and block, by its first warp (one per address and
         // warp made 3 same-address atomics per two tiles: 44 us on 47 k tiles)
         const unsigned gmask = __ballot_sync(0xffffffffu, new_gt);
@@ -400,23 +411,15 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
                 const int qs = q < per_block ? s_sid[q] : -1;
                 const unsigned m = __ballot_sync(0xffffffffu, qs >= 0);
                 if (qs >= 0) {
-                    const int qc = s_cnt[q], cls = qc > sh.split_min ? 0 : 1;
-                    const WarpAdd a_cur = warp_add_issue(&sh.cnt[qs].cursor, qc, m);
+                    const WarpAdd a_cur = warp_add_issue(&sh.cnt[qs].cursor, s_cnt[q], m);
                     const WarpAdd a_gt = warp_add_issue(sh.gcount, s_ng[q], m);
-                    WarpAdd a_cls{};
-                    if (sh.split_min >= 0) a_cls = warp_add_issue(sh.wcount + cls, 1, m);
                     s_off[q] = warp_add_finish(a_cur);
                     s_goff[q] = warp_add_finish(a_gt);
-                    if (sh.split_min >= 0) s_cat[q] = warp_add_finish(a_cls);
                 }
             }
         }
         __syncthreads();
         const int nxt_off = s_off[mine], at_g = s_goff[mine];
-        if (valid && r == 0 && sh.split_min >= 0) {  // dense tiles to the cell-sorted P2G, sparse ones to the fixed-point P2G
-            const int at = s_cat[mine];
-            if (at < sh.work_cap) sh.wlist[(cnt > sh.split_min ? 0 : 1) * sh.work_cap + at] = w;
-        }
         // the new grid tiles onto the flat grid-tile list, in lane order
         if (new_gt) {
             const int at = at_g + __popc(gmask & hbits & ((1u << lane) - 1u));
@@ -454,6 +457,27 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep(Shared sh) { prep_body(sh
 
 // ------------------------------------------------------------------- P2G
 
+constexpr int NWIN = TN * TN;  // nodes of a tile's window
+constexpr int NSLOT = 9;       // nodes a cell's particles reach (3 x 3)
+
+// A tile's partial window (PART_STRIDE floats): {m, m h, m vx, m vy} per node,
+// then {Fx, Fy} per node, then m vz per node (output steps): a node is one
+// 16-byte and one 8-byte access, and the pairs are operands of the two-wide
+// adds. Sum q (the order of NQ) and node of float k of it:
+__device__ __forceinline__ void part_slot(int k, int& q, int& node) {
+    if (k < 4 * NWIN) {
+        const int c = k & 3;
+        q = c == 0 ? 0 : (c == 1 ? 3 : c - 1);
+        node = k >> 2;
+    } else if (k < 6 * NWIN) {
+        q = 4 + (k & 1);
+        node = (k - 4 * NWIN) >> 1;
+    } else {
+        q = 6;
+        node = k - 6 * NWIN;
+    }
+}
+
 constexpr int P2G_THREADS = NCELL;  // one thread per cell slot; the CTA strides over its tile's particles
 constexpr int P2G_MIN_BLOCKS = NCELL == 64 ? 16 : 4;
 
@@ -490,25 +514,30 @@ struct PQ {
     int li, lj;
 };
 
-__device__ __forceinline__ PQ load_pq(const PBuf& B, int src, int li, int lj, const float4* dem, float g, float hod, bool outs) {
+// from the particle's two words and vz, its cell (li, lj) in the tile and the
+// tile's terrain window
+__device__ __forceinline__ PQ make_pq(float4 a, float4 b, float vz, int li, int lj, const float4* dem, float g, float hod) {
     PQ p;
-    const float2 f = B.f[src], v = B.v[src];
-    const float h = B.h[src], m = B.m[src];
-    const float4 dm = dem[(li + (f.x >= 1.f ? 1 : 0)) * (TILE + 1) + (lj + (f.y >= 1.f ? 1 : 0))];
+    const float4 dm = dem[(li + (a.x >= 1.f ? 1 : 0)) * (TILE + 1) + (lj + (a.y >= 1.f ? 1 : 0))];
+    const float h = b.x, m = b.y;
     const float K = m * g * dm.z * dm.z;
-    p.fx = f.x;
-    p.fy = f.y;
+    p.fx = a.x;
+    p.fy = a.y;
     p.m = m;
-    p.mvx = m * v.x;
-    p.mvy = m * v.y;
+    p.mvx = m * a.z;
+    p.mvy = m * a.w;
     p.mh = m * h;
-    p.mvz = outs ? m * B.vz[src] : 0.f;
+    p.mvz = m * vz;
     p.Kgx = K * dm.x;
     p.Kgy = K * dm.y;
     p.Khh = K * h * hod;
     p.li = li;
     p.lj = lj;
     return p;
+}
+
+__device__ __forceinline__ PQ load_pq(const PBuf& B, int src, int li, int lj, const float4* dem, float g, float hod, bool outs) {
+    return make_pq(B.a[src], B.b[src], outs ? B.vz[src] : 0.f, li, lj, dem, g, hod);
 }
 
 // K2: P2G of one tile (src/simulation.cpp:726-798), one thread per particle,
@@ -522,14 +551,12 @@ __device__ __forceinline__ PQ load_pq(const PBuf& B, int src, int li, int lj, co
 // than FP32 relative to the largest contribution. Pass B adds the
 // contributions; the window is converted back and written as the partials.
 template <int ACC>
-__global__ void __launch_bounds__(P2G_THREADS, P2G_MIN_BLOCKS) k_p2g(Shared sh, int cls) {
+__global__ void __launch_bounds__(P2G_THREADS, P2G_MIN_BLOCKS) k_p2g(Shared sh) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     P2GSmem& sm = *reinterpret_cast<P2GSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31;
-    int i0, i1;
-    work_range(p2g_count(sh, cls), i0, i1);
-    for (int i = i0; i < i1; ++i) {
-        const int w = p2g_item(sh, cls, i);
+    const WorkItems W = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
+    for (int w = W.w0; w < W.w1; w += W.step) {
         load_desc(sh.desc + w, &sm.d);
         for (int k = tid; k < NQ * TN * TN; k += P2G_THREADS) sm.node[k] = 0;
         int* node32 = reinterpret_cast<int*>(sm.node);  // ACC_I32: [q][node]; ACC_HILO: hi at [q][node], lo at NQ*TN*TN + [q][node]
@@ -556,7 +583,7 @@ __global__ void __launch_bounds__(P2G_THREADS, P2G_MIN_BLOCKS) k_p2g(Shared sh, 
         for (int k = tid; k < ncand; k += P2G_THREADS) {
             int d;
             const int src = cand_to_index(k, sm.d, d);
-            const int32_t cell = B.cell[src];
+            const int32_t cell = p_cell(B, src);
             const int li = cell_i(cell) - ti * TILE, lj = cell_j(cell) - tj * TILE;
             if ((unsigned)li >= TILE || (unsigned)lj >= TILE) {
                 if (d == 4) atomicOr(&S.ctl->err, ERR_MOVE);  // a stayer outside its tile
@@ -609,7 +636,7 @@ __global__ void __launch_bounds__(P2G_THREADS, P2G_MIN_BLOCKS) k_p2g(Shared sh, 
         for (int k = tid; k < ncand; k += P2G_THREADS) {
             int d;
             const int src = cand_to_index(k, sm.d, d);
-            const int32_t cell = B.cell[src];
+            const int32_t cell = p_cell(B, src);
             const int li = cell_i(cell) - ti * TILE, lj = cell_j(cell) - tj * TILE;
             if ((unsigned)li >= TILE || (unsigned)lj >= TILE) continue;
             const PQ p = load_pq(B, src, li, lj, sm.dem, g, hod, outs);
@@ -649,11 +676,14 @@ __global__ void __launch_bounds__(P2G_THREADS, P2G_MIN_BLOCKS) k_p2g(Shared sh, 
         __syncthreads();
         float* P = sh.part + (size_t)w * PART_STRIDE;
         for (int k = tid; k < PART_STRIDE; k += P2G_THREADS) {
-            const float is = sm.iscale[k / (TN * TN)];
+            int q, nd;
+            part_slot(k, q, nd);
+            const int at = q * NWIN + nd;
+            const float is = sm.iscale[q];
             float v;
-            if (ACC == ACC_I64) v = (float)((double)sm.node[k] * (double)is);
-            else if (ACC == ACC_HILO) v = (float)(((double)node32[k] + (double)node32[NQ * TN * TN + k] * lo_div) * (double)is);
-            else v = (float)node32[k] * is;
+            if (ACC == ACC_I64) v = (float)((double)sm.node[at] * (double)is);
+            else if (ACC == ACC_HILO) v = (float)(((double)node32[at] + (double)node32[NQ * NWIN + at] * lo_div) * (double)is);
+            else v = (float)node32[at] * is;
             P[k] = v;
         }
         __syncthreads();
@@ -678,9 +708,10 @@ __device__ __forceinline__ PQ warp_pq(const Shared& sh, const PBuf& B, const Til
                                       bool& valid, bool& stayer) {
     int d;
     const int src = cand_to_index(k, D, d);
-    const int32_t cell = B.cell[src];
-    const float2 f = B.f[src], v = B.v[src];
-    const float h = B.h[src], m = B.m[src];
+    const float4 pa = B.a[src], pb = B.b[src];
+    const int32_t cell = __float_as_int(pb.z);
+    const float2 f = make_float2(pa.x, pa.y), v = make_float2(pa.z, pa.w);
+    const float h = pb.x, m = pb.y;
     const float vz = outs ? B.vz[src] : 0.f;
     const int ci = cell_i(cell), cj = cell_j(cell);
     const int li = ci - ti * TILE, lj = cj - tj * TILE;
@@ -717,18 +748,17 @@ __device__ __forceinline__ PQ warp_pq(const Shared& sh, const PBuf& B, const Til
 // particles of one cell (mcc); a node's sum stays below 9 * mcc * 0.75 * b,
 // and the scale is the largest power of two that keeps that below 2^30; the
 // hi word is the rounded contribution, the lo word the rest at 2^-20.
-__global__ void __launch_bounds__(P2W_THREADS, 3) k_p2g_warp(Shared sh, int cls) {
+__global__ void __launch_bounds__(P2W_THREADS, 3) k_p2g_warp(Shared sh) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     P2WWarp& sw = reinterpret_cast<P2WWarp*>(smem_raw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int gw = blockIdx.x * P2W_WARPS + (threadIdx.x >> 5), nw = gridDim.x * P2W_WARPS;
-    const int nwork = p2g_count(sh, cls);
+    const int nwork = sh.work_pref[sh.nscn];
     const int per = (nwork + nw - 1) / nw;
     const int i0 = min(gw * per, nwork), i1 = min(i0 + per, nwork);
     int* hi = sw.node;
     int* lo = sw.node + NQ * TN * TN;
-    for (int i = i0; i < i1; ++i) {
-        const int w = p2g_item(sh, cls, i);
+    for (int w = i0; w < i1; ++w) {
         if (lane < (int)(sizeof(TileDesc) / 4)) reinterpret_cast<int*>(&sw.d)[lane] = reinterpret_cast<const int*>(sh.desc + w)[lane];
         for (int k = lane; k < 2 * NQ * TN * TN; k += 32) sw.node[k] = 0;
         for (int k = lane; k < NCELL; k += 32) sw.ccnt[k] = 0;
@@ -837,22 +867,21 @@ __global__ void __launch_bounds__(P2W_THREADS, 3) k_p2g_warp(Shared sh, int cls)
         __syncwarp();
         float* P = sh.part + (size_t)w * PART_STRIDE;
         for (int k = lane; k < PART_STRIDE; k += 32) {
-            const int q = k / (TN * TN);
+            int q, nd;
+            part_slot(k, q, nd);
             float is = isc[0];
 #pragma unroll
             for (int r = 1; r < NQ; ++r)
                 if (q == r) is = isc[r];
-            P[k] = (float)(((double)hi[k] + (double)lo[k] * lo_div) * (double)is);
+            P[k] = (float)(((double)hi[q * NWIN + nd] + (double)lo[q * NWIN + nd] * lo_div) * (double)is);
         }
         __syncwarp();
     }
 }
 
-// ------------------------------------------------ P2G over cell-sorted particles
-
 // Optional per-phase cycle counters of the P2G kernel (builds with
 // -DSLAB_PHASE_CLOCKS only): thread 0 of each CTA adds the clock64 cycles of
-// each phase of each tile to g_phase_clk[phase] (cell P2G 0-6, G2P 8-12);
+// each phase of each tile to g_phase_clk[phase] (P2G 0-5, G2P 8-11);
 // g_phase_clk[15] and [14] count their tiles.
 #ifdef SLAB_PHASE_CLOCKS
 __device__ unsigned long long g_phase_clk[16];
@@ -880,856 +909,553 @@ __device__ unsigned long long g_phase_clk[16];
 #define SLAB_PHASE_TILE_G2P()
 #endif
 
-// index of work item w in its scenario's list (pref: the prefix over scenarios)
-__device__ __forceinline__ int cached_work(const Shared& sh, const int32_t* pref, int w, WorkCache& c) {
-    if (w < c.lo || w >= c.hi) {
-        int loc;
-        find_work(pref, sh.nscn, w, c.sid, loc);
-        c.lo = pref[c.sid];
-        c.hi = pref[c.sid + 1];
-        const SCnt* n = sh.scn[c.sid].cnt;
-        c.seq = n->seq;
-        c.stepid = n->stepid;
-    }
-    return w - c.lo;
-}
+// --------------------------------------------------------- P2G over tiles
 
-
-constexpr int P2C_THREADS = NCELL;  // one thread per cell of the tile
-#ifndef SLAB_P2C_MIN_BLOCKS
-#define SLAB_P2C_MIN_BLOCKS (NCELL == 64 ? 12 : 3)
-#endif
-constexpr int P2C_MIN_BLOCKS = SLAB_P2C_MIN_BLOCKS;  // resident CTAs per SM the register budget is cut for
-constexpr int P2C_WARPS = P2C_THREADS / 32;
-constexpr int NSLOT = 9;            // nodes a cell's particles reach (3 x 3)
-constexpr int P2C_CAP = 6 * NCELL;  // candidates of a tile staged in shared memory (more go through global memory)
-
-struct P2CStage {
-    float4 sa[P2C_CAP];  // staged candidates, by candidate index: f.x, f.y, m, h
-    float2 sv[P2C_CAP];  //                                        v
-    float svz[P2C_CAP];  //                                        vz
-};
-
-struct P2CSmem {
-    P2CStage st;
-    float nsum[NQ * TN * TN];  // node sums of the tile's window, [q][node]
-    int16_t lc[P2C_CAP];   // local cell of each staged candidate (-1: not in the tile)
-    union {
-        int32_t ccell[P2C_CAP];  // phase 1: cell of each staged candidate
-        int16_t idx[P2C_CAP];    // phases 3-4: sorted position -> candidate index
-    };
-    alignas(128) float4 dem[(TILE + 1) * (TILE + 1)];  // a tensor copy's destination: 128-byte aligned
-    alignas(8) uint64_t dem_bar;  // completion of the terrain window's tensor copy (k_p2g_cell<false>)
-    int wcur[P2C_WARPS][NCELL];  // per-warp cell counts, then per-warp write cursors
-    int s_warp[33];
-    TileDesc d;
-    // the scenario of the CTA's current run of tiles (loaded when it changes)
-    PBuf B;             // current particle buffer
-    int32_t* nxt_cell;  // cell array of the next buffer (sorted index lists of large tiles)
-    Ctl* ctl;
-    float g, hod;
-    int csid, outs;
-};
-
-// Bulk-copy staging of the next tile (k_p2g_cell<true>): its 9 candidate
-// ranges of the particle arrays, each rounded out to 16-byte boundaries, and
-// its terrain window, copied by the TMA engine while the current tile is
-// summed. 4-byte arrays take at most 6 extra elements per range, 8-byte ones 2.
-constexpr int P2C_SCAP4 = (P2C_CAP + 9 * 6 + 3) / 4 * 4;
-constexpr int P2C_SCAP8 = (P2C_CAP + 9 * 2 + 1) / 2 * 2;
-constexpr int DEM_W = TILE + 1;  // terrain window edge (nodes)
-
-struct alignas(16) P2CTmaStage {
-    int32_t cell[P2C_SCAP4];
-    float h[P2C_SCAP4];
-    float m[P2C_SCAP4];
-    float vz[P2C_SCAP4];
-    float2 f[P2C_SCAP8];
-    float2 v[P2C_SCAP8];
-};
-static_assert(P2C_SCAP4 * 4 % 16 == 0 && P2C_SCAP8 * 8 % 16 == 0, "16-byte aligned stage arrays");
-
-struct P2CSmemTma : P2CSmem {
-    P2CTmaStage ts;                             // the tile's candidates (until its phase 1 has read them)
-    alignas(16) float4 dem2[2][DEM_W * DEM_W];  // terrain windows of this and the next tile
-    alignas(8) uint64_t bar;                    // completion of the staged copies
-    TileDesc dnext;                             // the next tile's descriptor
-    int lead4[9], lead8[9];                     // stage index of each range's first candidate (4-byte / 8-byte arrays)
-    int use_stage, dem_staged[2];               // the tile's candidates / terrain windows came by bulk copy
-};
-
-// Thread 0: lays out the 9 ranges of tile D in the stage and starts their
-// bulk copies (and the terrain window's rows into dem2[slot]) on sm.bar.
-// Candidates that do not fit leave the tile to the load path (use_stage 0).
-// The particle arrays are padded past Np, so a range rounded up to 16 bytes
-// stays inside its allocation.
-__device__ __forceinline__ void p2c_issue_stage(P2CSmemTma& sm, const TileDesc& D, const PBuf& B, bool outs, const Shared& sh, int slot) {
-    int o4 = 0, o8 = 0;
-    bool fit = D.rpref[9] <= P2C_CAP;
-    int a4[9], n4[9], a8[9], n8[9];
-#pragma unroll
-    for (int d = 0; d < 9; ++d) {
-        const int rs = D.rstart[d], rl = D.rpref[d + 1] - D.rpref[d];
-        a4[d] = rs & ~3;
-        n4[d] = rl > 0 ? ((rs + rl + 3) & ~3) - a4[d] : 0;
-        a8[d] = rs & ~1;
-        n8[d] = rl > 0 ? ((rs + rl + 1) & ~1) - a8[d] : 0;
-        sm.lead4[d] = o4 + (rs - a4[d]);
-        sm.lead8[d] = o8 + (rs - a8[d]);
-        o4 += n4[d];
-        o8 += n8[d];
-    }
-    if (o4 > P2C_SCAP4 || o8 > P2C_SCAP8) fit = false;
-    // the terrain window by rows when it lies inside the terrain
-    const int ti = D.t / sh.TY, tj = D.t % sh.TY;
-    const bool dem_in = ti * TILE + TILE < sh.Nx && tj * TILE + TILE < sh.Ny;
-    sm.dem_staged[slot] = dem_in ? 1 : 0;
-    sm.use_stage = fit ? 1 : 0;
-    uint32_t bytes = dem_in ? DEM_W * DEM_W * 16 : 0;
-    if (fit) bytes += (uint32_t)o4 * 4u * (outs ? 4u : 3u) + (uint32_t)o8 * 8u * 2u;
-    tma::fence_proxy_async();  // the CTA's earlier ordinary reads of these bytes come first
-    tma::mbar_arrive_expect_tx(&sm.bar, bytes);
-    if (dem_in)
-        for (int r = 0; r < DEM_W; ++r)
-            tma::bulk_g2s(&sm.dem2[slot][r * DEM_W], sh.dem + (int64_t)(ti * TILE + r) * sh.Ny + tj * TILE, DEM_W * 16, &sm.bar);
-    if (!fit) return;
-    int q4 = 0, q8 = 0;
-#pragma unroll
-    for (int d = 0; d < 9; ++d) {
-        if (n4[d]) {
-            tma::bulk_g2s(sm.ts.cell + q4, B.cell + a4[d], n4[d] * 4, &sm.bar);
-            tma::bulk_g2s(sm.ts.h + q4, B.h + a4[d], n4[d] * 4, &sm.bar);
-            tma::bulk_g2s(sm.ts.m + q4, B.m + a4[d], n4[d] * 4, &sm.bar);
-            if (outs) tma::bulk_g2s(sm.ts.vz + q4, B.vz + a4[d], n4[d] * 4, &sm.bar);
-            tma::bulk_g2s(sm.ts.f + q8, B.f + a8[d], n8[d] * 8, &sm.bar);
-            tma::bulk_g2s(sm.ts.v + q8, B.v + a8[d], n8[d] * 8, &sm.bar);
-        }
-        q4 += n4[d];
-        q8 += n8[d];
-    }
-}
-
-// P2G quantities of a staged particle (as load_pq)
-__device__ __forceinline__ PQ staged_pq(float4 a, float2 v, float vz, int li, int lj, const float4* dem, float g, float hod) {
-    PQ p;
-    const float4 dm = dem[(li + (a.x >= 1.f ? 1 : 0)) * (TILE + 1) + (lj + (a.y >= 1.f ? 1 : 0))];
-    const float K = a.z * g * dm.z * dm.z;
-    p.fx = a.x;
-    p.fy = a.y;
-    p.m = a.z;
-    p.mvx = a.z * v.x;
-    p.mvy = a.z * v.y;
-    p.mh = a.z * a.w;
-    p.mvz = a.z * vz;
-    p.Kgx = K * dm.x;
-    p.Kgy = K * dm.y;
-    p.Khh = K * a.w * hod;
-    p.li = li;
-    p.lj = lj;
-    return p;
-}
-
-// Sums of one particle over the 3 nodes of stencil rows A0 .. A0+NA-1 of its
-// cell (src/simulation.cpp:758-795); OUTS adds m vz. Every operation is
-// rounded as written (explicit multiply-adds), so both variants of the cell
-// P2G, and any later change of the code around them, sum the same bits.
-template <bool OUTS, int A0, int NA>
-__device__ __forceinline__ void add_particle_rows(float (&acc)[NA][NQ][3], const PQ& p) {
-    float wx[3], wy[3], dwx[3], dwy[3];
-    bspline3(p.fx, wx, dwx);
-    bspline3(p.fy, wy, dwy);
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int A = A0 + a;
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            const float wgt = __fmul_rn(wx[A], wy[b]);
-            if (wgt > 3e-3f) {  // the reference's weight cut-off (src/simulation.cpp:780)
-                acc[a][0][b] = __fmaf_rn(p.m, wgt, acc[a][0][b]);
-                acc[a][1][b] = __fmaf_rn(p.mvx, wgt, acc[a][1][b]);
-                acc[a][2][b] = __fmaf_rn(p.mvy, wgt, acc[a][2][b]);
-                acc[a][3][b] = __fmaf_rn(p.mh, wgt, acc[a][3][b]);
-                acc[a][4][b] = __fadd_rn(acc[a][4][b], __fmaf_rn(p.Khh, __fmul_rn(dwx[A], wy[b]), -__fmul_rn(p.Kgx, wgt)));
-                acc[a][5][b] = __fadd_rn(acc[a][5][b], __fmaf_rn(p.Khh, __fmul_rn(dwy[b], wx[A]), -__fmul_rn(p.Kgy, wgt)));
-                if (OUTS) acc[a][6][b] = __fmaf_rn(p.mvz, wgt, acc[a][6][b]);
-            }
-        }
-    }
-}
-
-// Rows A0 .. A0+NA-1 of one cell's particles, summed in sorted order: staged
-// in shared memory, or (tiles over P2C_CAP candidates) read through the
-// sorted index list in global memory.
-template <bool OUTS, int A0, int NA>
-__device__ __forceinline__ void cell_row_sums(float (&acc)[NA][NQ][3], bool staged, const P2CSmem& sm, const float4* dem,
-                                              const int32_t* order, int c0, int nn, const PBuf& B, int li, int lj, float g,
-                                              float hod) {
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) acc[a][q][b] = 0.f;
-    if (staged) {
-        for (int r = c0; r < c0 + nn; ++r) {
-            const int k = sm.idx[r];
-            add_particle_rows<OUTS, A0, NA>(acc, staged_pq(sm.st.sa[k], sm.st.sv[k], sm.st.svz[k], li, lj, dem, g, hod));
-        }
-        return;
-    }
-    int nsrc = nn > 0 ? order[c0] : 0;
-    for (int r = 0; r < nn; ++r) {
-        const int src = nsrc;
-        if (r + 1 < nn) nsrc = order[c0 + r + 1];
-        add_particle_rows<OUTS, A0, NA>(acc, load_pq(B, src, li, lj, dem, g, hod, OUTS));
-    }
-}
-
-// Stencil rows A0 .. A0+NA-1 of every cell into the node sums: in round
-// (A, b) each node receives the row sum of exactly one cell, so the rounds
-// need no atomics and every node adds its <= 9 cells in (a, b) order.
-template <bool OUTS, int A0, int NA>
-__device__ __forceinline__ void p2c_rowset(P2CSmem& sm, bool staged, const float4* dem, const int32_t* order, int c0,
-                                           int nn, const PBuf& B, int li, int lj, float g, float hod) {
-    float acc[NA][NQ][3];
-    cell_row_sums<OUTS, A0, NA>(acc, staged, sm, dem, order, c0, nn, B, li, lj, g, hod);
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            __syncthreads();
-            const int nd = (li + A0 + a) * TN + (lj + b);
-#pragma unroll
-            for (int q = 0; q < (OUTS ? NQ : NQ - 1); ++q) sm.nsum[q * TN * TN + nd] += acc[a][q][b];
-        }
-}
-
-// Rows per pass over a cell's particles: each pass evaluates the particles'
-// weights and quantities once; more rows per pass cost accumulator registers.
-#ifndef SLAB_P2C_ROWS
-#define SLAB_P2C_ROWS 2
-#endif
-template <bool OUTS>
-__device__ __forceinline__ void p2c_rows(P2CSmem& sm, bool staged, const float4* dem, const int32_t* order, int c0, int nn,
-                                         const PBuf& B, int li, int lj, float g, float hod) {
-    if constexpr (SLAB_P2C_ROWS == 3) {
-        p2c_rowset<OUTS, 0, 3>(sm, staged, dem, order, c0, nn, B, li, lj, g, hod);
-    } else if constexpr (SLAB_P2C_ROWS == 2) {
-        p2c_rowset<OUTS, 0, 2>(sm, staged, dem, order, c0, nn, B, li, lj, g, hod);
-        p2c_rowset<OUTS, 2, 1>(sm, staged, dem, order, c0, nn, B, li, lj, g, hod);
-    } else {
-        p2c_rowset<OUTS, 0, 1>(sm, staged, dem, order, c0, nn, B, li, lj, g, hod);
-        p2c_rowset<OUTS, 1, 1>(sm, staged, dem, order, c0, nn, B, li, lj, g, hod);
-        p2c_rowset<OUTS, 2, 1>(sm, staged, dem, order, c0, nn, B, li, lj, g, hod);
-    }
-}
-
-// K2: P2G of one tile (src/simulation.cpp:726-798) as a segmented reduction
-// over cell-sorted particles, with no atomics on floats. The tile's
-// descriptor comes from k_prep; then
-//  1. the tile's candidates and terrain window come into shared memory as
-//     per-thread asynchronous copies, all requested in one round (a tile
-//     with more than P2C_CAP candidates reads only their cells, chunk by
-//     chunk); then each warp walks a contiguous block of the candidates and
-//     counts particles per cell (lanes of one cell are grouped by
+// K2: P2G of the active tiles (src/simulation.cpp:726-798), one CTA per tile.
+// A tile with more than split_min particles is summed in FP32 over its
+// particles sorted by cell; one with fewer in exact fixed point (below). Which
+// scheme a tile gets depends only on its own particle count.
+//
+// Dense tiles. Threads = 3 x cells: thread (row, cell) owns stencil row `row`
+// of its cell's 3 x 3 nodes, so the sums of a cell's particles stay in 18
+// registers however many particles there are. Per pass of up to P2C_CAP
+// candidates (one pass, but for very dense tiles):
+//  1. the candidates (two float4 each) and the terrain window (one 2-D tensor
+//     copy) are in shared memory: both were requested while the tile before
+//     was summed, each thread the candidates that it reads itself. They are
+//     counted per cell and chunk of 32 (lanes of one cell grouped by
 //     __match_any_sync);
-//  2. thread = cell: per-warp write cursors and the cell's range (a scan);
-//  3. the warps walk their blocks again and give each particle its place --
-//     a stable counting sort by cell -- as an index in shared memory (large
-//     tiles: an index into the tile's segment of the next particle buffer,
-//     unused until G2P);
-//  4. thread = cell: FP32 sums of the cell's particles, in sorted order, for
-//     the 3 nodes of one stencil row at a time (21 accumulators, so 12 tiles
-//     fit on an SM), each row added into shared node sums in three rounds:
-//     every node adds its <= 9 cells in (a, b) order;
-//  5. the node sums are the tile's partial window.
+//  2. warp 0 turns the counts into each chunk's write cursors and the cells'
+//     ranges: a stable counting sort by cell;
+//  3. each thread writes its candidates' P2G quantities (mass, momentum, m h,
+//     force terms) straight to their sorted places, so these are computed
+//     once per particle and the sums read them in order. Places are XOR-
+//     swizzled: 4 particles per cell, the common filling, put the 8 threads of
+//     a 128-byte phase on 8 different 16-byte banks. The next tile's
+//     candidates are requested into the places just read;
+//  4. thread (row, cell) adds its cell's particles in sorted order over the 3
+//     nodes of its row (packed two-wide FP32: mass and m h, the momentum, the
+//     force). Every operation is rounded as written.
+// Then the 9 row sums of every cell go to shared memory (over the stage), and
+// one thread per node adds its <= 9 cells in (a, b) order and writes the
+// tile's partial window: no zeroed node sums, no rounds between barriers.
 // The candidates of a tile come in an order fixed by the previous step's G2P
 // (ordered placement), so every sum has a fixed order: results are bitwise
-// reproducible and the same alone or inside a batch. A tile costs one round
-// of global loads (its descriptor is read while the tile before it runs);
-// each CTA takes a contiguous run of work items.
-// With TMA = true the loads of a tile leave its critical path: while tile n
-// is summed (phases 2-5), thread 0 has the TMA engine copy tile n+1's
-// candidate ranges and terrain window into shared memory (p2c_issue_stage),
-// and the descriptor after that is read into registers. Tiles whose
-// candidates do not fit the stage load them as before.
+// reproducible and the same alone or inside a batch.
+constexpr int P2G_T = 3 * NCELL;        // threads of a CTA
+constexpr int P2C_CAP = 5 * NCELL;      // candidates of one pass
+constexpr int P2C_PER = (P2C_CAP + P2G_T - 1) / P2G_T;  // per thread
+constexpr int P2C_CHUNKS = P2C_CAP / 32;
+constexpr int P2C_HALVES = NCELL / 2;   // words of a chunk's 16-bit cell counts
+#ifndef SLAB_P2G_MIN_BLOCKS
+#define SLAB_P2G_MIN_BLOCKS (NCELL == 64 ? 6 : 1)
+#endif
 
-// the CTA's scenario values for a run of its tiles (thread 0)
-template <typename Sm> __device__ __forceinline__ void p2c_load_scenario(Sm& sm, const Shared& sh, int sid) {
-    const Scn& S = sh.scn[sid];
-    const SDyn& n = sh.dyn[sid];
-    const int cur = n.seq & 1;
-    const PBuf b0 = S.buf[0], b1 = S.buf[1];  // loaded beside seq
-    sm.B = cur ? b1 : b0;
-    sm.nxt_cell = cur ? b0.cell : b1.cell;
-    sm.ctl = S.ctl;
-    sm.g = S.g;
-    sm.hod = 0.5f * S.ood;
-    sm.outs = n.outs != 0;
-    sm.csid = sid;
-}
-
-// thread 0: the copies of the tile in sm.dnext, from its scenario's buffer
-__device__ __forceinline__ void p2c_issue_next(P2CSmemTma& sm, const Shared& sh, int slot) {
-    const TileDesc& D = sm.dnext;
-    if (D.sid == sm.csid) {
-        p2c_issue_stage(sm, D, sm.B, sm.outs != 0, sh, slot);
-    } else {
-        const Scn& S = sh.scn[D.sid];
-        const SCnt* n = S.cnt;
-        p2c_issue_stage(sm, D, S.buf[n->seq & 1], n->outs != 0, sh, slot);
-    }
-}
-
-// candidate k of tile D: its range and its position in that range
-__device__ __forceinline__ int cand_range(int k, const TileDesc& D, int& off) {
-    int d = 0;
-    while (d < 8 && D.rpref[d + 1] <= k) ++d;
-    off = k - D.rpref[d];
-    return d;
-}
-
-constexpr int P2C_TMA_MIN_BLOCKS = NCELL == 64 ? 6 : 2;  // the stage doubles the shared memory of a CTA
-
-// 8x8 tiles: a staged candidate's entry in sm.lc packs its local cell (6
-// bits) and its rank among the same cell's candidates in its warp's block
-// (the rest, up to 511 > P2C_CAP / 2), so the placement needs no warp votes.
-constexpr bool P2C_PACKED = NCELL == 64;
-
-// Count one chunk of a warp's candidates per cell: lanes of one cell are
-// grouped by __match_any_sync, the group's first lane adds the group to the
-// (warp, cell) count; returns each lane's rank among its cell's candidates
-// so far in this warp (lc < 0: not in the tile, rank 0).
-__device__ __forceinline__ int p2c_count(int (&wcur)[P2C_WARPS][NCELL], int warp, int lane, int lc) {
-    const unsigned vm = __ballot_sync(0xffffffffu, lc >= 0);
-    int rank = 0;
-    if (lc >= 0) {
-        const unsigned peers = __match_any_sync(vm, lc);
-        const int leader = __ffs(peers) - 1;
-        int base = 0;
-        if (lane == leader) {
-            base = wcur[warp][lc];
-            wcur[warp][lc] = base + __popc(peers);
-        }
-        rank = __shfl_sync(peers, base, leader) + __popc(peers & ((1u << lane) - 1u));
-    }
-    __syncwarp();
-    return rank;
-}
-// one candidate of phase 1: its range, cell and the quantities to stage
-struct P2CCand {
-    int d;
-    int32_t cell;
-    float2 f, v;
-    float m, h, vz;
-    bool valid;
-};
-
-template <bool TMA>
-__device__ __forceinline__ void p2g_cell_body(const Shared& sh, int cls, unsigned char* smem_raw, const CUtensorMap* dem_map) {
-    using Sm = typename std::conditional<TMA, P2CSmemTma, P2CSmem>::type;
-    Sm& sm = *reinterpret_cast<Sm*>(smem_raw);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    const int li = tid / TILE, lj = tid % TILE;
-    int i0, i1;
-    work_range(p2g_count(sh, cls), i0, i1);
-    // the first descriptor now; each later one is read while the tile before it runs
-    int w_cur = i0 < i1 ? p2g_item(sh, cls, i0) : 0;
-    int w_nxt = i0 + 1 < i1 ? p2g_item(sh, cls, i0 + 1) : 0;
-    if (i0 < i1) load_desc(sh.desc + w_cur, &sm.d);
-    if (tid == 0) {
-        sm.csid = -1;
-        if constexpr (TMA) {
-            tma::mbar_init(&sm.bar, 1);
-        } else {
-            tma::mbar_init(&sm.dem_bar, 1);
-        }
-        tma::fence_mbar_init();
-    }
-    __syncthreads();
-    uint32_t dem_phase = 0;  // parity of the terrain window's next completion
-    if constexpr (TMA) {
-        if (tid == 0 && i0 < i1) {  // the first tile's copies
-            p2c_load_scenario(sm, sh, sm.d.sid);
-            sm.dnext = sm.d;
-            p2c_issue_next(sm, sh, 0);
-        }
-    }
-    SLAB_PHASE_BEGIN;
-    for (int i = i0, n = 0; i < i1; ++i, ++n) {
-        const int w = w_cur;
-        for (int k = tid; k < P2C_WARPS * NCELL; k += P2C_THREADS) (&sm.wcur[0][0])[k] = 0;
-        for (int k = tid; k < NQ * TN * TN; k += P2C_THREADS) sm.nsum[k] = 0.f;
-        __syncthreads();
-        SLAB_PHASE_MARK(0);
-        // the next tile's descriptor (one word per thread) and the item after it
-        int dn = 0, w_nn = 0;
-        if (i + 1 < i1 && tid < DESC_WORDS) dn = reinterpret_cast<const int*>(sh.desc + w_nxt)[tid];
-        if (i + 2 < i1) w_nn = p2g_item(sh, cls, i + 2);
-        if (sm.d.sid != sm.csid) {  // uniform: a new scenario in this CTA's run
-            __syncthreads();
-            if (tid == 0) p2c_load_scenario(sm, sh, sm.d.sid);
-            __syncthreads();
-        }
-        const int t = sm.d.t;
-        const int ti = t / sh.TY, tj = t % sh.TY;
-        const bool outs = sm.outs != 0;
-        Ctl* const ctl = sm.ctl;
-        float4* dem;
-        bool from_stage = false;
-        if constexpr (TMA) {
-            const int slot = n & 1;
-            dem = sm.dem2[slot];
-            if (!tma::mbar_wait(&sm.bar, (uint32_t)(n & 1))) atomicOr(&ctl->err, ERR_TIMEOUT);  // this tile's copies
-            from_stage = sm.use_stage != 0;
-            if (!sm.dem_staged[slot])
-                for (int k = tid; k < DEM_W * DEM_W; k += P2C_THREADS) {
-                    const int i = ti * TILE + k / DEM_W, j = tj * TILE + k % DEM_W;
-                    dem[k] = (i < sh.Nx && j < sh.Ny) ? sh.dem[(int64_t)i * sh.Ny + j] : make_float4(0.f, 0.f, 1.f, 0.f);
-                }
-        } else {
-            // the terrain window: one 2-D tensor copy (TMA) of its 9 x 9 nodes,
-            // issued by one thread, completed before phase 4. The map sees the
-            // terrain as [Nx][4 Ny] floats, so x = 4 tj TILE (a multiple of 16
-            // bytes). Nodes past the terrain's far edges read as zero; no valid
-            // particle uses them (its stencil lies inside the terrain).
-            dem = sm.dem;
-            if (tid == 0) {
-                tma::fence_proxy_async();  // the previous tile's reads of the window come first
-                tma::mbar_arrive_expect_tx(&sm.dem_bar, DEM_W * DEM_W * 16);
-                tma::tensor_g2s_2d(dem, dem_map, 4 * tj * TILE, ti * TILE, &sm.dem_bar);
-            }
-        }
-        const int ncand = sm.d.rpref[9];
-        const int total = sm.d.total;
-        const bool staged = ncand <= P2C_CAP;
-        const PBuf B = sm.B;
-        const int per = (ncand + P2C_WARPS - 1) / P2C_WARPS;
-        const int k_lo = min(warp * per, ncand), k_hi = min(k_lo + per, ncand);
-        // 1. load (stage) and count per (warp, cell). A warp requests its next
-        // chunk of 32 candidates before it stages the current one, so the
-        // chunks' load rounds overlap.
-        auto load_cand = [&](int k, P2CCand& c) {
-            c.valid = k < k_hi;
-            c.d = 0;
-            c.cell = 0;
-            c.f = c.v = make_float2(0.f, 0.f);
-            c.m = c.h = c.vz = 0.f;
-            if (!c.valid) return;
-            if (TMA && from_stage) {  // from the bulk-copied stage
-                int off;
-                c.d = cand_range(k, sm.d, off);
-                if constexpr (TMA) {
-                    const int s4 = sm.lead4[c.d] + off, s8 = sm.lead8[c.d] + off;
-                    c.cell = sm.ts.cell[s4];
-                    c.f = sm.ts.f[s8];
-                    c.v = sm.ts.v[s8];
-                    c.m = sm.ts.m[s4];
-                    c.h = sm.ts.h[s4];
-                    if (outs) c.vz = sm.ts.vz[s4];
-                }
-            } else {
-                const int src = cand_to_index(k, sm.d, c.d);
-                c.cell = B.cell[src];
-                if (staged) {  // issued together with the cell load
-                    c.f = B.f[src];
-                    c.v = B.v[src];
-                    c.m = B.m[src];
-                    c.h = B.h[src];
-                    if (outs) c.vz = B.vz[src];
-                }
-            }
-        };
-        if (!TMA && staged) {
-            // every thread requests its share of the tile's candidates (and the
-            // terrain window above) as asynchronous copies into the stage: the
-            // whole gather is one load round, with no register held per value
-            int d = 0;  // range of candidate k: k only grows, so d is carried (rpref[9] = ncand > k bounds it by 8)
-            for (int k = tid; k < ncand; k += P2C_THREADS) {
-                while (sm.d.rpref[d + 1] <= k) ++d;
-                const int src = sm.d.rstart[d] + (k - sm.d.rpref[d]);
-                cpa::copy4(&sm.ccell[k], B.cell + src);
-                cpa::copy8(&sm.st.sa[k], B.f + src);  // f.x, f.y
-                cpa::copy4(&sm.st.sa[k].z, B.m + src);
-                cpa::copy4(&sm.st.sa[k].w, B.h + src);
-                cpa::copy8(&sm.st.sv[k], B.v + src);
-                if (outs) cpa::copy4(&sm.st.svz[k], B.vz + src);
-            }
-            cpa::wait_all();
-            __syncthreads();
-            // count per (warp, cell) over the warp's block, as below
-            for (int k0 = k_lo; k0 < k_hi; k0 += 32) {
-                const int k = k0 + lane;
-                int lc = -1;
-                if (k < k_hi) {
-                    const int32_t cell = sm.ccell[k];
-                    const int ci = cell_i(cell) - ti * TILE, cj = cell_j(cell) - tj * TILE;
-                    if ((unsigned)ci < TILE && (unsigned)cj < TILE) {
-                        lc = ci * TILE + cj;
-                    } else {
-                        int off;
-                        if (cand_range(k, sm.d, off) == 4) atomicOr(&ctl->err, ERR_MOVE);  // a stayer outside its tile
-                    }
-                }
-                const int rank = p2c_count(sm.wcur, warp, lane, lc);
-                if (k < k_hi) sm.lc[k] = (int16_t)(lc < 0 ? -1 : (P2C_PACKED ? (rank << 6) | lc : lc));
-            }
-        } else {
-            P2CCand nx;
-            load_cand(k_lo + lane, nx);
-            for (int k0 = k_lo; k0 < k_hi; k0 += 32) {
-                const int k = k0 + lane;
-                const P2CCand q = nx;
-                if (k0 + 32 < k_hi) load_cand(k0 + 32 + lane, nx);
-                int lc = -1;
-                if (q.valid) {
-                    const int ci = cell_i(q.cell) - ti * TILE, cj = cell_j(q.cell) - tj * TILE;
-                    if ((unsigned)ci < TILE && (unsigned)cj < TILE) lc = ci * TILE + cj;
-                    else if (q.d == 4) atomicOr(&ctl->err, ERR_MOVE);  // a stayer outside its tile
-                    if (staged && lc >= 0) {
-                        sm.st.sa[k] = make_float4(q.f.x, q.f.y, q.m, q.h);
-                        sm.st.sv[k] = q.v;
-                        sm.st.svz[k] = q.vz;
-                    }
-                }
-                const int rank = p2c_count(sm.wcur, warp, lane, lc);
-                if (staged && q.valid) sm.lc[k] = (int16_t)(lc < 0 ? -1 : (P2C_PACKED ? (rank << 6) | lc : lc));
-            }
-        }
-        if constexpr (TMA) {
-            if (tid < DESC_WORDS) reinterpret_cast<int*>(&sm.dnext)[tid] = dn;
-        } else {
-            // every thread waits for the terrain window's tensor copy
-            if (!tma::mbar_wait(&sm.dem_bar, dem_phase)) atomicOr(&ctl->err, ERR_TIMEOUT);
-            dem_phase ^= 1u;
-        }
-        __syncthreads();
-        if constexpr (TMA) {
-            // the stage is free: the next tile's copies run beside phases 2-5 of this one
-            if (tid == 0 && i + 1 < i1) p2c_issue_next(sm, sh, (n + 1) & 1);
-        }
-        SLAB_PHASE_MARK(1);
-        // 2. cursors: cell-major, warp-minor
-        int n_c = 0;
-#pragma unroll
-        for (int q = 0; q < P2C_WARPS; ++q) {
-            const int x = sm.wcur[q][tid];
-            sm.wcur[q][tid] = n_c;
-            n_c += x;
-        }
-        const int c0 = block_exclusive_scan(n_c, sm.s_warp);
-        if (tid == P2C_THREADS - 1 && c0 + n_c != total) atomicOr(&ctl->err, ERR_CAPACITY);
-#pragma unroll
-        for (int q = 0; q < P2C_WARPS; ++q) sm.wcur[q][tid] += c0;
-        __syncthreads();
-        SLAB_PHASE_MARK(2);
-        // 3. stable placement by cell: (warp, cell) cursor + rank
-        int32_t* order = sm.nxt_cell + sm.d.nxt_off;
-        if (P2C_PACKED && staged) {
-            for (int k = k_lo + lane; k < k_hi; k += 32) {
-                const int e = sm.lc[k];
-                if (e >= 0) {
-                    const int pos = sm.wcur[warp][e & 63] + (e >> 6);
-                    if (pos >= total) atomicOr(&ctl->err, ERR_CAPACITY);
-                    else sm.idx[pos] = (int16_t)k;
-                }
-            }
-        } else
-        for (int k0 = k_lo; k0 < k_hi; k0 += 32) {
-            const int k = k0 + lane;
-            int lc = -1, src = 0;
-            if (k < k_hi) {
-                if (staged) {
-                    lc = sm.lc[k];
-                } else {
-                    int d;
-                    src = cand_to_index(k, sm.d, d);
-                    const int32_t cell = B.cell[src];
-                    const int ci = cell_i(cell) - ti * TILE, cj = cell_j(cell) - tj * TILE;
-                    if ((unsigned)ci < TILE && (unsigned)cj < TILE) lc = ci * TILE + cj;
-                }
-            }
-            const unsigned vm = __ballot_sync(0xffffffffu, lc >= 0);
-            unsigned peers = 0;
-            if (lc >= 0) {
-                peers = __match_any_sync(vm, lc);
-                const int pos = sm.wcur[warp][lc] + __popc(peers & lt);
-                if (pos >= total) atomicOr(&ctl->err, ERR_CAPACITY);
-                else if (staged) sm.idx[pos] = (int16_t)k;
-                else order[pos] = src;
-            }
-            __syncwarp();
-            if (lc >= 0 && (peers & lt) == 0) sm.wcur[warp][lc] += __popc(peers);
-            __syncwarp();
-        }
-        __syncthreads();
-        SLAB_PHASE_MARK(3);
-        // 4. per-cell row sums into the node sums
-        {
-            const int nn = max(0, min(n_c, total - c0));
-            const float g = sm.g, hod = sm.hod;
-            if (outs) p2c_rows<true>(sm, staged, dem, order, c0, nn, B, li, lj, g, hod);
-            else p2c_rows<false>(sm, staged, dem, order, c0, nn, B, li, lj, g, hod);
-        }
-        __syncthreads();
-        SLAB_PHASE_MARK(4);
-        // 5. the tile's partial window
-        float* P = sh.part + (size_t)w * PART_STRIDE;
-        for (int k = tid; k < PART_STRIDE; k += P2C_THREADS) P[k] = sm.nsum[k];
-        __syncthreads();
-        if (i + 1 < i1 && tid < DESC_WORDS) reinterpret_cast<int*>(&sm.d)[tid] = dn;
-        w_cur = w_nxt;
-        w_nxt = w_nn;
-        SLAB_PHASE_MARK(5);
-        SLAB_PHASE_TILE();
-    }
-    SLAB_PHASE_MARK(6);
-    __syncthreads();
-    if (tid == 0) {  // every copy was waited for; the memory may serve another purpose next
-        if constexpr (TMA) tma::mbar_inval(&sm.bar);
-        else tma::mbar_inval(&sm.dem_bar);
-    }
-}
-
-template <bool TMA>
-__global__ void __launch_bounds__(P2C_THREADS, TMA ? P2C_TMA_MIN_BLOCKS : P2C_MIN_BLOCKS)
-    k_p2g_cell(Shared sh, int cls, const __grid_constant__ CUtensorMap dem_map) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    p2g_cell_body<TMA>(sh, cls, smem_raw, &dem_map);
-}
-
-// ----------------------------------------------------- P2G of sparse tiles
-
-// K2 for tiles with at most split_min particles (src/simulation.cpp:726-798).
-// Such a tile's time is load latency, not arithmetic, so the kernel:
-//  - keeps the scenario's buffer pointers across consecutive tiles of one
-//    scenario, and requests the next tile's descriptor while this one runs;
-//  - requests the terrain window and the first candidate of every thread in
-//    one round;
-//  - pass A: per particle quantities into shared memory, cell counts and the
-//    per-quantity bounds of one contribution (as k_p2g);
-//  - pass B: one (particle, stencil row) item per thread, three nodes each,
-//    added as the hi/lo 32-bit fixed-point pairs of k_p2g<ACC_HILO> with
-//    native shared-memory integer atomics. The integer sums are exact, so
-//    the result does not depend on arrival order.
-constexpr int P2S_THREADS = NCELL;
-constexpr int P2S_MIN_BLOCKS = NCELL == 64 ? 16 : 4;
 constexpr int P2S_CAP = NCELL;  // particles of a sparse tile (split_min is capped to it)
-constexpr int P2S_DEMW = (TILE + 1) * (TILE + 1);
-constexpr int P2S_DEM_PER = (P2S_DEMW + P2S_THREADS - 1) / P2S_THREADS;
-static_assert(DESC_WORDS <= P2S_THREADS, "one descriptor word per thread");
 
-struct P2SSmem {
-    int hi[NQ * TN * TN];  // fixed-point sums of the (TILE+2)^2 window, [q][node]: rounded part
-    int lo[NQ * TN * TN];  //                                                      2^-20 finer rest
-    float4 dem[P2S_DEMW];
-    PQ pq[P2S_CAP];
-    int ccnt[NCELL];
-    unsigned bmax[NQ];
-    int mcc, nv;
-    float scale[NQ], iscale[NQ];
-    TileDesc d;
+struct P2GTileSmem {
+    union {
+        struct {                // dense: a pass's particles in sorted, swizzled places
+            float4 a[P2C_CAP];  // f.x, f.y, m vx, m vy
+            float4 b[P2C_CAP];  // m, m h, -K gx, -K gy
+            float k[P2C_CAP];   // K h / (2 dx); then, on output steps, m vz
+        } st;
+        struct {                         // dense: row sums [row * 3 + b][cell]
+            float4 q4[NSLOT * NCELL];    // m, m h, m vx, m vy
+            float2 q2[NSLOT * NCELL];    // F; then, on output steps, m vz
+        } cs;
+        struct {                   // sparse
+            int hi[NQ * NWIN];     // fixed-point sums of the window, [q][node]: rounded part
+            int lo[NQ * NWIN];     //                                         finer rest
+            PQ pq[P2S_CAP];
+            int ccnt[NCELL];
+            unsigned bmax[NQ];
+            int mcc, nv;
+        } sp;
+    };
+    alignas(128) float4 dem[(TILE + 1) * (TILE + 1)];  // a tensor copy's destination: 128-byte aligned
+    float4 ra[P2C_CAP], rb[P2C_CAP];                   // candidates as they lie in the particle buffer
+    alignas(8) uint64_t dem_bar;                       // completion of the terrain window's copy
+    uint32_t cnt[P2C_CHUNKS][P2C_HALVES];              // cell counts of a chunk, two 16-bit halves per word
+    uint16_t cbeg[NCELL + 2];                          // first sorted place of each cell; [NCELL]: the pass's particles
+    TileDesc d[2];                                     // this tile and the next
+    ScnSm z;
 };
 
-__device__ __forceinline__ PQ make_pq(float2 f, float2 v, float m, float h, float vz, int li, int lj, const float4* dem, float g, float hod) {
-    PQ p;
-    const float4 dm = dem[(li + (f.x >= 1.f ? 1 : 0)) * (TILE + 1) + (lj + (f.y >= 1.f ? 1 : 0))];
-    const float K = m * g * dm.z * dm.z;
-    p.fx = f.x;
-    p.fy = f.y;
-    p.m = m;
-    p.mvx = m * v.x;
-    p.mvy = m * v.y;
-    p.mh = m * h;
-    p.mvz = m * vz;
-    p.Kgx = K * dm.x;
-    p.Kgy = K * dm.y;
-    p.Khh = K * h * hod;
-    p.li = li;
-    p.lj = lj;
-    return p;
+__device__ __forceinline__ int p2c_place(int p) { return p ^ ((p >> 3) & 7); }
+
+// node coordinates of a tile's first cell
+struct TileOrigin {
+    int i, j;
+};
+
+// Requests tile D's first candidates and terrain window. Thread t copies the
+// candidates t, t + P2G_T, ... and is their only reader, so it may call this
+// as soon as it has read the ones before; the terrain window is thread 0's,
+// after a barrier that follows its last reads.
+__device__ __forceinline__ void p2g_request(P2GTileSmem& sm, const Shared& sh, const TileDesc& D, const CUtensorMap* dem_map) {
+    const PBuf B = sm.z.cur();
+    const int nc = min(D.rpref[9], P2C_CAP);
+    for (int k = threadIdx.x; k < nc; k += P2G_T) {
+        int r;
+        const int src = cand_index(k, D, r);
+        cpa::copy16(&sm.ra[k], B.a + src);
+        cpa::copy16(&sm.rb[k], B.b + src);
+    }
+    if (threadIdx.x == 0) {
+        // one 2-D tensor copy (TMA) of 9 x 9 nodes. The map sees the terrain as
+        // [Nx][4 Ny] floats, so x = 4 tj TILE (a multiple of 16 bytes). Nodes
+        // past the terrain's far edges read as zero; no valid particle uses
+        // them (its stencil lies inside the terrain).
+        tma::fence_proxy_async();
+        tma::mbar_arrive_expect_tx(&sm.dem_bar, (TILE + 1) * (TILE + 1) * 16);
+        tma::tensor_g2s_2d(sm.dem, dem_map, 4 * (D.t % sh.TY) * TILE, (D.t / sh.TY) * TILE, &sm.dem_bar);
+    }
 }
 
-__device__ __forceinline__ void p2g_sparse_body(const Shared& sh, int cls, unsigned char* smem_raw) {
-    P2SSmem& sm = *reinterpret_cast<P2SSmem*>(smem_raw);
-    const int tid = threadIdx.x, lane = tid & 31;
-    int i0, i1;
-    work_range(p2g_count(sh, cls), i0, i1);
-    int w_cur = i0 < i1 ? p2g_item(sh, cls, i0) : 0;
-    int w_nxt = i0 + 1 < i1 ? p2g_item(sh, cls, i0 + 1) : 0;
-    if (i0 < i1) load_desc(sh.desc + w_cur, &sm.d);
-    int csid = -1;
-    PBuf B{};
-    Ctl* ctl = nullptr;
-    bool outs = false;
-    float g = 0.f, hod = 0.f;
-    for (int i = i0; i < i1; ++i) {
-        const int w = w_cur;
-        for (int k = tid; k < NQ * TN * TN; k += P2S_THREADS) {
-            sm.hi[k] = 0;
-            sm.lo[k] = 0;
-        }
-        for (int k = tid; k < NCELL; k += P2S_THREADS) sm.ccnt[k] = 0;
-        if (tid < NQ) sm.bmax[tid] = 0u;
-        if (tid == 0) {
-            sm.mcc = 0;
-            sm.nv = 0;
-        }
-        __syncthreads();
-        // the next tile's descriptor and the item after it, stored at the end
-        int dn = 0, w_nn = 0;
-        if (i + 1 < i1 && tid < DESC_WORDS) dn = reinterpret_cast<const int*>(sh.desc + w_nxt)[tid];
-        if (i + 2 < i1) w_nn = p2g_item(sh, cls, i + 2);
-        if (sm.d.sid != csid) {  // uniform: a new scenario in this CTA's run
-            csid = sm.d.sid;
-            const Scn& S = sh.scn[csid];
-            const SDyn& n = sh.dyn[csid];
-            const PBuf b0 = S.buf[0], b1 = S.buf[1];  // loaded beside seq
-            B = (n.seq & 1) ? b1 : b0;
-            outs = n.outs != 0;
-            g = S.g;
-            hod = 0.5f * S.ood;
-            ctl = S.ctl;
-        }
-        const int t = sm.d.t;
-        const int ti = t / sh.TY, tj = t % sh.TY;
-        const int ncand = sm.d.rpref[9];
-        // one round: the terrain window and each thread's first candidate
-        float4 dmr[P2S_DEM_PER];
+// The cells' sums into a partial window: thread (row, cell)'s row sums first,
+// then one thread per node.
+template <bool OUTS>
+__device__ __forceinline__ void p2g_cells_to_window(P2GTileSmem& sm, float* part, const float2 (&am)[3], const float2 (&av)[3],
+                                                    const float2 (&aF)[3], const float (&az)[3], int row, int cell) {
+    __syncthreads();  // the stage is no longer read
 #pragma unroll
-        for (int r = 0; r < P2S_DEM_PER; ++r) {
-            const int k = tid + r * P2S_THREADS;
-            const int ii = ti * TILE + k / (TILE + 1), jj = tj * TILE + k % (TILE + 1);
-            dmr[r] = (k < P2S_DEMW && ii < sh.Nx && jj < sh.Ny) ? sh.dem[(int64_t)ii * sh.Ny + jj] : make_float4(0.f, 0.f, 1.f, 0.f);
-        }
-        int d0 = 0;
-        int32_t cell0 = 0;
-        float2 f0 = make_float2(0.f, 0.f), v0 = make_float2(0.f, 0.f);
-        float m0 = 0.f, h0 = 0.f, vz0 = 0.f;
-        if (tid < ncand) {
-            const int src = cand_to_index(tid, sm.d, d0);
-            cell0 = B.cell[src];
-            f0 = B.f[src];
-            v0 = B.v[src];
-            m0 = B.m[src];
-            h0 = B.h[src];
-            if (outs) vz0 = B.vz[src];
-        }
+    for (int b = 0; b < 3; ++b) {
+        const int k = (row * 3 + b) * NCELL + cell;
+        sm.cs.q4[k] = make_float4(am[b].x, am[b].y, av[b].x, av[b].y);
+        sm.cs.q2[k] = aF[b];
+    }
+    __syncthreads();
+    const int n = threadIdx.x, i = n / TN, j = n % TN;
+    if (n < NWIN) {
+        float2 m = make_float2(0.f, 0.f), v = m, F = m;
 #pragma unroll
-        for (int r = 0; r < P2S_DEM_PER; ++r) {
-            const int k = tid + r * P2S_THREADS;
-            if (k < P2S_DEMW) sm.dem[k] = dmr[r];
-        }
-        __syncthreads();
-        // pass A: particle quantities, cell counts, bounds
-        float bm = 0.f, bvx = 0.f, bvy = 0.f, bh = 0.f, bvz = 0.f, bF = 0.f;
-        for (int k = tid; k < ncand; k += P2S_THREADS) {
-            int d = d0;
-            int32_t cell = cell0;
-            float2 f = f0, v = v0;
-            float m = m0, h = h0, vz = vz0;
-            if (k != tid) {
-                const int src = cand_to_index(k, sm.d, d);
-                cell = B.cell[src];
-                f = B.f[src];
-                v = B.v[src];
-                m = B.m[src];
-                h = B.h[src];
-                vz = outs ? B.vz[src] : 0.f;
-            }
-            const int li = cell_i(cell) - ti * TILE, lj = cell_j(cell) - tj * TILE;
-            if ((unsigned)li >= TILE || (unsigned)lj >= TILE) {
-                if (d == 4) atomicOr(&ctl->err, ERR_MOVE);  // a stayer outside its tile
-                continue;
-            }
-            const PQ p = make_pq(f, v, m, h, vz, li, lj, sm.dem, g, hod);
-            const int slot = atomicAdd(&sm.nv, 1);
-            if (slot < P2S_CAP) sm.pq[slot] = p;
-            else atomicOr(&ctl->err, ERR_CAPACITY);
-            const int c = atomicAdd(&sm.ccnt[li * TILE + lj], 1) + 1;
-            atomicMax(&sm.mcc, c);
-            bm = fmaxf(bm, p.m);
-            bvx = fmaxf(bvx, fabsf(p.mvx));
-            bvy = fmaxf(bvy, fabsf(p.mvy));
-            bh = fmaxf(bh, p.mh);
-            bvz = fmaxf(bvz, fabsf(p.mvz));
-            bF = fmaxf(bF, p.Khh + fmaxf(fabsf(p.Kgx), fabsf(p.Kgy)));
-        }
-        bm = warp_max(bm);
-        bvx = warp_max(bvx);
-        bvy = warp_max(bvy);
-        bh = warp_max(bh);
-        bvz = warp_max(bvz);
-        bF = warp_max(bF);
-        if (lane == 0) {
-            atomicMax(&sm.bmax[0], __float_as_uint(bm));
-            atomicMax(&sm.bmax[1], __float_as_uint(bvx));
-            atomicMax(&sm.bmax[2], __float_as_uint(bvy));
-            atomicMax(&sm.bmax[3], __float_as_uint(bh));
-            atomicMax(&sm.bmax[4], __float_as_uint(bF));
-            atomicMax(&sm.bmax[5], __float_as_uint(bF));
-            atomicMax(&sm.bmax[6], __float_as_uint(bvz));
-        }
-        __syncthreads();
-        if (tid < NQ) {
-            const float bound = 9.f * (float)sm.mcc * 0.75f * __uint_as_float(sm.bmax[tid]);
-            int e = 0;
-            if (bound > 0.f) {
-                int E;
-                frexpf(bound, &E);  // bound < 2^E
-                e = min(max(30 - E, -120), 120);
-            }
-            sm.scale[tid] = ldexpf(1.f, e);
-            sm.iscale[tid] = ldexpf(1.f, -e);
-        }
-        __syncthreads();
-        // pass B: (particle, stencil row) items
-        const int nv = min(sm.nv, P2S_CAP);
-        const int lob = lo_bits_for(9 * sm.mcc);  // lo sums of a node stay below 2^30 (20 bits for <= 64 particles)
-        const float lo_mul = ldexpf(1.f, lob);
-        const double lo_div = ldexp(1.0, -lob);
-        for (int it = tid; it < 3 * nv; it += P2S_THREADS) {
-            const int pi = it / 3, a = it - 3 * pi;
-            const PQ p = sm.pq[pi];
-            float wx[3], wy[3], dwx[3], dwy[3];
-            bspline3(p.fx, wx, dwx);
-            bspline3(p.fy, wy, dwy);
-            const float wxa = a == 0 ? wx[0] : (a == 1 ? wx[1] : wx[2]);
-            const float dwxa = a == 0 ? dwx[0] : (a == 1 ? dwx[1] : dwx[2]);
+        for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
-                const float wgt = wxa * wy[b];
-                if (wgt > 3e-3f) {  // the reference's weight cut-off (src/simulation.cpp:780)
-                    const int nd = (p.li + a) * TN + (p.lj + b);
-                    const float cq[NQ] = {p.m * wgt, p.mvx * wgt, p.mvy * wgt, p.mh * wgt, p.Khh * (dwxa * wy[b]) - p.Kgx * wgt,
-                                          p.Khh * (dwy[b] * wxa) - p.Kgy * wgt, p.mvz * wgt};
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q) {
-                        if (q == 6 && !outs) continue;
-                        const float x = cq[q] * sm.scale[q];
-                        const int h_ = __float2int_rn(x);
-                        atomicAdd(sm.hi + q * TN * TN + nd, h_);
-                        const int l_ = __float2int_rn((x - (float)h_) * lo_mul);
-                        if (l_) atomicAdd(sm.lo + q * TN * TN + nd, l_);
-                    }
+                const int ci = i - a, cj = j - b;
+                if ((unsigned)ci < TILE && (unsigned)cj < TILE) {
+                    const int k = (a * 3 + b) * NCELL + ci * TILE + cj;
+                    const float4 q = sm.cs.q4[k];
+                    m = f2add(m, make_float2(q.x, q.y));
+                    v = f2add(v, make_float2(q.z, q.w));
+                    F = f2add(F, sm.cs.q2[k]);
                 }
             }
+        reinterpret_cast<float4*>(part)[n] = make_float4(m.x, m.y, v.x, v.y);
+        reinterpret_cast<float2*>(part + 4 * NWIN)[n] = F;
+    }
+    if (OUTS) {
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < 3; ++b) sm.cs.q2[(row * 3 + b) * NCELL + cell].x = az[b];
+        __syncthreads();
+        if (n < NWIN) {
+            float z = 0.f;
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const int ci = i - a, cj = j - b;
+                    if ((unsigned)ci < TILE && (unsigned)cj < TILE) z = __fadd_rn(z, sm.cs.q2[(a * 3 + b) * NCELL + ci * TILE + cj].x);
+                }
+            part[6 * NWIN + n] = z;
         }
-        __syncthreads();
-        float* P = sh.part + (size_t)w * PART_STRIDE;
-        for (int k = tid; k < PART_STRIDE; k += P2S_THREADS)
-            P[k] = (float)(((double)sm.hi[k] + (double)sm.lo[k] * lo_div) * (double)sm.iscale[k / (TN * TN)]);
-        __syncthreads();
-        if (i + 1 < i1 && tid < DESC_WORDS) reinterpret_cast<int*>(&sm.d)[tid] = dn;
-        w_cur = w_nxt;
-        w_nxt = w_nn;
     }
 }
 
-__global__ void __launch_bounds__(P2S_THREADS, P2S_MIN_BLOCKS) k_p2g_sparse(Shared sh, int cls) {
+// Weights of one particle offset along y for the 3 nodes of a row, both
+// halves the same, and the row's along x: w = fma(sg, (hc t) t, w0), dw = dc t,
+// t = f - s, the operations of bspline3 (for row 0 with the sign of both
+// factors turned).
+struct RowSpline {
+    float s, hc, sg, w0, dc;
+    __device__ __forceinline__ explicit RowSpline(int row)
+        : s(row == 0 ? 1.5f : (row == 1 ? 1.0f : 0.5f)), hc(row == 1 ? 1.0f : 0.5f), sg(row == 1 ? -1.0f : 1.0f),
+          w0(row == 1 ? 0.75f : 0.0f), dc(row == 1 ? -2.0f : 1.0f) {}
+    __device__ __forceinline__ void x(float f, float& w, float& dw) const {
+        const float t = __fsub_rn(f, s);
+        w = __fmaf_rn(sg, __fmul_rn(__fmul_rn(hc, t), t), w0);
+        dw = __fmul_rn(dc, t);
+    }
+};
+__device__ __forceinline__ void spline_y(float f, float2 (&w)[3], float (&dw)[3]) {
+    const float2 fy = make_float2(f, f);
+    const float2 t0 = f2add(fy, make_float2(-1.5f, -1.5f)), t1 = f2add(fy, make_float2(-1.f, -1.f)), t2 = f2add(fy, make_float2(-0.5f, -0.5f));
+    const float2 hf = make_float2(0.5f, 0.5f);
+    w[0] = f2mul(f2mul(hf, t0), t0);
+    w[1] = f2fma(f2mul(t1, t1), make_float2(-1.f, -1.f), make_float2(0.75f, 0.75f));
+    w[2] = f2mul(f2mul(hf, t2), t2);
+    dw[0] = t0.x;
+    dw[1] = __fmul_rn(-2.0f, t1.x);
+    dw[2] = t2.x;
+}
+
+template <bool OUTS, typename Next>
+__device__ __forceinline__ void p2g_dense_tile(P2GTileSmem& sm, const TileDesc& D, float* part, uint32_t dem_phase, TileOrigin o,
+                                               Next request_next) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cell = tid % NCELL, row = tid / NCELL;  // row is the same in a whole warp
+    Ctl* const ctl = sm.z.s.ctl;
+    const int ncand = D.rpref[9];
+    uint16_t* const cnt = reinterpret_cast<uint16_t*>(&sm.cnt[0][0]);  // zero here
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 am[3] = {zero, zero, zero}, av[3] = {zero, zero, zero}, aF[3] = {zero, zero, zero};
+    float az[3] = {0.f, 0.f, 0.f};
+    int placed = 0;
+    SLAB_PHASE_BEGIN;
+    int base = 0;
+    do {
+        const int nc = min(P2C_CAP, ncand - base);
+        if (base) {  // a later pass of a very dense tile: its candidates were not requested ahead
+            const PBuf B = sm.z.cur();
+            for (int k = tid; k < nc; k += P2G_T) {
+                int r;
+                const int src = cand_index(base + k, D, r);
+                cpa::copy16(&sm.ra[k], B.a + src);
+                cpa::copy16(&sm.rb[k], B.b + src);
+            }
+            cpa::wait_all();
+            __syncthreads();  // the sums of the pass before are done with its places and ranges
+        }
+        SLAB_PHASE_MARK(0);
+        // 1. count: this thread's candidates as local cell | rank << 16, -1: not in the tile
+        int at[P2C_PER];
+#pragma unroll
+        for (int u = 0; u < P2C_PER; ++u) at[u] = -1;
+#pragma unroll
+        for (int u = 0; u < P2C_PER; ++u) {
+            const int k = tid + u * P2G_T;
+            if (k - lane >= nc) break;  // no candidate in the warp
+            if (k < nc) {
+                const int32_t c = __float_as_int(sm.rb[k].z);
+                const int ci = cell_i(c) - o.i, cj = cell_j(c) - o.j;
+                if ((unsigned)ci < TILE && (unsigned)cj < TILE) at[u] = ci * TILE + cj;
+                else if (base + k >= D.rpref[4] && base + k < D.rpref[5]) atomicOr(&ctl->err, ERR_MOVE);  // a stayer outside its tile
+            }
+            const unsigned vm = __ballot_sync(0xffffffffu, at[u] >= 0);
+            if (at[u] >= 0) {
+                const unsigned peers = __match_any_sync(vm, at[u]);
+                const int rank = __popc(peers & ((1u << lane) - 1u));
+                if (rank == 0) cnt[(warp + u * (P2G_T / 32)) * NCELL + at[u]] = (uint16_t)__popc(peers);
+                at[u] |= rank << 16;
+            }
+        }
+        __syncthreads();
+        SLAB_PHASE_MARK(1);
+        // 2. exclusive prefix over the chunks of every cell, then over the cells
+        if (warp == 0) {
+            constexpr int WPL = P2C_HALVES / 32;  // count words per lane
+            uint32_t sum[WPL];
+#pragma unroll
+            for (int q = 0; q < WPL; ++q) sum[q] = 0;
+#pragma unroll
+            for (int c = 0; c < P2C_CHUNKS; ++c)
+#pragma unroll
+                for (int q = 0; q < WPL; ++q) {
+                    const uint32_t x = sm.cnt[c][lane * WPL + q];
+                    sm.cnt[c][lane * WPL + q] = sum[q];
+                    sum[q] += x;  // halves stay below 2^16
+                }
+            int tot = 0;
+#pragma unroll
+            for (int q = 0; q < WPL; ++q) tot += (int)(sum[q] & 0xffffu) + (int)(sum[q] >> 16);
+            int e = tot;
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, e, s);
+                if (lane >= s) e += y;
+            }
+            if (lane == 31) sm.cbeg[NCELL] = (uint16_t)e;
+            e -= tot;
+#pragma unroll
+            for (int q = 0; q < WPL; ++q) {
+                sm.cbeg[2 * (lane * WPL + q)] = (uint16_t)e;
+                e += (int)(sum[q] & 0xffffu);
+                sm.cbeg[2 * (lane * WPL + q) + 1] = (uint16_t)e;
+                e += (int)(sum[q] >> 16);
+            }
+        }
+        if (base == 0 && !tma::mbar_wait(&sm.dem_bar, dem_phase)) atomicOr(&ctl->err, ERR_TIMEOUT);  // the terrain window
+        __syncthreads();
+        SLAB_PHASE_MARK(2);
+        // 3. quantities of every particle to its sorted place
+        const float g = sm.z.s.g, hod = 0.5f * sm.z.s.ood;
+#pragma unroll
+        for (int u = 0; u < P2C_PER; ++u) {
+            if (at[u] >= 0) {
+                const int k = tid + u * P2G_T, lc = at[u] & 0xffff;
+                const int p = p2c_place((int)sm.cbeg[lc] + (int)cnt[(warp + u * (P2G_T / 32)) * NCELL + lc] + (at[u] >> 16));
+                const float4 qa = sm.ra[k], qb = sm.rb[k];
+                const float4 qd = sm.dem[(lc / TILE + (qa.x >= 1.f ? 1 : 0)) * (TILE + 1) + (lc % TILE + (qa.y >= 1.f ? 1 : 0))];
+                const float h = qb.x, m = qb.y;
+                const float K = m * g * qd.z * qd.z;
+                sm.st.a[p] = make_float4(qa.x, qa.y, m * qa.z, m * qa.w);
+                sm.st.b[p] = make_float4(m, m * h, -(K * qd.x), -(K * qd.y));
+                sm.st.k[p] = K * h * hod;
+                at[u] = p;
+            }
+        }
+        placed += sm.cbeg[NCELL];
+        __syncthreads();
+        SLAB_PHASE_MARK(3);
+        for (int k = tid; k < P2C_CHUNKS * P2C_HALVES; k += P2G_T) (&sm.cnt[0][0])[k] = 0;  // for the next pass or tile
+        if (base + P2C_CAP >= ncand) request_next();
+        // 4. the cell's particles over the row's 3 nodes
+        const RowSpline rs(row);
+        const int r0 = sm.cbeg[cell], r1 = sm.cbeg[cell + 1];
+        for (int r = r0; r < r1; ++r) {
+            const int p = p2c_place(r);
+            const float4 a = sm.st.a[p], b = sm.st.b[p];
+            const float kh = sm.st.k[p];
+            float wx, dwx, dwy[3];
+            float2 wy[3];
+            rs.x(a.x, wx, dwx);
+            spline_y(a.y, wy, dwy);
+            const float2 wx2 = make_float2(wx, wx), kh2 = make_float2(kh, kh);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float2 w = f2mul(wx2, wy[k]);
+                if (w.x > 3e-3f) {  // the reference's weight cut-off (src/simulation.cpp:780)
+                    am[k] = f2fma(make_float2(b.x, b.y), w, am[k]);
+                    av[k] = f2fma(make_float2(a.z, a.w), w, av[k]);
+                    const float2 gr = make_float2(__fmul_rn(dwx, wy[k].x), __fmul_rn(dwy[k], wx));
+                    aF[k] = f2add(aF[k], f2fma(kh2, gr, f2mul(make_float2(b.z, b.w), w)));
+                }
+            }
+        }
+        if (OUTS) {  // m vz by a second walk, in the place of the force factor
+            __syncthreads();
+            const float* const gvz = sm.z.cur().vz;
+            const float4* const gb = sm.z.cur().b;
+#pragma unroll
+            for (int u = 0; u < P2C_PER; ++u)
+                if (at[u] >= 0) {
+                    int d;
+                    const int src = cand_index(base + tid + u * P2G_T, D, d);
+                    sm.st.k[at[u]] = gb[src].y * gvz[src];
+                }
+            __syncthreads();
+            for (int r = r0; r < r1; ++r) {
+                const int p = p2c_place(r);
+                const float4 a = sm.st.a[p];
+                const float mz = sm.st.k[p];
+                float wx, dwx, dwy[3];
+                float2 wy[3];
+                rs.x(a.x, wx, dwx);
+                spline_y(a.y, wy, dwy);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float w = __fmul_rn(wx, wy[k].x);
+                    if (w > 3e-3f) az[k] = __fmaf_rn(mz, w, az[k]);
+                }
+            }
+        }
+        base += P2C_CAP;
+        SLAB_PHASE_MARK(4);
+    } while (base < ncand);
+    if (tid == 0 && placed != D.total) atomicOr(&ctl->err, ERR_CAPACITY);
+    p2g_cells_to_window<OUTS>(sm, part, am, av, aF, az, row, cell);
+    SLAB_PHASE_MARK(5);
+    SLAB_PHASE_TILE();
+}
+
+// A tile with at most split_min particles. Its time is latency, not
+// arithmetic: pass A puts each particle's quantities in shared memory with the
+// bound of one contribution per quantity (as k_p2g); pass B gives each thread
+// one (particle, stencil row) item, three nodes each, added as the hi/lo
+// 32-bit fixed-point pairs of k_p2g<ACC_HILO> with native shared-memory
+// integer atomics. The integer sums are exact, so the result does not depend
+// on arrival order.
+template <typename Next>
+__device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc& D, float* part, uint32_t dem_phase, TileOrigin o,
+                                                Next request_next) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    auto& sp = sm.sp;
+    SLAB_PHASE_BEGIN;
+    const PBuf B = sm.z.cur();
+    Ctl* const ctl = sm.z.s.ctl;
+    const bool outs = sm.z.y.outs != 0;
+    const float g = sm.z.s.g, hod = 0.5f * sm.z.s.ood;
+    const int ncand = D.rpref[9];
+    float bm = 0.f, bvx = 0.f, bvy = 0.f, bh = 0.f, bvz = 0.f, bF = 0.f;
+    for (int k = tid; k < 2 * NQ * NWIN / 4; k += P2G_T) reinterpret_cast<int4*>(sp.hi)[k] = make_int4(0, 0, 0, 0);  // hi and lo
+    for (int k = tid; k < NCELL; k += P2G_T) sp.ccnt[k] = 0;
+    if (tid < NQ) sp.bmax[tid] = 0u;
+    if (tid == 0) {
+        sp.mcc = 0;
+        sp.nv = 0;
+    }
+    if (!tma::mbar_wait(&sm.dem_bar, dem_phase)) atomicOr(&ctl->err, ERR_TIMEOUT);
+    __syncthreads();  // (the window of the tile before was read before the barrier of that tile's caller)
+    // pass A: particle quantities, cell counts, bounds
+    for (int k = tid; k < ncand; k += P2G_T) {
+        int d;
+        const int src = cand_index(k, D, d);
+        const float4 a = k < P2C_CAP ? sm.ra[k] : B.a[src], b = k < P2C_CAP ? sm.rb[k] : B.b[src];
+        const float vz = outs ? B.vz[src] : 0.f;
+        const int32_t cell = __float_as_int(b.z);
+        const int li = cell_i(cell) - o.i, lj = cell_j(cell) - o.j;
+        if ((unsigned)li >= TILE || (unsigned)lj >= TILE) {
+            if (d == 4) atomicOr(&ctl->err, ERR_MOVE);  // a stayer outside its tile
+            continue;
+        }
+        const PQ p = make_pq(a, b, vz, li, lj, sm.dem, g, hod);
+        const int slot = atomicAdd(&sp.nv, 1);
+        if (slot < P2S_CAP) sp.pq[slot] = p;
+        else atomicOr(&ctl->err, ERR_CAPACITY);
+        const int c = atomicAdd(&sp.ccnt[li * TILE + lj], 1) + 1;
+        atomicMax(&sp.mcc, c);
+        bm = fmaxf(bm, p.m);
+        bvx = fmaxf(bvx, fabsf(p.mvx));
+        bvy = fmaxf(bvy, fabsf(p.mvy));
+        bh = fmaxf(bh, p.mh);
+        bvz = fmaxf(bvz, fabsf(p.mvz));
+        bF = fmaxf(bF, p.Khh + fmaxf(fabsf(p.Kgx), fabsf(p.Kgy)));
+    }
+    if ((tid & ~31) < ncand) {  // warps that hold a candidate; bounds are >= 0, so their bits order like the values
+        const unsigned v[6] = {__float_as_uint(bm), __float_as_uint(bvx), __float_as_uint(bvy),
+                               __float_as_uint(bh), __float_as_uint(bF), __float_as_uint(bvz)};
+        unsigned r[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) r[q] = __reduce_max_sync(0xffffffffu, v[q]);
+        if (lane == 0) {
+#pragma unroll
+            for (int q = 0; q < 5; ++q) atomicMax(&sp.bmax[q], r[q]);
+            atomicMax(&sp.bmax[5], r[4]);
+            atomicMax(&sp.bmax[6], r[5]);
+        }
+    }
+    __syncthreads();
+    SLAB_PHASE_MARK(6);
+    request_next();  // candidates and terrain window have been read
+    // scales 2^e of the sums from the exponents of their bounds (bound < 2^E,
+    // e = 30 - E, |e| <= 120), in every thread: integer operations instead of
+    // frexp / ldexp by 7 threads between two barriers
+    const int mcc = sp.mcc;
+    int ex[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const float bound = 9.f * (float)mcc * 0.75f * __uint_as_float(sp.bmax[q]);
+        const int E = (int)(__float_as_uint(bound) >> 23) - 126;
+        ex[q] = bound > 0.f ? min(max(30 - E, -120), 120) : 0;
+    }
+    // pass B: (particle, stencil row) items. The atomics are unconditional: a
+    // branch around an addition of zero kept the six sums' conversions from
+    // overlapping (3100 cycles for the pass in an idle SM).
+    const int nv = min(sp.nv, P2S_CAP);
+    const int nmax = 9 * mcc, c2 = nmax <= 1 ? 0 : 32 - __clz(nmax - 1);
+    const int lob = min(20, 31 - c2);  // lo_bits_for(nmax): lo sums of a node stay below 2^30 (20 bits for <= 64 particles)
+    const float lo_mul = __int_as_float((127 + lob) << 23);
+    for (int it = tid; it < 3 * nv; it += P2G_T) {
+        const int pi = it / 3, a = it - 3 * pi;
+        const PQ p = sp.pq[pi];
+        float wx[3], wy[3], dwx[3], dwy[3];
+        bspline3(p.fx, wx, dwx);
+        bspline3(p.fy, wy, dwy);
+        const float wxa = a == 0 ? wx[0] : (a == 1 ? wx[1] : wx[2]);
+        const float dwxa = a == 0 ? dwx[0] : (a == 1 ? dwx[1] : dwx[2]);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const float wgt = wxa * wy[b];
+            if (wgt > 3e-3f) {  // the reference's weight cut-off (src/simulation.cpp:780)
+                const int nd = (p.li + a) * TN + (p.lj + b);
+                const float cq[NQ] = {p.m * wgt, p.mvx * wgt, p.mvy * wgt, p.mh * wgt, p.Khh * (dwxa * wy[b]) - p.Kgx * wgt,
+                                      p.Khh * (dwy[b] * wxa) - p.Kgy * wgt, p.mvz * wgt};
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    if (q == 6 && !outs) continue;
+                    const float x = cq[q] * __int_as_float((127 + ex[q]) << 23);
+                    const int h_ = __float2int_rn(x);
+                    atomicAdd(sp.hi + q * NWIN + nd, h_);
+                    atomicAdd(sp.lo + q * NWIN + nd, __float2int_rn((x - (float)h_) * lo_mul));
+                }
+            }
+        }
+    }
+    __syncthreads();
+    SLAB_PHASE_MARK(12);
+    // the window, one node per thread
+    const double lo_div = __hiloint2double((1023 - lob) << 20, 0);
+    for (int n = tid; n < NWIN; n += P2G_T) {
+        float v[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+            v[q] = q < 6 || outs ? (float)(((double)sp.hi[q * NWIN + n] + (double)sp.lo[q * NWIN + n] * lo_div) *
+                                           (double)__int_as_float((127 - ex[q]) << 23))
+                                 : 0.f;
+        reinterpret_cast<float4*>(part)[n] = make_float4(v[0], v[3], v[1], v[2]);
+        reinterpret_cast<float2*>(part + 4 * NWIN)[n] = make_float2(v[4], v[5]);
+        if (outs) part[6 * NWIN + n] = v[6];
+    }
+    SLAB_PHASE_MARK(13);
+}
+
+// The active tiles of the step. Latency: the first
+// descriptor is read beside the work count (the guess blockIdx.x is right for
+// one scenario); a tile's candidates are requested while the tile
+// before it is summed, its descriptor one tile earlier; the scenario's values
+// stay in shared memory across a run of its tiles.
+__device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* smem_raw, const CUtensorMap* dem_map) {
+    P2GTileSmem& sm = *reinterpret_cast<P2GTileSmem*>(smem_raw);
+    const int tid = threadIdx.x;
+    int dn = 0;
+    const bool words = tid < DESC_WORDS;
+    if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
+    if (sh.nscn == 1) load_scn(sh, 0, sm.z, tid, P2G_T);
+    else if (tid == 0) sm.z.sid = -1;
+    const auto [w0, w1, step] = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
+    if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
+    for (int k = tid; k < P2C_CHUNKS * P2C_HALVES; k += P2G_T) (&sm.cnt[0][0])[k] = 0;
+    if (tid == 0) {
+        tma::mbar_init(&sm.dem_bar, 1);
+        tma::fence_mbar_init();
+    }
+    if (words) reinterpret_cast<int*>(&sm.d[0])[tid] = dn;
+    if (words && w0 + step < w1) dn = reinterpret_cast<const int*>(sh.desc + w0 + step)[tid];
+    __syncthreads();
+    uint32_t dem_phase = 0;  // parity of the terrain window's next completion
+    bool requested = false;  // the tile's candidates and terrain window are on their way (uniform)
+    for (int w = w0, cur = 0; w < w1; w += step, cur ^= 1) {
+        const TileDesc& D = sm.d[cur];
+        const TileDesc& N = sm.d[cur ^ 1];
+        if (D.sid != sm.z.sid) {  // uniform: a new scenario in this CTA's run
+            __syncthreads();
+            load_scn(sh, D.sid, sm.z, tid, P2G_T);
+            __syncthreads();
+        }
+        if (!requested) p2g_request(sm, sh, D, dem_map);
+        // the next descriptor; later barriers of this tile show it to the other threads
+        const bool more = w + step < w1;
+        if (words && more) reinterpret_cast<int*>(&sm.d[cur ^ 1])[tid] = dn;
+        if (words && w + 2 * step < w1) dn = reinterpret_cast<const int*>(sh.desc + w + 2 * step)[tid];
+        requested = false;
+        auto request_next = [&] {
+            if (more && N.sid == sm.z.sid) {
+                p2g_request(sm, sh, N, dem_map);
+                requested = true;
+            }
+        };
+        cpa::wait_all();
+        float* part = sh.part + (size_t)w * PART_STRIDE;
+        const TileOrigin o{(D.t / sh.TY) * TILE, (D.t % sh.TY) * TILE};
+        if (D.total <= sh.split_min) {
+            __syncthreads();  // the sums share memory with the row sums of the tile before
+            p2g_sparse_tile(sm, D, part, dem_phase, o, request_next);
+        } else if (sm.z.y.outs) {
+            p2g_dense_tile<true>(sm, D, part, dem_phase, o, request_next);
+        } else {
+            p2g_dense_tile<false>(sm, D, part, dem_phase, o, request_next);
+        }
+        dem_phase ^= 1u;
+    }
+    __syncthreads();
+    if (tid == 0) tma::mbar_inval(&sm.dem_bar);  // every copy was waited for; the memory may serve another purpose next
+}
+
+__global__ void __launch_bounds__(P2G_T, SLAB_P2G_MIN_BLOCKS) k_p2g_tiles(Shared sh, const __grid_constant__ CUtensorMap dem_map) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    p2g_sparse_body(sh, cls, smem_raw);
+    p2g_tiles_body(sh, smem_raw, &dem_map);
 }
 
 // ------------------------------------------------------------ grid update
@@ -1738,84 +1464,71 @@ __global__ void __launch_bounds__(P2S_THREADS, P2S_MIN_BLOCKS) k_p2g_sparse(Shar
 // nodes owned by one grid tile. A node's P2G sum is the partials of the
 // tiles whose window covers it, added in a fixed order (own, -x, -y, -xy).
 // h_max / v_max2 are updated in the node block; the FP64 grid mass sum and
-// the active-node count are diagnostics: every CTA adds them up over its run
-// of grid tiles and touches their two addresses once per run and scenario.
-// (Two atomics per grid tile on the same two addresses held the kernel up.)
-// Latency: the scenario's values stay in shared memory across a run of its
-// grid tiles, and thread 0 reads the grid-tile list two entries ahead.
+// the active-node count are diagnostics, added up over a warp's run of grid
+// tiles of one scenario.
+// One warp per grid tile and no block barriers: the kernel is two dependent
+// rounds of loads (the covering tiles' slots and the node block, then partials,
+// terrain and maxima), so what counts is how many grid tiles an SM has in
+// flight. The slots and block of the next grid tile are requested while one is
+// computed, and a window node is one 16-byte and one 8-byte load.
+constexpr int GRID_T = 128;
+constexpr int GRID_MAX_WARPS = 3 * NCELL / 32 > GRID_T / 32 ? 3 * NCELL / 32 : GRID_T / 32;  // the persistent kernel's CTAs run it too
+
 __device__ __forceinline__ void grid_body(const Shared& sh) {
-    __shared__ int s_gt, s_blk, s_sid;
-    __shared__ int s_slot[4];
-    __shared__ double s_red[NCELL / 32];
-    __shared__ unsigned s_act[NCELL / 32];
-    __shared__ ScnSm zs;
+    __shared__ ScnSm s_scn[GRID_MAX_WARPS];
+    constexpr int NPL = NCELL / 32;  // nodes per lane
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    ScnSm& zs = s_scn[warp];
     const Scn& Z = zs.s;
     const SDyn& Y = zs.y;
-    const int tid = threadIdx.x;
-    const int li = tid / TILE, lj = tid % TILE;
-    int w0, w1;
-    work_range(min(*sh.gcount, sh.gcap), w0, w1);
-    // thread 0: the current and the next entry of the flat grid-tile list
-    int2 e_cur = make_int2(-1, 0), e_nxt = make_int2(-1, 0);
-    if (tid == 0) {
-        if (w0 < w1) e_cur = reinterpret_cast<const int2*>(sh.gflat)[w0];
-        if (w0 + 1 < w1) e_nxt = reinterpret_cast<const int2*>(sh.gflat)[w0 + 1];
-    }
-    // mass and active nodes of this thread over the CTA's run of one scenario
+    const int nwork = min(*sh.gcount, sh.gcap);
+    const int gw = (int)blockIdx.x * nwarp + warp, gn = (int)gridDim.x * nwarp;
+    const auto [w0, w1, step] = work_items(sh, nwork, gw, gn);
+    if (w0 >= w1) return;  // warps run alone: no block barrier below
+    const int2* const list = reinterpret_cast<const int2*>(sh.gflat);
     int csid = -1;
-    double macc = 0.0;
+    double macc = 0.0;  // mass and active nodes of this lane over the run of one scenario
     unsigned nacc = 0;
     auto flush = [&] {
         nacc = __reduce_add_sync(0xffffffffu, nacc);
         for (int o = 16; o > 0; o >>= 1) macc += __shfl_xor_sync(0xffffffffu, macc, o);
-        if ((tid & 31) == 0) {
-            s_red[tid >> 5] = macc;
-            s_act[tid >> 5] = nacc;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double sum = 0.0;
-            unsigned na = 0;
-            for (int k = 0; k < NCELL / 32; ++k) {
-                sum += s_red[k];
-                na += s_act[k];
-            }
-            if (sum != 0.0) atomicAdd(&Z.cnt->grid_mass, sum);
-            if (na) atomicAdd(&Z.ctl->node_steps, (unsigned long long)na);
+        if (lane == 0) {
+            if (macc != 0.0) atomicAdd(&Z.cnt->grid_mass, macc);
+            if (nacc) atomicAdd(&Z.ctl->node_steps, (unsigned long long)nacc);
         }
         macc = 0.0;
         nacc = 0;
     };
-    for (int w = w0; w < w1; ++w) {
-        if (tid == 0) {
-            s_sid = e_cur.x;
-            s_gt = e_cur.y;
-            e_cur = e_nxt;
-            if (w + 2 < w1) e_nxt = reinterpret_cast<const int2*>(sh.gflat)[w + 2];
-        }
-        __syncthreads();
-        if (s_sid != csid) {  // uniform: a new scenario in this CTA's run
-            if (csid >= 0) flush();
-            csid = s_sid;
-            __syncthreads();
-            load_scn(sh, csid, zs, tid, NCELL);
-            __syncthreads();
-        }
-        Ctl* c = Z.ctl;
-        const int gt = s_gt;
-        const int gi = gt / sh.TY, gj = gt % sh.TY;
-        if (tid < 4) {
-            // contributor k: tile (gi - (k>>1), gj - (k&1)); slot if active this step
-            const int ti_ = gi - (tid >> 1), tj_ = gj - (tid & 1);
-            int slot = -1;
+    // lanes 0-3: slot of covering tile k (gi - (k >> 1), gj - (k & 1)), -1 if it is
+    // not active this step; lane 4: the node block
+    int st_ = -1, sl_ = -1;
+    auto request = [&](int gt) {
+        st_ = -1;
+        sl_ = -1;
+        if (lane < 4) {
+            const int ti_ = gt / sh.TY - (lane >> 1), tj_ = gt % sh.TY - (lane & 1);
             if (ti_ >= 0 && tj_ >= 0) {
                 const int tt = ti_ * sh.TY + tj_;
-                const int st_ = Z.act_stamp[tt], sl = Z.slot_of[tt];  // both loads in flight together
-                if (st_ == Y.seq) slot = sl;
+                st_ = Z.act_stamp[tt];
+                sl_ = Z.slot_of[tt];
             }
-            s_slot[tid] = slot;
-        } else if (tid == 32) {
-            int blk = Z.blk_of[gt];
+        } else if (lane == 4) {
+            sl_ = Z.blk_of[gt];
+        }
+    };
+    int2 e = list[w0], e_nxt = w0 + step < w1 ? list[w0 + step] : make_int2(-1, 0);
+    for (int w = w0; w < w1; w += step) {
+        if (e.x != csid) {  // a new scenario in this warp's run
+            if (csid >= 0) flush();
+            csid = e.x;
+            __syncwarp();
+            load_scn(sh, csid, zs, lane, 32);
+            __syncwarp();
+            request(e.y);
+        }
+        const int gt = e.y, gi = gt / sh.TY, gj = gt % sh.TY;
+        if (lane == 4) {
+            int blk = sl_;
             if (blk < 0) {
                 // a block released by a retired scenario, else a fresh one
                 const int f = atomicSub(sh.free_count, 1);
@@ -1826,97 +1539,110 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
                     blk = atomicAdd(sh.blk_count, 1);
                 }
                 if (blk >= sh.blk_cap) {
-                    atomicOr(&c->err, ERR_CAPACITY);
+                    atomicOr(&Z.ctl->err, ERR_CAPACITY);
                     blk = -1;
                 } else {
                     Z.blk_of[gt] = blk;
-                    sh.blk_owner[blk] = zs.sid;
+                    sh.blk_owner[blk] = csid;
                 }
             }
             if (blk >= 0) sh.blk_stamp[blk] = Y.stepid;
-            s_blk = blk;
+            sl_ = blk;
         }
-        __syncthreads();
-        const int blk = s_blk;
+        const int slot = lane < 4 ? (st_ == Y.seq ? sl_ : -1) : sl_;
+        const int blk = __shfl_sync(0xffffffffu, slot, 4);
+        int slots[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) slots[k] = __shfl_sync(0xffffffffu, slot, k);
         // the block of this grid tile is entry k of contributor k's window (for G2P)
-        if (tid < 4 && s_slot[tid] >= 0) sh.desc[s_slot[tid]].blk4[tid] = blk;
+        if (lane < 4 && slot >= 0) sh.desc[slot].blk4[lane] = blk;
+        // the next grid tile's slots and block, and the list entry after it
+        const int2 e_nn = w + 2 * step < w1 ? list[w + 2 * step] : make_int2(-1, 0);
+        if (e_nxt.x == csid) request(e_nxt.y);
         if (blk >= 0) {
-            float q[NQ];
 #pragma unroll
-            for (int k = 0; k < NQ; ++k) q[k] = 0.f;
-            auto add = [&](int slot, int a, int b) {
-                if (slot < 0) return;
-                const float* P = sh.part + (size_t)slot * PART_STRIDE + a * TN + b;
-#pragma unroll
-                for (int k = 0; k < NQ; ++k) q[k] += P[k * TN * TN];
-            };
-            const int i = gi * TILE + li, j = gj * TILE + lj;
-            const size_t bn = (size_t)blk * NCELL + tid;
-            const bool inside = i < sh.Nx && j < sh.Ny;
-            // terrain and maxima are requested with the partials (one round of loads)
-            const float4 dm = inside ? sh.dem[(int64_t)i * sh.Ny + j] : make_float4(0.f, 0.f, 1.f, 0.f);
-            const float hmax0 = sh.hmax[bn], vmax0 = sh.vmax2[bn];
-            add(s_slot[0], li, lj);
-            if (li < 2) add(s_slot[2], li + TILE, lj);
-            if (lj < 2) add(s_slot[1], li, lj + TILE);
-            if (li < 2 && lj < 2) add(s_slot[3], li + TILE, lj + TILE);
-            float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
-            float hn = 0.f, vzn = 0.f;
-            const float mi = q[0];
-            if (mi > 1e-6f && inside) {
-                const float vox = q[1] / mi, voy = q[2] / mi;
-                vzn = q[6] / mi;
-                hn = q[3] / mi;
-                const float dt = Y.dt;
-                const float vtx = vox + dt * (q[4] / mi), vty = voy + dt * (q[5] / mi);
-                const float vsq = vtx * vtx + vty * vty;
-                float nvx = 0.f, nvy = 0.f;
-                if (vsq > 1e-16f) {
-                    const float ct = dm.z;
-                    const float vz = vtx * dm.x + vty * dm.y;
-                    const float v3sq = vsq + vz * vz;
-                    const float v3 = sqrtf(v3sq);
-                    const float g = Z.g;
-                    float af;
-                    if (Z.fric == SLAB_COULOMB) {
-                        af = Z.mu_c * g * ct;
-                    } else if (Z.fric == SLAB_VOELLMY) {
-                        af = Z.mu_v * g * ct + g * v3sq / (Z.xi * hn * ct);
-                    } else {
-                        const float I = 5.f * Z.d * v3 / (2.f * hn * ct * ct * sqrtf(g * hn * Z.phi));
-                        const float muI = Z.mu1 + (Z.mu2 - Z.mu1) / (1.f + Z.I0 / I);
-                        af = muI * g * ct;
+            for (int u = 0; u < NPL; ++u) {
+                const int c = lane + 32 * u, li = c / TILE, lj = c % TILE;
+                const int i = gi * TILE + li, j = gj * TILE + lj;
+                const size_t bn = (size_t)blk * NCELL + c;
+                const bool inside = i < sh.Nx && j < sh.Ny;
+                // terrain and maxima are requested with the partials (one round of loads)
+                const float4 dm = inside ? sh.dem[(int64_t)i * sh.Ny + j] : make_float4(0.f, 0.f, 1.f, 0.f);
+                const float hmax0 = sh.hmax[bn], vmax0 = sh.vmax2[bn];
+                float2 m2 = make_float2(0.f, 0.f), v2 = m2, F2 = m2;  // m, m h; m v; F
+                float qz = 0.f;
+                auto add = [&](int s, int a, int b) {
+                    if (s < 0) return;
+                    const float* P = sh.part + (size_t)s * PART_STRIDE;
+                    const int n = a * TN + b;
+                    const float4 q = reinterpret_cast<const float4*>(P)[n];
+                    const float2 F = reinterpret_cast<const float2*>(P + 4 * NWIN)[n];
+                    m2 = f2add(m2, make_float2(q.x, q.y));
+                    v2 = f2add(v2, make_float2(q.z, q.w));
+                    F2 = f2add(F2, F);
+                    if (Y.outs) qz += P[6 * NWIN + n];
+                };
+                add(slots[0], li, lj);
+                if (li < 2) add(slots[2], li + TILE, lj);
+                if (lj < 2) add(slots[1], li, lj + TILE);
+                if (li < 2 && lj < 2) add(slots[3], li + TILE, lj + TILE);
+                float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+                float hn = 0.f, vzn = 0.f;
+                const float mi = m2.x;
+                if (mi > 1e-6f && inside) {
+                    const float vox = v2.x / mi, voy = v2.y / mi;
+                    if (Y.outs) vzn = qz / mi;
+                    hn = m2.y / mi;
+                    const float dt = Y.dt;
+                    const float vtx = vox + dt * (F2.x / mi), vty = voy + dt * (F2.y / mi);
+                    const float vsq = vtx * vtx + vty * vty;
+                    float nvx = 0.f, nvy = 0.f;
+                    if (vsq > 1e-16f) {
+                        const float ct = dm.z;
+                        const float vz = vtx * dm.x + vty * dm.y;
+                        const float v3sq = vsq + vz * vz;
+                        const float v3 = sqrtf(v3sq);
+                        const float g = Z.g;
+                        float af;
+                        if (Z.fric == SLAB_COULOMB) {
+                            af = Z.mu_c * g * ct;
+                        } else if (Z.fric == SLAB_VOELLMY) {
+                            af = Z.mu_v * g * ct + g * v3sq / (Z.xi * hn * ct);
+                        } else {
+                            const float I = 5.f * Z.d * v3 / (2.f * hn * ct * ct * sqrtf(g * hn * Z.phi));
+                            const float muI = Z.mu1 + (Z.mu2 - Z.mu1) / (1.f + Z.I0 / I);
+                            af = muI * g * ct;
+                        }
+                        const float dv = dt * af;
+                        if (dv < v3) {
+                            const float fct = 1.f - dv / v3;
+                            nvx = vtx * fct;
+                            nvy = vty * fct;
+                        }
                     }
-                    const float dv = dt * af;
-                    if (dv < v3) {
-                        const float fct = 1.f - dv / v3;
-                        nvx = vtx * fct;
-                        nvy = vty * fct;
-                    }
+                    out = make_float4(nvx, nvy, nvx - vox, nvy - voy);
+                    sh.hmax[bn] = fmaxf(hmax0, hn);
+                    sh.vmax2[bn] = fmaxf(vmax0, nvx * nvx + nvy * nvy);
+                    macc += (double)mi;
+                    nacc += 1u;
                 }
-                out = make_float4(nvx, nvy, nvx - vox, nvy - voy);
-                sh.hmax[bn] = fmaxf(hmax0, hn);
-                sh.vmax2[bn] = fmaxf(vmax0, nvx * nvx + nvy * nvy);
-                macc += (double)mi;
-                nacc += 1u;
-            }
-            sh.nv[bn] = out;
-            if (Y.outs) {
-                sh.oh[bn] = hn;
-                sh.om[bn] = inside ? mi : 0.f;
-                sh.ovz[bn] = vzn;
-                sh.oFx[bn] = inside ? q[4] : 0.f;
-                sh.oFy[bn] = inside ? q[5] : 0.f;
+                sh.nv[bn] = out;
+                if (Y.outs) {
+                    sh.oh[bn] = hn;
+                    sh.om[bn] = inside ? mi : 0.f;
+                    sh.ovz[bn] = vzn;
+                    sh.oFx[bn] = inside ? F2.x : 0.f;
+                    sh.oFy[bn] = inside ? F2.y : 0.f;
+                }
             }
         }
-        // (the shared values of this item are rewritten only after the next
-        // item's barriers, which every thread passes once it has read them)
+        e = e_nxt;
+        e_nxt = e_nn;
     }
-    if (csid >= 0) flush();
-    __syncthreads();  // the shared memory may serve another phase next
+    flush();
 }
 
-__global__ void __launch_bounds__(NCELL) k_grid(Shared sh) { grid_body(sh); }
+__global__ void __launch_bounds__(GRID_T) k_grid(Shared sh) { grid_body(sh); }
 
 // -------------------------------------------------------------------- G2P
 
@@ -1926,10 +1652,10 @@ __device__ __forceinline__ int dir_of(int ib, int jb, int ti, int tj) {
     return (di + 1) * 3 + (dj + 1);
 }
 
+constexpr int G2P_T = 2 * NCELL;  // threads of a CTA
 #ifndef SLAB_G2P_MIN_BLOCKS
-#define SLAB_G2P_MIN_BLOCKS (NCELL == 64 ? 14 : 3)
+#define SLAB_G2P_MIN_BLOCKS (NCELL == 64 ? 9 : 2)
 #endif
-constexpr int G2P_MIN_BLOCKS = SLAB_G2P_MIN_BLOCKS;  // resident G2P CTAs per SM the register budget is cut for
 
 // puts tile tt on the next step's active list, once
 __device__ __forceinline__ void g2p_activate(const ScnSm& z, int tt) {
@@ -1951,83 +1677,33 @@ __device__ __forceinline__ void g2p_flush_vmax2(const ScnSm& z, float vmax2) {
     if ((threadIdx.x & 31) == 0 && bits > *reinterpret_cast<volatile unsigned long long*>(acc)) atomicMax(acc, bits);
 }
 
-#ifndef SLAB_G2P_CAP
-#define SLAB_G2P_CAP (NCELL == 64 ? 5 * NCELL : 4 * NCELL)
-#endif
-constexpr int G2P_CAP = SLAB_G2P_CAP;  // candidates of a tile staged in shared memory (more are loaded chunk by chunk)
-
-// a tile's candidates, by candidate index
-struct G2PStage {
-    float2 f[G2P_CAP];
-    float2 v[G2P_CAP];
-    int32_t cell[G2P_CAP];
-    float h[G2P_CAP];
-    float m[G2P_CAP];
-    int32_t id[G2P_CAP];
-};
-
-struct G2PSmem {
-    G2PStage st;
-    float4 nv[TN * TN];
+template <int T> struct G2PSmem {
+    float4 nv[NWIN];
     float4 dem[(TILE + 1) * (TILE + 1)];
     int front, back;
-    int wst[2][NCELL / 32], wmv[2][NCELL / 32];  // per-warp stayer / mover counts of a chunk (double buffered)
+    alignas(16) int wcnt[2][(T / 32 + 3) / 4 * 4];  // stayers | movers << 16 of each warp of a chunk (double buffered)
     int dcnt[9];
     TileDesc d;
     ScnSm z;
-    double red[4][NCELL / 32];
+    double red[4][T / 32];
 };
 
-// one candidate of a tile in G2P: its index, data, and whether it is in the tile
+// one candidate of a tile: its two words, and whether it exists
 struct G2PCand {
-    int src;
-    int32_t cell, pid;
-    float2 f, v;
-    float h, m;
-    bool valid;
+    float4 a, b;
+    bool there;
 };
 
-__device__ __forceinline__ G2PCand load_g2p_cand(const TileDesc& D, const PBuf& B, int k, int ncand, int t, int TY) {
+__device__ __forceinline__ G2PCand load_g2p_cand(const TileDesc& D, const PBuf& B, int k, int ncand) {
     G2PCand q;
-    q.valid = k < ncand;
-    q.src = 0;
-    q.cell = 0;
-    q.pid = 0;
-    q.f = make_float2(1.f, 1.f);
-    q.v = make_float2(0.f, 0.f);
-    q.h = q.m = 0.f;
-    if (q.valid) {
+    q.there = k < ncand;
+    q.a = make_float4(1.f, 1.f, 0.f, 0.f);
+    q.b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (q.there) {
         int r;
-        q.src = cand_to_index(k, D, r);
-        q.cell = B.cell[q.src];  // the other loads go out with it; the filter is applied on use
-        q.f = B.f[q.src];
-        q.v = B.v[q.src];
-        q.h = B.h[q.src];
-        q.m = B.m[q.src];
-        q.pid = B.id[q.src];
-        q.valid = tile_of_cell(q.cell, TY) == t;
-    }
-    return q;
-}
-
-// candidate k of the tile from the stage (as load_g2p_cand)
-__device__ __forceinline__ G2PCand staged_g2p_cand(const G2PStage& st, int k, int ncand, int t, int TY) {
-    G2PCand q;
-    q.valid = k < ncand;
-    q.src = 0;
-    q.cell = 0;
-    q.pid = 0;
-    q.f = make_float2(1.f, 1.f);
-    q.v = make_float2(0.f, 0.f);
-    q.h = q.m = 0.f;
-    if (q.valid) {
-        q.cell = st.cell[k];
-        q.f = st.f[k];
-        q.v = st.v[k];
-        q.h = st.h[k];
-        q.m = st.m[k];
-        q.pid = st.id[k];
-        q.valid = tile_of_cell(q.cell, TY) == t;
+        const int src = cand_index(k, D, r);
+        q.a = B.a[src];
+        q.b = B.b[src];
     }
     return q;
 }
@@ -2035,37 +1711,40 @@ __device__ __forceinline__ G2PCand staged_g2p_cand(const G2PStage& st, int k, in
 // K4: G2P (src/simulation.cpp:877-940) of one tile: FLIP/PIC blend,
 // advection, depth update, and the write of the particle into the tile's
 // segment of the next buffer -- stayers from the front, particles that moved
-// to a neighbour tile from the back, with per-direction counts. The block
-// max of |v|^2 and the particle bounding box feed the next step's dt and
-// remesh box (K5). Latency: the scenario's values stay in shared memory
-// across a run of its tiles, the next tile's descriptor is requested while
-// this one runs, a tile's candidates (up to G2P_CAP), node window and terrain
-// come into shared memory by asynchronous copies requested in one round, and
-// a tile's neighbour activations (two dependent atomics) are issued while the
-// next tile's copies are in flight.
-__device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restrict__ z64, G2PSmem& sm) {
+// to a neighbour tile from the back, with per-direction counts. The max of
+// |v|^2 and the particle bounding box feed the next step's dt and remesh box
+// (K5). A particle is two 16-byte loads and two 16-byte stores; a thread
+// holds its candidate of this chunk and of the next in registers, so the
+// loads of a chunk go out with the node window's (asynchronous copies into
+// shared memory) or while the chunk before it is computed. The scenario's
+// values stay in shared memory across a run of its tiles, the next tile's
+// descriptor is requested while this one runs, and a tile's neighbour
+// activations (two dependent atomics) are issued while the next tile's loads
+// are in flight.
+template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restrict__ z64, G2PSmem<T>& sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nwork = sh.work_pref[sh.nscn];
-    int w0, w1;
-    work_range(nwork, w0, w1);
-    if (w0 < w1) load_desc(sh.desc + w0, &sm.d);
-    if (tid == 0) sm.z.sid = -1;
-    int pend_tt = -1;  // threads 0..8: neighbour tile the previous tile activates
-    float vmax2 = 0.f;  // largest |v|^2 of this thread's particles over the CTA's run of one scenario
-    SLAB_PHASE_BEGIN;
-    for (int w = w0; w < w1; ++w) {
+    int dn = 0;
+    const bool words = tid < DESC_WORDS;
+    if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
+    if (sh.nscn == 1) load_scn(sh, 0, sm.z, tid, T);
+    else if (tid == 0) sm.z.sid = -1;
+    const auto [w0, w1, step] = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
+    if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
+    int pend_tt = -1;    // threads 0..8: neighbour tile the previous tile activates
+    float vmax2 = 0.f;   // largest |v|^2 of this thread's particles over the CTA's run of one scenario
+    for (int w = w0; w < w1; w += step) {
+        __syncthreads();  // the tile before is done with the shared memory
+        if (words) reinterpret_cast<int*>(&sm.d)[tid] = dn;
         if (tid < 9) sm.dcnt[tid] = 0;
         __syncthreads();
-        SLAB_PHASE_MARK(8);
-        int dn = 0;
-        if (w + 1 < w1 && tid < DESC_WORDS) dn = reinterpret_cast<const int*>(sh.desc + w + 1)[tid];
+        if (w + step < w1 && words) dn = reinterpret_cast<const int*>(sh.desc + w + step)[tid];
         if (sm.d.sid != sm.z.sid) {  // uniform: a new scenario in this CTA's run
             if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);
             pend_tt = -1;
             if (w > w0) g2p_flush_vmax2(sm.z, vmax2);
             vmax2 = 0.f;
             __syncthreads();
-            load_scn(sh, sm.d.sid, sm.z, tid, NCELL);
+            load_scn(sh, sm.d.sid, sm.z, tid, T);
             __syncthreads();
         }
         const ScnSm& Z = sm.z;
@@ -2075,31 +1754,11 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
         const bool outs = Z.y.outs != 0;
         const bool need_vz = Z.y.need_vz != 0;
         const int ncand = sm.d.rpref[9];
-        const bool staged = ncand <= G2P_CAP;
-        // the tile's candidates (the first chunk's, for a tile over the stage),
-        // the node window and the terrain are requested together; the stage
-        // and the windows fill by asynchronous copies
-        G2PCand pre = {};
-        if (staged) {
-            const PBuf& B = Z.s.buf[Z.y.seq & 1];
-            for (int k = tid; k < ncand; k += NCELL) {
-                int r;
-                const int src = cand_to_index(k, sm.d, r);
-                cpa::copy8(&sm.st.f[k], B.f + src);
-                cpa::copy8(&sm.st.v[k], B.v + src);
-                cpa::copy4(&sm.st.cell[k], B.cell + src);
-                cpa::copy4(&sm.st.h[k], B.h + src);
-                cpa::copy4(&sm.st.m[k], B.m + src);
-                cpa::copy4(&sm.st.id[k], B.id + src);
-            }
-        } else {
-            pre = load_g2p_cand(sm.d, Z.cur(), tid, ncand, t, sh.TY);
-        }
-        // the node window by per-thread asynchronous copies; a part whose grid tile
-        // has no block this step (or past the terrain edge) is zero. (Bulk copies
-        // of the blocks' rows, issued by warp 0 on an mbarrier, gave the same
-        // bits but made the kernel 6 % slower.)
-        for (int k = tid; k < TN * TN; k += NCELL) {
+        // the first candidates, the node window and the terrain in one round
+        SLAB_PHASE_BEGIN;
+        G2PCand nxt = load_g2p_cand(sm.d, Z.cur(), tid, ncand);
+        // a part of the window whose grid tile has no block this step (or past the terrain edge) is zero
+        for (int k = tid; k < NWIN; k += T) {
             const int a = k / TN, b = k % TN;
             const int i = ti * TILE + a, j = tj * TILE + b;
             const int blk = (i < sh.Nx && j < sh.Ny) ? sm.d.blk4[(a >= TILE ? 2 : 0) + (b >= TILE ? 1 : 0)] : -1;
@@ -2107,7 +1766,7 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
             else sm.nv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if (need_vz) {
-            for (int k = tid; k < (TILE + 1) * (TILE + 1); k += NCELL) {
+            for (int k = tid; k < (TILE + 1) * (TILE + 1); k += T) {
                 const int i = ti * TILE + k / (TILE + 1), j = tj * TILE + k % (TILE + 1);
                 if (i < sh.Nx && j < sh.Ny) cpa::copy16(&sm.dem[k], sh.dem + (int64_t)i * sh.Ny + j);
                 else sm.dem[k] = make_float4(0.f, 0.f, 1.f, 0.f);
@@ -2115,63 +1774,51 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
         }
         if (pend_tt >= 0) g2p_activate(Z, pend_tt);  // the previous tile's, while the loads above are in flight
         pend_tt = -1;
-        SLAB_PHASE_MARK(9);
+        SLAB_PHASE_MARK(8);
         cpa::wait_all();
         __syncthreads();
-        SLAB_PHASE_MARK(10);
+        SLAB_PHASE_MARK(9);
         const int total = sm.d.total;
         const int base = sm.d.nxt_off;
-        const PBuf& B = Z.s.buf[Z.y.seq & 1];
-        const PBuf O = Z.next();
-        const float dt = Z.y.dt;
-        const float dt_ood = Z.y.dt_ood;
-        const double dx = sh.dx;
         const bool edge = ti < Z.y.in_i0 || ti > Z.y.in_i1 || tj < Z.y.in_j0 || tj > Z.y.in_j1;  // uniform: may change the particle box
+        const bool inner = (ti + 1) * TILE + 1 <= sh.Nx - 1 && (tj + 1) * TILE + 1 <= sh.Ny - 1;  // uniform
         double mnx = INFINITY, mxx = 0.0, mny = INFINITY, mxy = 0.0;
         int front = 0, back = 0;  // stayers / movers placed so far (same in every thread)
-        G2PCand nxt = pre;
-        for (int k0 = 0; k0 < ncand; k0 += NCELL) {
-            // this chunk's candidates, and the next chunk's requested before this one is computed
-            G2PCand q;
-            if (staged) {
-                q = staged_g2p_cand(sm.st, k0 + tid, ncand, t, sh.TY);
-            } else {
-                q = nxt;
-                if (k0 + NCELL < ncand) nxt = load_g2p_cand(sm.d, B, k0 + NCELL + tid, ncand, t, sh.TY);
-            }
-            const bool valid = q.valid;
-            const int32_t cell = q.cell;
+        for (int k0 = 0; k0 < ncand; k0 += T) {
+            // this chunk's candidate, and the next chunk's requested before this one is computed
+            const G2PCand q = nxt;
+            if (k0 + T < ncand) nxt = load_g2p_cand(sm.d, Z.cur(), k0 + T + tid, ncand);
+            const int32_t cell = __float_as_int(q.b.z);
+            const int ci = cell_i(cell) - ti * TILE, cj = cell_j(cell) - tj * TILE;
+            const bool valid = q.there && (unsigned)ci < TILE && (unsigned)cj < TILE;
             int d = 4, ib = 0, jb = 0;
             float2 fn = make_float2(1.f, 1.f), vn = make_float2(0.f, 0.f);
-            float hn = 0.f, m = 0.f, vzp = 0.f;
+            float hn = 0.f, vzp = 0.f;
             double zp = 0.0;
-            int32_t pid = 0;
+            const float dt = Z.y.dt, dt_ood = Z.y.dt_ood;
             if (valid) {
-                const float2 f = q.f;
-                const float2 v = q.v;
-                const float h = q.h;
-                m = q.m;
-                pid = q.pid;
-                const int ci = cell_i(cell) - ti * TILE, cj = cell_j(cell) - tj * TILE;
+                const float2 f = make_float2(q.a.x, q.a.y);
+                const float2 v = make_float2(q.a.z, q.a.w);
+                const float h = q.b.x;
                 float wx[3], wy[3], dwx[3], dwy[3];
                 bspline3(f.x, wx, dwx);
                 bspline3(f.y, wy, dwy);
-                float picx = 0.f, picy = 0.f, flx = 0.f, fly = 0.f, div = 0.f;
+                float2 pic = make_float2(0.f, 0.f), fl = make_float2(0.f, 0.f);
+                float div = 0.f;
 #pragma unroll
                 for (int a = 0; a < 3; ++a)
 #pragma unroll
                     for (int b = 0; b < 3; ++b) {
                         const float wgt = wx[a] * wy[b];
                         const float4 nv = sm.nv[(ci + a) * TN + (cj + b)];
-                        picx += nv.x * wgt;
-                        picy += nv.y * wgt;
-                        flx += nv.z * wgt;
-                        fly += nv.w * wgt;
+                        const float2 w2 = make_float2(wgt, wgt);
+                        pic = f2fma(make_float2(nv.x, nv.y), w2, pic);
+                        fl = f2fma(make_float2(nv.z, nv.w), w2, fl);
                         div += (dwx[a] * wy[b]) * nv.x + (dwy[b] * wx[a]) * nv.y;
                     }
                 div *= Z.s.ood;
                 const float fr = Z.s.fr;
-                vn = make_float2(fr * (v.x + flx) + (1.f - fr) * picx, fr * (v.y + fly) + (1.f - fr) * picy);
+                vn = make_float2(fr * (v.x + fl.x) + (1.f - fr) * pic.x, fr * (v.y + fl.y) + (1.f - fr) * pic.y);
                 hn = h / (1.f + dt * div);
                 if (need_vz) {
                     const float4 dm = sm.dem[(ci + (f.x >= 1.f ? 1 : 0)) * (TILE + 1) + (cj + (f.y >= 1.f ? 1 : 0))];
@@ -2185,11 +1832,14 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
                         for (int b = 0; b < 3; ++b) zp += (double)(wx[a] * wy[b]) * z64[(int64_t)(i0 + a) * sh.Ny + (j0 + b)];
                 }
                 // advection with the PIC velocity and re-anchoring of the offset
-                const float ux = f.x + dt_ood * picx, uy = f.y + dt_ood * picy;
+                const float ux = f.x + dt_ood * pic.x, uy = f.y + dt_ood * pic.y;
                 const int ki = (int)floorf(ux - 0.5f), kj = (int)floorf(uy - 0.5f);
                 ib = cell_i(cell) + ki;
                 jb = cell_j(cell) + kj;
                 fn = make_float2(ux - (float)ki, uy - (float)kj);
+                // most particles stay in a tile whose stencils all lie inside the
+                // terrain: nothing else to check
+                if (!inner || (unsigned)(ci + ki) >= TILE || (unsigned)(cj + kj) >= TILE) {
                 d = dir_of(ib, jb, ti, tj);
                 if (d < 0) {
                     atomicOr(&c->err, ERR_MOVE);
@@ -2202,39 +1852,37 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
                     d = dir_of(ib, jb, ti, tj);
                     if (d < 0) d = 4;
                 }
+                }
                 if (edge) {
-                    const double px = ((double)ib + (double)fn.x) * dx, py = ((double)jb + (double)fn.y) * dx;
+                    const double px = ((double)ib + (double)fn.x) * sh.dx, py = ((double)jb + (double)fn.y) * sh.dx;
                     mnx = fmin(mnx, px);
                     mxx = fmax(mxx, px);
                     mny = fmin(mny, py);
                     mxy = fmax(mxy, py);
                 }
                 vmax2 = fmaxf(vmax2, vn.x * vn.x + vn.y * vn.y);
-                if (!isfinite(vn.x) || !isfinite(vn.y) || !isfinite(hn) || !isfinite(fn.x) || !isfinite(fn.y))
-                    atomicOr(&c->err, ERR_NONFINITE);
+                // 0 unless one of them is infinite or NaN
+                const float bad = fmaf(vn.x, 0.f, fmaf(vn.y, 0.f, fmaf(hn, 0.f, fmaf(fn.x, 0.f, fn.y * 0.f))));
+                if (bad != 0.f) atomicOr(&c->err, ERR_NONFINITE);
             }
             // stayers to the front of the segment, movers to the back, both in
             // candidate order (a block prefix of the warps' counts), so the next
             // step sees the tile's particles in an order fixed by the data
             const bool stay = valid && d == 4, move = valid && d != 4;
             const unsigned ms = __ballot_sync(0xffffffffu, stay), mm = __ballot_sync(0xffffffffu, move);
-            const int par = (k0 / NCELL) & 1;
-            if (lane == 0) {
-                sm.wst[par][warp] = __popc(ms);
-                sm.wmv[par][warp] = __popc(mm);
-            }
+            const int par = (k0 / T) & 1;
+            if (lane == 0) sm.wcnt[par][warp] = __popc(ms) | __popc(mm) << 16;
             __syncthreads();
-            int bs = front, bm = back;
+            int before = 0, all = 0;  // stayers | movers << 16: of the warps before this one, of all
 #pragma unroll
-            for (int q = 0; q < NCELL / 32; ++q) {
-                const int a = sm.wst[par][q], b = sm.wmv[par][q];
-                if (q < warp) {
-                    bs += a;
-                    bm += b;
-                }
-                front += a;
-                back += b;
+            for (int q_ = 0; q_ < T / 32; ++q_) {
+                const int a = sm.wcnt[par][q_];
+                if (q_ < warp) before += a;
+                all += a;
             }
+            const int bs = front + (before & 0xffff), bm = back + (before >> 16);
+            front += all & 0xffff;
+            back += all >> 16;
             const unsigned lt = (1u << lane) - 1u;
             if (valid) {
                 int pos;
@@ -2244,17 +1892,14 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
                     pos = base + total - 1 - (bm + __popc(mm & lt));
                     atomicAdd(&sm.dcnt[d], 1);
                 }
-                O.cell[pos] = pack_cell(ib, jb);
-                O.f[pos] = fn;
-                O.v[pos] = vn;
-                O.h[pos] = hn;
-                O.m[pos] = m;
-                O.id[pos] = pid;
+                const PBuf O = Z.next();
+                O.a[pos] = make_float4(fn.x, fn.y, vn.x, vn.y);
+                O.b[pos] = make_float4(hn, q.b.y, __int_as_float(pack_cell(ib, jb)), q.b.w);
                 if (need_vz) O.vz[pos] = vzp;
                 if (outs) O.z[pos] = (float)zp;
             }
         }
-        SLAB_PHASE_MARK(11);
+        SLAB_PHASE_MARK(10);
         if (tid == 0) {
             sm.front = front;
             sm.back = back;
@@ -2286,7 +1931,7 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
             }
             __syncthreads();
             if (tid == 0 && total > 0) {
-                for (int k = 1; k < NCELL / 32; ++k) {
+                for (int k = 1; k < T / 32; ++k) {
                     mnx = fmin(mnx, sm.red[0][k]);
                     mxx = fmax(mxx, sm.red[1][k]);
                     mny = fmin(mny, sm.red[2][k]);
@@ -2298,18 +1943,16 @@ __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restr
                 atomicMax(reinterpret_cast<unsigned long long*>(&c->pos_acc[3]), (unsigned long long)__double_as_longlong(mxy));
             }
         }
-        __syncthreads();
-        if (w + 1 < w1 && tid < DESC_WORDS) reinterpret_cast<int*>(&sm.d)[tid] = dn;
-        SLAB_PHASE_MARK(12);
+        SLAB_PHASE_MARK(11);
         SLAB_PHASE_TILE_G2P();
     }
     if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);  // the last tile's
     if (w0 < w1) g2p_flush_vmax2(sm.z, vmax2);
 }
 
-__global__ void __launch_bounds__(NCELL, G2P_MIN_BLOCKS) k_g2p(Shared sh, const double* __restrict__ z64) {
-    __shared__ G2PSmem sm;
-    g2p_body(sh, z64, sm);
+__global__ void __launch_bounds__(G2P_T, SLAB_G2P_MIN_BLOCKS) k_g2p(Shared sh, const double* __restrict__ z64) {
+    __shared__ G2PSmem<G2P_T> sm;
+    g2p_body<G2P_T>(sh, z64, sm);
 }
 
 // K5: end of the step for every running scenario (the per-step reductions
@@ -2370,17 +2013,16 @@ __device__ __forceinline__ bool grid_sync(const Shared& sh, GridBar* bar, long l
 
 // Shared memory of the persistent kernel: the largest phase's, reused by
 // every phase (each phase initialises what it reads).
-constexpr size_t PERSIST_SMEM = sizeof(P2CSmem) > sizeof(P2SSmem) ? (sizeof(P2CSmem) > sizeof(G2PSmem) ? sizeof(P2CSmem) : sizeof(G2PSmem))
-                                                                  : (sizeof(P2SSmem) > sizeof(G2PSmem) ? sizeof(P2SSmem) : sizeof(G2PSmem));
+constexpr size_t PERSIST_SMEM = sizeof(P2GTileSmem) > sizeof(G2PSmem<P2G_T>) ? sizeof(P2GTileSmem) : sizeof(G2PSmem<P2G_T>);
 
-// Up to nsteps whole steps (K1 tile bookkeeping, K2 both P2G classes, K3 grid
-// update, K4 G2P, K5 end of step) in one launch, the phases separated by
-// grid_sync instead of kernel boundaries. The same phase bodies as the
-// separate kernels, over the same work lists and in the same per-tile order,
-// so a step gives the same bits either way. The launch ends early once no
-// scenario has work (every one stopped at its frame, step budget or end).
-__global__ void __launch_bounds__(NCELL, P2C_MIN_BLOCKS) k_persist(Shared sh, const double* __restrict__ z64, int nsteps, long long limit,
-                                                                   GridBar* bar, const __grid_constant__ CUtensorMap dem_map) {
+// Up to nsteps whole steps (K1 tile bookkeeping, K2 P2G, K3 grid update, K4
+// G2P, K5 end of step) in one launch, the phases separated by grid_sync
+// instead of kernel boundaries. The same phase bodies as the separate kernels,
+// over the same work lists and in the same per-tile order, so a step gives
+// the same bits either way. The launch ends early once no scenario has work
+// (every one stopped at its frame, step budget or end).
+__global__ void __launch_bounds__(P2G_T, SLAB_P2G_MIN_BLOCKS) k_persist(Shared sh, const double* __restrict__ z64, int nsteps, long long limit,
+                                                                        GridBar* bar, const __grid_constant__ CUtensorMap dem_map) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // after a launch whose waits ran out, the tile bookkeeping of the step it
     // left is half done: no phase may run on it again
@@ -2388,13 +2030,11 @@ __global__ void __launch_bounds__(NCELL, P2C_MIN_BLOCKS) k_persist(Shared sh, co
     for (int s = 0; s < nsteps; ++s) {
         prep_body(sh);
         if (!grid_sync(sh, bar, limit)) return;
-        p2g_cell_body<false>(sh, 0, smem_raw, &dem_map);
-        __syncthreads();  // the shared memory passes to the next phase
-        p2g_sparse_body(sh, 1, smem_raw);
+        p2g_tiles_body(sh, smem_raw, &dem_map);
         if (!grid_sync(sh, bar, limit)) return;
         grid_body(sh);
         if (!grid_sync(sh, bar, limit)) return;
-        g2p_body(sh, z64, *reinterpret_cast<G2PSmem*>(smem_raw));
+        g2p_body<P2G_T>(sh, z64, *reinterpret_cast<G2PSmem<P2G_T>*>(smem_raw));
         if (!grid_sync(sh, bar, limit)) return;
         if (blockIdx.x == 0) control_scenarios(sh, CTL_END);
         if (!grid_sync(sh, bar, limit)) return;
@@ -2407,8 +2047,9 @@ __global__ void __launch_bounds__(NCELL, P2C_MIN_BLOCKS) k_persist(Shared sh, co
 // containing cell, z from the quadratic stencil of FP64 terrain heights.
 __global__ void k_refresh_vz_z(Shared sh, PBuf B, int Np, const double* __restrict__ z64) {
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < Np; q += gridDim.x * blockDim.x) {
-        const int32_t cell = B.cell[q];
-        const float2 f = B.f[q], v = B.v[q];
+        const int32_t cell = p_cell(B, q);
+        const float4 pa = B.a[q];
+        const float2 f = make_float2(pa.x, pa.y), v = make_float2(pa.z, pa.w);
         const int i0 = cell_i(cell), j0 = cell_j(cell);
         float wx[3], wy[3], dwx[3], dwy[3];
         bspline3(f.x, wx, dwx);
