@@ -112,6 +112,22 @@ struct Terrain {
     dptr<float4> dem32;    // FP32 copy for the split path: gx, gy, cos(theta), z
 };
 
+// Launches kernel k of a chain whose kernels all call chain_wait() first: it
+// may start before the kernel launched last on the stream is over.
+template <typename... P, typename... A> void launch_chained(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*k)(P...), A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    SLAB_CUDA(cudaLaunchKernelEx(&c, k, std::forward<A>(args)...));
+}
+
 // CUDA graphs of `chunk` consecutive steps, one per chunk size used.
 struct StepGraphs {
     std::map<int, cudaGraphExec_t> g;

@@ -75,6 +75,7 @@ __device__ __forceinline__ void stencil_weights(const Phys& P, double xp, int ba
 }
 
 __global__ void k64_begin(Ctl* c, int Nx, int Ny) {
+    chain_wait<true>();
     if (threadIdx.x == 0 && blockIdx.x == 0) ctl_begin(c, Nx, Ny);
 }
 __global__ void k64_begin_t0(Ctl* c, int Nx, int Ny) {
@@ -83,8 +84,9 @@ __global__ void k64_begin_t0(Ctl* c, int Nx, int Ny) {
 
 // P2G (src/simulation.cpp:726-798) with atomicAdd(double) scatter. Slope
 // terms of the particle's containing cell (src/complex_terrain.cpp:113-130).
-__global__ void __launch_bounds__(256) k64_p2g(const Ctl* __restrict__ c, P64 p, N64 n, const double2* __restrict__ grad,
+__global__ void __launch_bounds__(256) k64_p2g(const Ctl* c, P64 p, N64 n, const double2* __restrict__ grad,
                                                const double* __restrict__ cos_t, Phys P, int Np) {
+    chain_wait<true>();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= Np || !c->active) return;
     const double2 x = p.x[q], v = p.v[q];
@@ -164,6 +166,7 @@ __global__ void k64_pack_grid(N64 n, int Ny, int i0, int j0, int nI, int nJ, flo
 // the accumulators are zeroed for the next step.
 __global__ void __launch_bounds__(256) k64_grid(Ctl* c, N64 n, const double2* __restrict__ grad,
                                                 const double* __restrict__ cos_t, Phys P) {
+    chain_wait<true>();
     if (!c->active) return;
     const int i0 = c->box[0], j0 = c->box[2];
     const int nI = c->box[1] - i0 + 1, nJ = c->box[3] - j0 + 1;
@@ -282,6 +285,7 @@ __device__ void block_epilogue(Ctl* c, bool valid, double px, double py, double 
 // G2P (src/simulation.cpp:877-940).
 __global__ void __launch_bounds__(256) k64_g2p(Ctl* c, P64 p, N64 n, const double2* __restrict__ grad, const double* __restrict__ z,
                                                Phys P, int Np) {
+    chain_wait<true>();
     if (!c->active) return;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = q < Np;
@@ -436,10 +440,10 @@ struct Plain64 final : Path {
     void launch_kernel(int k) {
         const int pb = (Np + 255) / 256;
         switch (k) {
-            case 0: k64_begin<<<1, 32, 0, st>>>(dc, T.Nx, T.Ny); break;
-            case 1: k64_p2g<<<pb, 256, 0, st>>>(dc, parts(), nodes(), T.grad.get(), T.cos_t.get(), P, Np); break;
-            case 2: k64_grid<<<grid_blocks(), 256, 0, st>>>(dc, nodes(), T.grad.get(), T.cos_t.get(), P); break;
-            case 3: k64_g2p<<<pb, 256, 0, st>>>(dc, parts(), nodes(), T.grad.get(), T.z.get(), P, Np); break;
+            case 0: launch_chained(st, 1, 32, 0, k64_begin, dc, T.Nx, T.Ny); break;
+            case 1: launch_chained(st, pb, 256, 0, k64_p2g, dc, parts(), nodes(), T.grad.get(), T.cos_t.get(), P, Np); break;
+            case 2: launch_chained(st, grid_blocks(), 256, 0, k64_grid, dc, nodes(), T.grad.get(), T.cos_t.get(), P); break;
+            case 3: launch_chained(st, pb, 256, 0, k64_g2p, dc, parts(), nodes(), T.grad.get(), T.z.get(), P, Np); break;
         }
     }
     void launch_step() {

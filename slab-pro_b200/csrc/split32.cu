@@ -617,9 +617,7 @@ void Engine32::launch_begin(int t0) {
 void Engine32::launch_t0() {
     const Shared sh = shared();
     k32::k_begin<<<1, k32::CTL_THREADS, 0, st>>>(sh, 1);
-    k32::k_prep<<<grid_prep, 256, 0, st>>>(sh);
-    launch_p2g(sh);
-    k32::k_grid<<<grid_grid, k32::GRID_T, 0, st>>>(sh);
+    for (int k = 0; k < 3; ++k) launch_kernel(k, sh);
     SLAB_CUDA(cudaGetLastError());
     nlaunch += 4;
     pending_blocks = 0;  // later reads of the pool count see these blocks
@@ -628,7 +626,7 @@ void Engine32::launch_t0() {
 void Engine32::launch_p2g(const Shared& sh) {
     if (acc_mode == k32::ACC_MIXED || acc_mode == k32::ACC_CELL) {  // dense and sparse tiles, or every tile as a dense one
         const int grid = std::max(grid_p2g_cell, grid_p2g_sparse);
-        k32::k_p2g_tiles<<<grid, k32::P2G_T, sizeof(k32::P2GTileSmem), st>>>(sh, dem_map);
+        launch_chained(st, grid, k32::P2G_T, sizeof(k32::P2GTileSmem), k32::k_p2g_tiles, sh, dem_map);
     } else if (acc_mode == k32::ACC_WARP) {
         k32::k_p2g_warp<<<grid_p2g, k32::P2W_THREADS, k32::P2W_WARPS * sizeof(k32::P2WWarp), st>>>(sh);
     } else if (acc_mode == k32::ACC_I32) {
@@ -642,11 +640,11 @@ void Engine32::launch_p2g(const Shared& sh) {
 
 void Engine32::launch_kernel(int k, const Shared& sh) {
     switch (k) {
-        case 0: k32::k_prep<<<grid_prep, 256, 0, st>>>(sh); break;
+        case 0: launch_chained(st, grid_prep, k32::PREP_THREADS, 0, k32::k_prep, sh); break;
         case 1: launch_p2g(sh); break;
-        case 2: k32::k_grid<<<grid_grid, k32::GRID_T, 0, st>>>(sh); break;
-        case 3: k32::k_g2p<<<grid_g2p, k32::G2P_T, 0, st>>>(sh, T.z.get()); break;
-        case 4: k32::k_end<<<1, k32::CTL_THREADS, 0, st>>>(sh); break;
+        case 2: launch_chained(st, grid_grid, k32::GRID_T, 0, k32::k_grid, sh); break;
+        case 3: launch_chained(st, grid_g2p, k32::G2P_T, 0, k32::k_g2p, sh, T.z.get()); break;
+        case 4: launch_chained(st, 1, k32::CTL_THREADS, 0, k32::k_end, sh); break;
     }
 }
 
@@ -714,16 +712,16 @@ void Engine32::fix_shapes(const int32_t* grids, bool tune_on) {
 // One MIXED step with an event before each kernel and after the last.
 void Engine32::launch_step_timed(const Shared& sh, cudaEvent_t* e) {
     SLAB_CUDA(cudaEventRecord(e[0], st));
-    k32::k_prep<<<grid_prep, 256, 0, st>>>(sh);
+    launch_kernel(0, sh);
     SLAB_CUDA(cudaEventRecord(e[1], st));
-    launch_p2g(sh);
+    launch_kernel(1, sh);
     SLAB_CUDA(cudaEventRecord(e[2], st));  // (shape 2, the sparse tiles', goes with shape 1: one kernel runs both)
     SLAB_CUDA(cudaEventRecord(e[3], st));
-    k32::k_grid<<<grid_grid, k32::GRID_T, 0, st>>>(sh);
+    launch_kernel(2, sh);
     SLAB_CUDA(cudaEventRecord(e[4], st));
-    k32::k_g2p<<<grid_g2p, k32::G2P_T, 0, st>>>(sh, T.z.get());
+    launch_kernel(3, sh);
     SLAB_CUDA(cudaEventRecord(e[5], st));
-    k32::k_end<<<1, k32::CTL_THREADS, 0, st>>>(sh);
+    launch_kernel(4, sh);
     SLAB_CUDA(cudaEventRecord(e[6], st));
 }
 

@@ -268,11 +268,15 @@ __device__ __forceinline__ void control_scenarios(const Shared& sh, int what, in
 
 constexpr int CTL_THREADS = 256;  // one thread per scenario; enough registers for the control block
 
-__global__ void __launch_bounds__(CTL_THREADS) k_begin(Shared sh, int t0_pass) { control_scenarios(sh, t0_pass ? CTL_T0 : CTL_BEGIN); }
+__global__ void __launch_bounds__(CTL_THREADS) k_begin(Shared sh, int t0_pass) {
+    chain_wait<true>();
+    control_scenarios(sh, t0_pass ? CTL_T0 : CTL_BEGIN);
+}
 
 // Start of an advance call: every scenario gets the step budget and the
 // frame-stop rule, then the first step begins.
 __global__ void __launch_bounds__(CTL_THREADS) k_arm_begin(Shared sh, int64_t steps_left, int stop_at_frame) {
+    chain_wait<true>();
     control_scenarios(sh, CTL_ARM, steps_left, stop_at_frame);
 }
 
@@ -289,14 +293,23 @@ struct ScnSm {
 };
 static_assert(sizeof(Scn) % 16 == 0 && sizeof(SDyn) % 16 == 0, "loaded as 16-byte words");
 
-__device__ __forceinline__ void load_scn(const Shared& sh, int sid, ScnSm& z, int t, int nt) {
-    constexpr int A = sizeof(Scn) / 16, B = sizeof(SDyn) / 16;
-    for (int k = t; k < A + B; k += nt) {
-        if (k < A) reinterpret_cast<int4*>(&z.s)[k] = reinterpret_cast<const int4*>(sh.scn + sid)[k];
-        else reinterpret_cast<int4*>(&z.y)[k - A] = reinterpret_cast<const int4*>(sh.dyn + sid)[k - A];
-    }
+__device__ __forceinline__ void load_scn_static(const Shared& sh, int sid, ScnSm& z, int t, int nt) {
+    for (int k = t; k < (int)(sizeof(Scn) / 16); k += nt) reinterpret_cast<int4*>(&z.s)[k] = reinterpret_cast<const int4*>(sh.scn + sid)[k];
     if (t == 0) z.sid = sid;
 }
+__device__ __forceinline__ void load_scn_step(const Shared& sh, int sid, ScnSm& z, int t) {
+    if (t < (int)(sizeof(SDyn) / 16)) reinterpret_cast<int4*>(&z.y)[t] = reinterpret_cast<const int4*>(sh.dyn + sid)[t];
+}
+__device__ __forceinline__ void load_scn(const Shared& sh, int sid, ScnSm& z, int t, int nt) {
+    load_scn_static(sh, sid, z, t, nt);
+    load_scn_step(sh, sid, z, t);
+}
+
+// Start of a kernel of the step chain. With one scenario (the small runs,
+// where a step is a chain of dependent loads more than anything else) its
+// descriptor, which no kernel of the chain writes, is in shared memory before
+// the kernel before is over, and the step values are requested beside the
+// work count and the first work item, which the caller guesses.
 
 // The work items w0, w0 + step, ... < w1 of one of n workers. Of several
 // scenarios a worker takes a contiguous run of the flat list, so that
@@ -335,53 +348,77 @@ static_assert(sizeof(TileDesc) == 28 * 4 && offsetof(TileDesc, rstart) == 4 * 4 
 __device__ __forceinline__ void prep_body(const Shared& sh) {
     __shared__ int s_sid[PREP_MAX_TILES], s_cnt[PREP_MAX_TILES], s_ng[PREP_MAX_TILES];  // of the block's tiles
     __shared__ int s_off[PREP_MAX_TILES], s_goff[PREP_MAX_TILES];
-    const int nwork = sh.work_pref[sh.nscn];
+    __shared__ ScnSm s_one;
     const int lane = threadIdx.x & 31, r = lane & (PREP_LANES - 1);
     const int per_block = (int)blockDim.x / PREP_LANES, mine = threadIdx.x / PREP_LANES;
     const int stride = gridDim.x * per_block;
+    const bool one = sh.nscn == 1;
+    if (one) {
+        load_scn_static(sh, 0, s_one, threadIdx.x, blockDim.x);
+        __syncthreads();
+    }
+    chain_wait<false>();
+    // one scenario: the tile's entry in both lists, before the step's parity and
+    // the work count are known; later ones while the tile before is handled
+    int e0 = 0, e1 = 0;
+    auto entries = [&](int w) {
+        if (one && w < s_one.s.act_cap) {
+            e0 = s_one.s.act_list[0][w];
+            e1 = s_one.s.act_list[1][w];
+        }
+    };
+    entries((int)blockIdx.x * per_block + mine);
+    const int nwork = sh.work_pref[sh.nscn];
     // whole blocks run every iteration (barriers and shuffles); a half warp
     // without a tile computes with valid = false
     for (int w0 = blockIdx.x * per_block; w0 < nwork; w0 += stride) {
         const int w = w0 + mine;
         const bool valid = w < nwork;
         int sid = 0, loc = 0;
-        if (valid) find_work(sh.work_pref, sh.nscn, w, sid, loc);
-        const Scn& S = sh.scn[sid];
+        if (valid && !one) find_work(sh.work_pref, sh.nscn, w, sid, loc);
+        const Scn& S = one ? s_one.s : sh.scn[sid];
         const SDyn& n = sh.dyn[sid];
         int seq = 0, stamp = 0, t = 0;
         if (valid) {
-            const int32_t *l0 = S.act_list[0], *l1 = S.act_list[1];  // loaded beside seq
             seq = n.seq;
             stamp = n.stepid;
-            t = ((seq & 1) ? l1 : l0)[loc];
+            if (one) {
+                t = (seq & 1) ? e1 : e0;
+            } else {
+                const int32_t *l0 = S.act_list[0], *l1 = S.act_list[1];  // loaded beside seq
+                t = ((seq & 1) ? l1 : l0)[loc];
+            }
         }
+        entries(w + stride);
         const int cur = seq & 1;
         const int ti = t / sh.TY, tj = t % sh.TY;
-        // lanes 0-8: the record of neighbour d = r (its particles that moved to t)
-        int rs = 0, rl = 0, c = 0;
+        // lanes 0-8: the record of neighbour d = r (its particles that moved to t);
+        // lanes 9-12: the grid tiles of t's node window, stamped with this step.
+        // All requests go out before the first answer is looked at.
+        int4 g = make_int4(0, 0, 0, 0);
+        int gc = 0, gst = -1;
         if (valid && r < 9) {
             const int si = ti - dir_i(r), sj = tj - dir_j(r);
             if (si >= 0 && sj >= 0 && si < sh.TX && sj < sh.TY) {
                 const int32_t* G = S.grp[cur] + (size_t)(si * sh.TY + sj) * GRP_STRIDE;
-                if (G[GRP_STAMP] == seq) {
-                    const int g0 = G[0], g1 = G[1], g2 = G[2];
-                    rs = r == 4 ? g0 : g1;
-                    rl = r == 4 ? g1 - g0 : g2 - g1;
-                    c = G[3 + r];
-                }
+                g = *reinterpret_cast<const int4*>(G);
+                gc = G[3 + r];
+                gst = G[GRP_STAMP];
             }
         }
-        // lanes 9-12: the grid tiles of t's node window, stamped with this step
-        bool new_gt = false;
-        int gt = 0;
+        int gt = 0, was = 0x7fffffff;
         if (valid && r >= 9 && r < 13) {
             const int k = r - 9;
             const int gi = ti + (k >> 1), gj = tj + (k & 1);
             if (gi < sh.TX && gj < sh.TY) {
                 gt = gi * sh.TY + gj;
-                new_gt = atomicMax(&S.gt_stamp[gt], stamp) < stamp;
+                was = atomicMax(&S.gt_stamp[gt], stamp);
             }
         }
+        if (valid && r == 0) S.slot_of[t] = w;
+        const bool live = gst == seq && r < 9 && valid;
+        const int rs = live ? (r == 4 ? g.x : g.y) : 0, rl = live ? (r == 4 ? g.y - g.x : g.z - g.y) : 0, c = live ? gc : 0;
+        const bool new_gt = was < stamp && valid;
         // half-warp shuffles: the tile's particle count and the range prefixes
         int incl = rl;
 #pragma unroll
@@ -402,10 +439,33 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
             s_sid[mine] = valid ? sid : -1;
             s_cnt[mine] = cnt;
             s_ng[mine] = __popc(gmask & hbits);
-            if (valid) S.slot_of[t] = w;
         }
         __syncthreads();
-        if (threadIdx.x < 32) {
+        if (one && threadIdx.x < 32) {
+            // one scenario: both counters by a warp prefix and one atomic each
+            for (int q0 = 0; q0 < per_block; q0 += 32) {
+                const int q = q0 + lane;
+                const bool has = q < per_block && s_sid[q] >= 0;
+                const int qc = has ? s_cnt[q] : 0, qg = has ? s_ng[q] : 0;
+                int ic = qc, ig = qg;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int yc = __shfl_up_sync(0xffffffffu, ic, o), yg = __shfl_up_sync(0xffffffffu, ig, o);
+                    if (lane >= o) {
+                        ic += yc;
+                        ig += yg;
+                    }
+                }
+                const int totg = __shfl_sync(0xffffffffu, ig, 31), totc = __shfl_sync(0xffffffffu, ic, 31);
+                int base = 0;
+                if (lane < 2) base = atomicAdd(lane == 0 ? &sh.cnt[0].cursor : sh.gcount, lane == 0 ? totc : totg);
+                const int bc = __shfl_sync(0xffffffffu, base, 0), bg = __shfl_sync(0xffffffffu, base, 1);
+                if (has) {
+                    s_off[q] = bc + ic - qc;
+                    s_goff[q] = bg + ig - qg;
+                }
+            }
+        } else if (threadIdx.x < 32) {
             for (int q0 = 0; q0 < per_block; q0 += 32) {
                 const int q = q0 + lane;
                 const int qs = q < per_block ? s_sid[q] : -1;
@@ -554,6 +614,7 @@ template <int ACC>
 __global__ void __launch_bounds__(P2G_THREADS, P2G_MIN_BLOCKS) k_p2g(Shared sh) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     P2GSmem& sm = *reinterpret_cast<P2GSmem*>(smem_raw);
+    chain_wait<true>();
     const int tid = threadIdx.x, lane = tid & 31;
     const WorkItems W = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
     for (int w = W.w0; w < W.w1; w += W.step) {
@@ -752,6 +813,7 @@ __global__ void __launch_bounds__(P2W_THREADS, 3) k_p2g_warp(Shared sh) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     P2WWarp& sw = reinterpret_cast<P2WWarp*>(smem_raw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
+    chain_wait<true>();
     const int gw = blockIdx.x * P2W_WARPS + (threadIdx.x >> 5), nw = gridDim.x * P2W_WARPS;
     const int nwork = sh.work_pref[sh.nscn];
     const int per = (nwork + nw - 1) / nw;
@@ -1401,16 +1463,18 @@ __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* 
     const int tid = threadIdx.x;
     int dn = 0;
     const bool words = tid < DESC_WORDS;
-    if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
-    if (sh.nscn == 1) load_scn(sh, 0, sm.z, tid, P2G_T);
+    if (sh.nscn == 1) load_scn_static(sh, 0, sm.z, tid, P2G_T);
     else if (tid == 0) sm.z.sid = -1;
-    const auto [w0, w1, step] = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
-    if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
     for (int k = tid; k < P2C_CHUNKS * P2C_HALVES; k += P2G_T) (&sm.cnt[0][0])[k] = 0;
     if (tid == 0) {
         tma::mbar_init(&sm.dem_bar, 1);
         tma::fence_mbar_init();
     }
+    chain_wait<true>();
+    if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
+    if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
+    const auto [w0, w1, step] = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
+    if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
     if (words) reinterpret_cast<int*>(&sm.d[0])[tid] = dn;
     if (words && w0 + step < w1) dn = reinterpret_cast<const int*>(sh.desc + w0 + step)[tid];
     __syncthreads();
@@ -1481,12 +1545,25 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
     ScnSm& zs = s_scn[warp];
     const Scn& Z = zs.s;
     const SDyn& Y = zs.y;
-    const int nwork = min(*sh.gcount, sh.gcap);
     const int gw = (int)blockIdx.x * nwarp + warp, gn = (int)gridDim.x * nwarp;
-    const auto [w0, w1, step] = work_items(sh, nwork, gw, gn);
-    if (w0 >= w1) return;  // warps run alone: no block barrier below
     const int2* const list = reinterpret_cast<const int2*>(sh.gflat);
     int csid = -1;
+    if (sh.nscn == 1) load_scn_static(sh, 0, zs, lane, 32);
+    chain_wait<false>();
+    int2 e = make_int2(-1, 0), e_nxt = make_int2(-1, 0);
+    if (sh.nscn == 1) {  // the entries that this warp will have, before the count is known
+        if (gw < sh.gcap) e = list[gw];
+        if (gw + gn < sh.gcap) e_nxt = list[gw + gn];
+        load_scn_step(sh, 0, zs, lane);
+    }
+    const int nwork = min(*sh.gcount, sh.gcap);
+    const auto [w0, w1, step] = work_items(sh, nwork, gw, gn);
+    if (w0 >= w1) return;  // warps run alone: no block barrier below
+    if (sh.nscn != 1) {
+        e = list[w0];
+        if (w0 + step < w1) e_nxt = list[w0 + step];
+    }
+    if (w0 + step >= w1) e_nxt = make_int2(-1, 0);
     double macc = 0.0;  // mass and active nodes of this lane over the run of one scenario
     unsigned nacc = 0;
     auto flush = [&] {
@@ -1516,7 +1593,11 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
             sl_ = Z.blk_of[gt];
         }
     };
-    int2 e = list[w0], e_nxt = w0 + step < w1 ? list[w0 + step] : make_int2(-1, 0);
+    if (sh.nscn == 1) {
+        csid = 0;
+        __syncwarp();
+        request(e.y);
+    }
     for (int w = w0; w < w1; w += step) {
         if (e.x != csid) {  // a new scenario in this warp's run
             if (csid >= 0) flush();
@@ -1569,23 +1650,34 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
                 // terrain and maxima are requested with the partials (one round of loads)
                 const float4 dm = inside ? sh.dem[(int64_t)i * sh.Ny + j] : make_float4(0.f, 0.f, 1.f, 0.f);
                 const float hmax0 = sh.hmax[bn], vmax0 = sh.vmax2[bn];
+                // the covering tiles' partials, all requested before the first is
+                // added (a branch per tile made them four rounds of loads); one
+                // that does not cover the node adds zero
+                float4 pq[4];
+                float2 pF[4];
+                float pz[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    // tile k: 0 own, 1 -y, 2 -x, 3 -xy
+                    const int a = li + (k >> 1) * TILE, b = lj + (k & 1) * TILE;
+                    const bool covers = slots[k] >= 0 && a < TN && b < TN;
+                    const float* P = sh.part + (size_t)(covers ? slots[k] : 0) * PART_STRIDE;
+                    const int n = covers ? a * TN + b : 0;
+                    pq[k] = covers ? reinterpret_cast<const float4*>(P)[n] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    pF[k] = covers ? reinterpret_cast<const float2*>(P + 4 * NWIN)[n] : make_float2(0.f, 0.f);
+                    pz[k] = covers && Y.outs ? P[6 * NWIN + n] : 0.f;
+                }
                 float2 m2 = make_float2(0.f, 0.f), v2 = m2, F2 = m2;  // m, m h; m v; F
                 float qz = 0.f;
-                auto add = [&](int s, int a, int b) {
-                    if (s < 0) return;
-                    const float* P = sh.part + (size_t)s * PART_STRIDE;
-                    const int n = a * TN + b;
-                    const float4 q = reinterpret_cast<const float4*>(P)[n];
-                    const float2 F = reinterpret_cast<const float2*>(P + 4 * NWIN)[n];
-                    m2 = f2add(m2, make_float2(q.x, q.y));
-                    v2 = f2add(v2, make_float2(q.z, q.w));
-                    F2 = f2add(F2, F);
-                    if (Y.outs) qz += P[6 * NWIN + n];
-                };
-                add(slots[0], li, lj);
-                if (li < 2) add(slots[2], li + TILE, lj);
-                if (lj < 2) add(slots[1], li, lj + TILE);
-                if (li < 2 && lj < 2) add(slots[3], li + TILE, lj + TILE);
+                constexpr int order[4] = {0, 2, 1, 3};
+#pragma unroll
+                for (int u_ = 0; u_ < 4; ++u_) {
+                    const int k = order[u_];
+                    m2 = f2add(m2, make_float2(pq[k].x, pq[k].y));
+                    v2 = f2add(v2, make_float2(pq[k].z, pq[k].w));
+                    F2 = f2add(F2, pF[k]);
+                    qz += pz[k];
+                }
                 float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
                 float hn = 0.f, vzn = 0.f;
                 const float mi = m2.x;
@@ -1668,13 +1760,14 @@ __device__ __forceinline__ void g2p_activate(const ScnSm& z, int tt) {
 }
 
 // the largest |v|^2 of a run of tiles into the scenario's control block: one
-// atomic per warp, and only if it raises the value seen (speeds squared are
-// >= 0, so their bit patterns order like the values)
+// atomic per warp that does not wait for an answer (speeds squared are >= 0,
+// so their bit patterns order like the values)
 __device__ __forceinline__ void g2p_flush_vmax2(const ScnSm& z, float vmax2) {
-    const double v = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(vmax2)));
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-    unsigned long long* acc = reinterpret_cast<unsigned long long*>(&z.s.ctl->vmax2_acc);
-    if ((threadIdx.x & 31) == 0 && bits > *reinterpret_cast<volatile unsigned long long*>(acc)) atomicMax(acc, bits);
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(vmax2));
+    if ((threadIdx.x & 31) == 0 && m) {
+        const double v = (double)__uint_as_float(m);
+        atomicMax(reinterpret_cast<unsigned long long*>(&z.s.ctl->vmax2_acc), (unsigned long long)__double_as_longlong(v));
+    }
 }
 
 template <int T> struct G2PSmem {
@@ -1725,9 +1818,11 @@ template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, cons
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int dn = 0;
     const bool words = tid < DESC_WORDS;
-    if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
-    if (sh.nscn == 1) load_scn(sh, 0, sm.z, tid, T);
+    if (sh.nscn == 1) load_scn_static(sh, 0, sm.z, tid, T);
     else if (tid == 0) sm.z.sid = -1;
+    chain_wait<true>();
+    if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
+    if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
     const auto [w0, w1, step] = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
     if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
     int pend_tt = -1;    // threads 0..8: neighbour tile the previous tile activates
@@ -1946,8 +2041,8 @@ template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, cons
         SLAB_PHASE_MARK(11);
         SLAB_PHASE_TILE_G2P();
     }
-    if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);  // the last tile's
     if (w0 < w1) g2p_flush_vmax2(sm.z, vmax2);
+    if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);  // the last tile's
 }
 
 __global__ void __launch_bounds__(G2P_T, SLAB_G2P_MIN_BLOCKS) k_g2p(Shared sh, const double* __restrict__ z64) {
@@ -1958,7 +2053,10 @@ __global__ void __launch_bounds__(G2P_T, SLAB_G2P_MIN_BLOCKS) k_g2p(Shared sh, c
 // K5: end of the step for every running scenario (the per-step reductions
 // of G2P into dt, time and the remesh box), then the next step's dt, stop
 // rules and work list. One CTA, after G2P.
-__global__ void __launch_bounds__(CTL_THREADS) k_end(Shared sh) { control_scenarios(sh, CTL_END); }
+__global__ void __launch_bounds__(CTL_THREADS) k_end(Shared sh) {
+    chain_wait<true>();
+    control_scenarios(sh, CTL_END);
+}
 
 // ------------------------------------------------------- persistent steps
 
