@@ -192,10 +192,16 @@ slab_status slab_batch_run(slab_batch* b, int64_t max_steps, int64_t* steps_out)
         run_t0(b);
         b->E->arm(max_steps, 0);
         int64_t done = 0;
+        pull_all(b);
         while (done < max_steps) {
-            const int k = (int)std::min<int64_t>(b->chunk, max_steps - done);
-            b->E->enqueue_steps(k);
-            done += k;
+            // a chunk, or what the scenario with most steps to go still needs
+            int64_t need = 1;
+            for (int s = 0; s < b->E->nscn; ++s)
+                if (b->h_ctl[s].time < b->h_ctl[s].total_time && !b->h_ctl[s].err) need = std::max(need, steps_until(b->h_ctl[s], b->h_ctl[s].total_time));
+            const int64_t todo = std::min<int64_t>({(int64_t)b->chunk, max_steps - done, need < b->chunk ? (need + 3) / 4 * 4 : (int64_t)b->chunk});
+            if (todo < b->chunk && todo < max_steps - done) enqueue_planned(todo, b->chunk, [&](int k) { b->E->enqueue_steps(k); });
+            else b->E->enqueue_steps((int)todo);
+            done += todo;
             b->E->check_capacity();
             pull_all(b);
             bool all_stopped = true, gave_up = false;

@@ -169,7 +169,13 @@ void advance(slab_ctx* c, int64_t nsteps, bool stop_at_frame, int64_t* steps_out
         double last_time = c->h_ctl->time;
         int stalled = 0;
         for (;;) {
-            c->path->enqueue_steps(c->chunk);
+            // the steps to the frame if dt stays as it is, without a look at the
+            // control block in between. Steps past the frame do nothing but cost
+            // their launches (28 of 128 for a frame of 100); if dt shrinks, the
+            // next round does the rest.
+            const double frame_time = std::min(c->h_ctl->output_dt * (c->h_ctl->frame + 1), c->h_ctl->total_time);
+            enqueue_planned(std::min<int64_t>(steps_until(*c->h_ctl, frame_time), 8 * (int64_t)c->chunk), c->chunk,
+                            [&](int k) { c->path->enqueue_steps(k); });
             pull_ctl(c);
             if (c->h_ctl->stop) break;
             // dt > 0 always moves time forward; a chunk without progress
@@ -269,16 +275,26 @@ namespace {
 void upload_arrays(slab_ctx* c, int32_t Np, const double* x, const double* v, const double* vz, const double* h, const double* A,
                    const double* m, const double* z) {
     c->uploaded = false;
-    c->path.reset();
+    // the path of the run before, with its step graphs (capturing and
+    // instantiating them takes 1-2 ms), serves again when it can; the
+    // parameters are the same, since slab_set_params drops the path
+    if (c->path && !c->path->reusable()) c->path.reset();
     reset_ctl(c);
-    if (c->params.precision == SLAB_FP64_PLAIN)
-        c->path = make_plain64(c->terrain, c->params, c->stream, c->d_ctl, c->h_ctl);
-    else
-        c->path = make_split32(c->terrain, c->params, c->stream, c->d_ctl, c->h_ctl);
-    if (c->persist >= 0 && c->params.precision != SLAB_FP64_PLAIN) c->path->set_persistent(c->persist != 0, c->persist_limit);
-    c->path->upload(Np, x, v, vz, h, A, m, z);
-    pull_ctl(c);
-    raise_device_errors(c);
+    try {
+        if (!c->path) {
+            if (c->params.precision == SLAB_FP64_PLAIN)
+                c->path = make_plain64(c->terrain, c->params, c->stream, c->d_ctl, c->h_ctl);
+            else
+                c->path = make_split32(c->terrain, c->params, c->stream, c->d_ctl, c->h_ctl);
+        }
+        if (c->persist >= 0 && c->params.precision != SLAB_FP64_PLAIN) c->path->set_persistent(c->persist != 0, c->persist_limit);
+        c->path->upload(Np, x, v, vz, h, A, m, z);
+        pull_ctl(c);
+        raise_device_errors(c);
+    } catch (...) {
+        c->path.reset();  // nothing of a failed upload is kept
+        throw;
+    }
     c->Np = Np;
     c->uploaded = true;
     c->initial_done = false;

@@ -4,6 +4,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
 #include "slab_gpu.h"
 
 namespace slab {
@@ -162,6 +166,18 @@ __device__ inline void ctl_end(Ctl* c) {
         c->frame += 1;
         c->frame_hit = 1;
     }
+}
+
+// Host: the steps from control block c to `time` if dt stays what updateDt
+// gives for the last G2P's speed, rounded up; at least 1.
+inline int64_t steps_until(const Ctl& c, double time) {
+    double vmax2;
+    static_assert(sizeof vmax2 == sizeof c.vmax2_bits, "double bits");
+    std::memcpy(&vmax2, &c.vmax2_bits, sizeof vmax2);
+    const double speed = std::sqrt(vmax2);
+    const double dt = speed > 0.0 ? std::min(c.dt_max, c.C_cfl * c.dx / speed) : c.dt_max;
+    const double left = (time - c.time) / dt;
+    return left > 1.0 ? (int64_t)std::ceil(std::min(left, 1e9) - 1e-6) : 1;
 }
 
 // Same as ctl_begin for simulate()'s t=0 pass: dt = 0, no time advance.

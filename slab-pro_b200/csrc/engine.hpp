@@ -210,10 +210,26 @@ struct PhaseTimer {
     }
 };
 
+// Enqueues `todo` steps as whole chunks, then halving ones down to 4 (few
+// different step graphs), rounding the last one up.
+template <typename F> void enqueue_planned(int64_t todo, int chunk, F enqueue) {
+    for (int k = chunk; todo > 0;) {
+        if (todo >= k || k <= 4) {
+            enqueue(k);
+            todo -= k;
+        } else {
+            k /= 2;
+        }
+    }
+}
+
 struct Path {
     virtual ~Path() = default;
     virtual void upload(int Np, const double* x, const double* v, const double* vz, const double* h, const double* A, const double* m,
                         const double* z) = 0;
+    // whether upload() may be called again on this path: its buffers, step
+    // graphs and launch shapes then serve the next run
+    virtual bool reusable() const { return false; }
     virtual void initial_pass() = 0;
     // enqueue up to `chunk` steps; the device control block decides which run
     virtual void enqueue_steps(int chunk) = 0;

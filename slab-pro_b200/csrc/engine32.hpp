@@ -66,6 +66,7 @@ class Engine32 {
     // free a finished scenario's slot: its memory, its node blocks (back to
     // the pool, zeroed) and its control block (replaced by empty_ctl)
     void retire(int sid, const Ctl& empty_ctl);
+    void restart_counts();
     // node box covered by the scenario's blocks; box[1] < box[0] if none
     void box_of_blocks(int sid, int box[4]);
     void download_max_box(int sid, const int box[4], double* hmax, double* vmax2);

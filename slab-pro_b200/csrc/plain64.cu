@@ -393,6 +393,10 @@ struct Plain64 final : Path {
         gflip = dalloc<double2>(nn);
         out5 = dalloc<double>(5 * nn);
         maxes = dalloc<double>(2 * nn);
+        clear_nodes();
+    }
+    void clear_nodes() {
+        const size_t nn = (size_t)T.Nx * T.Ny;
         SLAB_CUDA(cudaMemsetAsync(acc.get(), 0, 7 * nn * sizeof(double), st));
         SLAB_CUDA(cudaMemsetAsync(gv.get(), 0, nn * sizeof(double2), st));
         SLAB_CUDA(cudaMemsetAsync(gflip.get(), 0, nn * sizeof(double2), st));
@@ -411,14 +415,24 @@ struct Plain64 final : Path {
 
     void upload(int np, const double* hx, const double* hv, const double* hvz, const double* hh, const double* hA, const double* hm,
                 const double* hz) override {
-        Np = np;
-        x = dalloc<double2>(np);
-        v = dalloc<double2>(np);
-        vz = dalloc<double>(np);
-        h = dalloc<double>(np);
-        A = dalloc<double>(np);
-        m = dalloc<double>(np);
-        z = dalloc<double>(np);
+        if (Np > 0) {  // another run on this path: the nodes as a new one has them
+            clear_nodes();
+            timer.collect();
+            timer.reset();
+            timer.on = false;
+            nlaunch = 0;
+        }
+        if (np != Np) {  // the step graphs carry the count and the buffers
+            graphs.clear();
+            Np = np;
+            x = dalloc<double2>(np);
+            v = dalloc<double2>(np);
+            vz = dalloc<double>(np);
+            h = dalloc<double>(np);
+            A = dalloc<double>(np);
+            m = dalloc<double>(np);
+            z = dalloc<double>(np);
+        }
         // host arrays, or device arrays of a release generated on the device
         SLAB_CUDA(cudaMemcpyAsync(x.get(), hx, np * sizeof(double2), cudaMemcpyDefault, st));
         SLAB_CUDA(cudaMemcpyAsync(v.get(), hv, np * sizeof(double2), cudaMemcpyDefault, st));
@@ -432,8 +446,8 @@ struct Plain64 final : Path {
         SLAB_CUDA(cudaGetLastError());
         ++nlaunch;
         SLAB_CUDA(cudaMemcpyAsync(&dc->vmax2_bits, &dc->vmax2_acc, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
-        graphs.clear();
     }
+    bool reusable() const override { return true; }
 
     int grid_blocks() const { return 148 * 4; }
 

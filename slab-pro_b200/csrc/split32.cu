@@ -675,7 +675,9 @@ void Engine32::tune_key_for(int Np) {
     int dev = 0;
     SLAB_CUDA(cudaGetDevice(&dev));
     const int bucket = Np > 0 ? (int)std::floor(2.0 * std::log2((double)Np)) : 0;
-    tune.key = std::to_string(dev) + ":" + std::to_string(TILE) + ":" + std::to_string(ntiles) + ":" + std::to_string(bucket);
+    const std::string key = std::to_string(dev) + ":" + std::to_string(TILE) + ":" + std::to_string(ntiles) + ":" + std::to_string(bucket);
+    if (key == tune.key) return;  // another run of the same size: its shapes, graphs and cadence go on
+    tune.key = key;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     const auto it = g_tune_cache.find(tune.key);
     if (it == g_tune_cache.end() || !tune.enabled) return;
@@ -756,6 +758,14 @@ void Engine32::tune_pick() {
     tune.state = 0;
     tune.tunes += 1;
     tune.next = std::max<int64_t>(4 * tune.steps, tune.steps + 256);
+}
+
+// launch and profile counts start anew with a new run
+void Engine32::restart_counts() {
+    timer.collect();
+    timer.reset();
+    timer.on = false;
+    nlaunch = 0;
 }
 
 void Engine32::set_persistent(bool on, long long limit_cycles) {
@@ -1134,9 +1144,16 @@ struct Split32 final : Path {
     void upload(int Np, const double* x, const double* v, const double* vz, const double* h, const double* A, const double* m,
                 const double* z) override {
         (void)A;
+        if (sid >= 0) {  // the run before gives its slot and node blocks back
+            Ctl empty = *hc;
+            E.retire(sid, empty);
+            E.restart_counts();
+            sid = -1;
+        }
         sid = E.add_scenario(prm, dc, hc, Np, x, v, vz, h, m, z);
         E.tune_key_for(Np);
     }
+    bool reusable() const override { return !E.dead; }
     void initial_pass() override { E.launch_t0(); }
     void enqueue_steps(int chunk) override { E.enqueue_steps(chunk); }
     bool arm(int64_t steps_left, int stop_at_frame) override {
