@@ -98,7 +98,7 @@ __global__ void k_bin_gather(int Np, const int32_t* __restrict__ order, const in
 // segment record of occupied tile r (stamp 0) and its place on the first
 // active list
 __global__ void k_bin_records(int n, const uint32_t* __restrict__ tiles, const int32_t* __restrict__ counts,
-                              const int32_t* __restrict__ starts, int32_t* grp, int32_t* act_list, int32_t* act_stamp) {
+                              const int32_t* __restrict__ starts, int32_t* grp, int32_t* act_list, int2* act) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         const int t = (int)tiles[r];
         int32_t* G = grp + (size_t)t * GRP_STRIDE;
@@ -109,7 +109,7 @@ __global__ void k_bin_records(int n, const uint32_t* __restrict__ tiles, const i
         G[3 + 4] = counts[r];
         G[GRP_STAMP] = 0;
         act_list[r] = t;
-        act_stamp[t] = 0;
+        act[t] = make_int2(0, r);
     }
 }
 
@@ -122,7 +122,7 @@ template <typename T> void cpy_h2d(T* d, const T* h, size_t n, cudaStream_t s) {
 
 BinResult bin_particles(const Terrain& T, int TY, int ntiles, cudaStream_t st, int Np, const double* x, const double* v, const double* vz,
                         const double* h, const double* m, const double* z, const PBuf& out, int32_t* grp0, int32_t* act_list0,
-                        int32_t* act_stamp, int act_cap, Scratch& scratch) {
+                        int2* act, int act_cap, Scratch& scratch) {
     BinResult res;
     if (Np <= 0) return res;
     int end_bit = 1;
@@ -183,7 +183,7 @@ BinResult bin_particles(const Terrain& T, int TY, int ntiles, cudaStream_t st, i
     if (n > act_cap) throw Error{SLAB_E_OOM, "active tile capacity"};
     SLAB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, t_bytes, counts, starts, n, st));
     k_bin_gather<<<blocks, 256, 0, st>>>(Np, val_s, cell, f, dv, dvz, dh, dm, dz, out);
-    k_bin_records<<<std::max(1, std::min((n + 127) / 128, 148 * 8)), 128, 0, st>>>(n, uniq, counts, starts, grp0, act_list0, act_stamp);
+    k_bin_records<<<std::max(1, std::min((n + 127) / 128, 148 * 8)), 128, 0, st>>>(n, uniq, counts, starts, grp0, act_list0, act);
     SLAB_CUDA(cudaGetLastError());
     res.tiles.resize(n);
     SLAB_CUDA(cudaMemcpyAsync(res.tiles.data(), uniq, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));

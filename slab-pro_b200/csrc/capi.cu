@@ -118,6 +118,7 @@ void reset_ctl(slab_ctx* c) {
 void pull_ctl(slab_ctx* c) {
     SLAB_CUDA(cudaMemcpyAsync(c->h_ctl, c->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->stream));
     SLAB_CUDA(cudaStreamSynchronize(c->stream));
+    if (c->path) c->path->observe(*c->h_ctl);
 }
 
 void raise_device_errors(slab_ctx* c) {

@@ -128,16 +128,17 @@ template <typename... P, typename... A> void launch_chained(cudaStream_t st, dim
     SLAB_CUDA(cudaLaunchKernelEx(&c, k, std::forward<A>(args)...));
 }
 
-// CUDA graphs of `chunk` consecutive steps, one per chunk size used.
+// CUDA graphs of `chunk` consecutive steps, one per chunk size and kind of step used.
 struct StepGraphs {
-    std::map<int, cudaGraphExec_t> g;
+    std::map<std::pair<int, int>, cudaGraphExec_t> g;
     ~StepGraphs() { clear(); }
     void clear() {
         for (auto& kv : g) cudaGraphExecDestroy(kv.second);
         g.clear();
     }
-    void launch(int chunk, cudaStream_t st, const std::function<void()>& one_step) {
-        auto it = g.find(chunk);
+    void launch(int chunk, cudaStream_t st, const std::function<void()>& one_step, int kind = 0) {
+        const std::pair<int, int> key{chunk, kind};
+        auto it = g.find(key);
         if (it == g.end()) {
             cudaGraph_t gr;
             SLAB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -147,7 +148,7 @@ struct StepGraphs {
             cudaError_t e = cudaGraphInstantiate(&ex, gr, 0);
             cudaGraphDestroy(gr);
             SLAB_CUDA(e);
-            it = g.emplace(chunk, ex).first;
+            it = g.emplace(key, ex).first;
         }
         SLAB_CUDA(cudaGraphLaunch(it->second, st));
     }
@@ -247,6 +248,8 @@ struct Path {
     // d_part Np x 8 float32 vertices (x y vx vy vz z h A, upload order),
     // d_grid 6 GeoTIFF bands over box {i0, i1, j0, j1} (slab_frame)
     virtual void pack_frame(float* d_part, float* d_grid, const int32_t box[4]) = 0;
+    // the control block as the host last read it, between chunks of steps
+    virtual void observe(const Ctl&) {}
     virtual int64_t launches() const = 0;
     virtual void phase_times(double out[5]) { for (int k = 0; k < 5; ++k) out[k] = 0; }
     virtual void set_profiling(bool) {}

@@ -27,7 +27,8 @@ class Engine32 {
         dptr<int32_t> grp[2], act_list[2];
         dptr<float4> a[2], b[2];  // PBuf
         dptr<float> vz[2], z[2];
-        dptr<int32_t> act_stamp, slot_of, nxt_off, gt_stamp, blk_of;
+        dptr<int2> act;
+        dptr<int32_t> nxt_off, gt_stamp, blk_of;
         SCnt* cnt = nullptr;  // in the engine's counter array
     };
 
@@ -40,7 +41,17 @@ class Engine32 {
     void launch_begin(int t0);
     void launch_t0();
     void launch_step();
+    static constexpr int NKERNELS = 5;  // of a step: k_prep, P2G, grid update, G2P, k_end
     void launch_kernel(int k, const Shared& sh);
+    // Steps of few active tiles run the grid update inside G2P (k_g2p<true>),
+    // with the same bits: per step 17 against 21 us at 12 tiles, 26 against 30
+    // at 734, 68 against 71 at 1 900, but 132 against 129 at 7 900 (8 000 tiles
+    // of a thin flow: 98 against 93), where computing the nodes on the tiles'
+    // edges up to four times costs more than a kernel. tiles_seen is what the
+    // host saw last.
+    static constexpr int64_t FUSED_MAX_TILES = 4096;
+    int64_t tiles_seen = 0;
+    bool fused() const { return tiles_seen <= FUSED_MAX_TILES; }
     void launch_p2g(const Shared& sh);
     CUtensorMap dem_map;   // the FP32 terrain as [Nx][4 Ny] floats, 9 x 9-node boxes (P2G's terrain window)
     // persistent steps: a chunk of steps as one cooperative launch of k_persist
@@ -153,7 +164,7 @@ class Engine32 {
                                     bool with_v);
     dptr<float4> d_nv;
     dptr<float> d_hmax, d_vmax2, d_oh, d_om, d_ovz, d_oFx, d_oFy;
-    dptr<int32_t> d_blk_stamp, d_blk_owner, d_misc, d_work_pref, d_gflat, d_free_blocks;
+    dptr<int32_t> d_blk_stamp, d_blk_owner, d_misc, d_work_pref, d_xlist, d_free_blocks;
     dptr<Scn> d_scn;
     dptr<SCnt> d_cnt;
     dptr<SDyn> d_dyn;

@@ -274,7 +274,7 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     if (const char* e = std::getenv("SLAB_P2G_ACC")) acc_mode = std::atoi(e);
     if (const char* e = std::getenv("SLAB_P2G_SPLIT")) split_min = std::atoi(e);
     split_min = std::min(split_min, k32::P2S_CAP);
-    int dev = 0, sms = 0, occ_p = 0, occ_g = 0, occ_u = 0;
+    int dev = 0, sms = 0, occ_p = 0, occ_g = 0;
     SLAB_CUDA(cudaGetDevice(&dev));
     SLAB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, k32::k_p2g_warp, k32::P2W_THREADS,
@@ -282,13 +282,14 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     int occ_c = 0, occ_h = 0;
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k32::k_p2g_tiles, k32::P2G_T, sizeof(k32::P2GTileSmem)));
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k32::k_p2g<k32::ACC_HILO>, k32::P2G_THREADS, sizeof(k32::P2GSmem)));
-    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p, k32::G2P_T, 0));
-    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k32::k_grid, k32::GRID_T, 0));
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p<false>, k32::G2P_T, 0));
     grid_p2g = sms * std::max(occ_p, 1);
     grid_p2g_cell = sms * std::max(occ_c, 1);
     grid_p2g_hilo = sms * std::max(occ_h, 1);
     grid_p2g_sparse = grid_p2g_cell;  // sparse tiles run in the same kernel
     grid_g2p = sms * std::max(occ_g, 1);
+    int occ_u = 0;
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k32::k_grid, k32::GRID_T, 0));
     grid_grid = sms * std::max(occ_u, 1);
     int occ_d = 0;
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_d, k32::k_prep, 256, 0));
@@ -304,9 +305,9 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_ps, k32::k_persist, k32::P2G_T, k32::PERSIST_SMEM));
     grid_persist = coop ? sms * occ_ps : 0;
     if (const char* e = std::getenv("SLAB_PERSIST")) persist = std::atoi(e) != 0 && grid_persist > 0;
-    timer.nk = 5;  // k_prep, P2G, grid update, G2P, k_end
-    const int phase_map[5] = {1, 2, 3, 4, 0};
-    for (int k = 0; k < 5; ++k) timer.phase_of[k] = phase_map[k];
+    timer.nk = NKERNELS;  // k_prep, P2G, grid update (unless G2P does it), G2P, k_end
+    const int phase_map[NKERNELS] = {1, 2, 3, 4, 0};
+    for (int k = 0; k < NKERNELS; ++k) timer.phase_of[k] = phase_map[k];
 }
 
 Engine32::~Engine32() {}
@@ -338,11 +339,11 @@ Shared Engine32::shared() const {
     sh.dyn = d_dyn.get();
     sh.work_pref = d_work_pref.get();
     sh.split_min = acc_mode == k32::ACC_MIXED ? split_min : -1;
-    sh.gflat = d_gflat.get();
-    sh.gcount = d_misc.get() + 6;
-    sh.gcap = 4 * work_cap;
     sh.desc = d_desc.get();
     sh.part = d_part.get();
+    sh.xlist = d_xlist.get();
+    sh.xcount = d_misc.get() + 6;
+    sh.use_xlist = fused() ? 0 : 1;
     sh.work_cap = work_cap;
     sh.free_blocks = d_free_blocks.get();
     sh.free_count = d_misc.get() + 4;
@@ -463,7 +464,7 @@ void Engine32::ensure_work_cap(int64_t need) {
     SLAB_CUDA(cudaStreamSynchronize(st));
     d_desc = dalloc<TileDesc>(cap);
     d_part = dalloc<float>((size_t)cap * PART_STRIDE);
-    d_gflat = dalloc<int32_t>((size_t)8 * cap);  // up to 4 grid tiles per active tile, 2 ints each
+    d_xlist = dalloc<int32_t>((size_t)3 * cap);  // up to 3 grid tiles without particles per active tile
     work_cap = (int)cap;
     graphs.clear();
 }
@@ -516,8 +517,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     if (new_lists) S.act_alloc = S.act_cap;
     else S.act_cap = S.act_alloc;  // a reused list keeps its full length
     if (new_tiles) {
-        S.act_stamp = dalloc<int32_t>(ntiles);
-        S.slot_of = dalloc<int32_t>(ntiles);
+        S.act = dalloc<int2>(ntiles);
         S.nxt_off = dalloc<int32_t>(ntiles);
         S.gt_stamp = dalloc<int32_t>(ntiles);
         S.blk_of = dalloc<int32_t>(ntiles);
@@ -535,10 +535,10 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     const double ood = 1.0 / T.dx;
     for (int b = 0; b < 2; ++b)  // every record stale (stamp -1)
         SLAB_CUDA(cudaMemsetAsync(S.grp[b].get(), 0xff, (size_t)ntiles * GRP_STRIDE * sizeof(int32_t), st));
-    SLAB_CUDA(cudaMemsetAsync(S.act_stamp.get(), 0xff, ntiles * sizeof(int32_t), st));
+    SLAB_CUDA(cudaMemsetAsync(S.act.get(), 0xff, ntiles * sizeof(int2), st));
     const PBuf out0{S.a[0].get(), S.b[0].get(), S.vz[0].get(), S.z[0].get()};
     const BinResult bin = bin_particles(T, TY, ntiles, st, Np, x, v, vz, h, m, z, out0, S.grp[0].get(), S.act_list[0].get(),
-                                        S.act_stamp.get(), S.act_cap, scratch);
+                                        S.act.get(), S.act_cap, scratch);
     const std::vector<uint32_t>& alist = bin.tiles;
     // node blocks the t=0 pass will take (the grid tiles of the active tiles'
     // node windows): grow the pool now, as the pass runs before any check
@@ -560,6 +560,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
         const int64_t need = (int64_t)(misc[0] - misc[4]) + pending_blocks;
         if (2 * need > blk_cap) grow_blocks((int)std::min<int64_t>(std::max<int64_t>(2 * (int64_t)blk_cap, 2 * need), INT32_MAX / NCELL));
     }
+    tiles_seen = (batch ? tiles_seen : 0) + (int64_t)alist.size();
     SLAB_CUDA(cudaMemsetAsync(S.gt_stamp.get(), 0xff, ntiles * sizeof(int32_t), st));
     SLAB_CUDA(cudaMemsetAsync(S.blk_of.get(), 0xff, ntiles * sizeof(int32_t), st));
     SCnt c0{};
@@ -595,8 +596,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
         D.grp[b] = S.grp[b].get();
         D.act_list[b] = S.act_list[b].get();
     }
-    D.act_stamp = S.act_stamp.get();
-    D.slot_of = S.slot_of.get();
+    D.act = S.act.get();
     D.nxt_off = S.nxt_off.get();
     D.gt_stamp = S.gt_stamp.get();
     D.blk_of = S.blk_of.get();
@@ -615,7 +615,8 @@ void Engine32::launch_begin(int t0) {
 }
 
 void Engine32::launch_t0() {
-    const Shared sh = shared();
+    Shared sh = shared();
+    sh.use_xlist = 1;  // the pass has no G2P to run the grid update in
     k32::k_begin<<<1, k32::CTL_THREADS, 0, st>>>(sh, 1);
     for (int k = 0; k < 3; ++k) launch_kernel(k, sh);
     SLAB_CUDA(cudaGetLastError());
@@ -643,7 +644,7 @@ void Engine32::launch_kernel(int k, const Shared& sh) {
         case 0: launch_chained(st, grid_prep, k32::PREP_THREADS, 0, k32::k_prep, sh); break;
         case 1: launch_p2g(sh); break;
         case 2: launch_chained(st, grid_grid, k32::GRID_T, 0, k32::k_grid, sh); break;
-        case 3: launch_chained(st, grid_g2p, k32::G2P_T, 0, k32::k_g2p, sh, T.z.get()); break;
+        case 3: launch_chained(st, grid_g2p, k32::G2P_T, 0, fused() ? k32::k_g2p<true> : k32::k_g2p<false>, sh, T.z.get()); break;
         case 4: launch_chained(st, 1, k32::CTL_THREADS, 0, k32::k_end, sh); break;
     }
 }
@@ -656,7 +657,8 @@ void Engine32::arm(int64_t steps_left, int stop_at_frame) {
 
 void Engine32::launch_step() {
     const Shared sh = shared();
-    for (int k = 0; k < 5; ++k) launch_kernel(k, sh);
+    for (int k = 0; k < NKERNELS; ++k)
+        if (k != 2 || !fused()) launch_kernel(k, sh);
 }
 
 constexpr int Engine32::Tuner::FACTOR4[];
@@ -719,7 +721,7 @@ void Engine32::launch_step_timed(const Shared& sh, cudaEvent_t* e) {
     launch_kernel(1, sh);
     SLAB_CUDA(cudaEventRecord(e[2], st));  // (shape 2, the sparse tiles', goes with shape 1: one kernel runs both)
     SLAB_CUDA(cudaEventRecord(e[3], st));
-    launch_kernel(2, sh);
+    if (!fused()) launch_kernel(2, sh);
     SLAB_CUDA(cudaEventRecord(e[4], st));
     launch_kernel(3, sh);
     SLAB_CUDA(cudaEventRecord(e[5], st));
@@ -749,6 +751,7 @@ void Engine32::tune_pick() {
         tune.pick[k] = best;
     }
     tune.pick[2] = tune.pick[1];
+    if (fused()) tune.pick[3] = 2;  // the kernel did not run: its occupancy grid
     apply_shapes(tune.pick);
     graphs.clear();  // the step graphs carry the grid sizes
     if (!tune.key.empty()) {
@@ -849,14 +852,16 @@ void Engine32::enqueue_steps(int chunk) {
     if (k < chunk) {
         if (timer.on) {
             const Shared sh = shared();
-            for (; k < chunk; ++k) timer.profiled_step(st, [&](int kk) { launch_kernel(kk, sh); });
+            for (; k < chunk; ++k) timer.profiled_step(st, [&](int kk) {
+                if (kk != 2 || !fused()) launch_kernel(kk, sh);
+            });
             SLAB_CUDA(cudaGetLastError());
         } else {
-            graphs.launch(chunk, st, [&] { launch_step(); });
+            graphs.launch(chunk, st, [&] { launch_step(); }, fused() ? 1 : 0);
         }
     }
     tune.steps += chunk;
-    nlaunch += 5 * (int64_t)chunk;
+    nlaunch += (NKERNELS - (fused() ? 1 : 0)) * (int64_t)chunk;
 }
 
 SCnt Engine32::counters(int sid) {
@@ -896,6 +901,7 @@ bool Engine32::check_capacity() {
         }
     }
     tune.active = active;
+    tiles_seen = active;
     if (grew) ensure_work_cap(work_cap_total);
     if (2 * (int64_t)used_blocks > blk_cap) {
         grow_blocks((int)std::min<int64_t>((int64_t)blk_cap * 2, INT32_MAX / NCELL));
@@ -1154,6 +1160,9 @@ struct Split32 final : Path {
         E.tune_key_for(Np);
     }
     bool reusable() const override { return !E.dead; }
+    void observe(const Ctl& c) override {
+        if (c.active || c.steps) E.tiles_seen = c.tiles;
+    }
     void initial_pass() override { E.launch_t0(); }
     void enqueue_steps(int chunk) override { E.enqueue_steps(chunk); }
     bool arm(int64_t steps_left, int stop_at_frame) override {

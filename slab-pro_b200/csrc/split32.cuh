@@ -78,8 +78,8 @@ struct alignas(16) SDyn {
     int32_t pad_[2];
 };
 
-// Work descriptor of one active tile t for the running step (written by
-// k_prep). Its particles are found in 9 candidate ranges of the current
+// Work descriptor of one active tile t for the running step, written by
+// k_prep. Its particles are found in 9 candidate ranges of the current
 // buffer: range 4 holds the stayers of t's own segment, range d != 4 the
 // movers of neighbour t - dir(d) (of which only those now in t are used);
 // rpref[d] is the number of candidates before range d; total is the exact
@@ -88,9 +88,13 @@ struct TileDesc {
     int32_t t, total, nxt_off, sid;
     int32_t rstart[9];
     int32_t rpref[10];
-    int32_t blk4[4];  // node blocks of the tile's node window (own, +y, +x, +xy grid tile), written by k_grid
-    int32_t pad_;
+    int32_t fresh;    // bit k > 0: grid tile k of the node window is no particle tile of this step, and this tile is the first to touch it
+    int32_t blk4[4];  // node blocks of the window's grid tiles (own, +y, +x, +xy); -1: off the terrain, BLK_LATER: look it up
+    int32_t nb[9];    // partial windows of the 3 x 3 tiles around t active this step (-1: not active)
+    int32_t pad_[3];
 };
+constexpr int BLK_LATER = -2;  // the block was being allocated while the descriptor was written (a grid tile's first step)
+static_assert(sizeof(TileDesc) % 16 == 0, "descriptors lie on 16-byte boundaries");
 
 // Segment record of a tile in a particle buffer (GRP_STRIDE ints, one
 // 64-byte line): [0] first stayer, [1] first mover (= end of stayers),
@@ -111,9 +115,8 @@ struct alignas(16) Scn {
     int32_t Np;
     PBuf buf[2];
     int32_t* grp[2];        // [ntiles][GRP_STRIDE] segment records (see GRP_STRIDE)
-    int32_t* act_stamp;     // [ntiles] last seq the tile was put on an active list
+    int2* act;              // [ntiles] {last seq the tile was put on an active list, its place on that list}
     int32_t* act_list[2];   // active tiles of each parity
-    int32_t* slot_of;       // [ntiles] work index (partial slot) of the tile in the running step
     int32_t* nxt_off;       // [ntiles] start of the tile's segment in the next buffer
     int32_t* gt_stamp;      // [ntiles] stepid at which the tile joined the grid list
     int32_t* blk_of;        // [ntiles] node block of the tile, -1 if none yet
@@ -147,12 +150,12 @@ struct Shared {
     int32_t* work_pref;   // [nscn+1] prefix of active tiles (P2G / G2P work)
     int32_t split_min;    // tiles with more particles take the cell-sorted P2G, the others the fixed-point one
     int32_t pad3_;
-    int32_t* gflat;       // [gcap][2] grid tiles of the running step: (scenario, grid tile)
-    int32_t* gcount;      // entries in gflat
-    int32_t gcap;
-    int32_t pad2_;
     TileDesc* desc;       // [work_cap] descriptors of the running step
     float* part;          // [work_cap][PART_STRIDE] P2G partial sums
+    int32_t* xlist;       // [3 work_cap] grid tiles of the step without particles of their own: work item << 2 | k (TileDesc::fresh)
+    int32_t* xcount;      // their count
+    int32_t use_xlist;    // the step has a grid update of its own
+    int32_t pad2_;
     int32_t work_cap;
     int32_t pad_;
     int32_t* free_blocks; // node blocks released by retired scenarios

@@ -1,14 +1,15 @@
 // Kernels of the FP32 split-precision step loop, shared by the
 // single-scenario path and the batched / served paths. One step is
-//   k_prep   (grid)    one thread per active tile: its 9 candidate ranges,
-//                      its segment in the next buffer, its grid tiles on the
-//                      flat grid-tile list
-//   k_p2g_cell, k_p2g_sparse (grid)
-//                      one CTA per active tile: P2G partial sums, tiles of
-//                      more than split_min particles by the cell-sorted
-//                      kernel, the others by the sparse-tile kernel
-//   k_grid   (grid)    one CTA per grid tile: grid update + friction
-//   k_g2p    (grid)    one CTA per active tile: G2P, advection, regrouping
+//   k_prep   (grid)    16 lanes per active tile: its 9 candidate ranges, its
+//                      segment in the next buffer, node blocks of new grid tiles
+//   k_p2g_tiles (grid) one CTA per active tile: P2G partial sums, tiles of
+//                      more than split_min particles sorted by cell, the
+//                      others in fixed point
+//   k_grid   (grid)    steps of many tiles: grid update + friction, a warp per
+//                      half grid tile
+//   k_g2p    (grid)    one CTA per active tile: (steps of few tiles: grid update
+//                      of the tile's node window, then) G2P, advection,
+//                      regrouping
 //   k_end    (1 CTA)   per scenario: end of the step, then the next step's
 //                      dt / stop rules and work-list prefix (k_arm_begin does
 //                      the same at the start of an advance call)
@@ -97,32 +98,6 @@ __device__ int warp_atomic_add(int* addr, int val, unsigned mask) {
     return base + prefix;
 }
 
-// warp_atomic_add in two halves, so that several atomics are in flight
-// before the first result is used: issue (the leader's atomic), then finish
-// (the broadcast of its result)
-struct WarpAdd {
-    unsigned peers;
-    int leader, prefix, base;
-};
-__device__ __forceinline__ WarpAdd warp_add_issue(int* addr, int val, unsigned mask) {
-    WarpAdd a;
-    a.peers = __match_any_sync(mask, (unsigned long long)addr);
-    const int lane = threadIdx.x & 31;
-    a.leader = __ffs(a.peers) - 1;
-    a.prefix = 0;
-    int total = 0;
-    for (unsigned m = a.peers; m; m &= m - 1) {
-        const int l = __ffs(m) - 1;
-        const int v = __shfl_sync(a.peers, val, l);
-        if (l < lane) a.prefix += v;
-        total += v;
-    }
-    a.base = 0;
-    if (lane == a.leader) a.base = atomicAdd(addr, total);
-    return a;
-}
-__device__ __forceinline__ int warp_add_finish(const WarpAdd& a) { return __shfl_sync(a.peers, a.base, a.leader) + a.prefix; }
-
 // candidate index -> particle index in the current buffer (range d)
 __device__ __forceinline__ int cand_to_index(int q, const TileDesc& D, int& d) {
     d = 0;
@@ -150,7 +125,7 @@ __device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) { return _
 
 constexpr int DESC_WORDS = (int)(sizeof(TileDesc) / 4);
 
-// copy a descriptor to shared memory (threads 0..27)
+// copy a descriptor to shared memory (its first threads)
 __device__ __forceinline__ void load_desc(const TileDesc* g, TileDesc* s) {
     if (threadIdx.x < (int)(sizeof(TileDesc) / 4)) reinterpret_cast<int*>(s)[threadIdx.x] = reinterpret_cast<const int*>(g)[threadIdx.x];
 }
@@ -208,6 +183,7 @@ __device__ __forceinline__ int step_control(const Shared& sh, int s, int what, i
         const double nft = __dmul_rn(k.output_dt, (double)(frame_after + 1));
         n.vz_next = (k.keep_outputs || __dadd_rn(k.new_time, k.dt_max) > nft - 1e-12) ? 1 : 0;
         cnt = (n.seq & 1) ? n.act_count[1] : n.act_count[0];
+        k.tiles = cnt;
         SDyn y;
         y.seq = n.seq;
         y.stepid = n.stepid;
@@ -261,8 +237,8 @@ __device__ __forceinline__ void control_scenarios(const Shared& sh, int what, in
     }
     if (tid == 0) {
         sh.work_pref[sh.nscn] = min(total, sh.work_cap);
+        *sh.xcount = 0;
         if (total > sh.work_cap) atomicOr(&sh.ctl[0].err, ERR_CAPACITY);
-        *sh.gcount = 0;
     }
 }
 
@@ -288,6 +264,7 @@ struct ScnSm {
     Scn s;
     SDyn y;
     int sid;
+    int base;  // first work item of the scenario
     __device__ __forceinline__ PBuf cur() const { return s.buf[y.seq & 1]; }
     __device__ __forceinline__ PBuf next() const { return s.buf[(y.seq & 1) ^ 1]; }
 };
@@ -298,6 +275,7 @@ __device__ __forceinline__ void load_scn_static(const Shared& sh, int sid, ScnSm
     if (t == 0) z.sid = sid;
 }
 __device__ __forceinline__ void load_scn_step(const Shared& sh, int sid, ScnSm& z, int t) {
+    if (t == 0) z.base = sh.nscn == 1 ? 0 : sh.work_pref[sid];
     if (t < (int)(sizeof(SDyn) / 16)) reinterpret_cast<int4*>(&z.y)[t] = reinterpret_cast<const int4*>(sh.dyn + sid)[t];
 }
 __device__ __forceinline__ void load_scn(const Shared& sh, int sid, ScnSm& z, int t, int nt) {
@@ -331,23 +309,22 @@ __device__ __forceinline__ WorkItems work_items(const Shared& sh, int nwork, int
 // segment in the current buffer plus the movers of the 8 neighbour segments
 // that moved to it (those are filtered by cell when read). The descriptor
 // records these 9 candidate ranges and the exact count, reserves the tile's
-// segment in the next buffer, and puts the 4 tiles owning its node window on
-// the grid-tile list.
+// segment in the next buffer, and gives node blocks to the grid tiles of its
+// node window that have none.
 // Sixteen lanes (half a warp) per active tile, so that its independent
 // global accesses go out together: lanes 0-8 read the 9 segment records,
-// lanes 9-12 stamp the 4 grid tiles, lane 0 takes the segment cursor and the
-// class-list slot; the counts and range prefixes are half-warp shuffles, and
-// the lanes write the descriptor's words side by side.
+// lanes 9-12 stamp the 4 grid tiles and see to their node blocks; the counts
+// and range prefixes are half-warp shuffles, and the lanes write the
+// descriptor's words side by side.
 constexpr int PREP_LANES = 16;
 constexpr int PREP_THREADS = 256;
 constexpr int PREP_MAX_TILES = 1024 / PREP_LANES;  // tiles of one block pass (the persistent kernel runs larger blocks)
-static_assert(sizeof(TileDesc) == 28 * 4 && offsetof(TileDesc, rstart) == 4 * 4 && offsetof(TileDesc, rpref) == 13 * 4 &&
-                  offsetof(TileDesc, blk4) == 23 * 4,
+static_assert(offsetof(TileDesc, rstart) == 4 * 4 && offsetof(TileDesc, rpref) == 13 * 4 && offsetof(TileDesc, fresh) == 23 * 4 &&
+                  offsetof(TileDesc, nb) == 28 * 4,
               "k_prep writes the descriptor word by word");
 
 __device__ __forceinline__ void prep_body(const Shared& sh) {
-    __shared__ int s_sid[PREP_MAX_TILES], s_cnt[PREP_MAX_TILES], s_ng[PREP_MAX_TILES];  // of the block's tiles
-    __shared__ int s_off[PREP_MAX_TILES], s_goff[PREP_MAX_TILES];
+    __shared__ int s_sid[PREP_MAX_TILES], s_cnt[PREP_MAX_TILES], s_off[PREP_MAX_TILES];  // of the block's tiles
     __shared__ ScnSm s_one;
     const int lane = threadIdx.x & 31, r = lane & (PREP_LANES - 1);
     const int per_block = (int)blockDim.x / PREP_LANES, mine = threadIdx.x / PREP_LANES;
@@ -396,7 +373,7 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
         // lanes 9-12: the grid tiles of t's node window, stamped with this step.
         // All requests go out before the first answer is looked at.
         int4 g = make_int4(0, 0, 0, 0);
-        int gc = 0, gst = -1;
+        int gc = 0, gst = -1, ast = -1, aslot = 0;
         if (valid && r < 9) {
             const int si = ti - dir_i(r), sj = tj - dir_j(r);
             if (si >= 0 && sj >= 0 && si < sh.TX && sj < sh.TY) {
@@ -404,21 +381,25 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
                 g = *reinterpret_cast<const int4*>(G);
                 gc = G[3 + r];
                 gst = G[GRP_STAMP];
+                const int2 ac = S.act[si * sh.TY + sj];
+                ast = ac.x;
+                aslot = ac.y;
             }
         }
-        int gt = 0, was = 0x7fffffff;
+        int gt = 0, was = 0x7fffffff, blk = -1;
         if (valid && r >= 9 && r < 13) {
             const int k = r - 9;
             const int gi = ti + (k >> 1), gj = tj + (k & 1);
             if (gi < sh.TX && gj < sh.TY) {
                 gt = gi * sh.TY + gj;
+                blk = S.blk_of[gt];
                 was = atomicMax(&S.gt_stamp[gt], stamp);
             }
         }
-        if (valid && r == 0) S.slot_of[t] = w;
         const bool live = gst == seq && r < 9 && valid;
         const int rs = live ? (r == 4 ? g.x : g.y) : 0, rl = live ? (r == 4 ? g.y - g.x : g.z - g.y) : 0, c = live ? gc : 0;
         const bool new_gt = was < stamp && valid;
+        const int nb = ast == seq && r < 9 && valid ? (one ? 0 : w - loc) + aslot : -1;  // that tile's partial window
         // half-warp shuffles: the tile's particle count and the range prefixes
         int incl = rl;
 #pragma unroll
@@ -430,79 +411,89 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
 #pragma unroll
         for (int o = PREP_LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o, PREP_LANES);
         const int ncand = __shfl_sync(0xffffffffu, incl, 8, PREP_LANES);
-        // the segment cursor and the flat grid-tile list: one
-        // atomic per address and block, by its first warp (one per address and
-        // warp made 3 same-address atomics per two tiles: 44 us on 47 k tiles)
-        const unsigned gmask = __ballot_sync(0xffffffffu, new_gt);
-        const unsigned hbits = (lane < PREP_LANES ? 0x0000ffffu : 0xffff0000u);
+        // a new grid tile's node block: the one it has, else one released by a
+        // retired scenario, else a fresh one
+        if (new_gt) {
+            if (blk < 0) {
+                const int f = atomicSub(sh.free_count, 1);
+                if (f > 0) {
+                    blk = sh.free_blocks[f - 1];
+                } else {
+                    atomicAdd(sh.free_count, 1);
+                    blk = atomicAdd(sh.blk_count, 1);
+                }
+                if (blk >= sh.blk_cap) {
+                    atomicOr(&S.ctl->err, ERR_CAPACITY);
+                    blk = -1;
+                } else {
+                    S.blk_of[gt] = blk;
+                    sh.blk_owner[blk] = sid;
+                }
+            }
+            if (blk >= 0) sh.blk_stamp[blk] = stamp;
+        } else if (blk < 0 && was != 0x7fffffff) {
+            blk = BLK_LATER;  // another tile is giving it one
+        }
+        // grid tile k = r - 9 (its particle tile is neighbour t + (k >> 1, k & 1),
+        // whose record lane 8 - direction read)
+        const int gk = r - 9, from = (lane & ~(PREP_LANES - 1)) + 8 - (((gk >> 1) + 1) * 3 + (gk & 1) + 1);
+        const int gnb = __shfl_sync(0xffffffffu, nb, r >= 9 && r < 13 ? from : lane);
+        const bool fresh = new_gt && gnb < 0;
+        const unsigned gmask = __ballot_sync(0xffffffffu, fresh);
+        if (gmask && sh.use_xlist) {  // the grid update's list of these
+            int at = 0;
+            if (lane == __ffs(gmask) - 1) at = atomicAdd(sh.xcount, __popc(gmask));
+            at = __shfl_sync(0xffffffffu, at, __ffs(gmask) - 1) + __popc(gmask & ((1u << lane) - 1u));
+            if (fresh) sh.xlist[at] = w << 2 | gk;
+        }
+        // the segment cursor: one atomic per scenario and block, by its first
+        // warp (one per warp, with the counters of the step's lists, made 3
+        // same-address atomics per two tiles: 44 us on 47 k tiles)
         if (r == 0) {
             s_sid[mine] = valid ? sid : -1;
             s_cnt[mine] = cnt;
-            s_ng[mine] = __popc(gmask & hbits);
         }
         __syncthreads();
         if (one && threadIdx.x < 32) {
-            // one scenario: both counters by a warp prefix and one atomic each
             for (int q0 = 0; q0 < per_block; q0 += 32) {
                 const int q = q0 + lane;
                 const bool has = q < per_block && s_sid[q] >= 0;
-                const int qc = has ? s_cnt[q] : 0, qg = has ? s_ng[q] : 0;
-                int ic = qc, ig = qg;
+                const int qc = has ? s_cnt[q] : 0;
+                int ic = qc;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    const int yc = __shfl_up_sync(0xffffffffu, ic, o), yg = __shfl_up_sync(0xffffffffu, ig, o);
-                    if (lane >= o) {
-                        ic += yc;
-                        ig += yg;
-                    }
+                    const int yc = __shfl_up_sync(0xffffffffu, ic, o);
+                    if (lane >= o) ic += yc;
                 }
-                const int totg = __shfl_sync(0xffffffffu, ig, 31), totc = __shfl_sync(0xffffffffu, ic, 31);
                 int base = 0;
-                if (lane < 2) base = atomicAdd(lane == 0 ? &sh.cnt[0].cursor : sh.gcount, lane == 0 ? totc : totg);
-                const int bc = __shfl_sync(0xffffffffu, base, 0), bg = __shfl_sync(0xffffffffu, base, 1);
-                if (has) {
-                    s_off[q] = bc + ic - qc;
-                    s_goff[q] = bg + ig - qg;
-                }
+                if (lane == 31) base = atomicAdd(&sh.cnt[0].cursor, ic);
+                base = __shfl_sync(0xffffffffu, base, 31);
+                if (has) s_off[q] = base + ic - qc;
             }
         } else if (threadIdx.x < 32) {
             for (int q0 = 0; q0 < per_block; q0 += 32) {
                 const int q = q0 + lane;
                 const int qs = q < per_block ? s_sid[q] : -1;
                 const unsigned m = __ballot_sync(0xffffffffu, qs >= 0);
-                if (qs >= 0) {
-                    const WarpAdd a_cur = warp_add_issue(&sh.cnt[qs].cursor, s_cnt[q], m);
-                    const WarpAdd a_gt = warp_add_issue(sh.gcount, s_ng[q], m);
-                    s_off[q] = warp_add_finish(a_cur);
-                    s_goff[q] = warp_add_finish(a_gt);
-                }
+                if (qs >= 0) s_off[q] = warp_atomic_add(&sh.cnt[qs].cursor, s_cnt[q], m);
             }
         }
         __syncthreads();
-        const int nxt_off = s_off[mine], at_g = s_goff[mine];
-        // the new grid tiles onto the flat grid-tile list, in lane order
-        if (new_gt) {
-            const int at = at_g + __popc(gmask & hbits & ((1u << lane) - 1u));
-            if (at < sh.gcap) {
-                sh.gflat[2 * at] = sid;
-                sh.gflat[2 * at + 1] = gt;
-            } else {
-                atomicOr(&S.ctl->err, ERR_CAPACITY);
-            }
-        }
+        const int nxt_off = s_off[mine];
         // the descriptor, word by word (TileDesc: t, total, nxt_off, sid,
-        // rstart[9], rpref[10], blk4[4], pad)
+        // rstart[9], rpref[10], fresh, blk4[4], nb[9])
         if (valid) {
             int* D = reinterpret_cast<int*>(sh.desc + w);
             if (r < 9) {
                 D[4 + r] = rs;
                 D[13 + r] = incl - rl;  // candidates before range r
-            } else if (r == 9) {
+                D[28 + 8 - r] = nb;     // (lane r read the tile at -direction r)
+            } else if (r < 13) {
+                D[24 + r - 9] = blk;
+            } else if (r == 13) {
                 D[22] = ncand;
-            } else if (r < 14) {
-                D[23 + (r - 10)] = -1;  // grid tiles off the terrain keep -1; k_grid fills the others
             } else if (r == 14) {
-                D[27] = 0;
+                D[23] = (int)(gmask >> ((lane & ~(PREP_LANES - 1)) + 9)) & 0xf;
             } else {
                 D[0] = t;
                 D[1] = cnt;
@@ -535,6 +526,28 @@ __device__ __forceinline__ void part_slot(int k, int& q, int& node) {
     } else {
         q = 6;
         node = k - 6 * NWIN;
+    }
+}
+
+// A grid tile's node block, looked up where k_prep could not name it yet.
+__device__ __forceinline__ int node_block(const Shared& sh, const Scn& S, const TileDesc& D, int k) {
+    const int blk = D.blk4[k];
+    return blk != BLK_LATER ? blk : S.blk_of[(D.t / sh.TY + (k >> 1)) * sh.TY + D.t % sh.TY + (k & 1)];
+}
+
+// Clears the nodes of the grid tiles that are no particle tiles of this step
+// and that tile D touches first: their nodes are then written one by one by
+// the tiles that reach them, the others keep zero. (t: thread of nt)
+__device__ __forceinline__ void p2g_clear_fresh(const Shared& sh, const Scn& S, const TileDesc& D, bool outs, int t, int nt) {
+    for (int k = 1; k < 4; ++k) {
+        if (!(D.fresh >> k & 1)) continue;
+        const int blk = node_block(sh, S, D, k);
+        if (blk < 0) continue;
+        for (int c = t; c < NCELL; c += nt) {
+            const size_t bn = (size_t)blk * NCELL + c;
+            sh.nv[bn] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (outs) sh.oh[bn] = sh.om[bn] = sh.ovz[bn] = sh.oFx[bn] = sh.oFy[bn] = 0.f;
+        }
     }
 }
 
@@ -629,6 +642,7 @@ __global__ void __launch_bounds__(P2G_THREADS, P2G_MIN_BLOCKS) k_p2g(Shared sh) 
         const int t = sm.d.t;
         const int ti = t / sh.TY, tj = t % sh.TY;
         SCnt* n = S.cnt;
+        p2g_clear_fresh(sh, S, sm.d, n->outs != 0, tid, P2G_THREADS);
         const int cur = n->seq & 1;
         const bool outs = n->outs != 0;
         for (int k = tid; k < (TILE + 1) * (TILE + 1); k += P2G_THREADS) {
@@ -821,7 +835,7 @@ __global__ void __launch_bounds__(P2W_THREADS, 3) k_p2g_warp(Shared sh) {
     int* hi = sw.node;
     int* lo = sw.node + NQ * TN * TN;
     for (int w = i0; w < i1; ++w) {
-        if (lane < (int)(sizeof(TileDesc) / 4)) reinterpret_cast<int*>(&sw.d)[lane] = reinterpret_cast<const int*>(sh.desc + w)[lane];
+        for (int k = lane; k < DESC_WORDS; k += 32) reinterpret_cast<int*>(&sw.d)[k] = reinterpret_cast<const int*>(sh.desc + w)[k];
         for (int k = lane; k < 2 * NQ * TN * TN; k += 32) sw.node[k] = 0;
         for (int k = lane; k < NCELL; k += 32) sw.ccnt[k] = 0;
         __syncwarp();
@@ -830,6 +844,7 @@ __global__ void __launch_bounds__(P2W_THREADS, 3) k_p2g_warp(Shared sh) {
         const SCnt* n = S.cnt;
         const int cur = n->seq & 1;
         const bool outs = n->outs != 0;
+        p2g_clear_fresh(sh, S, D, outs, lane, 32);
         const int ti = D.t / sh.TY, tj = D.t % sh.TY;
         const int ncand = D.rpref[9];
         const PBuf B = S.buf[cur];
@@ -1470,10 +1485,11 @@ __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* 
         tma::mbar_init(&sm.dem_bar, 1);
         tma::fence_mbar_init();
     }
-    chain_wait<true>();
+    chain_wait<false>();
     if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
     if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
-    const auto [w0, w1, step] = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
+    const WorkItems W = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
+    const int w0 = W.w0, w1 = W.w1, step = W.step;
     if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
     if (words) reinterpret_cast<int*>(&sm.d[0])[tid] = dn;
     if (words && w0 + step < w1) dn = reinterpret_cast<const int*>(sh.desc + w0 + step)[tid];
@@ -1500,6 +1516,7 @@ __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* 
                 requested = true;
             }
         };
+        if (D.fresh) p2g_clear_fresh(sh, sm.z.s, D, sm.z.y.outs != 0, tid, P2G_T);
         cpa::wait_all();
         float* part = sh.part + (size_t)w * PART_STRIDE;
         const TileOrigin o{(D.t / sh.TY) * TILE, (D.t % sh.TY) * TILE};
@@ -1524,217 +1541,204 @@ __global__ void __launch_bounds__(P2G_T, SLAB_P2G_MIN_BLOCKS) k_p2g_tiles(Shared
 
 // ------------------------------------------------------------ grid update
 
-// K3 + K6: computeGridVelocity (src/simulation.cpp:800-875) for the TILE^2
-// nodes owned by one grid tile. A node's P2G sum is the partials of the
-// tiles whose window covers it, added in a fixed order (own, -x, -y, -xy).
-// h_max / v_max2 are updated in the node block; the FP64 grid mass sum and
-// the active-node count are diagnostics, added up over a warp's run of grid
-// tiles of one scenario.
-// One warp per grid tile and no block barriers: the kernel is two dependent
-// rounds of loads (the covering tiles' slots and the node block, then partials,
-// terrain and maxima), so what counts is how many grid tiles an SM has in
-// flight. The slots and block of the next grid tile are requested while one is
-// computed, and a window node is one 16-byte and one 8-byte load.
+// computeGridVelocity (src/simulation.cpp:800-875) for node (li, lj) of grid
+// tile (gi, gj): velocity and FLIP increment. The P2G sum is the partials of
+// the tiles whose window covers the node -- slot[k]: 0 own, 1 -y, 2 -x, 3 -xy
+// tile of the grid tile, -1 if it has no particles this step -- added in the
+// order own, -x, -y, -xy, so everyone who computes the node gets the same
+// bits. blk >= 0: the caller owns the node and writes its maxima, its entry
+// of the node block and the output fields, and counts its mass.
+__device__ __forceinline__ float4 grid_node(const Shared& sh, const Scn& Z, const SDyn& Y, int gi, int gj, int li, int lj, const int (&slot)[4],
+                                            int blk, double& macc, unsigned& nacc) {
+    const int i = gi * TILE + li, j = gj * TILE + lj;
+    const bool inside = i < sh.Nx && j < sh.Ny;
+    // all partials requested before the first is added (a branch per tile made
+    // them four rounds of loads); a tile that does not cover the node adds zero
+    float4 pq[4];
+    float2 pF[4];
+    float pz[4];
+    constexpr int order[4] = {0, 2, 1, 3};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int k = order[u];
+        const bool covers = slot[k] >= 0;
+        const float* P = sh.part + (size_t)(covers ? slot[k] : 0) * PART_STRIDE;
+        const int pn = covers ? (li + (k >> 1) * TILE) * TN + lj + (k & 1) * TILE : 0;
+        pq[u] = covers ? reinterpret_cast<const float4*>(P)[pn] : make_float4(0.f, 0.f, 0.f, 0.f);
+        pF[u] = covers ? reinterpret_cast<const float2*>(P + 4 * NWIN)[pn] : make_float2(0.f, 0.f);
+        pz[u] = covers && Y.outs ? P[6 * NWIN + pn] : 0.f;
+    }
+    const size_t bn = (size_t)max(blk, 0) * NCELL + li * TILE + lj;
+    const float4 dm = inside ? sh.dem[(int64_t)i * sh.Ny + j] : make_float4(0.f, 0.f, 1.f, 0.f);
+    const float hmax0 = blk >= 0 ? sh.hmax[bn] : 0.f, vmax0 = blk >= 0 ? sh.vmax2[bn] : 0.f;
+    float2 m2 = make_float2(0.f, 0.f), v2 = m2, F2 = m2;  // m, m h; m v; F
+    float qz = 0.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        m2 = f2add(m2, make_float2(pq[u].x, pq[u].y));
+        v2 = f2add(v2, make_float2(pq[u].z, pq[u].w));
+        F2 = f2add(F2, pF[u]);
+        qz += pz[u];
+    }
+    float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+    float hn = 0.f, vzn = 0.f;
+    const float mi = m2.x;
+    if (mi > 1e-6f && inside) {
+        const float vox = v2.x / mi, voy = v2.y / mi;
+        if (Y.outs) vzn = qz / mi;
+        hn = m2.y / mi;
+        const float dt = Y.dt;
+        const float vtx = vox + dt * (F2.x / mi), vty = voy + dt * (F2.y / mi);
+        const float vsq = vtx * vtx + vty * vty;
+        float nvx = 0.f, nvy = 0.f;
+        if (vsq > 1e-16f) {
+            const float ct = dm.z;
+            const float vz = vtx * dm.x + vty * dm.y;
+            const float v3sq = vsq + vz * vz;
+            const float v3 = sqrtf(v3sq);
+            const float g = Z.g;
+            float af;
+            if (Z.fric == SLAB_COULOMB) {
+                af = Z.mu_c * g * ct;
+            } else if (Z.fric == SLAB_VOELLMY) {
+                af = Z.mu_v * g * ct + g * v3sq / (Z.xi * hn * ct);
+            } else {
+                const float I = 5.f * Z.d * v3 / (2.f * hn * ct * ct * sqrtf(g * hn * Z.phi));
+                const float muI = Z.mu1 + (Z.mu2 - Z.mu1) / (1.f + Z.I0 / I);
+                af = muI * g * ct;
+            }
+            const float dv = dt * af;
+            if (dv < v3) {
+                const float fct = 1.f - dv / v3;
+                nvx = vtx * fct;
+                nvy = vty * fct;
+            }
+        }
+        out = make_float4(nvx, nvy, nvx - vox, nvy - voy);
+        if (blk >= 0) {
+            sh.hmax[bn] = fmaxf(hmax0, hn);
+            sh.vmax2[bn] = fmaxf(vmax0, nvx * nvx + nvy * nvy);
+            macc += (double)mi;
+            nacc += 1u;
+        }
+    }
+    if (blk >= 0) {
+        sh.nv[bn] = out;
+        if (Y.outs) {
+            sh.oh[bn] = hn;
+            sh.om[bn] = inside ? mi : 0.f;
+            sh.ovz[bn] = vzn;
+            sh.oFx[bn] = inside ? F2.x : 0.f;
+            sh.oFy[bn] = inside ? F2.y : 0.f;
+        }
+    }
+    return out;
+}
+
+// whether the window of tile k (grid_node) covers node (li, lj) of the grid tile
+__device__ __forceinline__ bool covers_node(int k, int li, int lj) { return li + (k >> 1) * TILE < TN && lj + (k & 1) * TILE < TN; }
+
+// Node n of tile D's window, for its G2P. Owner of a node is the first active
+// tile, in the order of the sum, whose window covers it.
+__device__ __forceinline__ float4 window_node(const Shared& sh, const Scn& Z, const SDyn& Y, const TileDesc& D, int n, double& macc,
+                                              unsigned& nacc) {
+    const int a = n / TN, b = n % TN, qi = a >= TILE ? 1 : 0, qj = b >= TILE ? 1 : 0, li = a - qi * TILE, lj = b - qj * TILE;
+    int slot[4], first = -1;
+    constexpr int order[4] = {0, 2, 1, 3};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int k = order[u];
+        slot[k] = covers_node(k, li, lj) ? D.nb[(qi - (k >> 1) + 1) * 3 + (qj - (k & 1) + 1)] : -1;
+        if (slot[k] >= 0 && first < 0) first = k;
+    }
+    const int blk = first == 2 * qi + qj ? node_block(sh, Z, D, 2 * qi + qj) : -1;
+    return grid_node(sh, Z, Y, D.t / sh.TY + qi, D.t % sh.TY + qj, li, lj, slot, blk, macc, nacc);
+}
+
+// K3 + K6 as a kernel of its own, for steps of many tiles: a warp per 32 nodes
+// of a grid tile -- the particle tiles' own, then those without particles
+// (xlist). The kernel is a round of loads after the descriptor's words (which
+// the lanes hold, the next item's requested ahead) and the friction law's chain
+// of divisions, so what counts is how many warps an SM has in flight. Mass and
+// active nodes (diagnostics) are added up over a warp's run of one scenario.
 constexpr int GRID_T = 128;
-constexpr int GRID_MAX_WARPS = 3 * NCELL / 32 > GRID_T / 32 ? 3 * NCELL / 32 : GRID_T / 32;  // the persistent kernel's CTAs run it too
+constexpr int GRID_MAX_WARPS = GRID_T / 32;
 
 __device__ __forceinline__ void grid_body(const Shared& sh) {
     __shared__ ScnSm s_scn[GRID_MAX_WARPS];
-    constexpr int NPL = NCELL / 32;  // nodes per lane
+    constexpr int PARTS = NCELL / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     ScnSm& zs = s_scn[warp];
-    const Scn& Z = zs.s;
-    const SDyn& Y = zs.y;
     const int gw = (int)blockIdx.x * nwarp + warp, gn = (int)gridDim.x * nwarp;
-    const int2* const list = reinterpret_cast<const int2*>(sh.gflat);
-    int csid = -1;
     if (sh.nscn == 1) load_scn_static(sh, 0, zs, lane, 32);
     chain_wait<false>();
-    int2 e = make_int2(-1, 0), e_nxt = make_int2(-1, 0);
-    if (sh.nscn == 1) {  // the entries that this warp will have, before the count is known
-        if (gw < sh.gcap) e = list[gw];
-        if (gw + gn < sh.gcap) e_nxt = list[gw + gn];
+    // lane's word of a descriptor: nb, blk4, then t, sid
+    const int word = lane < 9 ? 28 + lane : (lane < 13 ? 24 + lane - 9 : (lane == 13 ? 0 : 3));
+    int v = 0, q_nxt = 0, csid = -1;
+    if (sh.nscn == 1) {
+        if (gw < sh.work_cap * PARTS) v = reinterpret_cast<const int*>(sh.desc + gw / PARTS)[word];  // a guess until the count is known
         load_scn_step(sh, 0, zs, lane);
+        csid = 0;
+        __syncwarp();
     }
-    const int nwork = min(*sh.gcount, sh.gcap);
-    const auto [w0, w1, step] = work_items(sh, nwork, gw, gn);
+    const int ntile = sh.work_pref[sh.nscn];
+    const WorkItems W = work_items(sh, (ntile + *sh.xcount) * PARTS, gw, gn);
+    const int w0 = W.w0, w1 = W.w1, step = W.step;
+    auto request = [&](int it) {
+        int w = it / PARTS;
+        q_nxt = 0;
+        if (w >= ntile) {
+            const int e = sh.xlist[w - ntile];
+            w = e >> 2;
+            q_nxt = e & 3;
+        }
+        v = reinterpret_cast<const int*>(sh.desc + w)[word];
+    };
     if (w0 >= w1) return;  // warps run alone: no block barrier below
-    if (sh.nscn != 1) {
-        e = list[w0];
-        if (w0 + step < w1) e_nxt = list[w0 + step];
-    }
-    if (w0 + step >= w1) e_nxt = make_int2(-1, 0);
-    double macc = 0.0;  // mass and active nodes of this lane over the run of one scenario
+    if (sh.nscn != 1 || w0 / PARTS >= ntile) request(w0);
+    double macc = 0.0;
     unsigned nacc = 0;
     auto flush = [&] {
         nacc = __reduce_add_sync(0xffffffffu, nacc);
         for (int o = 16; o > 0; o >>= 1) macc += __shfl_xor_sync(0xffffffffu, macc, o);
         if (lane == 0) {
-            if (macc != 0.0) atomicAdd(&Z.cnt->grid_mass, macc);
-            if (nacc) atomicAdd(&Z.ctl->node_steps, (unsigned long long)nacc);
+            if (macc != 0.0) atomicAdd(&zs.s.cnt->grid_mass, macc);
+            if (nacc) atomicAdd(&zs.s.ctl->node_steps, (unsigned long long)nacc);
         }
         macc = 0.0;
         nacc = 0;
     };
-    // lanes 0-3: slot of covering tile k (gi - (k >> 1), gj - (k & 1)), -1 if it is
-    // not active this step; lane 4: the node block
-    int st_ = -1, sl_ = -1;
-    auto request = [&](int gt) {
-        st_ = -1;
-        sl_ = -1;
-        if (lane < 4) {
-            const int ti_ = gt / sh.TY - (lane >> 1), tj_ = gt % sh.TY - (lane & 1);
-            if (ti_ >= 0 && tj_ >= 0) {
-                const int tt = ti_ * sh.TY + tj_;
-                st_ = Z.act_stamp[tt];
-                sl_ = Z.slot_of[tt];
-            }
-        } else if (lane == 4) {
-            sl_ = Z.blk_of[gt];
-        }
-    };
-    if (sh.nscn == 1) {
-        csid = 0;
-        __syncwarp();
-        request(e.y);
-    }
     for (int w = w0; w < w1; w += step) {
-        if (e.x != csid) {  // a new scenario in this warp's run
+        const int cur = v, q = q_nxt, sid = __shfl_sync(0xffffffffu, cur, 14), t = __shfl_sync(0xffffffffu, cur, 13);
+        if (w + step < w1) request(w + step);
+        if (sid != csid) {  // a new scenario in this warp's run
             if (csid >= 0) flush();
-            csid = e.x;
+            csid = sid;
             __syncwarp();
             load_scn(sh, csid, zs, lane, 32);
             __syncwarp();
-            request(e.y);
         }
-        const int gt = e.y, gi = gt / sh.TY, gj = gt % sh.TY;
-        if (lane == 4) {
-            int blk = sl_;
-            if (blk < 0) {
-                // a block released by a retired scenario, else a fresh one
-                const int f = atomicSub(sh.free_count, 1);
-                if (f > 0) {
-                    blk = sh.free_blocks[f - 1];
-                } else {
-                    atomicAdd(sh.free_count, 1);
-                    blk = atomicAdd(sh.blk_count, 1);
-                }
-                if (blk >= sh.blk_cap) {
-                    atomicOr(&Z.ctl->err, ERR_CAPACITY);
-                    blk = -1;
-                } else {
-                    Z.blk_of[gt] = blk;
-                    sh.blk_owner[blk] = csid;
-                }
-            }
-            if (blk >= 0) sh.blk_stamp[blk] = Y.stepid;
-            sl_ = blk;
+        if (w / PARTS < ntile && w % PARTS == 0 && cur == BLK_LATER && lane >= 9 && lane < 13)  // named now, for G2P
+            sh.desc[w / PARTS].blk4[lane - 9] = zs.s.blk_of[(t / sh.TY + ((lane - 9) >> 1)) * sh.TY + t % sh.TY + ((lane - 9) & 1)];
+        const int c = (w % PARTS) * 32 + lane, li = c / TILE, lj = c % TILE;
+        const int qi = q >> 1, qj = q & 1, gi = t / sh.TY + qi, gj = t % sh.TY + qj;
+        int blk = __shfl_sync(0xffffffffu, cur, 9 + q);
+        if (blk == BLK_LATER) blk = zs.s.blk_of[gi * sh.TY + gj];
+        int slot[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int s = __shfl_sync(0xffffffffu, cur, (qi - (k >> 1) + 1) * 3 + (qj - (k & 1) + 1));
+            slot[k] = covers_node(k, li, lj) ? s : -1;
         }
-        const int slot = lane < 4 ? (st_ == Y.seq ? sl_ : -1) : sl_;
-        const int blk = __shfl_sync(0xffffffffu, slot, 4);
-        int slots[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) slots[k] = __shfl_sync(0xffffffffu, slot, k);
-        // the block of this grid tile is entry k of contributor k's window (for G2P)
-        if (lane < 4 && slot >= 0) sh.desc[slot].blk4[lane] = blk;
-        // the next grid tile's slots and block, and the list entry after it
-        const int2 e_nn = w + 2 * step < w1 ? list[w + 2 * step] : make_int2(-1, 0);
-        if (e_nxt.x == csid) request(e_nxt.y);
-        if (blk >= 0) {
-#pragma unroll
-            for (int u = 0; u < NPL; ++u) {
-                const int c = lane + 32 * u, li = c / TILE, lj = c % TILE;
-                const int i = gi * TILE + li, j = gj * TILE + lj;
-                const size_t bn = (size_t)blk * NCELL + c;
-                const bool inside = i < sh.Nx && j < sh.Ny;
-                // terrain and maxima are requested with the partials (one round of loads)
-                const float4 dm = inside ? sh.dem[(int64_t)i * sh.Ny + j] : make_float4(0.f, 0.f, 1.f, 0.f);
-                const float hmax0 = sh.hmax[bn], vmax0 = sh.vmax2[bn];
-                // the covering tiles' partials, all requested before the first is
-                // added (a branch per tile made them four rounds of loads); one
-                // that does not cover the node adds zero
-                float4 pq[4];
-                float2 pF[4];
-                float pz[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    // tile k: 0 own, 1 -y, 2 -x, 3 -xy
-                    const int a = li + (k >> 1) * TILE, b = lj + (k & 1) * TILE;
-                    const bool covers = slots[k] >= 0 && a < TN && b < TN;
-                    const float* P = sh.part + (size_t)(covers ? slots[k] : 0) * PART_STRIDE;
-                    const int n = covers ? a * TN + b : 0;
-                    pq[k] = covers ? reinterpret_cast<const float4*>(P)[n] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    pF[k] = covers ? reinterpret_cast<const float2*>(P + 4 * NWIN)[n] : make_float2(0.f, 0.f);
-                    pz[k] = covers && Y.outs ? P[6 * NWIN + n] : 0.f;
-                }
-                float2 m2 = make_float2(0.f, 0.f), v2 = m2, F2 = m2;  // m, m h; m v; F
-                float qz = 0.f;
-                constexpr int order[4] = {0, 2, 1, 3};
-#pragma unroll
-                for (int u_ = 0; u_ < 4; ++u_) {
-                    const int k = order[u_];
-                    m2 = f2add(m2, make_float2(pq[k].x, pq[k].y));
-                    v2 = f2add(v2, make_float2(pq[k].z, pq[k].w));
-                    F2 = f2add(F2, pF[k]);
-                    qz += pz[k];
-                }
-                float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
-                float hn = 0.f, vzn = 0.f;
-                const float mi = m2.x;
-                if (mi > 1e-6f && inside) {
-                    const float vox = v2.x / mi, voy = v2.y / mi;
-                    if (Y.outs) vzn = qz / mi;
-                    hn = m2.y / mi;
-                    const float dt = Y.dt;
-                    const float vtx = vox + dt * (F2.x / mi), vty = voy + dt * (F2.y / mi);
-                    const float vsq = vtx * vtx + vty * vty;
-                    float nvx = 0.f, nvy = 0.f;
-                    if (vsq > 1e-16f) {
-                        const float ct = dm.z;
-                        const float vz = vtx * dm.x + vty * dm.y;
-                        const float v3sq = vsq + vz * vz;
-                        const float v3 = sqrtf(v3sq);
-                        const float g = Z.g;
-                        float af;
-                        if (Z.fric == SLAB_COULOMB) {
-                            af = Z.mu_c * g * ct;
-                        } else if (Z.fric == SLAB_VOELLMY) {
-                            af = Z.mu_v * g * ct + g * v3sq / (Z.xi * hn * ct);
-                        } else {
-                            const float I = 5.f * Z.d * v3 / (2.f * hn * ct * ct * sqrtf(g * hn * Z.phi));
-                            const float muI = Z.mu1 + (Z.mu2 - Z.mu1) / (1.f + Z.I0 / I);
-                            af = muI * g * ct;
-                        }
-                        const float dv = dt * af;
-                        if (dv < v3) {
-                            const float fct = 1.f - dv / v3;
-                            nvx = vtx * fct;
-                            nvy = vty * fct;
-                        }
-                    }
-                    out = make_float4(nvx, nvy, nvx - vox, nvy - voy);
-                    sh.hmax[bn] = fmaxf(hmax0, hn);
-                    sh.vmax2[bn] = fmaxf(vmax0, nvx * nvx + nvy * nvy);
-                    macc += (double)mi;
-                    nacc += 1u;
-                }
-                sh.nv[bn] = out;
-                if (Y.outs) {
-                    sh.oh[bn] = hn;
-                    sh.om[bn] = inside ? mi : 0.f;
-                    sh.ovz[bn] = vzn;
-                    sh.oFx[bn] = inside ? F2.x : 0.f;
-                    sh.oFy[bn] = inside ? F2.y : 0.f;
-                }
-            }
-        }
-        e = e_nxt;
-        e_nxt = e_nn;
+        if (blk >= 0) grid_node(sh, zs.s, zs.y, gi, gj, li, lj, slot, blk, macc, nacc);
     }
     flush();
 }
 
-__global__ void __launch_bounds__(GRID_T) k_grid(Shared sh) { grid_body(sh); }
+#ifndef SLAB_GRID_MIN_BLOCKS
+#define SLAB_GRID_MIN_BLOCKS 8
+#endif
+__global__ void __launch_bounds__(GRID_T, SLAB_GRID_MIN_BLOCKS) k_grid(Shared sh) { grid_body(sh); }
 
 // -------------------------------------------------------------------- G2P
 
@@ -1748,27 +1752,47 @@ constexpr int G2P_T = 2 * NCELL;  // threads of a CTA
 #ifndef SLAB_G2P_MIN_BLOCKS
 #define SLAB_G2P_MIN_BLOCKS (NCELL == 64 ? 9 : 2)
 #endif
+#ifndef SLAB_G2P_FUSED_MIN_BLOCKS
+#define SLAB_G2P_FUSED_MIN_BLOCKS (NCELL == 64 ? 7 : 1)
+#endif
 
-// puts tile tt on the next step's active list, once
+// puts tile tt on the next step's active list, once; its place there is also
+// the place of its partial window
 __device__ __forceinline__ void g2p_activate(const ScnSm& z, int tt) {
     const int seq1 = z.y.seq + 1;
-    if (atomicMax(&z.s.act_stamp[tt], seq1) < seq1) {
+    if (atomicMax(&z.s.act[tt].x, seq1) < seq1) {
         const int kk = atomicAdd(&z.s.cnt->act_count[seq1 & 1], 1);
+        z.s.act[tt].y = kk;
         if (kk < z.s.act_cap) z.s.act_list[seq1 & 1][kk] = tt;
         else atomicOr(&z.s.ctl->err, ERR_CAPACITY);
     }
 }
 
-// the largest |v|^2 of a run of tiles into the scenario's control block: one
-// atomic per warp that does not wait for an answer (speeds squared are >= 0,
-// so their bit patterns order like the values)
-__device__ __forceinline__ void g2p_flush_vmax2(const ScnSm& z, float vmax2) {
-    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(vmax2));
-    if ((threadIdx.x & 31) == 0 && m) {
-        const double v = (double)__uint_as_float(m);
-        atomicMax(reinterpret_cast<unsigned long long*>(&z.s.ctl->vmax2_acc), (unsigned long long)__double_as_longlong(v));
+// What a thread gathers over a run of tiles of one scenario: its particles'
+// largest |v|^2, and mass and number of the active nodes it owns (the FP64 grid
+// mass and the node count are diagnostics).
+struct G2PRun {
+    float vmax2 = 0.f;
+    unsigned nodes = 0;
+    double mass = 0.0;
+    // into the scenario's control block: one atomic of each per warp, without
+    // waiting for an answer (speeds squared are >= 0, so their bit patterns
+    // order like the values)
+    __device__ __forceinline__ void flush(const ScnSm& z) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(vmax2));
+        nodes = __reduce_add_sync(0xffffffffu, nodes);
+        for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+        if ((threadIdx.x & 31) == 0) {
+            const double v = (double)__uint_as_float(m);
+            if (m) atomicMax(reinterpret_cast<unsigned long long*>(&z.s.ctl->vmax2_acc), (unsigned long long)__double_as_longlong(v));
+            if (nodes) atomicAdd(&z.s.ctl->node_steps, (unsigned long long)nodes);
+            if (mass != 0.0) atomicAdd(&z.s.cnt->grid_mass, mass);
+        }
+        vmax2 = 0.f;
+        nodes = 0;
+        mass = 0.0;
     }
-}
+};
 
 template <int T> struct G2PSmem {
     float4 nv[NWIN];
@@ -1801,20 +1825,26 @@ __device__ __forceinline__ G2PCand load_g2p_cand(const TileDesc& D, const PBuf& 
     return q;
 }
 
-// K4: G2P (src/simulation.cpp:877-940) of one tile: FLIP/PIC blend,
+// K4, one CTA per tile. FUSED, for steps of few tiles: K3 and K6 first, the grid
+// update of the tile's node window into shared memory (window_node). 100 nodes
+// for 64 cells, nodes near an edge computed by up to 4 tiles, but no kernel of
+// its own between P2G and G2P: per step 22 -> 18.5 us at 1 600 particles, 30 ->
+// 27 at 180 k (734 tiles); at 2 M particles (8 000 tiles) the pass through
+// memory is the cheaper one, 129 against 140 us. Otherwise the window comes from the node blocks.
+// Then G2P (src/simulation.cpp:877-940): FLIP/PIC blend,
 // advection, depth update, and the write of the particle into the tile's
 // segment of the next buffer -- stayers from the front, particles that moved
 // to a neighbour tile from the back, with per-direction counts. The max of
 // |v|^2 and the particle bounding box feed the next step's dt and remesh box
 // (K5). A particle is two 16-byte loads and two 16-byte stores; a thread
 // holds its candidate of this chunk and of the next in registers, so the
-// loads of a chunk go out with the node window's (asynchronous copies into
-// shared memory) or while the chunk before it is computed. The scenario's
+// loads of a chunk go out with the node window's or while the chunk before it
+// is computed. The scenario's
 // values stay in shared memory across a run of its tiles, the next tile's
 // descriptor is requested while this one runs, and a tile's neighbour
 // activations (two dependent atomics) are issued while the next tile's loads
 // are in flight.
-template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restrict__ z64, G2PSmem<T>& sm) {
+template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restrict__ z64, G2PSmem<T>& sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int dn = 0;
     const bool words = tid < DESC_WORDS;
@@ -1823,10 +1853,11 @@ template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, cons
     chain_wait<true>();
     if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
     if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
-    const auto [w0, w1, step] = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
+    const WorkItems W = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
+    const int w0 = W.w0, w1 = W.w1, step = W.step;
     if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
     int pend_tt = -1;    // threads 0..8: neighbour tile the previous tile activates
-    float vmax2 = 0.f;   // largest |v|^2 of this thread's particles over the CTA's run of one scenario
+    G2PRun run;
     for (int w = w0; w < w1; w += step) {
         __syncthreads();  // the tile before is done with the shared memory
         if (words) reinterpret_cast<int*>(&sm.d)[tid] = dn;
@@ -1836,30 +1867,25 @@ template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, cons
         if (sm.d.sid != sm.z.sid) {  // uniform: a new scenario in this CTA's run
             if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);
             pend_tt = -1;
-            if (w > w0) g2p_flush_vmax2(sm.z, vmax2);
-            vmax2 = 0.f;
+            if (w > w0) run.flush(sm.z);
             __syncthreads();
             load_scn(sh, sm.d.sid, sm.z, tid, T);
             __syncthreads();
         }
         const ScnSm& Z = sm.z;
+        const TileDesc& D = sm.d;
         Ctl* c = Z.s.ctl;
-        const int t = sm.d.t;
+        const int t = D.t;
         const int ti = t / sh.TY, tj = t % sh.TY;
         const bool outs = Z.y.outs != 0;
         const bool need_vz = Z.y.need_vz != 0;
-        const int ncand = sm.d.rpref[9];
+        const int ncand = D.rpref[9];
         // the first candidates, the node window and the terrain in one round
+        // (requested while the tile before ran, they took as long: the kernel is
+        // bound by instruction issue, and the second window's shared memory and
+        // the longer-lived registers cost what the wait did)
         SLAB_PHASE_BEGIN;
-        G2PCand nxt = load_g2p_cand(sm.d, Z.cur(), tid, ncand);
-        // a part of the window whose grid tile has no block this step (or past the terrain edge) is zero
-        for (int k = tid; k < NWIN; k += T) {
-            const int a = k / TN, b = k % TN;
-            const int i = ti * TILE + a, j = tj * TILE + b;
-            const int blk = (i < sh.Nx && j < sh.Ny) ? sm.d.blk4[(a >= TILE ? 2 : 0) + (b >= TILE ? 1 : 0)] : -1;
-            if (blk >= 0) cpa::copy16(&sm.nv[k], &sh.nv[(size_t)blk * NCELL + (a % TILE) * TILE + (b % TILE)]);
-            else sm.nv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        G2PCand nxt = load_g2p_cand(D, Z.cur(), tid, ncand);
         if (need_vz) {
             for (int k = tid; k < (TILE + 1) * (TILE + 1); k += T) {
                 const int i = ti * TILE + k / (TILE + 1), j = tj * TILE + k % (TILE + 1);
@@ -1869,12 +1895,22 @@ template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, cons
         }
         if (pend_tt >= 0) g2p_activate(Z, pend_tt);  // the previous tile's, while the loads above are in flight
         pend_tt = -1;
+        for (int k = tid; k < NWIN; k += T) {
+            if constexpr (FUSED) {
+                sm.nv[k] = window_node(sh, Z.s, Z.y, D, k, run.mass, run.nodes);
+            } else {
+                // a part of the window whose grid tile has no block (past the terrain edge) is zero
+                const int a = k / TN, b = k % TN;
+                const int blk = ti * TILE + a < sh.Nx && tj * TILE + b < sh.Ny ? D.blk4[(a >= TILE ? 2 : 0) + (b >= TILE ? 1 : 0)] : -1;
+                if (blk >= 0) cpa::copy16(&sm.nv[k], &sh.nv[(size_t)blk * NCELL + (a % TILE) * TILE + (b % TILE)]);
+                else sm.nv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
         SLAB_PHASE_MARK(8);
         cpa::wait_all();
         __syncthreads();
         SLAB_PHASE_MARK(9);
-        const int total = sm.d.total;
-        const int base = sm.d.nxt_off;
+        const int total = D.total, base = D.nxt_off;
         const bool edge = ti < Z.y.in_i0 || ti > Z.y.in_i1 || tj < Z.y.in_j0 || tj > Z.y.in_j1;  // uniform: may change the particle box
         const bool inner = (ti + 1) * TILE + 1 <= sh.Nx - 1 && (tj + 1) * TILE + 1 <= sh.Ny - 1;  // uniform
         double mnx = INFINITY, mxx = 0.0, mny = INFINITY, mxy = 0.0;
@@ -1882,7 +1918,7 @@ template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, cons
         for (int k0 = 0; k0 < ncand; k0 += T) {
             // this chunk's candidate, and the next chunk's requested before this one is computed
             const G2PCand q = nxt;
-            if (k0 + T < ncand) nxt = load_g2p_cand(sm.d, Z.cur(), k0 + T + tid, ncand);
+            if (k0 + T < ncand) nxt = load_g2p_cand(D, Z.cur(), k0 + T + tid, ncand);
             const int32_t cell = __float_as_int(q.b.z);
             const int ci = cell_i(cell) - ti * TILE, cj = cell_j(cell) - tj * TILE;
             const bool valid = q.there && (unsigned)ci < TILE && (unsigned)cj < TILE;
@@ -1955,7 +1991,7 @@ template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, cons
                     mny = fmin(mny, py);
                     mxy = fmax(mxy, py);
                 }
-                vmax2 = fmaxf(vmax2, vn.x * vn.x + vn.y * vn.y);
+                run.vmax2 = fmaxf(run.vmax2, vn.x * vn.x + vn.y * vn.y);
                 // 0 unless one of them is infinite or NaN
                 const float bad = fmaf(vn.x, 0.f, fmaf(vn.y, 0.f, fmaf(hn, 0.f, fmaf(fn.x, 0.f, fn.y * 0.f))));
                 if (bad != 0.f) atomicOr(&c->err, ERR_NONFINITE);
@@ -2041,13 +2077,14 @@ template <int T> __device__ __forceinline__ void g2p_body(const Shared& sh, cons
         SLAB_PHASE_MARK(11);
         SLAB_PHASE_TILE_G2P();
     }
-    if (w0 < w1) g2p_flush_vmax2(sm.z, vmax2);
+    if (w0 < w1) run.flush(sm.z);
     if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);  // the last tile's
 }
 
-__global__ void __launch_bounds__(G2P_T, SLAB_G2P_MIN_BLOCKS) k_g2p(Shared sh, const double* __restrict__ z64) {
+template <bool FUSED>
+__global__ void __launch_bounds__(G2P_T, FUSED ? SLAB_G2P_FUSED_MIN_BLOCKS : SLAB_G2P_MIN_BLOCKS) k_g2p(Shared sh, const double* __restrict__ z64) {
     __shared__ G2PSmem<G2P_T> sm;
-    g2p_body<G2P_T>(sh, z64, sm);
+    g2p_body<G2P_T, FUSED>(sh, z64, sm);
 }
 
 // K5: end of the step for every running scenario (the per-step reductions
@@ -2113,8 +2150,8 @@ __device__ __forceinline__ bool grid_sync(const Shared& sh, GridBar* bar, long l
 // every phase (each phase initialises what it reads).
 constexpr size_t PERSIST_SMEM = sizeof(P2GTileSmem) > sizeof(G2PSmem<P2G_T>) ? sizeof(P2GTileSmem) : sizeof(G2PSmem<P2G_T>);
 
-// Up to nsteps whole steps (K1 tile bookkeeping, K2 P2G, K3 grid update, K4
-// G2P, K5 end of step) in one launch, the phases separated by grid_sync
+// Up to nsteps whole steps (K1 tile bookkeeping, K2 P2G, K3 grid update and
+// K4 G2P, K5 end of step) in one launch, the phases separated by grid_sync
 // instead of kernel boundaries. The same phase bodies as the separate kernels,
 // over the same work lists and in the same per-tile order, so a step gives
 // the same bits either way. The launch ends early once no scenario has work
@@ -2130,9 +2167,7 @@ __global__ void __launch_bounds__(P2G_T, SLAB_P2G_MIN_BLOCKS) k_persist(Shared s
         if (!grid_sync(sh, bar, limit)) return;
         p2g_tiles_body(sh, smem_raw, &dem_map);
         if (!grid_sync(sh, bar, limit)) return;
-        grid_body(sh);
-        if (!grid_sync(sh, bar, limit)) return;
-        g2p_body<P2G_T>(sh, z64, *reinterpret_cast<G2PSmem<P2G_T>*>(smem_raw));
+        g2p_body<P2G_T, true>(sh, z64, *reinterpret_cast<G2PSmem<P2G_T>*>(smem_raw));
         if (!grid_sync(sh, bar, limit)) return;
         if (blockIdx.x == 0) control_scenarios(sh, CTL_END);
         if (!grid_sync(sh, bar, limit)) return;
