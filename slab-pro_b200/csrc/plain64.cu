@@ -74,9 +74,25 @@ __device__ __forceinline__ void stencil_weights(const Phys& P, double xp, int ba
     }
 }
 
-__global__ void k64_begin(Ctl* c, int Nx, int Ny) {
+// Control of a step, after its G2P: the step's end, then the start of the next
+// one; arm: the start of an advance call instead (its budget and frame stop).
+// One thread, with the control block in registers: read and written once. (As
+// G2P's last block and a kernel before P2G, field by field, the two took 3 us
+// of a 22 us step at 1 600 particles.)
+__global__ void k64_control(Ctl* c, int Nx, int Ny, int arm, int64_t steps_left, int stop_at_frame) {
     chain_wait<true>();
-    if (threadIdx.x == 0 && blockIdx.x == 0) ctl_begin(c, Nx, Ny);
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    Ctl k = *c;
+    if (arm) {
+        k.stop = 0;
+        k.frame_hit = 0;
+        k.steps_left = steps_left;
+        k.stop_at_frame = stop_at_frame;
+    } else if (k.active) {
+        ctl_end(&k);
+    }
+    ctl_begin(&k, Nx, Ny);
+    *c = k;
 }
 __global__ void k64_begin_t0(Ctl* c, int Nx, int Ny) {
     if (threadIdx.x == 0 && blockIdx.x == 0) ctl_begin_t0(c, Nx, Ny);
@@ -84,6 +100,11 @@ __global__ void k64_begin_t0(Ctl* c, int Nx, int Ny) {
 
 // P2G (src/simulation.cpp:726-798) with atomicAdd(double) scatter. Slope
 // terms of the particle's containing cell (src/complex_terrain.cpp:113-130).
+// The atomics bound it (L2 at 71 % of its peak, 2 M particles 238 us), so the
+// sum of m vz, which only output fields use, is left out of the other steps.
+// (Summing each 8 x 8-cell tile of periodically ordered particles in shared
+// memory first, 3 atomics per particle instead of 63, was bound by FP64
+// issue: 218 us, and 354 instead of 134 us where cells hold 4 to 15 particles.)
 __global__ void __launch_bounds__(256) k64_p2g(const Ctl* c, P64 p, N64 n, const double2* __restrict__ grad,
                                                const double* __restrict__ cos_t, Phys P, int Np) {
     chain_wait<true>();
@@ -91,8 +112,9 @@ __global__ void __launch_bounds__(256) k64_p2g(const Ctl* c, P64 p, N64 n, const
     if (q >= Np || !c->active) return;
     const double2 x = p.x[q], v = p.v[q];
     const double h = p.h[q], A = p.A[q], m = p.m[q];
+    const bool outs = c->write_outputs;
     const double vmx = v.x * m, vmy = v.y * m;
-    const double vzm = p.vz[q] * m, hm = h * m, hA = h * A;
+    const double vzm = outs ? p.vz[q] * m : 0.0, hm = h * m, hA = h * A;
     const int ib = (int)floor(x.x * P.one_over_dx - 0.5), jb = (int)floor(x.y * P.one_over_dx - 0.5);
     const int cell = (int)floor(x.x * P.one_over_dx) * P.Ny + (int)floor(x.y * P.one_over_dx);
     const double2 gr = grad[cell];
@@ -114,7 +136,7 @@ __global__ void __launch_bounds__(256) k64_p2g(const Ctl* c, P64 p, N64 n, const
                 atomicAdd(n.m + k, m * w);
                 atomicAdd(n.px + k, vmx * w);
                 atomicAdd(n.py + k, vmy * w);
-                atomicAdd(n.pvz + k, vzm * w);
+                if (outs) atomicAdd(n.pvz + k, vzm * w);
                 atomicAdd(n.hm + k, hm * w);
                 atomicAdd(n.Fx + k, mbx * w - hA * (s00 * gwx + 0.0 * gwy));
                 atomicAdd(n.Fy + k, mby * w - hA * (s00 * gwy + 0.0 * gwx));
@@ -182,7 +204,7 @@ __global__ void __launch_bounds__(256) k64_grid(Ctl* c, N64 n, const double2* __
         double hn = 0.0, vzn = 0.0;
         if (mi > 1e-6) {
             const double vox = n.px[k] / mi, voy = n.py[k] / mi;
-            vzn = n.pvz[k] / mi;
+            if (outs) vzn = n.pvz[k] / mi;
             hn = n.hm[k] / mi;
             const double ax = n.Fx[k] / mi, ay = n.Fy[k] / mi;
             const double vtx = vox + dt * ax, vty = voy + dt * ay;
@@ -227,7 +249,7 @@ __global__ void __launch_bounds__(256) k64_grid(Ctl* c, N64 n, const double2* __
         n.m[k] = 0.0;
         n.px[k] = 0.0;
         n.py[k] = 0.0;
-        n.pvz[k] = 0.0;
+        if (outs) n.pvz[k] = 0.0;
         n.hm[k] = 0.0;
         n.Fx[k] = 0.0;
         n.Fy[k] = 0.0;
@@ -238,9 +260,12 @@ __global__ void __launch_bounds__(256) k64_grid(Ctl* c, N64 n, const double2* __
 
 __device__ __forceinline__ uint64_t dbits(double v) { return (uint64_t)__double_as_longlong(v); }
 
-// Block-reduce the particle bounding box and max |v|^2 into the control
-// block; the last block to finish closes the step.
-__device__ void block_epilogue(Ctl* c, bool valid, double px, double py, double v2, bool close_step) {
+// Block-reduce the particle bounding box and max |v|^2 into the control block,
+// by atomics that no one waits for. (With the last block, found by a fence and
+// a counter, closing the step here, G2P took 138 us for 2 M particles instead
+// of 116; skipping atomics that cannot widen the box costs more registers than
+// the atomics.)
+__device__ void block_epilogue(Ctl* c, bool valid, double px, double py, double v2) {
     __shared__ double s_red[5][8];
     double mnx = valid ? px : INFINITY, mxx = valid ? px : 0.0, mny = valid ? py : INFINITY, mxy = valid ? py : 0.0;
     double vv = valid ? v2 : 0.0;
@@ -271,14 +296,6 @@ __device__ void block_epilogue(Ctl* c, bool valid, double px, double py, double 
         atomicMin(reinterpret_cast<unsigned long long*>(&c->pos_acc[2]), (unsigned long long)dbits(mny));
         atomicMax(reinterpret_cast<unsigned long long*>(&c->pos_acc[3]), (unsigned long long)dbits(mxy));
         atomicMax(reinterpret_cast<unsigned long long*>(&c->vmax2_acc), (unsigned long long)dbits(vv));
-        if (close_step) {
-            __threadfence();
-            const unsigned prev = atomicAdd(&c->done_blocks, 1u);
-            if (prev == gridDim.x - 1) {
-                __threadfence();
-                ctl_end(c);
-            }
-        }
     }
 }
 
@@ -334,7 +351,7 @@ __global__ void __launch_bounds__(256) k64_g2p(Ctl* c, P64 p, N64 n, const doubl
         if (!isfinite(nx.x) || !isfinite(nx.y) || !isfinite(v2) || !isfinite(hn)) atomicOr(&c->err, ERR_NONFINITE);
         if (nx.x < 0.0 || nx.y < 0.0) atomicOr(&c->err, ERR_DOMAIN);
     }
-    block_epilogue(c, valid, nx.x, nx.y, v2, true);
+    block_epilogue(c, valid, nx.x, nx.y, v2);
 }
 
 // Particle box and max |v|^2 of freshly uploaded particles.
@@ -349,7 +366,7 @@ __global__ void k64_stats(Ctl* c, P64 p, int Np) {
         v2 = v.x * v.x + v.y * v.y;
         if (x.x < 0.0 || x.y < 0.0) atomicOr(&c->err, ERR_DOMAIN);
     }
-    block_epilogue(c, valid, x.x, x.y, v2, false);
+    block_epilogue(c, valid, x.x, x.y, v2);
 }
 
 struct Plain64 final : Path {
@@ -392,6 +409,8 @@ struct Plain64 final : Path {
         gv = dalloc<double2>(nn);
         gflip = dalloc<double2>(nn);
         out5 = dalloc<double>(5 * nn);
+        const int phase_map[4] = {2, 3, 4, 0};  // P2G, grid update, G2P, control
+        std::copy(phase_map, phase_map + 4, timer.phase_of);
         maxes = dalloc<double>(2 * nn);
         clear_nodes();
     }
@@ -448,16 +467,22 @@ struct Plain64 final : Path {
         SLAB_CUDA(cudaMemcpyAsync(&dc->vmax2_bits, &dc->vmax2_acc, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
     }
     bool reusable() const override { return true; }
+    bool arm(int64_t steps_left, int stop_at_frame) override {
+        k64_control<<<1, 32, 0, st>>>(dc, T.Nx, T.Ny, 1, steps_left, stop_at_frame);
+        SLAB_CUDA(cudaGetLastError());
+        ++nlaunch;
+        return true;
+    }
 
     int grid_blocks() const { return 148 * 4; }
 
     void launch_kernel(int k) {
         const int pb = (Np + 255) / 256;
         switch (k) {
-            case 0: launch_chained(st, 1, 32, 0, k64_begin, dc, T.Nx, T.Ny); break;
-            case 1: launch_chained(st, pb, 256, 0, k64_p2g, dc, parts(), nodes(), T.grad.get(), T.cos_t.get(), P, Np); break;
-            case 2: launch_chained(st, grid_blocks(), 256, 0, k64_grid, dc, nodes(), T.grad.get(), T.cos_t.get(), P); break;
-            case 3: launch_chained(st, pb, 256, 0, k64_g2p, dc, parts(), nodes(), T.grad.get(), T.z.get(), P, Np); break;
+            case 0: launch_chained(st, pb, 256, 0, k64_p2g, dc, parts(), nodes(), T.grad.get(), T.cos_t.get(), P, Np); break;
+            case 1: launch_chained(st, grid_blocks(), 256, 0, k64_grid, dc, nodes(), T.grad.get(), T.cos_t.get(), P); break;
+            case 2: launch_chained(st, pb, 256, 0, k64_g2p, dc, parts(), nodes(), T.grad.get(), T.z.get(), P, Np); break;
+            case 3: launch_chained(st, 1, 32, 0, k64_control, dc, T.Nx, T.Ny, 0, (int64_t)0, 0); break;
         }
     }
     void launch_step() {
@@ -466,8 +491,7 @@ struct Plain64 final : Path {
 
     void initial_pass() override {
         k64_begin_t0<<<1, 32, 0, st>>>(dc, T.Nx, T.Ny);
-        k64_p2g<<<(Np + 255) / 256, 256, 0, st>>>(dc, parts(), nodes(), T.grad.get(), T.cos_t.get(), P, Np);
-        k64_grid<<<grid_blocks(), 256, 0, st>>>(dc, nodes(), T.grad.get(), T.cos_t.get(), P);
+        for (int k = 0; k < 2; ++k) launch_kernel(k);
         SLAB_CUDA(cudaGetLastError());
         nlaunch += 3;
     }
