@@ -91,7 +91,8 @@ struct TileDesc {
     int32_t fresh;    // bit k > 0: grid tile k of the node window is no particle tile of this step, and this tile is the first to touch it
     int32_t blk4[4];  // node blocks of the window's grid tiles (own, +y, +x, +xy); -1: off the terrain, BLK_LATER: look it up
     int32_t nb[9];    // partial windows of the 3 x 3 tiles around t active this step (-1: not active)
-    int32_t pad_[3];
+    int32_t tij;      // t's row and column, as pack_cell (a division per tile and thread otherwise)
+    int32_t pad_[2];
 };
 constexpr int BLK_LATER = -2;  // the block was being allocated while the descriptor was written (a grid tile's first step)
 static_assert(sizeof(TileDesc) % 16 == 0, "descriptors lie on 16-byte boundaries");

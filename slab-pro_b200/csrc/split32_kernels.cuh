@@ -320,7 +320,7 @@ constexpr int PREP_LANES = 16;
 constexpr int PREP_THREADS = 256;
 constexpr int PREP_MAX_TILES = 1024 / PREP_LANES;  // tiles of one block pass (the persistent kernel runs larger blocks)
 static_assert(offsetof(TileDesc, rstart) == 4 * 4 && offsetof(TileDesc, rpref) == 13 * 4 && offsetof(TileDesc, fresh) == 23 * 4 &&
-                  offsetof(TileDesc, nb) == 28 * 4,
+                  offsetof(TileDesc, nb) == 28 * 4 && offsetof(TileDesc, tij) == 37 * 4,
               "k_prep writes the descriptor word by word");
 
 __device__ __forceinline__ void prep_body(const Shared& sh) {
@@ -499,6 +499,7 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
                 D[1] = cnt;
                 D[2] = nxt_off;
                 D[3] = sid;
+                D[37] = pack_cell(ti, tj);
             }
         }
     }
@@ -532,7 +533,7 @@ __device__ __forceinline__ void part_slot(int k, int& q, int& node) {
 // A grid tile's node block, looked up where k_prep could not name it yet.
 __device__ __forceinline__ int node_block(const Shared& sh, const Scn& S, const TileDesc& D, int k) {
     const int blk = D.blk4[k];
-    return blk != BLK_LATER ? blk : S.blk_of[(D.t / sh.TY + (k >> 1)) * sh.TY + D.t % sh.TY + (k & 1)];
+    return blk != BLK_LATER ? blk : S.blk_of[(cell_i(D.tij) + (k >> 1)) * sh.TY + cell_j(D.tij) + (k & 1)];
 }
 
 // Clears the nodes of the grid tiles that are no particle tiles of this step
@@ -1086,7 +1087,7 @@ __device__ __forceinline__ void p2g_request(P2GTileSmem& sm, const Shared& sh, c
         // them (its stencil lies inside the terrain).
         tma::fence_proxy_async();
         tma::mbar_arrive_expect_tx(&sm.dem_bar, (TILE + 1) * (TILE + 1) * 16);
-        tma::tensor_g2s_2d(sm.dem, dem_map, 4 * (D.t % sh.TY) * TILE, (D.t / sh.TY) * TILE, &sm.dem_bar);
+        tma::tensor_g2s_2d(sm.dem, dem_map, 4 * cell_j(D.tij) * TILE, cell_i(D.tij) * TILE, &sm.dem_bar);
     }
 }
 
@@ -1519,7 +1520,7 @@ __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* 
         if (D.fresh) p2g_clear_fresh(sh, sm.z.s, D, sm.z.y.outs != 0, tid, P2G_T);
         cpa::wait_all();
         float* part = sh.part + (size_t)w * PART_STRIDE;
-        const TileOrigin o{(D.t / sh.TY) * TILE, (D.t % sh.TY) * TILE};
+        const TileOrigin o{cell_i(D.tij) * TILE, cell_j(D.tij) * TILE};
         if (D.total <= sh.split_min) {
             __syncthreads();  // the sums share memory with the row sums of the tile before
             p2g_sparse_tile(sm, D, part, dem_phase, o, request_next);
@@ -1652,7 +1653,7 @@ __device__ __forceinline__ float4 window_node(const Shared& sh, const Scn& Z, co
         if (slot[k] >= 0 && first < 0) first = k;
     }
     const int blk = first == 2 * qi + qj ? node_block(sh, Z, D, 2 * qi + qj) : -1;
-    return grid_node(sh, Z, Y, D.t / sh.TY + qi, D.t % sh.TY + qj, li, lj, slot, blk, macc, nacc);
+    return grid_node(sh, Z, Y, cell_i(D.tij) + qi, cell_j(D.tij) + qj, li, lj, slot, blk, macc, nacc);
 }
 
 // K3 + K6 as a kernel of its own, for steps of many tiles: a warp per 32 nodes
@@ -1672,8 +1673,8 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
     const int gw = (int)blockIdx.x * nwarp + warp, gn = (int)gridDim.x * nwarp;
     if (sh.nscn == 1) load_scn_static(sh, 0, zs, lane, 32);
     chain_wait<false>();
-    // lane's word of a descriptor: nb, blk4, then t, sid
-    const int word = lane < 9 ? 28 + lane : (lane < 13 ? 24 + lane - 9 : (lane == 13 ? 0 : 3));
+    // lane's word of a descriptor: nb, blk4, then tij, sid
+    const int word = lane < 9 ? 28 + lane : (lane < 13 ? 24 + lane - 9 : (lane == 13 ? 37 : 3));
     int v = 0, q_nxt = 0, csid = -1;
     if (sh.nscn == 1) {
         if (gw < sh.work_cap * PARTS) v = reinterpret_cast<const int*>(sh.desc + gw / PARTS)[word];  // a guess until the count is known
@@ -1709,7 +1710,7 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
         nacc = 0;
     };
     for (int w = w0; w < w1; w += step) {
-        const int cur = v, q = q_nxt, sid = __shfl_sync(0xffffffffu, cur, 14), t = __shfl_sync(0xffffffffu, cur, 13);
+        const int cur = v, q = q_nxt, sid = __shfl_sync(0xffffffffu, cur, 14), tij = __shfl_sync(0xffffffffu, cur, 13);
         if (w + step < w1) request(w + step);
         if (sid != csid) {  // a new scenario in this warp's run
             if (csid >= 0) flush();
@@ -1719,9 +1720,9 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
             __syncwarp();
         }
         if (w / PARTS < ntile && w % PARTS == 0 && cur == BLK_LATER && lane >= 9 && lane < 13)  // named now, for G2P
-            sh.desc[w / PARTS].blk4[lane - 9] = zs.s.blk_of[(t / sh.TY + ((lane - 9) >> 1)) * sh.TY + t % sh.TY + ((lane - 9) & 1)];
+            sh.desc[w / PARTS].blk4[lane - 9] = zs.s.blk_of[(cell_i(tij) + ((lane - 9) >> 1)) * sh.TY + cell_j(tij) + ((lane - 9) & 1)];
         const int c = (w % PARTS) * 32 + lane, li = c / TILE, lj = c % TILE;
-        const int qi = q >> 1, qj = q & 1, gi = t / sh.TY + qi, gj = t % sh.TY + qj;
+        const int qi = q >> 1, qj = q & 1, gi = cell_i(tij) + qi, gj = cell_j(tij) + qj;
         int blk = __shfl_sync(0xffffffffu, cur, 9 + q);
         if (blk == BLK_LATER) blk = zs.s.blk_of[gi * sh.TY + gj];
         int slot[4];
@@ -1875,8 +1876,7 @@ template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shar
         const ScnSm& Z = sm.z;
         const TileDesc& D = sm.d;
         Ctl* c = Z.s.ctl;
-        const int t = D.t;
-        const int ti = t / sh.TY, tj = t % sh.TY;
+        const int t = D.t, ti = cell_i(D.tij), tj = cell_j(D.tij);
         const bool outs = Z.y.outs != 0;
         const bool need_vz = Z.y.need_vz != 0;
         const int ncand = D.rpref[9];
