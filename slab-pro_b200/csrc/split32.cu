@@ -233,7 +233,7 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     d_oFy = dalloc<float>((size_t)this->blk_cap * NCELL);
     d_blk_stamp = dalloc<int32_t>(this->blk_cap);
     d_blk_owner = dalloc<int32_t>(this->blk_cap);
-    d_misc = dalloc<int32_t>(8);
+    d_misc = dalloc<int32_t>(16);
     d_work_pref = dalloc<int32_t>(max_scn + 1);
     d_scn = dalloc<Scn>(max_scn);
     d_cnt = dalloc<SCnt>(max_scn);
@@ -246,7 +246,7 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     SLAB_CUDA(cudaMemsetAsync(d_hmax.get(), 0, (size_t)this->blk_cap * NCELL * sizeof(float), st));
     SLAB_CUDA(cudaMemsetAsync(d_vmax2.get(), 0, (size_t)this->blk_cap * NCELL * sizeof(float), st));
     SLAB_CUDA(cudaMemsetAsync(d_blk_stamp.get(), 0xff, (size_t)this->blk_cap * sizeof(int32_t), st));
-    SLAB_CUDA(cudaMemsetAsync(d_misc.get(), 0, 8 * sizeof(int32_t), st));
+    SLAB_CUDA(cudaMemsetAsync(d_misc.get(), 0, 16 * sizeof(int32_t), st));
     SLAB_CUDA(cudaMemsetAsync(d_work_pref.get(), 0, (max_scn + 1) * sizeof(int32_t), st));
     host_scn.resize(max_scn);
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g<k32::ACC_I32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GSmem)));
@@ -342,8 +342,10 @@ Shared Engine32::shared() const {
     sh.desc = d_desc.get();
     sh.part = d_part.get();
     sh.xlist = d_xlist.get();
-    sh.xcount = d_misc.get() + 6;
+    static_assert(NLISTCNT <= 8);
+    sh.lists = d_misc.get() + 8;
     sh.use_xlist = fused() ? 0 : 1;
+    sh.p2g_ctas = tune.base[1];
     sh.work_cap = work_cap;
     sh.free_blocks = d_free_blocks.get();
     sh.free_count = d_misc.get() + 4;

@@ -57,8 +57,9 @@ __device__ __forceinline__ int32_t p_id(const PBuf& B, int q) { return reinterpr
 
 // Per-scenario counters (device).
 struct SCnt {
+    int64_t cursor;        // low 32 bits: particles placed in the next buffer; then two 16-bit counts: descriptors placed
+                           // from the front and from the back of the order of work (ordered_by_size)
     int32_t act_count[2];  // active tiles of the list of each parity
-    int32_t cursor;        // particles placed in the next buffer
     int32_t seq;           // completed G2P passes (buffer parity = seq & 1)
     int32_t stepid;        // P2G passes so far (stamps grid tiles / blocks)
     int32_t vz_next;       // the running G2P must store vz (a frame may follow)
@@ -92,7 +93,8 @@ struct TileDesc {
     int32_t blk4[4];  // node blocks of the window's grid tiles (own, +y, +x, +xy); -1: off the terrain, BLK_LATER: look it up
     int32_t nb[9];    // partial windows of the 3 x 3 tiles around t active this step (-1: not active)
     int32_t tij;      // t's row and column, as pack_cell (a division per tile and thread otherwise)
-    int32_t pad_[2];
+    int32_t slot;     // the tile's place on the active list: that of its partial window
+    int32_t pad_;
 };
 constexpr int BLK_LATER = -2;  // the block was being allocated while the descriptor was written (a grid tile's first step)
 static_assert(sizeof(TileDesc) % 16 == 0, "descriptors lie on 16-byte boundaries");
@@ -125,6 +127,11 @@ struct alignas(16) Scn {
     int32_t pad_;
 };
 
+// Counters of a step over all tiles, zeroed at its start: entries of xlist; of
+// one scenario, descriptors placed from the front and from the back of the
+// order of work, and tiles taken from it by P2G and by G2P.
+enum : int { LIST_X = 0, LIST_P2G = 1, LIST_G2P = 2, NLISTCNT = 3 };
+
 // Shared by all scenarios of a context: terrain and node-block pool.
 struct Shared {
     int32_t Nx, Ny, TX, TY;
@@ -154,9 +161,9 @@ struct Shared {
     TileDesc* desc;       // [work_cap] descriptors of the running step
     float* part;          // [work_cap][PART_STRIDE] P2G partial sums
     int32_t* xlist;       // [3 work_cap] grid tiles of the step without particles of their own: work item << 2 | k (TileDesc::fresh)
-    int32_t* xcount;      // their count
+    int32_t* lists;       // [NLISTCNT] counters of the running step, see LIST_X
     int32_t use_xlist;    // the step has a grid update of its own
-    int32_t pad2_;
+    int32_t p2g_ctas;     // CTAs of P2G that the device holds at once
     int32_t work_cap;
     int32_t pad_;
     int32_t* free_blocks; // node blocks released by retired scenarios

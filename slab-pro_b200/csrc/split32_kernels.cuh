@@ -154,7 +154,7 @@ __device__ __forceinline__ int step_control(const Shared& sh, int s, int what, i
         k.stop_at_frame = stop_at_frame;
     }
     if (what == CTL_END && k.active) {
-        if (n.cursor != Np) k.err |= ERR_CAPACITY;
+        if ((int32_t)n.cursor != Np) k.err |= ERR_CAPACITY;
         ctl_end(&k);
         n.seq += 1;
         n.vz_valid = n.outs;
@@ -237,7 +237,7 @@ __device__ __forceinline__ void control_scenarios(const Shared& sh, int what, in
     }
     if (tid == 0) {
         sh.work_pref[sh.nscn] = min(total, sh.work_cap);
-        *sh.xcount = 0;
+        for (int k = 0; k < NLISTCNT; ++k) sh.lists[k] = 0;
         if (total > sh.work_cap) atomicOr(&sh.ctl[0].err, ERR_CAPACITY);
     }
 }
@@ -294,7 +294,8 @@ __device__ __forceinline__ void load_scn(const Shared& sh, int sid, ScnSm& z, in
 // consecutive items mostly belong to the same scenario. Of one scenario it
 // takes every n-th item: the list is roughly in the order of space, so runs of
 // it are all dense tiles for one worker and all sparse ones for the next (300 k
-// particles in a thin tongue: P2G 62 us with runs, 49 us with strides).
+// particles in a thin tongue: P2G 62 us with runs, 49 us with strides). P2G and
+// G2P leave this order in some steps, see many_rounds.
 struct WorkItems {
     int w0, w1, step;
 };
@@ -304,6 +305,28 @@ __device__ __forceinline__ WorkItems work_items(const Shared& sh, int nwork, int
     const int w0 = min(me * per, nwork);
     return {w0, min(w0 + per, nwork), 1};
 }
+
+// Steps of one scenario whose descriptors k_prep orders by size: tiles with more
+// than 5/4 of the mean particle count from the front, the others from the back.
+// These are steps of a few tiles per P2G CTA (more than one, at most about 5),
+// where the heaviest tiles decide when the last CTA is done: 637 k particles in
+// 1 905 tiles of 1 to 980, P2G 44 us in list order, 39 us so. Longer steps keep
+// the list order, which is that of space: ordered, 12 M particles (47 k tiles)
+// took 72 us instead of 69 in the grid update and 25 instead of 21 in k_prep.
+__device__ __forceinline__ bool ordered_by_size(const Shared& sh, int nwork) {
+    return sh.nscn == 1 && !sh.use_xlist && nwork > sh.p2g_ctas && nwork < (1 << 16);
+}
+
+// Steps of one scenario in which a CTA takes, after its first tile, the next
+// one that no CTA has taken, instead of every gridDim.x-th: ordered ones (P2G
+// only: G2P, with its smaller CTAs, 27 us either way), and those of many tiles
+// per CTA. There CTAs drift apart, so that strided tiles that lie side by side
+// run at different times; in turn, they run together and the next step's list
+// comes out in the order of space. 12 M particles (54 tiles per P2G CTA, 36 per
+// G2P CTA): P2G 305 -> 297 us, G2P 221 -> 214, grid update 72 -> 69; 2 M (9 and
+// 6): P2G 60.0 and 59.4, G2P 44.2 and 45.9 us.
+constexpr int TURN_ROUNDS = 16;
+__device__ __forceinline__ bool many_rounds(const Shared& sh, int nwork) { return sh.nscn == 1 && nwork >= TURN_ROUNDS * (int)gridDim.x; }
 
 // K1 (bookkeeping half): a tile's particles are the stayers of its own
 // segment in the current buffer plus the movers of the 8 neighbour segments
@@ -320,11 +343,12 @@ constexpr int PREP_LANES = 16;
 constexpr int PREP_THREADS = 256;
 constexpr int PREP_MAX_TILES = 1024 / PREP_LANES;  // tiles of one block pass (the persistent kernel runs larger blocks)
 static_assert(offsetof(TileDesc, rstart) == 4 * 4 && offsetof(TileDesc, rpref) == 13 * 4 && offsetof(TileDesc, fresh) == 23 * 4 &&
-                  offsetof(TileDesc, nb) == 28 * 4 && offsetof(TileDesc, tij) == 37 * 4,
+                  offsetof(TileDesc, nb) == 28 * 4 && offsetof(TileDesc, tij) == 37 * 4 &&
+                  offsetof(TileDesc, slot) == 38 * 4,
               "k_prep writes the descriptor word by word");
 
 __device__ __forceinline__ void prep_body(const Shared& sh) {
-    __shared__ int s_sid[PREP_MAX_TILES], s_cnt[PREP_MAX_TILES], s_off[PREP_MAX_TILES];  // of the block's tiles
+    __shared__ int s_sid[PREP_MAX_TILES], s_cnt[PREP_MAX_TILES], s_off[PREP_MAX_TILES], s_pos[PREP_MAX_TILES];  // of the block's tiles
     __shared__ ScnSm s_one;
     const int lane = threadIdx.x & 31, r = lane & (PREP_LANES - 1);
     const int per_block = (int)blockDim.x / PREP_LANES, mine = threadIdx.x / PREP_LANES;
@@ -440,11 +464,11 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
         const int gnb = __shfl_sync(0xffffffffu, nb, r >= 9 && r < 13 ? from : lane);
         const bool fresh = new_gt && gnb < 0;
         const unsigned gmask = __ballot_sync(0xffffffffu, fresh);
+        int xat = 0;
         if (gmask && sh.use_xlist) {  // the grid update's list of these
             int at = 0;
-            if (lane == __ffs(gmask) - 1) at = atomicAdd(sh.xcount, __popc(gmask));
-            at = __shfl_sync(0xffffffffu, at, __ffs(gmask) - 1) + __popc(gmask & ((1u << lane) - 1u));
-            if (fresh) sh.xlist[at] = w << 2 | gk;
+            if (lane == __ffs(gmask) - 1) at = atomicAdd(&sh.lists[LIST_X], __popc(gmask));
+            xat = __shfl_sync(0xffffffffu, at, __ffs(gmask) - 1) + __popc(gmask & ((1u << lane) - 1u));
         }
         // the segment cursor: one atomic per scenario and block, by its first
         // warp (one per warp, with the counters of the step's lists, made 3
@@ -452,9 +476,12 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
         if (r == 0) {
             s_sid[mine] = valid ? sid : -1;
             s_cnt[mine] = cnt;
+            s_pos[mine] = w;
         }
         __syncthreads();
         if (one && threadIdx.x < 32) {
+            const bool by_size = ordered_by_size(sh, nwork);
+            const int heavy = by_size ? (int)__fdividef(1.25f * (float)s_one.s.Np, (float)nwork) : 0;
             for (int q0 = 0; q0 < per_block; q0 += 32) {
                 const int q = q0 + lane;
                 const bool has = q < per_block && s_sid[q] >= 0;
@@ -465,25 +492,34 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
                     const int yc = __shfl_up_sync(0xffffffffu, ic, o);
                     if (lane >= o) ic += yc;
                 }
-                int base = 0;
-                if (lane == 31) base = atomicAdd(&sh.cnt[0].cursor, ic);
-                base = __shfl_sync(0xffffffffu, base, 31);
-                if (has) s_off[q] = base + ic - qc;
+                const unsigned hm = __ballot_sync(0xffffffffu, by_size && has && qc > heavy), lm = __ballot_sync(0xffffffffu, by_size && has && qc <= heavy);
+                unsigned long long old = 0;
+                if (lane == 31)
+                    old = atomicAdd(reinterpret_cast<unsigned long long*>(&sh.cnt[0].cursor),
+                                    (unsigned long long)ic + ((unsigned long long)__popc(hm) << 32) + ((unsigned long long)__popc(lm) << 48));
+                old = __shfl_sync(0xffffffffu, old, 31);
+                if (has) {
+                    const unsigned lt = (1u << lane) - 1u;
+                    s_off[q] = (int)(unsigned)old + ic - qc;
+                    if (by_size)
+                        s_pos[q] = qc > heavy ? (int)(old >> 32 & 0xffff) + __popc(hm & lt) : nwork - 1 - ((int)(old >> 48) + __popc(lm & lt));
+                }
             }
         } else if (threadIdx.x < 32) {
             for (int q0 = 0; q0 < per_block; q0 += 32) {
                 const int q = q0 + lane;
                 const int qs = q < per_block ? s_sid[q] : -1;
                 const unsigned m = __ballot_sync(0xffffffffu, qs >= 0);
-                if (qs >= 0) s_off[q] = warp_atomic_add(&sh.cnt[qs].cursor, s_cnt[q], m);
+                if (qs >= 0) s_off[q] = warp_atomic_add(reinterpret_cast<int*>(&sh.cnt[qs].cursor), s_cnt[q], m);  // its low word
             }
         }
         __syncthreads();
-        const int nxt_off = s_off[mine];
+        const int nxt_off = s_off[mine], pos = s_pos[mine];
+        if (fresh && sh.use_xlist) sh.xlist[xat] = pos << 2 | gk;
         // the descriptor, word by word (TileDesc: t, total, nxt_off, sid,
-        // rstart[9], rpref[10], fresh, blk4[4], nb[9])
+        // rstart[9], rpref[10], fresh, blk4[4], nb[9], tij, slot)
         if (valid) {
-            int* D = reinterpret_cast<int*>(sh.desc + w);
+            int* D = reinterpret_cast<int*>(sh.desc + pos);
             if (r < 9) {
                 D[4 + r] = rs;
                 D[13 + r] = incl - rl;  // candidates before range r
@@ -500,6 +536,7 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
                 D[2] = nxt_off;
                 D[3] = sid;
                 D[37] = pack_cell(ti, tj);
+                D[38] = w;
             }
         }
     }
@@ -750,7 +787,7 @@ __global__ void __launch_bounds__(P2G_THREADS, P2G_MIN_BLOCKS) k_p2g(Shared sh) 
             }
         }
         __syncthreads();
-        float* P = sh.part + (size_t)w * PART_STRIDE;
+        float* P = sh.part + (size_t)sm.d.slot * PART_STRIDE;
         for (int k = tid; k < PART_STRIDE; k += P2G_THREADS) {
             int q, nd;
             part_slot(k, q, nd);
@@ -943,7 +980,7 @@ __global__ void __launch_bounds__(P2W_THREADS, 3) k_p2g_warp(Shared sh) {
             }
         }
         __syncwarp();
-        float* P = sh.part + (size_t)w * PART_STRIDE;
+        float* P = sh.part + (size_t)D.slot * PART_STRIDE;
         for (int k = lane; k < PART_STRIDE; k += 32) {
             int q, nd;
             part_slot(k, q, nd);
@@ -1009,8 +1046,8 @@ __device__ unsigned long long g_phase_clk[16];
 //     force terms) straight to their sorted places, so these are computed
 //     once per particle and the sums read them in order. Places are XOR-
 //     swizzled: 4 particles per cell, the common filling, put the 8 threads of
-//     a 128-byte phase on 8 different 16-byte banks. The next tile's
-//     candidates are requested into the places just read;
+//     a 128-byte phase on 8 different 16-byte banks. The next pass's or
+//     tile's candidates are requested into the places just read;
 //  4. thread (row, cell) adds its cell's particles in sorted order over the 3
 //     nodes of its row (packed two-wide FP32: mass and m h, the momentum, the
 //     force). Every operation is rounded as written.
@@ -1021,7 +1058,8 @@ __device__ unsigned long long g_phase_clk[16];
 // (ordered placement), so every sum has a fixed order: results are bitwise
 // reproducible and the same alone or inside a batch.
 constexpr int P2G_T = 3 * NCELL;        // threads of a CTA
-constexpr int P2C_CAP = 5 * NCELL;      // candidates of one pass
+constexpr int P2C_CAP = 6 * NCELL;      // candidates of one pass, two per thread (tiles of 1 to 980 particles: 40 us with 5 x 64
+                                        // and 38 with 6 x 64; with 7 x 64 a third one per thread spills: 12 M particles 309 against 296)
 constexpr int P2C_PER = (P2C_CAP + P2G_T - 1) / P2G_T;  // per thread
 constexpr int P2C_CHUNKS = P2C_CAP / 32;
 constexpr int P2C_HALVES = NCELL / 2;   // words of a chunk's 16-bit cell counts
@@ -1057,6 +1095,7 @@ struct P2GTileSmem {
     uint32_t cnt[P2C_CHUNKS][P2C_HALVES];              // cell counts of a chunk, two 16-bit halves per word
     uint16_t cbeg[NCELL + 2];                          // first sorted place of each cell; [NCELL]: the pass's particles
     TileDesc d[2];                                     // this tile and the next
+    int next_w;                                        // the next tile's place in the order of work
     ScnSm z;
 };
 
@@ -1067,19 +1106,24 @@ struct TileOrigin {
     int i, j;
 };
 
-// Requests tile D's first candidates and terrain window. Thread t copies the
-// candidates t, t + P2G_T, ... and is their only reader, so it may call this
-// as soon as it has read the ones before; the terrain window is thread 0's,
-// after a barrier that follows its last reads.
-__device__ __forceinline__ void p2g_request(P2GTileSmem& sm, const Shared& sh, const TileDesc& D, const CUtensorMap* dem_map) {
+// Requests tile D's candidates base, base + 1, ... of one pass. Thread t copies
+// the pass's candidates t, t + P2G_T, ... and is their only reader, so it may
+// call this as soon as it has read the ones before.
+__device__ __forceinline__ void p2g_request_cands(P2GTileSmem& sm, const TileDesc& D, int base) {
     const PBuf B = sm.z.cur();
-    const int nc = min(D.rpref[9], P2C_CAP);
+    const int nc = min(D.rpref[9] - base, P2C_CAP);
     for (int k = threadIdx.x; k < nc; k += P2G_T) {
         int r;
-        const int src = cand_index(k, D, r);
+        const int src = cand_index(base + k, D, r);
         cpa::copy16(&sm.ra[k], B.a + src);
         cpa::copy16(&sm.rb[k], B.b + src);
     }
+}
+
+// Requests tile D's first candidates and its terrain window (by thread 0, after
+// a barrier that follows the last reads of the one before).
+__device__ __forceinline__ void p2g_request(P2GTileSmem& sm, const Shared& sh, const TileDesc& D, const CUtensorMap* dem_map) {
+    p2g_request_cands(sm, D, 0);
     if (threadIdx.x == 0) {
         // one 2-D tensor copy (TMA) of 9 x 9 nodes. The map sees the terrain as
         // [Nx][4 Ny] floats, so x = 4 tj TILE (a multiple of 16 bytes). Nodes
@@ -1171,7 +1215,7 @@ __device__ __forceinline__ void spline_y(float f, float2 (&w)[3], float (&dw)[3]
 
 template <bool OUTS, typename Next>
 __device__ __forceinline__ void p2g_dense_tile(P2GTileSmem& sm, const TileDesc& D, float* part, uint32_t dem_phase, TileOrigin o,
-                                               Next request_next) {
+                                               Next& next) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cell = tid % NCELL, row = tid / NCELL;  // row is the same in a whole warp
     Ctl* const ctl = sm.z.s.ctl;
@@ -1185,14 +1229,7 @@ __device__ __forceinline__ void p2g_dense_tile(P2GTileSmem& sm, const TileDesc& 
     int base = 0;
     do {
         const int nc = min(P2C_CAP, ncand - base);
-        if (base) {  // a later pass of a very dense tile: its candidates were not requested ahead
-            const PBuf B = sm.z.cur();
-            for (int k = tid; k < nc; k += P2G_T) {
-                int r;
-                const int src = cand_index(base + k, D, r);
-                cpa::copy16(&sm.ra[k], B.a + src);
-                cpa::copy16(&sm.rb[k], B.b + src);
-            }
+        if (base) {  // a later pass of a very dense tile
             cpa::wait_all();
             __syncthreads();  // the sums of the pass before are done with its places and ranges
         }
@@ -1220,6 +1257,7 @@ __device__ __forceinline__ void p2g_dense_tile(P2GTileSmem& sm, const TileDesc& 
             }
         }
         __syncthreads();
+        if (base == 0) next.fetch();
         SLAB_PHASE_MARK(1);
         // 2. exclusive prefix over the chunks of every cell, then over the cells
         if (warp == 0) {
@@ -1275,10 +1313,12 @@ __device__ __forceinline__ void p2g_dense_tile(P2GTileSmem& sm, const TileDesc& 
             }
         }
         placed += sm.cbeg[NCELL];
+        if (base == 0) next.store();
         __syncthreads();
         SLAB_PHASE_MARK(3);
         for (int k = tid; k < P2C_CHUNKS * P2C_HALVES; k += P2G_T) (&sm.cnt[0][0])[k] = 0;  // for the next pass or tile
-        if (base + P2C_CAP >= ncand) request_next();
+        if (base + P2C_CAP >= ncand) next.request();
+        else p2g_request_cands(sm, D, base + P2C_CAP);
         // 4. the cell's particles over the row's 3 nodes
         const RowSpline rs(row);
         const int r0 = sm.cbeg[cell], r1 = sm.cbeg[cell + 1];
@@ -1347,7 +1387,7 @@ __device__ __forceinline__ void p2g_dense_tile(P2GTileSmem& sm, const TileDesc& 
 // on arrival order.
 template <typename Next>
 __device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc& D, float* part, uint32_t dem_phase, TileOrigin o,
-                                                Next request_next) {
+                                                Next& next) {
     const int tid = threadIdx.x, lane = tid & 31;
     auto& sp = sm.sp;
     SLAB_PHASE_BEGIN;
@@ -1366,6 +1406,7 @@ __device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc&
     }
     if (!tma::mbar_wait(&sm.dem_bar, dem_phase)) atomicOr(&ctl->err, ERR_TIMEOUT);
     __syncthreads();  // (the window of the tile before was read before the barrier of that tile's caller)
+    next.fetch();
     // pass A: particle quantities, cell counts, bounds
     for (int k = tid; k < ncand; k += P2G_T) {
         int d;
@@ -1404,9 +1445,10 @@ __device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc&
             atomicMax(&sp.bmax[6], r[5]);
         }
     }
+    next.store();
     __syncthreads();
     SLAB_PHASE_MARK(6);
-    request_next();  // candidates and terrain window have been read
+    next.request();  // candidates and terrain window have been read
     // scales 2^e of the sums from the exponents of their bounds (bound < 2^E,
     // e = 30 - E, |e| <= 120), in every thread: integer operations instead of
     // frexp / ldexp by 7 threads between two barriers
@@ -1469,11 +1511,39 @@ __device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc&
     SLAB_PHASE_MARK(13);
 }
 
-// The active tiles of the step. Latency: the first
-// descriptor is read beside the work count (the guess blockIdx.x is right for
-// one scenario); a tile's candidates are requested while the tile
-// before it is summed, its descriptor one tile earlier; the scenario's values
-// stay in shared memory across a run of its tiles.
+// The tile after the one that a P2G CTA sums. Its place in the order of work is
+// known to thread 0 (wn: of one scenario, the next that no CTA has taken, the
+// atomic issued a tile ahead) and shown to the others by the tile's first
+// barrier; then come its descriptor and, when this tile's candidates have been
+// read, its own candidates.
+struct P2GNext {
+    P2GTileSmem& sm;
+    const Shared& sh;
+    const CUtensorMap* dem_map;
+    int w, w1, step, cur, wn, dn;
+    bool in_turn, requested;
+    __device__ __forceinline__ void take() {  // thread 0
+        if (in_turn) wn = (int)gridDim.x + atomicAdd(&sh.lists[LIST_P2G], 1);
+    }
+    __device__ __forceinline__ void fetch() {
+        w = in_turn ? sm.next_w : w + step;
+        if (threadIdx.x < DESC_WORDS && w < w1) dn = reinterpret_cast<const int*>(sh.desc + w)[threadIdx.x];
+    }
+    __device__ __forceinline__ void store() {
+        if (threadIdx.x < DESC_WORDS && w < w1) reinterpret_cast<int*>(&sm.d[cur ^ 1])[threadIdx.x] = dn;
+        if (threadIdx.x == 0 && w < w1) take();
+    }
+    __device__ __forceinline__ void request() {
+        const TileDesc& N = sm.d[cur ^ 1];
+        requested = w < w1 && N.sid == sm.z.sid;
+        if (requested) p2g_request(sm, sh, N, dem_map);
+    }
+};
+
+// The active tiles of the step. Latency: the first descriptor is read beside
+// the work count (the guess blockIdx.x is right for one scenario); a tile's
+// candidates are requested while the tile before it is summed; the scenario's
+// values stay in shared memory across a run of its tiles.
 __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* smem_raw, const CUtensorMap* dem_map) {
     P2GTileSmem& sm = *reinterpret_cast<P2GTileSmem*>(smem_raw);
     const int tid = threadIdx.x;
@@ -1489,45 +1559,34 @@ __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* 
     chain_wait<false>();
     if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
     if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
-    const WorkItems W = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
-    const int w0 = W.w0, w1 = W.w1, step = W.step;
-    if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
+    const int nwork = sh.work_pref[sh.nscn];
+    const WorkItems W = work_items(sh, nwork, blockIdx.x, gridDim.x);
+    P2GNext next{sm, sh, dem_map, W.w0, W.w1, W.step, 0, W.w1, 0, many_rounds(sh, nwork) || ordered_by_size(sh, nwork), false};
+    if (tid == 0 && next.w < next.w1) next.take();
+    if (words && next.w < next.w1 && next.w != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + next.w)[tid];
     if (words) reinterpret_cast<int*>(&sm.d[0])[tid] = dn;
-    if (words && w0 + step < w1) dn = reinterpret_cast<const int*>(sh.desc + w0 + step)[tid];
     __syncthreads();
     uint32_t dem_phase = 0;  // parity of the terrain window's next completion
-    bool requested = false;  // the tile's candidates and terrain window are on their way (uniform)
-    for (int w = w0, cur = 0; w < w1; w += step, cur ^= 1) {
-        const TileDesc& D = sm.d[cur];
-        const TileDesc& N = sm.d[cur ^ 1];
+    for (; next.w < next.w1; next.cur ^= 1) {
+        const TileDesc& D = sm.d[next.cur];
+        if (tid == 0) sm.next_w = next.wn;
         if (D.sid != sm.z.sid) {  // uniform: a new scenario in this CTA's run
             __syncthreads();
             load_scn(sh, D.sid, sm.z, tid, P2G_T);
             __syncthreads();
         }
-        if (!requested) p2g_request(sm, sh, D, dem_map);
-        // the next descriptor; later barriers of this tile show it to the other threads
-        const bool more = w + step < w1;
-        if (words && more) reinterpret_cast<int*>(&sm.d[cur ^ 1])[tid] = dn;
-        if (words && w + 2 * step < w1) dn = reinterpret_cast<const int*>(sh.desc + w + 2 * step)[tid];
-        requested = false;
-        auto request_next = [&] {
-            if (more && N.sid == sm.z.sid) {
-                p2g_request(sm, sh, N, dem_map);
-                requested = true;
-            }
-        };
+        if (!next.requested) p2g_request(sm, sh, D, dem_map);
         if (D.fresh) p2g_clear_fresh(sh, sm.z.s, D, sm.z.y.outs != 0, tid, P2G_T);
         cpa::wait_all();
-        float* part = sh.part + (size_t)w * PART_STRIDE;
+        float* part = sh.part + (size_t)D.slot * PART_STRIDE;
         const TileOrigin o{cell_i(D.tij) * TILE, cell_j(D.tij) * TILE};
         if (D.total <= sh.split_min) {
             __syncthreads();  // the sums share memory with the row sums of the tile before
-            p2g_sparse_tile(sm, D, part, dem_phase, o, request_next);
+            p2g_sparse_tile(sm, D, part, dem_phase, o, next);
         } else if (sm.z.y.outs) {
-            p2g_dense_tile<true>(sm, D, part, dem_phase, o, request_next);
+            p2g_dense_tile<true>(sm, D, part, dem_phase, o, next);
         } else {
-            p2g_dense_tile<false>(sm, D, part, dem_phase, o, request_next);
+            p2g_dense_tile<false>(sm, D, part, dem_phase, o, next);
         }
         dem_phase ^= 1u;
     }
@@ -1683,7 +1742,7 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
         __syncwarp();
     }
     const int ntile = sh.work_pref[sh.nscn];
-    const WorkItems W = work_items(sh, (ntile + *sh.xcount) * PARTS, gw, gn);
+    const WorkItems W = work_items(sh, (ntile + sh.lists[LIST_X]) * PARTS, gw, gn);
     const int w0 = W.w0, w1 = W.w1, step = W.step;
     auto request = [&](int it) {
         int w = it / PARTS;
@@ -1799,6 +1858,7 @@ template <int T> struct G2PSmem {
     float4 nv[NWIN];
     float4 dem[(TILE + 1) * (TILE + 1)];
     int front, back;
+    int next_w;  // the next tile's place in the order of work
     alignas(16) int wcnt[2][(T / 32 + 3) / 4 * 4];  // stayers | movers << 16 of each warp of a chunk (double buffered)
     int dcnt[9];
     TileDesc d;
@@ -1855,20 +1915,29 @@ template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shar
     if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
     if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
     const WorkItems W = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
-    const int w0 = W.w0, w1 = W.w1, step = W.step;
-    if (words && w0 < w1 && w0 != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w0)[tid];
+    const int w1 = W.w1, step = W.step;
+    const bool in_turn = many_rounds(sh, w1);
+    int w = W.w0, wn = w1;  // this tile's place in the order of work, the next one's (thread 0)
+    auto take = [&] {
+        if (tid == 0) wn = (int)gridDim.x + atomicAdd(&sh.lists[LIST_G2P], 1);
+    };
+    if (in_turn && w < w1) take();
+    if (words && w < w1 && w != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w)[tid];
     int pend_tt = -1;    // threads 0..8: neighbour tile the previous tile activates
     G2PRun run;
-    for (int w = w0; w < w1; w += step) {
+    while (w < w1) {
         __syncthreads();  // the tile before is done with the shared memory
         if (words) reinterpret_cast<int*>(&sm.d)[tid] = dn;
         if (tid < 9) sm.dcnt[tid] = 0;
+        if (in_turn && tid == 0) sm.next_w = wn;
         __syncthreads();
-        if (w + step < w1 && words) dn = reinterpret_cast<const int*>(sh.desc + w + step)[tid];
+        w = in_turn ? sm.next_w : w + step;
+        if (w < w1 && words) dn = reinterpret_cast<const int*>(sh.desc + w)[tid];
+        if (in_turn && w < w1) take();
         if (sm.d.sid != sm.z.sid) {  // uniform: a new scenario in this CTA's run
             if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);
             pend_tt = -1;
-            if (w > w0) run.flush(sm.z);
+            run.flush(sm.z);  // (nothing yet before the first)
             __syncthreads();
             load_scn(sh, sm.d.sid, sm.z, tid, T);
             __syncthreads();
@@ -2077,7 +2146,7 @@ template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shar
         SLAB_PHASE_MARK(11);
         SLAB_PHASE_TILE_G2P();
     }
-    if (w0 < w1) run.flush(sm.z);
+    run.flush(sm.z);
     if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);  // the last tile's
 }
 
