@@ -43,7 +43,7 @@ class Engine32 {
     void launch_step();
     static constexpr int NKERNELS = 5;  // of a step: k_prep, P2G, grid update, G2P, k_end
     void launch_kernel(int k, const Shared& sh);
-    // Steps of few active tiles run the grid update inside G2P (k_g2p<true>),
+    // Steps of few active tiles run the grid update inside G2P (k_g2p_fused),
     // with the same bits: per step 17 against 21 us at 12 tiles, 26 against 30
     // at 734, 68 against 71 at 1 900, but 132 against 129 at 7 900 (8 000 tiles
     // of a thin flow: 98 against 93), where computing the nodes on the tiles'
@@ -99,7 +99,7 @@ class Engine32 {
     int TX = 0, TY = 0, ntiles = 0;
     int blk_cap = 0;
     int64_t pending_blocks = 0;  // node blocks of scenarios added since the last t=0 pass (an estimate)
-    int grid_p2g = 0, grid_p2g_cell = 0, grid_p2g_hilo = 0, grid_p2g_sparse = 0, grid_g2p = 0, grid_grid = 0, grid_prep = 0;
+    int grid_p2g = 0, grid_p2g_cell = 0, grid_p2g_hilo = 0, grid_p2g_sparse = 0, grid_g2p = 0, grid_g2p_fused = 0, grid_grid = 0, grid_prep = 0;
 
     // Launch-shape tuner of the step's work kernels (k_prep, k_p2g_tiles --
     // shapes 1 and 2, its dense and sparse tiles, go together --, k_grid, k_g2p). Each CTA of these kernels takes a
@@ -122,6 +122,7 @@ class Engine32 {
         int64_t active = 0;    // active tiles seen by the last capacity check
         int64_t active_at = 0; // active tiles when the last schedule started
         int base[NK] = {};     // occupancy-derived grids
+        int base_fused = 0;    // of G2P with the grid update (k_g2p_fused); shares its pick with k_g2p
         int pick[NK] = {2, 2, 2, 2, 2};
         int fixed[NK] = {};    // > 0: grid set by the caller, not tuned
         int tunes = 0;

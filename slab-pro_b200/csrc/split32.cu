@@ -282,12 +282,14 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     int occ_c = 0, occ_h = 0;
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k32::k_p2g_tiles, k32::P2G_T, sizeof(k32::P2GTileSmem)));
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k32::k_p2g<k32::ACC_HILO>, k32::P2G_THREADS, sizeof(k32::P2GSmem)));
-    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p<false>, k32::G2P_T, 0));
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p, 32, 0));
     grid_p2g = sms * std::max(occ_p, 1);
     grid_p2g_cell = sms * std::max(occ_c, 1);
     grid_p2g_hilo = sms * std::max(occ_h, 1);
     grid_p2g_sparse = grid_p2g_cell;  // sparse tiles run in the same kernel
     grid_g2p = sms * std::max(occ_g, 1);
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p_fused, k32::G2P_T, 0));
+    tune.base_fused = grid_g2p_fused = sms * std::max(occ_g, 1);
     int occ_u = 0;
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k32::k_grid, k32::GRID_T, 0));
     grid_grid = sms * std::max(occ_u, 1);
@@ -646,7 +648,10 @@ void Engine32::launch_kernel(int k, const Shared& sh) {
         case 0: launch_chained(st, grid_prep, k32::PREP_THREADS, 0, k32::k_prep, sh); break;
         case 1: launch_p2g(sh); break;
         case 2: launch_chained(st, grid_grid, k32::GRID_T, 0, k32::k_grid, sh); break;
-        case 3: launch_chained(st, grid_g2p, k32::G2P_T, 0, fused() ? k32::k_g2p<true> : k32::k_g2p<false>, sh, T.z.get()); break;
+        case 3:
+            if (fused()) launch_chained(st, grid_g2p_fused, k32::G2P_T, 0, k32::k_g2p_fused, sh, T.z.get());
+            else launch_chained(st, grid_g2p, 32, 0, k32::k_g2p, sh, T.z.get());
+            break;
         case 4: launch_chained(st, 1, k32::CTL_THREADS, 0, k32::k_end, sh); break;
     }
 }
@@ -700,10 +705,11 @@ int Engine32::tuned_grid(int k, int c) const {
 void Engine32::apply_shapes(const int* c) {
     int* g[Tuner::NK] = {&grid_prep, &grid_p2g_cell, &grid_p2g_sparse, &grid_grid, &grid_g2p};
     for (int k = 0; k < Tuner::NK; ++k) *g[k] = tuned_grid(k, c[k]);
+    grid_g2p_fused = tune.fixed[4] > 0 ? tune.fixed[4] : std::max(1, tune.base_fused * Tuner::FACTOR4[c[4]] / 4);
 }
 
 void Engine32::launch_shapes(int out[5]) const {
-    const int g[Tuner::NK] = {grid_prep, grid_p2g_cell, grid_p2g_sparse, grid_grid, grid_g2p};
+    const int g[Tuner::NK] = {grid_prep, grid_p2g_cell, grid_p2g_sparse, grid_grid, fused() ? grid_g2p_fused : grid_g2p};
     for (int k = 0; k < Tuner::NK; ++k) out[k] = g[k];
 }
 

@@ -127,10 +127,9 @@ struct alignas(16) Scn {
     int32_t pad_;
 };
 
-// Counters of a step over all tiles, zeroed at its start: entries of xlist; of
-// one scenario, descriptors placed from the front and from the back of the
-// order of work, and tiles taken from it by P2G and by G2P.
-enum : int { LIST_X = 0, LIST_P2G = 1, LIST_G2P = 2, NLISTCNT = 3 };
+// Counters of a step over all tiles, zeroed at its start: entries of xlist, and
+// (of one scenario) tiles that P2G took in turn.
+enum : int { LIST_X = 0, LIST_P2G = 1, NLISTCNT = 2 };
 
 // Shared by all scenarios of a context: terrain and node-block pool.
 struct Shared {

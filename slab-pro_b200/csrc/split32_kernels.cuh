@@ -294,8 +294,8 @@ __device__ __forceinline__ void load_scn(const Shared& sh, int sid, ScnSm& z, in
 // consecutive items mostly belong to the same scenario. Of one scenario it
 // takes every n-th item: the list is roughly in the order of space, so runs of
 // it are all dense tiles for one worker and all sparse ones for the next (300 k
-// particles in a thin tongue: P2G 62 us with runs, 49 us with strides). P2G and
-// G2P leave this order in some steps, see many_rounds.
+// particles in a thin tongue: P2G 62 us with runs, 49 us with strides). P2G
+// leaves this order in some steps, see many_rounds.
 struct WorkItems {
     int w0, w1, step;
 };
@@ -317,14 +317,11 @@ __device__ __forceinline__ bool ordered_by_size(const Shared& sh, int nwork) {
     return sh.nscn == 1 && !sh.use_xlist && nwork > sh.p2g_ctas && nwork < (1 << 16);
 }
 
-// Steps of one scenario in which a CTA takes, after its first tile, the next
-// one that no CTA has taken, instead of every gridDim.x-th: ordered ones (P2G
-// only: G2P, with its smaller CTAs, 27 us either way), and those of many tiles
-// per CTA. There CTAs drift apart, so that strided tiles that lie side by side
-// run at different times; in turn, they run together and the next step's list
-// comes out in the order of space. 12 M particles (54 tiles per P2G CTA, 36 per
-// G2P CTA): P2G 305 -> 297 us, G2P 221 -> 214, grid update 72 -> 69; 2 M (9 and
-// 6): P2G 60.0 and 59.4, G2P 44.2 and 45.9 us.
+// Steps of one scenario in which a P2G CTA takes, after its first tile, the next
+// one that no CTA has taken, instead of every gridDim.x-th: ordered ones, and
+// those of many tiles per CTA, where CTAs drift apart and strided tiles that lie
+// side by side run at different times. 12 M particles (54 tiles per CTA): 305 ->
+// 297 us; 2 M (9): 60.0 and 59.4. (G2P in turn: no gain.)
 constexpr int TURN_ROUNDS = 16;
 __device__ __forceinline__ bool many_rounds(const Shared& sh, int nwork) { return sh.nscn == 1 && nwork >= TURN_ROUNDS * (int)gridDim.x; }
 
@@ -1808,9 +1805,9 @@ __device__ __forceinline__ int dir_of(int ib, int jb, int ti, int tj) {
     return (di + 1) * 3 + (dj + 1);
 }
 
-constexpr int G2P_T = 2 * NCELL;  // threads of a CTA
+constexpr int G2P_T = 2 * NCELL;  // threads of a CTA with the grid update
 #ifndef SLAB_G2P_MIN_BLOCKS
-#define SLAB_G2P_MIN_BLOCKS (NCELL == 64 ? 9 : 2)
+#define SLAB_G2P_MIN_BLOCKS (NCELL == 64 ? 32 : 8)
 #endif
 #ifndef SLAB_G2P_FUSED_MIN_BLOCKS
 #define SLAB_G2P_FUSED_MIN_BLOCKS (NCELL == 64 ? 7 : 1)
@@ -1858,7 +1855,6 @@ template <int T> struct G2PSmem {
     float4 nv[NWIN];
     float4 dem[(TILE + 1) * (TILE + 1)];
     int front, back;
-    int next_w;  // the next tile's place in the order of work
     alignas(16) int wcnt[2][(T / 32 + 3) / 4 * 4];  // stayers | movers << 16 of each warp of a chunk (double buffered)
     int dcnt[9];
     TileDesc d;
@@ -1886,13 +1882,26 @@ __device__ __forceinline__ G2PCand load_g2p_cand(const TileDesc& D, const PBuf& 
     return q;
 }
 
-// K4, one CTA per tile. FUSED, for steps of few tiles: K3 and K6 first, the grid
+// K4, one tile per CTA of T threads. Two kernels:
+//
+// k_g2p_fused (T = 128), for steps of few tiles: K3 and K6 first, the grid
 // update of the tile's node window into shared memory (window_node). 100 nodes
 // for 64 cells, nodes near an edge computed by up to 4 tiles, but no kernel of
 // its own between P2G and G2P: per step 22 -> 18.5 us at 1 600 particles, 30 ->
-// 27 at 180 k (734 tiles); at 2 M particles (8 000 tiles) the pass through
-// memory is the cheaper one, 129 against 140 us. Otherwise the window comes from the node blocks.
-// Then G2P (src/simulation.cpp:877-940): FLIP/PIC blend,
+// 27 at 180 k (734 tiles), 76 -> 63 at 637 k (1 900 tiles); at 2 M particles
+// (8 000 tiles) the pass through memory is the cheaper one.
+//
+// k_g2p (T = 32), for steps of many: the window comes from the node blocks. One
+// warp per CTA, because the rounds of a tile (descriptor, candidates and window,
+// chunks, records) depend on one another and all warps of a larger CTA wait in
+// the same place: with 128 / 96 / 64 / 32 threads and the same number of warps
+// per SM, 12 M particles take 214 / 205 / 187 / 172 us, 2 M 44 / 42 / 40 / 37
+// and 300 k in a thin flow 27 / 25 / 23 / 20. The stayers' and movers' places
+// then need no block prefix either. (Several such warps in one CTA of 128 lose
+// it again: the tile number is no longer the same in the whole CTA, so
+// addresses that were uniform take registers, 250 us with the spills.)
+//
+// G2P itself (src/simulation.cpp:877-940): FLIP/PIC blend,
 // advection, depth update, and the write of the particle into the tile's
 // segment of the next buffer -- stayers from the front, particles that moved
 // to a neighbour tile from the back, with per-direction counts. The max of
@@ -1900,47 +1909,44 @@ __device__ __forceinline__ G2PCand load_g2p_cand(const TileDesc& D, const PBuf& 
 // (K5). A particle is two 16-byte loads and two 16-byte stores; a thread
 // holds its candidate of this chunk and of the next in registers, so the
 // loads of a chunk go out with the node window's or while the chunk before it
-// is computed. The scenario's
-// values stay in shared memory across a run of its tiles, the next tile's
-// descriptor is requested while this one runs, and a tile's neighbour
-// activations (two dependent atomics) are issued while the next tile's loads
-// are in flight.
+// is computed. The scenario's values stay in shared memory across a run of its
+// tiles, the next tile's descriptor is requested while this one runs, and a
+// tile's neighbour activations (two dependent atomics) are issued while the
+// next tile's loads are in flight.
 template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shared& sh, const double* __restrict__ z64, G2PSmem<T>& sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int dn = 0;
-    const bool words = tid < DESC_WORDS;
+    constexpr int PER = (DESC_WORDS + T - 1) / T;  // descriptor words per thread
+    int dn[PER] = {};
+    auto load_words = [&](int w) {
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            if (tid + u * T < DESC_WORDS) dn[u] = reinterpret_cast<const int*>(sh.desc + w)[tid + u * T];
+    };
     if (sh.nscn == 1) load_scn_static(sh, 0, sm.z, tid, T);
     else if (tid == 0) sm.z.sid = -1;
     chain_wait<true>();
-    if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
+    if ((int)blockIdx.x < sh.work_cap) load_words(blockIdx.x);
     if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
     const WorkItems W = work_items(sh, sh.work_pref[sh.nscn], blockIdx.x, gridDim.x);
-    const int w1 = W.w1, step = W.step;
-    const bool in_turn = many_rounds(sh, w1);
-    int w = W.w0, wn = w1;  // this tile's place in the order of work, the next one's (thread 0)
-    auto take = [&] {
-        if (tid == 0) wn = (int)gridDim.x + atomicAdd(&sh.lists[LIST_G2P], 1);
-    };
-    if (in_turn && w < w1) take();
-    if (words && w < w1 && w != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + w)[tid];
+    const int w0 = W.w0, w1 = W.w1, step = W.step;
+    if (w0 < w1 && w0 != (int)blockIdx.x) load_words(w0);
     int pend_tt = -1;    // threads 0..8: neighbour tile the previous tile activates
     G2PRun run;
-    while (w < w1) {
-        __syncthreads();  // the tile before is done with the shared memory
-        if (words) reinterpret_cast<int*>(&sm.d)[tid] = dn;
+    for (int w = w0; w < w1; w += step) {
+        g2p_sync<T>();  // the tile before is done with the shared memory
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            if (tid + u * T < DESC_WORDS) reinterpret_cast<int*>(&sm.d)[tid + u * T] = dn[u];
         if (tid < 9) sm.dcnt[tid] = 0;
-        if (in_turn && tid == 0) sm.next_w = wn;
-        __syncthreads();
-        w = in_turn ? sm.next_w : w + step;
-        if (w < w1 && words) dn = reinterpret_cast<const int*>(sh.desc + w)[tid];
-        if (in_turn && w < w1) take();
+        g2p_sync<T>();
+        if (w + step < w1) load_words(w + step);
         if (sm.d.sid != sm.z.sid) {  // uniform: a new scenario in this CTA's run
             if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);
             pend_tt = -1;
             run.flush(sm.z);  // (nothing yet before the first)
-            __syncthreads();
+            g2p_sync<T>();
             load_scn(sh, sm.d.sid, sm.z, tid, T);
-            __syncthreads();
+            g2p_sync<T>();
         }
         const ScnSm& Z = sm.z;
         const TileDesc& D = sm.d;
@@ -1977,7 +1983,7 @@ template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shar
         }
         SLAB_PHASE_MARK(8);
         cpa::wait_all();
-        __syncthreads();
+        g2p_sync<T>();
         SLAB_PHASE_MARK(9);
         const int total = D.total, base = D.nxt_off;
         const bool edge = ti < Z.y.in_i0 || ti > Z.y.in_i1 || tj < Z.y.in_j0 || tj > Z.y.in_j1;  // uniform: may change the particle box
@@ -2070,15 +2076,18 @@ template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shar
             // step sees the tile's particles in an order fixed by the data
             const bool stay = valid && d == 4, move = valid && d != 4;
             const unsigned ms = __ballot_sync(0xffffffffu, stay), mm = __ballot_sync(0xffffffffu, move);
-            const int par = (k0 / T) & 1;
-            if (lane == 0) sm.wcnt[par][warp] = __popc(ms) | __popc(mm) << 16;
-            __syncthreads();
-            int before = 0, all = 0;  // stayers | movers << 16: of the warps before this one, of all
+            int before = 0, all = __popc(ms) | __popc(mm) << 16;  // stayers | movers << 16: of the warps before this one, of all
+            if (T > 32) {
+                const int par = (k0 / T) & 1;
+                if (lane == 0) sm.wcnt[par][warp] = all;
+                g2p_sync<T>();
+                all = 0;
 #pragma unroll
-            for (int q_ = 0; q_ < T / 32; ++q_) {
-                const int a = sm.wcnt[par][q_];
-                if (q_ < warp) before += a;
-                all += a;
+                for (int q_ = 0; q_ < T / 32; ++q_) {
+                    const int a = sm.wcnt[par][q_];
+                    if (q_ < warp) before += a;
+                    all += a;
+                }
             }
             const int bs = front + (before & 0xffff), bm = back + (before >> 16);
             front += all & 0xffff;
@@ -2104,7 +2113,7 @@ template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shar
             sm.front = front;
             sm.back = back;
         }
-        __syncthreads();
+        g2p_sync<T>();
         if (tid < 9) {
             int32_t* G = Z.s.grp[(Z.y.seq & 1) ^ 1] + (size_t)t * GRP_STRIDE;
             const int cnt = tid == 4 ? sm.front : sm.dcnt[tid];
@@ -2129,7 +2138,7 @@ template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shar
                 sm.red[2][warp] = mny;
                 sm.red[3][warp] = mxy;
             }
-            __syncthreads();
+            g2p_sync<T>();
             if (tid == 0 && total > 0) {
                 for (int k = 1; k < T / 32; ++k) {
                     mnx = fmin(mnx, sm.red[0][k]);
@@ -2150,10 +2159,14 @@ template <int T, bool FUSED> __device__ __forceinline__ void g2p_body(const Shar
     if (pend_tt >= 0) g2p_activate(sm.z, pend_tt);  // the last tile's
 }
 
-template <bool FUSED>
-__global__ void __launch_bounds__(G2P_T, FUSED ? SLAB_G2P_FUSED_MIN_BLOCKS : SLAB_G2P_MIN_BLOCKS) k_g2p(Shared sh, const double* __restrict__ z64) {
+__global__ void __launch_bounds__(G2P_T, SLAB_G2P_FUSED_MIN_BLOCKS) k_g2p_fused(Shared sh, const double* __restrict__ z64) {
     __shared__ G2PSmem<G2P_T> sm;
-    g2p_body<G2P_T, FUSED>(sh, z64, sm);
+    g2p_body<G2P_T, true>(sh, z64, sm);
+}
+
+__global__ void __launch_bounds__(32, SLAB_G2P_MIN_BLOCKS) k_g2p(Shared sh, const double* __restrict__ z64) {
+    __shared__ G2PSmem<32> sm;
+    g2p_body<32, false>(sh, z64, sm);
 }
 
 // K5: end of the step for every running scenario (the per-step reductions
