@@ -1882,6 +1882,12 @@ __device__ __forceinline__ G2PCand load_g2p_cand(const TileDesc& D, const PBuf& 
     return q;
 }
 
+// G2P's barrier: of the block, or of its only warp
+template <int T> __device__ __forceinline__ void g2p_sync() {
+    if (T == 32) __syncwarp();
+    else __syncthreads();
+}
+
 // K4, one tile per CTA of T threads. Two kernels:
 //
 // k_g2p_fused (T = 128), for steps of few tiles: K3 and K6 first, the grid
