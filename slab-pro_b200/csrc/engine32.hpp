@@ -99,7 +99,7 @@ class Engine32 {
     int TX = 0, TY = 0, ntiles = 0;
     int blk_cap = 0;
     int64_t pending_blocks = 0;  // node blocks of scenarios added since the last t=0 pass (an estimate)
-    int grid_p2g = 0, grid_p2g_cell = 0, grid_p2g_hilo = 0, grid_p2g_sparse = 0, grid_g2p = 0, grid_g2p_fused = 0, grid_grid = 0, grid_prep = 0;
+    int grid_p2g = 0, grid_p2g_cell = 0, grid_p2g_hilo = 0, grid_p2g_sparse = 0, grid_p2g_fused = 0, grid_g2p = 0, grid_g2p_fused = 0, grid_grid = 0, grid_prep = 0;
 
     // Launch-shape tuner of the step's work kernels (k_prep, k_p2g_tiles --
     // shapes 1 and 2, its dense and sparse tiles, go together --, k_grid, k_g2p). Each CTA of these kernels takes a
@@ -122,7 +122,7 @@ class Engine32 {
         int64_t active = 0;    // active tiles seen by the last capacity check
         int64_t active_at = 0; // active tiles when the last schedule started
         int base[NK] = {};     // occupancy-derived grids
-        int base_fused = 0;    // of G2P with the grid update (k_g2p_fused); shares its pick with k_g2p
+        int base_fused[NK] = {};  // of the kernels of short steps (P2G and G2P have two each, which share a pick)
         int pick[NK] = {2, 2, 2, 2, 2};
         int fixed[NK] = {};    // > 0: grid set by the caller, not tuned
         int tunes = 0;
@@ -133,7 +133,7 @@ class Engine32 {
             for (auto e : ev) cudaEventDestroy(e);
         }
     } tune;
-    int tuned_grid(int k, int c) const;
+    int tuned_grid(int k, int c, int base) const;
     void apply_shapes(const int* c);
     void tune_pick();
     void launch_step_timed(const Shared& sh, cudaEvent_t* e);

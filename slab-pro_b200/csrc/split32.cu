@@ -253,6 +253,7 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g<k32::ACC_HILO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GSmem)));
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g<k32::ACC_I64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GSmem)));
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GTileSmem)));
+    SLAB_CUDA(cudaFuncSetAttribute(k32::k_p2g_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(k32::P2GCellSmem)));
     {
         // the terrain window of the cell P2G as one tensor copy per tile: the
         // float4 terrain seen as [Nx][4 Ny] floats (rows 16 Ny bytes apart), boxes
@@ -284,12 +285,14 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k32::k_p2g<k32::ACC_HILO>, k32::P2G_THREADS, sizeof(k32::P2GSmem)));
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p, 32, 0));
     grid_p2g = sms * std::max(occ_p, 1);
+    tune.base_fused[1] = grid_p2g_fused = sms * std::max(occ_c, 1);
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, k32::k_p2g_cells, k32::P2X_T, sizeof(k32::P2GCellSmem)));
     grid_p2g_cell = sms * std::max(occ_c, 1);
     grid_p2g_hilo = sms * std::max(occ_h, 1);
     grid_p2g_sparse = grid_p2g_cell;  // sparse tiles run in the same kernel
     grid_g2p = sms * std::max(occ_g, 1);
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k32::k_g2p_fused, k32::G2P_T, 0));
-    tune.base_fused = grid_g2p_fused = sms * std::max(occ_g, 1);
+    tune.base_fused[4] = grid_g2p_fused = sms * std::max(occ_g, 1);
     int occ_u = 0;
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k32::k_grid, k32::GRID_T, 0));
     grid_grid = sms * std::max(occ_u, 1);
@@ -347,7 +350,7 @@ Shared Engine32::shared() const {
     static_assert(NLISTCNT <= 8);
     sh.lists = d_misc.get() + 8;
     sh.use_xlist = fused() ? 0 : 1;
-    sh.p2g_ctas = tune.base[1];
+    sh.p2g_ctas = tune.base_fused[1];
     sh.work_cap = work_cap;
     sh.free_blocks = d_free_blocks.get();
     sh.free_count = d_misc.get() + 4;
@@ -630,8 +633,9 @@ void Engine32::launch_t0() {
 
 void Engine32::launch_p2g(const Shared& sh) {
     if (acc_mode == k32::ACC_MIXED || acc_mode == k32::ACC_CELL) {  // dense and sparse tiles, or every tile as a dense one
-        const int grid = std::max(grid_p2g_cell, grid_p2g_sparse);
-        launch_chained(st, grid, k32::P2G_T, sizeof(k32::P2GTileSmem), k32::k_p2g_tiles, sh, dem_map);
+        const int grid = std::max(fused() ? grid_p2g_fused : grid_p2g_cell, tune.fixed[2]);
+        if (fused()) launch_chained(st, grid, k32::P2G_T, sizeof(k32::P2GTileSmem), k32::k_p2g_tiles, sh, dem_map);
+        else launch_chained(st, grid, k32::P2X_T, sizeof(k32::P2GCellSmem), k32::k_p2g_cells, sh, dem_map);
     } else if (acc_mode == k32::ACC_WARP) {
         k32::k_p2g_warp<<<grid_p2g, k32::P2W_THREADS, k32::P2W_WARPS * sizeof(k32::P2WWarp), st>>>(sh);
     } else if (acc_mode == k32::ACC_I32) {
@@ -697,19 +701,21 @@ void Engine32::tune_key_for(int Np) {
     tune.next = 256;  // no schedule on the first steps; the usual cadence after them
 }
 
-int Engine32::tuned_grid(int k, int c) const {
+int Engine32::tuned_grid(int k, int c, int base) const {
     if (tune.fixed[k] > 0) return tune.fixed[k];
-    return std::max(1, tune.base[k] * Tuner::FACTOR4[c] / 4);
+    return std::max(1, base * Tuner::FACTOR4[c] / 4);
 }
 
 void Engine32::apply_shapes(const int* c) {
     int* g[Tuner::NK] = {&grid_prep, &grid_p2g_cell, &grid_p2g_sparse, &grid_grid, &grid_g2p};
-    for (int k = 0; k < Tuner::NK; ++k) *g[k] = tuned_grid(k, c[k]);
-    grid_g2p_fused = tune.fixed[4] > 0 ? tune.fixed[4] : std::max(1, tune.base_fused * Tuner::FACTOR4[c[4]] / 4);
+    for (int k = 0; k < Tuner::NK; ++k) *g[k] = tuned_grid(k, c[k], tune.base[k]);
+    grid_p2g_fused = tuned_grid(1, c[1], tune.base_fused[1]);
+    grid_g2p_fused = tuned_grid(4, c[4], tune.base_fused[4]);
 }
 
 void Engine32::launch_shapes(int out[5]) const {
-    const int g[Tuner::NK] = {grid_prep, grid_p2g_cell, grid_p2g_sparse, grid_grid, fused() ? grid_g2p_fused : grid_g2p};
+    const int p2g = fused() ? grid_p2g_fused : grid_p2g_cell;
+    const int g[Tuner::NK] = {grid_prep, p2g, tune.fixed[2] > 0 ? tune.fixed[2] : p2g, grid_grid, fused() ? grid_g2p_fused : grid_g2p};
     for (int k = 0; k < Tuner::NK; ++k) out[k] = g[k];
 }
 

@@ -320,8 +320,8 @@ __device__ __forceinline__ bool ordered_by_size(const Shared& sh, int nwork) {
 // Steps of one scenario in which a P2G CTA takes, after its first tile, the next
 // one that no CTA has taken, instead of every gridDim.x-th: ordered ones, and
 // those of many tiles per CTA, where CTAs drift apart and strided tiles that lie
-// side by side run at different times. 12 M particles (54 tiles per CTA): 305 ->
-// 297 us; 2 M (9): 60.0 and 59.4. (G2P in turn: no gain.)
+// side by side run at different times. 12 M particles (40 tiles per CTA of
+// k_p2g_cells): 235 -> 231 us. (G2P in turn: no gain.)
 constexpr int TURN_ROUNDS = 16;
 __device__ __forceinline__ bool many_rounds(const Shared& sh, int nwork) { return sh.nscn == 1 && nwork >= TURN_ROUNDS * (int)gridDim.x; }
 
@@ -1023,12 +1023,15 @@ __device__ unsigned long long g_phase_clk[16];
 
 // --------------------------------------------------------- P2G over tiles
 
-// K2: P2G of the active tiles (src/simulation.cpp:726-798), one CTA per tile.
+// K2: P2G of the active tiles (src/simulation.cpp:726-798), one CTA per tile, in
+// two kernels with the same bits: k_p2g_tiles here, for steps of few tiles and for
+// persistent steps, and k_p2g_cells below, for steps of many.
 // A tile with more than split_min particles is summed in FP32 over its
 // particles sorted by cell; one with fewer in exact fixed point (below). Which
 // scheme a tile gets depends only on its own particle count.
 //
-// Dense tiles. Threads = 3 x cells: thread (row, cell) owns stencil row `row`
+// Dense tiles of k_p2g_tiles. Threads = 3 x cells, which keeps the chain of one
+// tile short: thread (row, cell) owns stencil row `row`
 // of its cell's 3 x 3 nodes, so the sums of a cell's particles stay in 18
 // registers however many particles there are. Per pass of up to P2C_CAP
 // candidates (one pass, but for very dense tiles):
@@ -1066,6 +1069,15 @@ constexpr int P2C_HALVES = NCELL / 2;   // words of a chunk's 16-bit cell counts
 
 constexpr int P2S_CAP = NCELL;  // particles of a sparse tile (split_min is capped to it)
 
+struct P2GSparseSmem {
+    int hi[NQ * NWIN];  // fixed-point sums of the window, [q][node]: rounded part
+    int lo[NQ * NWIN];  //                                         finer rest
+    PQ pq[P2S_CAP];
+    int ccnt[NCELL];
+    unsigned bmax[NQ];
+    int mcc, nv;
+};
+
 struct P2GTileSmem {
     union {
         struct {                // dense: a pass's particles in sorted, swizzled places
@@ -1077,14 +1089,7 @@ struct P2GTileSmem {
             float4 q4[NSLOT * NCELL];    // m, m h, m vx, m vy
             float2 q2[NSLOT * NCELL];    // F; then, on output steps, m vz
         } cs;
-        struct {                   // sparse
-            int hi[NQ * NWIN];     // fixed-point sums of the window, [q][node]: rounded part
-            int lo[NQ * NWIN];     //                                         finer rest
-            PQ pq[P2S_CAP];
-            int ccnt[NCELL];
-            unsigned bmax[NQ];
-            int mcc, nv;
-        } sp;
+        P2GSparseSmem sp;
     };
     alignas(128) float4 dem[(TILE + 1) * (TILE + 1)];  // a tensor copy's destination: 128-byte aligned
     float4 ra[P2C_CAP], rb[P2C_CAP];                   // candidates as they lie in the particle buffer
@@ -1119,7 +1124,7 @@ __device__ __forceinline__ void p2g_request_cands(P2GTileSmem& sm, const TileDes
 
 // Requests tile D's first candidates and its terrain window (by thread 0, after
 // a barrier that follows the last reads of the one before).
-__device__ __forceinline__ void p2g_request(P2GTileSmem& sm, const Shared& sh, const TileDesc& D, const CUtensorMap* dem_map) {
+__device__ __forceinline__ void p2g_request(P2GTileSmem& sm, const Shared& sh, const TileDesc& D, int, int, const CUtensorMap* dem_map) {
     p2g_request_cands(sm, D, 0);
     if (threadIdx.x == 0) {
         // one 2-D tensor copy (TMA) of 9 x 9 nodes. The map sees the terrain as
@@ -1382,33 +1387,59 @@ __device__ __forceinline__ void p2g_dense_tile(P2GTileSmem& sm, const TileDesc& 
 // 32-bit fixed-point pairs of k_p2g<ACC_HILO> with native shared-memory
 // integer atomics. The integer sums are exact, so the result does not depend
 // on arrival order.
-template <typename Next>
-__device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc& D, float* part, uint32_t dem_phase, TileOrigin o,
+// T threads; OVER: the sums lie over the candidates (ra, rb), which each thread
+// reads first (its first two; of a tile with more than 2 T candidates, almost
+// all of them other tiles' movers, the others come from the particle buffer).
+template <int T, bool OVER, typename Next>
+__device__ __forceinline__ void p2g_sparse_tile(P2GSparseSmem& sp, const float4* ra, const float4* rb, const float4* dem, uint64_t* dem_bar,
+                                                uint32_t dem_phase, const ScnSm& Z, const TileDesc& D, float* part, TileOrigin o,
                                                 Next& next) {
+    constexpr int AHEAD = OVER ? 2 : 0;
     const int tid = threadIdx.x, lane = tid & 31;
-    auto& sp = sm.sp;
     SLAB_PHASE_BEGIN;
-    const PBuf B = sm.z.cur();
-    Ctl* const ctl = sm.z.s.ctl;
-    const bool outs = sm.z.y.outs != 0;
-    const float g = sm.z.s.g, hod = 0.5f * sm.z.s.ood;
+    const PBuf B = Z.cur();
+    Ctl* const ctl = Z.s.ctl;
+    const bool outs = Z.y.outs != 0;
+    const float g = Z.s.g, hod = 0.5f * Z.s.ood;
     const int ncand = D.rpref[9];
     float bm = 0.f, bvx = 0.f, bvy = 0.f, bh = 0.f, bvz = 0.f, bF = 0.f;
-    for (int k = tid; k < 2 * NQ * NWIN / 4; k += P2G_T) reinterpret_cast<int4*>(sp.hi)[k] = make_int4(0, 0, 0, 0);  // hi and lo
-    for (int k = tid; k < NCELL; k += P2G_T) sp.ccnt[k] = 0;
+    float4 ca[2], cb[2];
+    if (OVER) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int k = tid + u * T;
+            if (k < ncand) {
+                ca[u] = ra[k];
+                cb[u] = rb[k];
+            }
+        }
+        __syncthreads();
+    }
+    for (int k = tid; k < 2 * NQ * NWIN / 4; k += T) reinterpret_cast<int4*>(sp.hi)[k] = make_int4(0, 0, 0, 0);  // hi and lo
+    for (int k = tid; k < NCELL; k += T) sp.ccnt[k] = 0;
     if (tid < NQ) sp.bmax[tid] = 0u;
     if (tid == 0) {
         sp.mcc = 0;
         sp.nv = 0;
     }
-    if (!tma::mbar_wait(&sm.dem_bar, dem_phase)) atomicOr(&ctl->err, ERR_TIMEOUT);
+    if (!tma::mbar_wait(dem_bar, dem_phase)) atomicOr(&ctl->err, ERR_TIMEOUT);
     __syncthreads();  // (the window of the tile before was read before the barrier of that tile's caller)
     next.fetch();
     // pass A: particle quantities, cell counts, bounds
-    for (int k = tid; k < ncand; k += P2G_T) {
+    for (int k = tid; k < ncand; k += T) {
         int d;
         const int src = cand_index(k, D, d);
-        const float4 a = k < P2C_CAP ? sm.ra[k] : B.a[src], b = k < P2C_CAP ? sm.rb[k] : B.b[src];
+        float4 a, b;
+        if (OVER && k < AHEAD * T) {
+            a = k < T ? ca[0] : ca[1];
+            b = k < T ? cb[0] : cb[1];
+        } else if (!OVER && k < P2C_CAP) {
+            a = ra[k];
+            b = rb[k];
+        } else {
+            a = B.a[src];
+            b = B.b[src];
+        }
         const float vz = outs ? B.vz[src] : 0.f;
         const int32_t cell = __float_as_int(b.z);
         const int li = cell_i(cell) - o.i, lj = cell_j(cell) - o.j;
@@ -1416,7 +1447,7 @@ __device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc&
             if (d == 4) atomicOr(&ctl->err, ERR_MOVE);  // a stayer outside its tile
             continue;
         }
-        const PQ p = make_pq(a, b, vz, li, lj, sm.dem, g, hod);
+        const PQ p = make_pq(a, b, vz, li, lj, dem, g, hod);
         const int slot = atomicAdd(&sp.nv, 1);
         if (slot < P2S_CAP) sp.pq[slot] = p;
         else atomicOr(&ctl->err, ERR_CAPACITY);
@@ -1464,7 +1495,7 @@ __device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc&
     const int nmax = 9 * mcc, c2 = nmax <= 1 ? 0 : 32 - __clz(nmax - 1);
     const int lob = min(20, 31 - c2);  // lo_bits_for(nmax): lo sums of a node stay below 2^30 (20 bits for <= 64 particles)
     const float lo_mul = __int_as_float((127 + lob) << 23);
-    for (int it = tid; it < 3 * nv; it += P2G_T) {
+    for (int it = tid; it < 3 * nv; it += T) {
         const int pi = it / 3, a = it - 3 * pi;
         const PQ p = sp.pq[pi];
         float wx[3], wy[3], dwx[3], dwy[3];
@@ -1494,7 +1525,7 @@ __device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc&
     SLAB_PHASE_MARK(12);
     // the window, one node per thread
     const double lo_div = __hiloint2double((1023 - lob) << 20, 0);
-    for (int n = tid; n < NWIN; n += P2G_T) {
+    for (int n = tid; n < NWIN; n += T) {
         float v[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q)
@@ -1513,12 +1544,13 @@ __device__ __forceinline__ void p2g_sparse_tile(P2GTileSmem& sm, const TileDesc&
 // atomic issued a tile ahead) and shown to the others by the tile's first
 // barrier; then come its descriptor and, when this tile's candidates have been
 // read, its own candidates.
-struct P2GNext {
-    P2GTileSmem& sm;
+template <typename Sm> struct P2GNext {
+    Sm& sm;
     const Shared& sh;
     const CUtensorMap* dem_map;
     int w, w1, step, cur, wn, dn;
     bool in_turn, requested;
+    int buf;  // where the next pass's candidates go (P2GCellSmem)
     __device__ __forceinline__ void take() {  // thread 0
         if (in_turn) wn = (int)gridDim.x + atomicAdd(&sh.lists[LIST_P2G], 1);
     }
@@ -1533,7 +1565,7 @@ struct P2GNext {
     __device__ __forceinline__ void request() {
         const TileDesc& N = sm.d[cur ^ 1];
         requested = w < w1 && N.sid == sm.z.sid;
-        if (requested) p2g_request(sm, sh, N, dem_map);
+        if (requested) p2g_request(sm, sh, N, cur ^ 1, buf, dem_map);
     }
 };
 
@@ -1558,7 +1590,7 @@ __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* 
     if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
     const int nwork = sh.work_pref[sh.nscn];
     const WorkItems W = work_items(sh, nwork, blockIdx.x, gridDim.x);
-    P2GNext next{sm, sh, dem_map, W.w0, W.w1, W.step, 0, W.w1, 0, many_rounds(sh, nwork) || ordered_by_size(sh, nwork), false};
+    P2GNext<P2GTileSmem> next{sm, sh, dem_map, W.w0, W.w1, W.step, 0, W.w1, 0, many_rounds(sh, nwork) || ordered_by_size(sh, nwork), false, 0};
     if (tid == 0 && next.w < next.w1) next.take();
     if (words && next.w < next.w1 && next.w != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + next.w)[tid];
     if (words) reinterpret_cast<int*>(&sm.d[0])[tid] = dn;
@@ -1572,14 +1604,14 @@ __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* 
             load_scn(sh, D.sid, sm.z, tid, P2G_T);
             __syncthreads();
         }
-        if (!next.requested) p2g_request(sm, sh, D, dem_map);
+        if (!next.requested) p2g_request(sm, sh, D, next.cur, 0, dem_map);
         if (D.fresh) p2g_clear_fresh(sh, sm.z.s, D, sm.z.y.outs != 0, tid, P2G_T);
         cpa::wait_all();
         float* part = sh.part + (size_t)D.slot * PART_STRIDE;
         const TileOrigin o{cell_i(D.tij) * TILE, cell_j(D.tij) * TILE};
         if (D.total <= sh.split_min) {
             __syncthreads();  // the sums share memory with the row sums of the tile before
-            p2g_sparse_tile(sm, D, part, dem_phase, o, next);
+            p2g_sparse_tile<P2G_T, false>(sm.sp, sm.ra, sm.rb, sm.dem, &sm.dem_bar, dem_phase, sm.z, D, part, o, next);
         } else if (sm.z.y.outs) {
             p2g_dense_tile<true>(sm, D, part, dem_phase, o, next);
         } else {
@@ -1594,6 +1626,320 @@ __device__ __forceinline__ void p2g_tiles_body(const Shared& sh, unsigned char* 
 __global__ void __launch_bounds__(P2G_T, SLAB_P2G_MIN_BLOCKS) k_p2g_tiles(Shared sh, const __grid_constant__ CUtensorMap dem_map) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     p2g_tiles_body(sh, smem_raw, &dem_map);
+}
+
+// ---------------------------------------- P2G over tiles, a thread per cell
+
+// K2 of steps of many tiles, where k_p2g_tiles is bound by how many instructions
+// it issues (59 % of the slots, 4 200 warp instructions per tile of 253
+// particles): its three threads per cell each read a particle's staged
+// quantities and compute its weights along y, and 6 warps run the steps around
+// the sums. Here a thread owns a cell and all 9 nodes it reaches (54 sums in
+// registers), so
+// a particle's quantities and weights are computed once, where they are used,
+// and nothing is staged but the order of the candidates by cell. Per pass of up
+// to P2X_CAP candidates:
+//  1. count them per cell and chunk of 32 (as k_p2g_tiles);
+//  2. each thread turns its cell's counts into the chunks' write cursors, each
+//     warp the counts of its cells into places in its own list;
+//  3. every candidate's offset goes to its place (a stable counting sort); the
+//     next pass's or tile's candidates are requested into the other buffer;
+//  4. each thread adds its cell's particles in that order.
+// Then the 9 x 64 sums go to shared memory and 100 nodes add theirs in (a, b)
+// order. The operations and their order are those of k_p2g_tiles.
+// 3 000 warp instructions per tile; 8 CTAs of 2 warps per SM at 128 registers.
+// 12 M particles: 297 -> 231 us, 2 M: 59.6 -> 50.2, 300 k in a thin flow: 46.2 ->
+// 38.4. Fewer tiles are a matter of one tile's latency: 637 k in 1 900 uneven
+// tiles 47 us against 38, 12 tiles 10.5 against 10.2. Not better: the next
+// particle's values requested a turn ahead (249 us; registers), 9 CTAs (262;
+// spills), two rounds of the node sums in the space of one (240).
+constexpr int P2X_T = NCELL;                    // threads of a CTA
+constexpr int P2X_CAP = NCELL * 9 / 2;          // candidates of one pass: two float4 each are as large as the cells' float4 sums
+constexpr int P2X_PER = (P2X_CAP + P2X_T - 1) / P2X_T;
+constexpr int P2X_CHUNKS = P2X_CAP / 32;
+constexpr int P2X_DEM = ((TILE + 1) * (TILE + 1) + 7) / 8 * 8;  // a tensor copy's destination starts on 128 bytes
+#ifndef SLAB_P2X_MIN_BLOCKS
+#define SLAB_P2X_MIN_BLOCKS (NCELL == 64 ? 8 : 1)
+#endif
+
+struct P2GCellSmem {
+    union Buf {
+        struct {
+            float4 a[P2X_CAP], b[P2X_CAP];  // candidates as they lie in the particle buffer
+        } r;
+        float4 q4[NSLOT * NCELL];           // sums [row * 3 + b][cell]: m, m h, m vx, m vy
+        float q1[NSLOT * NCELL];            // then, on output steps, m vz
+        P2GSparseSmem sp;
+    };
+    alignas(128) float4 dem[2][P2X_DEM];
+    Buf buf[2];                                // this pass's candidates and the next one's
+    alignas(8) uint64_t dem_bar[2];
+    uint16_t cnt[P2X_CHUNKS][NCELL];           // cell counts of a chunk of 32 candidates
+    union {
+        uint16_t order[NCELL / 32][P2X_CAP];   // the pass's candidates by cell, for each warp's cells
+        float2 q2[NSLOT * NCELL];              // sums F, as q4
+    };
+    uint16_t cbeg[NCELL];                      // first place of a cell in order
+    int wtot[NCELL / 32];
+    TileDesc d[2];
+    int next_w;
+    ScnSm z;
+};
+
+__device__ __forceinline__ void p2x_request_cands(P2GCellSmem& sm, const TileDesc& D, int base, int buf) {
+    const PBuf B = sm.z.cur();
+    const int nc = min(D.rpref[9] - base, P2X_CAP);
+    for (int k = threadIdx.x; k < nc; k += P2X_T) {
+        int r;
+        const int src = cand_index(base + k, D, r);
+        cpa::copy16(&sm.buf[buf].r.a[k], B.a + src);
+        cpa::copy16(&sm.buf[buf].r.b[k], B.b + src);
+    }
+}
+
+// Requests tile D's first candidates and its terrain window (descriptor slot q).
+__device__ __forceinline__ void p2g_request(P2GCellSmem& sm, const Shared& sh, const TileDesc& D, int q, int buf, const CUtensorMap* dem_map) {
+    p2x_request_cands(sm, D, 0, buf);
+    if (threadIdx.x == 0) {
+        tma::fence_proxy_async();
+        tma::mbar_arrive_expect_tx(&sm.dem_bar[q], (TILE + 1) * (TILE + 1) * 16);
+        tma::tensor_g2s_2d(sm.dem[q], dem_map, 4 * cell_j(D.tij) * TILE, cell_i(D.tij) * TILE, &sm.dem_bar[q]);
+    }
+}
+
+template <bool OUTS, typename Next>
+__device__ __forceinline__ void p2g_cell_tile(P2GCellSmem& sm, const TileDesc& D, float* part, uint32_t dem_phase, TileOrigin o, int& cb,
+                                              Next& next) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int q = next.cur;
+    Ctl* const ctl = sm.z.s.ctl;
+    const int ncand = D.rpref[9];
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 am[NSLOT], av[NSLOT], aF[NSLOT];
+    float az[OUTS ? NSLOT : 1];
+#pragma unroll
+    for (int k = 0; k < NSLOT; ++k) {
+        am[k] = av[k] = aF[k] = zero;
+        if (OUTS) az[k] = 0.f;
+    }
+    const unsigned origin = (unsigned)pack_cell(o.i, o.j);
+    int placed = 0;
+    int base = 0;
+    do {
+        const int nc = min(P2X_CAP, ncand - base);
+        if (base) {
+            cpa::wait_all();
+            __syncthreads();  // the pass before is done with its order and counts
+        }
+        const float4* const ra = sm.buf[cb].r.a;
+        const float4* const rb = sm.buf[cb].r.b;
+        // 1. count: this thread's candidates as local cell | rank << 16, -1: not in the tile
+        int at[P2X_PER];
+#pragma unroll
+        for (int u = 0; u < P2X_PER; ++u) at[u] = -1;
+#pragma unroll
+        for (int u = 0; u < P2X_PER; ++u) {
+            const int k = tid + u * P2X_T;
+            if (k - lane >= nc) break;  // no candidate in the warp
+            if (k < nc) {
+                // both coordinates at once: a borrow leaves more than TILE - 1 in the lower half
+                const unsigned c = (unsigned)__float_as_int(rb[k].z) - origin;
+                if ((c & ~((TILE - 1u) << 16 | (TILE - 1u))) == 0u) at[u] = (int)((c >> 16) * TILE + (c & 0xffffu));
+                else if (base + k >= D.rpref[4] && base + k < D.rpref[5]) atomicOr(&ctl->err, ERR_MOVE);  // a stayer outside its tile
+            }
+            const unsigned vm = __ballot_sync(0xffffffffu, at[u] >= 0);
+            if (at[u] >= 0) {
+                const unsigned peers = __match_any_sync(vm, at[u]);
+                const int rank = __popc(peers & ((1u << lane) - 1u));
+                if (rank == 0) sm.cnt[warp + u * (P2X_T / 32)][at[u]] = (uint16_t)__popc(peers);
+                at[u] |= rank << 16;
+            }
+        }
+        __syncthreads();
+        if (base == 0) next.fetch();
+        // 2. exclusive prefix over the chunks of the thread's cell, then over the warp's cells
+        int num = 0;
+#pragma unroll
+        for (int c = 0; c < P2X_CHUNKS; ++c) {
+            const int x = sm.cnt[c][tid];
+            sm.cnt[c][tid] = (uint16_t)num;
+            num += x;
+        }
+        int e = num;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, e, s);
+            if (lane >= s) e += y;
+        }
+        if (lane == 31) sm.wtot[warp] = e;
+        e -= num;
+        sm.cbeg[tid] = (uint16_t)e;
+        if (base == 0 && !tma::mbar_wait(&sm.dem_bar[q], dem_phase)) atomicOr(&ctl->err, ERR_TIMEOUT);  // the terrain window
+        __syncthreads();
+        // 3. the candidates' order by cell, as byte offsets
+#pragma unroll
+        for (int u = 0; u < P2X_PER; ++u)
+            if (at[u] >= 0) {
+                const int lc = at[u] & 0xffff;
+                const int p = (int)sm.cbeg[lc] + (int)sm.cnt[warp + u * (P2X_T / 32)][lc] + (at[u] >> 16);
+                sm.order[lc >> 5][p] = (uint16_t)(16 * (tid + u * P2X_T));
+            }
+        if (tid == 0)
+            for (int w = 0; w < NCELL / 32; ++w) placed += sm.wtot[w];
+        if (base == 0) next.store();
+        __syncthreads();
+        for (int k = tid; k < P2X_CHUNKS * NCELL / 2; k += P2X_T) reinterpret_cast<uint32_t*>(&sm.cnt[0][0])[k] = 0;  // for the next pass or tile
+        next.buf = cb ^ 1;
+        if (base + P2X_CAP >= ncand) next.request();
+        else p2x_request_cands(sm, D, base + P2X_CAP, cb ^ 1);
+        // 4. the cell's particles over its 9 nodes
+        const uint16_t* const ord = sm.order[warp] + e;
+        const float4* const dem = sm.dem[q] + (tid / TILE) * (TILE + 1) + tid % TILE;
+        const float g = sm.z.s.g, hod = 0.5f * sm.z.s.ood;
+        for (int r = 0; r < num; ++r) {
+            const int k16 = ord[r];
+            const float4* const pa = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(ra) + k16);
+            const float4 a = pa[0], b = pa[P2X_CAP];
+            const float4 qd = dem[(a.x >= 1.f ? TILE + 1 : 0) + (a.y >= 1.f ? 1 : 0)];
+            const float h = b.x, m = b.y;
+            const float K = m * g * qd.z * qd.z;
+            const float2 pm = make_float2(m, m * h), pv = make_float2(m * a.z, m * a.w), pk = make_float2(-(K * qd.x), -(K * qd.y));
+            const float khs = K * h * hod;
+            const float2 kh = make_float2(khs, khs);
+            float2 wx[3], wy[3];
+            float dwx[3], dwy[3];
+            spline_y(a.x, wx, dwx);
+            spline_y(a.y, wy, dwy);
+            float mz = 0.f;
+            if (OUTS) {
+                int d;
+                const int src = cand_index(base + k16 / 16, D, d);
+                mz = m * sm.z.cur().vz[src];
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const int k = 3 * i + j;
+                    const float2 w = f2mul(wx[i], wy[j]);
+                    if (w.x > 3e-3f) {  // the reference's weight cut-off (src/simulation.cpp:780)
+                        am[k] = f2fma(pm, w, am[k]);
+                        av[k] = f2fma(pv, w, av[k]);
+                        const float2 gr = f2mul(make_float2(dwx[i], wx[i].x), make_float2(wy[j].x, dwy[j]));
+                        aF[k] = f2add(aF[k], f2fma(kh, gr, f2mul(pk, w)));
+                        if (OUTS) az[k] = __fmaf_rn(mz, w.x, az[k]);
+                    }
+                }
+        }
+        base += P2X_CAP;
+        cb ^= 1;
+    } while (base < ncand);
+    if (tid == 0 && placed != D.total) atomicOr(&ctl->err, ERR_CAPACITY);
+    // the cells' sums into the window, over the candidates just summed
+    auto& cs = sm.buf[cb ^ 1];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NSLOT; ++k) {
+        cs.q4[k * NCELL + tid] = make_float4(am[k].x, am[k].y, av[k].x, av[k].y);
+        sm.q2[k * NCELL + tid] = aF[k];
+    }
+    __syncthreads();
+    for (int n = tid; n < NWIN; n += P2X_T) {
+        const int i = n / TN, j = n % TN;
+        float2 m = zero, v = zero, F = zero;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const int ci = i - a, cj = j - b;
+                if ((unsigned)ci < TILE && (unsigned)cj < TILE) {
+                    const int k = (a * 3 + b) * NCELL + ci * TILE + cj;
+                    const float4 x = cs.q4[k];
+                    m = f2add(m, make_float2(x.x, x.y));
+                    v = f2add(v, make_float2(x.z, x.w));
+                    F = f2add(F, sm.q2[k]);
+                }
+            }
+        reinterpret_cast<float4*>(part)[n] = make_float4(m.x, m.y, v.x, v.y);
+        reinterpret_cast<float2*>(part + 4 * NWIN)[n] = F;
+    }
+    if (OUTS) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < NSLOT; ++k) cs.q1[k * NCELL + tid] = az[k];
+        __syncthreads();
+        for (int n = tid; n < NWIN; n += P2X_T) {
+            const int i = n / TN, j = n % TN;
+            float z = 0.f;
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const int ci = i - a, cj = j - b;
+                    if ((unsigned)ci < TILE && (unsigned)cj < TILE) z = __fadd_rn(z, cs.q1[(a * 3 + b) * NCELL + ci * TILE + cj]);
+                }
+            part[6 * NWIN + n] = z;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(P2X_T, SLAB_P2X_MIN_BLOCKS) k_p2g_cells(Shared sh, const __grid_constant__ CUtensorMap dem_map) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    P2GCellSmem& sm = *reinterpret_cast<P2GCellSmem*>(smem_raw);
+    const int tid = threadIdx.x;
+    int dn = 0;
+    const bool words = tid < DESC_WORDS;
+    if (sh.nscn == 1) load_scn_static(sh, 0, sm.z, tid, P2X_T);
+    else if (tid == 0) sm.z.sid = -1;
+    for (int k = tid; k < P2X_CHUNKS * NCELL / 2; k += P2X_T) reinterpret_cast<uint32_t*>(&sm.cnt[0][0])[k] = 0;
+    if (tid == 0) {
+        tma::mbar_init(&sm.dem_bar[0], 1);
+        tma::mbar_init(&sm.dem_bar[1], 1);
+        tma::fence_mbar_init();
+    }
+    chain_wait<false>();
+    if (words && (int)blockIdx.x < sh.work_cap) dn = reinterpret_cast<const int*>(sh.desc + blockIdx.x)[tid];
+    if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
+    const int nwork = sh.work_pref[sh.nscn];
+    const WorkItems W = work_items(sh, nwork, blockIdx.x, gridDim.x);
+    P2GNext<P2GCellSmem> next{sm, sh, &dem_map, W.w0, W.w1, W.step, 0, W.w1, 0, many_rounds(sh, nwork), false, 0};
+    if (tid == 0 && next.w < next.w1) next.take();
+    if (words && next.w < next.w1 && next.w != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + next.w)[tid];
+    if (words) reinterpret_cast<int*>(&sm.d[0])[tid] = dn;
+    __syncthreads();
+    uint32_t phases = 0;  // bit q: parity of the next completion of terrain window q
+    int cb = 0;           // buffer of the running pass
+    for (; next.w < next.w1; next.cur ^= 1) {
+        const int q = next.cur;
+        const TileDesc& D = sm.d[q];
+        if (tid == 0) sm.next_w = next.wn;
+        if (D.sid != sm.z.sid) {  // uniform: a new scenario in this CTA's run
+            __syncthreads();
+            load_scn(sh, D.sid, sm.z, tid, P2X_T);
+            __syncthreads();
+        }
+        if (!next.requested) p2g_request(sm, sh, D, q, cb, &dem_map);
+        if (D.fresh) p2g_clear_fresh(sh, sm.z.s, D, sm.z.y.outs != 0, tid, P2X_T);
+        cpa::wait_all();
+        float* part = sh.part + (size_t)D.slot * PART_STRIDE;
+        const TileOrigin o{cell_i(D.tij) * TILE, cell_j(D.tij) * TILE};
+        const uint32_t phase = phases >> q & 1u;
+        if (D.total <= sh.split_min) {
+            next.buf = cb ^ 1;
+            p2g_sparse_tile<P2X_T, true>(sm.buf[cb].sp, sm.buf[cb].r.a, sm.buf[cb].r.b, sm.dem[q], &sm.dem_bar[q], phase, sm.z, D, part, o, next);
+            cb ^= 1;
+        } else if (sm.z.y.outs) {
+            p2g_cell_tile<true>(sm, D, part, phase, o, cb, next);
+        } else {
+            p2g_cell_tile<false>(sm, D, part, phase, o, cb, next);
+        }
+        phases ^= 1u << q;
+    }
+    __syncthreads();
+    if (tid == 0) {  // every copy was waited for
+        tma::mbar_inval(&sm.dem_bar[0]);
+        tma::mbar_inval(&sm.dem_bar[1]);
+    }
 }
 
 // ------------------------------------------------------------ grid update

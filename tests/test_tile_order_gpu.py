@@ -58,6 +58,32 @@ def test_alone_equals_beside_another(kind):
     b.close()
 
 
+def test_thread_per_cell_equals_thread_per_row():
+    """Steps of more than 4 096 tiles sum with a thread per cell, in passes of
+    288 candidates; persistent steps with three. The same operations in the same
+    order: the same bits, also of the grid members of an output step."""
+    rng = np.random.default_rng(21)
+    counts = rng.permutation(np.concatenate([rng.integers(1, 120, 4300), [48, 49, 287, 288, 289, 575, 576, 577, 1000]]))
+    P = _scenario(70, counts, 22)
+    i = np.arange(8 * 70)
+    out = []
+    for persistent in (False, True):
+        s = slab.Slab(-0.3 * i[:, None] * DX + 0.2 * np.sin(0.2 * i)[None, :], DX)
+        s.set_params(CFG, slab.FP32_SPLIT)
+        s.set_persistent(persistent)
+        s.upload(P)
+        s.initial_pass()
+        g = s.grid()
+        s.advance_to_frame()
+        out.append((s.particles(), g, s.grid(), s.state()))
+        s.close()
+    (Pa, ga, fa, sa), (Pb, gb, fb, sb) = out
+    assert sa == sb
+    for a, b in ((Pa, Pb), (ga, gb), (fa, fb)):
+        for k in a:
+            assert np.array_equal(a[k], b[k]), k
+
+
 @pytest.mark.parametrize("n", [383, 384, 385, 768, 769])
 def test_pass_edges_against_fp64(n):
     tiles.test_tile_sums_against_fp64(n, True)
