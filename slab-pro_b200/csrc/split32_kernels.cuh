@@ -595,12 +595,13 @@ constexpr int P2G_MIN_BLOCKS = NCELL == 64 ? 16 : 4;
 //            part below one quantum -- each contribution keeps about FP32
 //            precision relative to itself; two plain (non-returning) atomics
 //  ACC_I64   one int64 per sum at 2^-52 of the bound
-//  ACC_CELL  no fixed point: k_p2g_cell, FP32 sums over cell-sorted particles
+//  ACC_CELL  no fixed point: every tile by k_p2g_tiles / k_p2g_cells, FP32
+//            sums over cell-sorted particles
 //  ACC_WARP  k_p2g_warp: ACC_HILO sums with one warp per tile
-//  ACC_MIXED dense tiles (more than split_min particles) by k_p2g_cell, the
-//            others by k_p2g_sparse (64-bit fixed point): each tile's scheme
-//            depends only on its particle count, so results are still
-//            reproducible
+//  ACC_MIXED dense tiles (more than split_min particles) as ACC_CELL, the
+//            others in fixed point (p2g_sparse_tile), in the same launch: a
+//            tile's scheme depends only on its particle count, so results are
+//            still reproducible
 enum { ACC_I32 = 0, ACC_HILO = 1, ACC_I64 = 2, ACC_CELL = 3, ACC_WARP = 4, ACC_MIXED = 5 };
 
 struct P2GSmem {
