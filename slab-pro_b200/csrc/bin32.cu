@@ -187,7 +187,10 @@ BinResult bin_particles(const Terrain& T, int TY, int ntiles, cudaStream_t st, i
     SLAB_CUDA(cudaGetLastError());
     res.tiles.resize(n);
     SLAB_CUDA(cudaMemcpyAsync(res.tiles.data(), uniq, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    std::vector<int32_t> held(n <= FUSED_MAX_TILES ? n : 0);
+    if (!held.empty()) SLAB_CUDA(cudaMemcpyAsync(held.data(), counts, held.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     SLAB_CUDA(cudaStreamSynchronize(st));  // the scratch is free again on return
+    for (const int32_t c : held) res.heaviest = std::max(res.heaviest, (int)c);
     for (int k = 0; k < 4; ++k) res.box_bits[k] = hred[k];
     res.vmax2_bits = hred[4];
     return res;

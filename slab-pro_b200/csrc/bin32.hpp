@@ -10,6 +10,7 @@ namespace slab {
 
 struct BinResult {
     std::vector<uint32_t> tiles;  // occupied tiles in increasing order (the first active list)
+    int heaviest = 0;             // most particles in a tile; counted for at most FUSED_MAX_TILES tiles
     uint64_t box_bits[4] = {0x7ff0000000000000ull, 0, 0x7ff0000000000000ull, 0};  // min x, max x, min y, max y (double bits)
     uint64_t vmax2_bits = 0;      // max |v|^2 of the FP32 velocities (double bits)
 };

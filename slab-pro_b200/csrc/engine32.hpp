@@ -43,15 +43,23 @@ class Engine32 {
     void launch_step();
     static constexpr int NKERNELS = 5;  // of a step: k_prep, P2G, grid update, G2P, k_end
     void launch_kernel(int k, const Shared& sh);
-    // Steps of few active tiles run the grid update inside G2P (k_g2p_fused),
-    // with the same bits: per step 17 against 21 us at 12 tiles, 26 against 30
-    // at 734, 68 against 71 at 1 900, but 132 against 129 at 7 900 (8 000 tiles
-    // of a thin flow: 98 against 93), where computing the nodes on the tiles'
-    // edges up to four times costs more than a kernel. tiles_seen is what the
-    // host saw last.
-    static constexpr int64_t FUSED_MAX_TILES = 4096;
+    // Whether a step runs k_p2g_tiles and the grid update inside G2P, or
+    // k_p2g_cells, k_grid and k_g2p; the same bits. The first chain is shorter
+    // for one tile, the second costs fewer instructions per tile, so the line
+    // depends on how many tiles there are and how long the heaviest takes. us per
+    // step, first / second: 12 tiles 17 / 21, 734 of up to 256 particles 24 / 31,
+    // 1 700 36.5 / 39.8, 3 260 57.5 / 54.5, 4 080 68 / 62; of up to 90 particles
+    // 2 900 43 / 40; of up to 360 2 134 44 / 45 and 3 371 56 / 54; of up to 565
+    // 1 967 45 / 54 and 3 317 66 / 67; of up to 810 3 318 81 / 85; of up to 1 060
+    // 2 516 76 / 92. Equal at about 1 500 tiles and 3 for each particle of the
+    // heaviest. Of several scenarios the heaviest tile is not known; there the
+    // line is at FUSED_MAX_TILES. Both numbers are what the host saw last.
+    static constexpr int64_t FUSED_TILES = 1500, FUSED_TILES_PER_PARTICLE = 3;
     int64_t tiles_seen = 0;
-    bool fused() const { return tiles_seen <= FUSED_MAX_TILES; }
+    int64_t heaviest_seen = 0;  // 0: nobody counted, steps of more than FUSED_MAX_TILES tiles
+    bool fused() const {
+        return tiles_seen <= FUSED_MAX_TILES && (batch || tiles_seen <= FUSED_TILES + FUSED_TILES_PER_PARTICLE * heaviest_seen);
+    }
     void launch_p2g(const Shared& sh);
     CUtensorMap dem_map;   // the FP32 terrain as [Nx][4 Ny] floats, 9 x 9-node boxes (P2G's terrain window)
     // persistent steps: a chunk of steps as one cooperative launch of k_persist

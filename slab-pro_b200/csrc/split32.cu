@@ -568,6 +568,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
         if (2 * need > blk_cap) grow_blocks((int)std::min<int64_t>(std::max<int64_t>(2 * (int64_t)blk_cap, 2 * need), INT32_MAX / NCELL));
     }
     tiles_seen = (batch ? tiles_seen : 0) + (int64_t)alist.size();
+    heaviest_seen = bin.heaviest;
     SLAB_CUDA(cudaMemsetAsync(S.gt_stamp.get(), 0xff, ntiles * sizeof(int32_t), st));
     SLAB_CUDA(cudaMemsetAsync(S.blk_of.get(), 0xff, ntiles * sizeof(int32_t), st));
     SCnt c0{};
@@ -1175,7 +1176,9 @@ struct Split32 final : Path {
     }
     bool reusable() const override { return !E.dead; }
     void observe(const Ctl& c) override {
-        if (c.active || c.steps) E.tiles_seen = c.tiles;
+        if (!c.active && !c.steps) return;
+        E.tiles_seen = c.tiles;
+        if (c.heaviest) E.heaviest_seen = c.heaviest;
     }
     void initial_pass() override { E.launch_t0(); }
     void enqueue_steps(int chunk) override { E.enqueue_steps(chunk); }

@@ -66,6 +66,8 @@ struct SCnt {
     int32_t outs;          // the running step writes output fields
     double grid_mass;      // FP64 sum of node masses of the last grid update
     int32_t t0_pending;    // the scenario still needs simulate()'s t=0 pass
+    int32_t heaviest;      // most particles in a tile of the running step (k_prep, steps of at most FUSED_MAX_TILES tiles)
+    int32_t pad_;
     int32_t vz_valid;      // buffer vz / z were written by the last G2P (an output step)
 };
 
@@ -96,6 +98,7 @@ struct TileDesc {
     int32_t slot;     // the tile's place on the active list: that of its partial window
     int32_t pad_;
 };
+constexpr int FUSED_MAX_TILES = 4096;  // most active tiles of a step whose grid update runs inside G2P (Engine32::fused)
 constexpr int BLK_LATER = -2;  // the block was being allocated while the descriptor was written (a grid tile's first step)
 static_assert(sizeof(TileDesc) % 16 == 0, "descriptors lie on 16-byte boundaries");
 

@@ -4,7 +4,7 @@
 //                      segment in the next buffer, node blocks of new grid tiles
 //   k_p2g_tiles (grid) one CTA per active tile: P2G partial sums, tiles of
 //                      more than split_min particles sorted by cell, the
-//                      others in fixed point
+//                      others in fixed point; k_p2g_cells in steps of many tiles
 //   k_grid   (grid)    steps of many tiles: grid update + friction, a warp per
 //                      half grid tile
 //   k_g2p    (grid)    one CTA per active tile: (steps of few tiles: grid update
@@ -177,6 +177,8 @@ __device__ __forceinline__ int step_control(const Shared& sh, int s, int what, i
         n.act_count[0] = (n.seq & 1) ? 0 : n.act_count[0];  // the next step's list starts empty
         n.act_count[1] = (n.seq & 1) ? n.act_count[1] : 0;
         n.cursor = 0;
+        if (n.heaviest) k.heaviest = n.heaviest;
+        n.heaviest = 0;
         n.grid_mass = 0.0;
         n.outs = k.write_outputs;
         const int frame_after = k.frame + (k.frame_end ? 1 : 0);
@@ -490,6 +492,10 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
                     if (lane >= o) ic += yc;
                 }
                 const unsigned hm = __ballot_sync(0xffffffffu, by_size && has && qc > heavy), lm = __ballot_sync(0xffffffffu, by_size && has && qc <= heavy);
+                if (nwork <= FUSED_MAX_TILES) {  // the host chooses the step's kernels by it
+                    const unsigned top = __reduce_max_sync(0xffffffffu, (unsigned)qc);
+                    if (lane == 0) atomicMax(&sh.cnt[0].heaviest, (int)top);
+                }
                 unsigned long long old = 0;
                 if (lane == 31)
                     old = atomicAdd(reinterpret_cast<unsigned long long*>(&sh.cnt[0].cursor),
@@ -2242,7 +2248,7 @@ template <int T> __device__ __forceinline__ void g2p_sync() {
 // for 64 cells, nodes near an edge computed by up to 4 tiles, but no kernel of
 // its own between P2G and G2P: per step 22 -> 18.5 us at 1 600 particles, 30 ->
 // 27 at 180 k (734 tiles), 76 -> 63 at 637 k (1 900 tiles); at 2 M particles
-// (8 000 tiles) the pass through memory is the cheaper one.
+// (8 000 tiles) the pass through memory is the cheaper one (Engine32::fused).
 //
 // k_g2p (T = 32), for steps of many: the window comes from the node blocks. One
 // warp per CTA, because the rounds of a tile (descriptor, candidates and window,
