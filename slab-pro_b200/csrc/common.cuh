@@ -47,7 +47,6 @@ struct Ctl {
     // The reference's remeshed grid box for the current step
     // (src/simulation.cpp:602-612): nodes [box[0], box[1]] x [box[2], box[3]].
     int32_t box[4];
-    uint32_t done_blocks;  // last-block-done counter
     int32_t tiles;         // FP32: active tiles of the current step
     int32_t heaviest;      // FP32: particles of its heaviest tile, 0 where nobody counted (steps of many tiles)
     int32_t keep_outputs;  // write grid output fields every step (tests); else frame steps only
@@ -153,11 +152,10 @@ __device__ inline void ctl_begin(Ctl* c, int Nx, int Ny) {
     c->pos_acc[2] = 0x7ff0000000000000ull;
     c->pos_acc[3] = 0;
     c->vmax2_acc = 0;
-    c->done_blocks = 0;
     c->active = 1;
 }
 
-// End of a step, one thread (the last block of G2P): time += dt and the frame
+// End of a step, one thread of the control kernel: time += dt and the frame
 // bump of simulate() (src/simulation.cpp:503-505).
 __device__ inline void ctl_end(Ctl* c) {
     c->time = c->new_time;

@@ -298,7 +298,7 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     grid_grid = sms * std::max(occ_u, 1);
     int occ_d = 0;
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_d, k32::k_prep, 256, 0));
-    grid_prep = sms * std::max(occ_d, 1);  // one resident wave, one thread per active tile
+    grid_prep = sms * std::max(occ_d, 1);  // one resident wave
     const int base[Tuner::NK] = {grid_prep, grid_p2g_cell, grid_p2g_sparse, grid_grid, grid_g2p};
     std::copy(base, base + Tuner::NK, tune.base);
     if (const char* e = std::getenv("SLAB_TUNE")) tune.enabled = std::atoi(e) != 0;

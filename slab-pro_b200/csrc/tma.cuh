@@ -1,13 +1,11 @@
-// Bulk asynchronous copies (the TMA engine's 1-D form, cp.async.bulk) from
-// global into shared memory, completed on an mbarrier, for sm_100a. Used to
-// stage the next work item's contiguous particle ranges and terrain rows
-// while the current one is computed. Only this GPU's own memory is ever a
-// source, and no copy is multicast.
+// Asynchronous tensor copies (cp.async.bulk.tensor) from global into shared
+// memory, completed on an mbarrier, for sm_100a. Used to stage the next tile's
+// terrain window while the current one is computed. Only this GPU's own memory
+// is ever a source, and no copy is multicast.
 //
-// Rules of the instruction that the callers keep: source and destination
-// 16-byte aligned, size a positive multiple of 16; a thread that issues copies
-// into a buffer first orders the CTA's earlier ordinary accesses of it with
-// fence_proxy_async(); every wait is bounded.
+// Rules that the callers keep: a thread that issues a copy into a buffer first
+// orders the CTA's earlier ordinary accesses of it with fence_proxy_async();
+// every wait is bounded.
 #pragma once
 
 #include <cuda.h>  // CUtensorMap
@@ -32,7 +30,7 @@ __device__ __forceinline__ void mbar_inval(uint64_t* bar) {
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
 // order the CTA's earlier ordinary shared-memory accesses (after a barrier)
-// before later bulk copies into the same bytes
+// before later tensor copies into the same bytes
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // one arrival that also announces `bytes` of copies to come
@@ -64,14 +62,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int li
     return false;
 }
 
-// bytes (a multiple of 16) from global src to shared dst (both 16-byte
-// aligned), completing on bar
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-
 // A box of a 2-D tensor (map built on the host by cuTensorMapEncodeTiled)
 // into shared memory (128-byte aligned), completing on bar. x is the inner
 // coordinate in elements; x times the element size must be a multiple of 16.
@@ -88,17 +78,10 @@ __device__ __forceinline__ void tensor_g2s_2d(void* dst, const CUtensorMap* map,
 
 // Per-thread asynchronous copies global -> shared (cp.async): a thread
 // requests many small copies without holding the values in registers, so a
-// whole work item's gather goes out in one round. Each copy is 4, 8 or 16
-// bytes with both addresses aligned to its size; wait_all() completes the
-// thread's own copies, and a CTA barrier after it shows them to the others.
+// whole work item's gather goes out in one round. Both addresses are 16-byte
+// aligned; wait_all() completes the thread's own copies, and a CTA barrier after it shows them to the others.
 namespace cpa {
 
-__device__ __forceinline__ void copy4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(tma::smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(tma::smem_addr(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void copy16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tma::smem_addr(dst)), "l"(src) : "memory");
 }
