@@ -41,6 +41,7 @@ namespace {
 
 template <typename F> slab_status bguard(slab_batch* b, F&& f) {
     try {
+        const BlockScope scope(b ? b->stream : nullptr);
         f();
         if (b) b->err.clear();
         return SLAB_OK;
@@ -356,13 +357,16 @@ const char* slab_batch_last_error(const slab_batch* b) { return b ? b->err.c_str
 void slab_batch_destroy(slab_batch* b) {
     if (!b) return;
     if (b->stream) cudaStreamSynchronize(b->stream);
-    b->E.reset();
-    b->terrain.z.reset();
-    b->terrain.grad.reset();
-    b->terrain.cos_t.reset();
-    b->terrain.dem32.reset();
-    release_device(b->d_ctl);
-    release_pinned(b->h_ctl);
+    {
+        const BlockScope scope(b->stream);
+        b->E.reset();
+        b->terrain.z.reset();
+        b->terrain.grad.reset();
+        b->terrain.cos_t.reset();
+        b->terrain.dem32.reset();
+        release_device(b->d_ctl);
+        release_pinned(b->h_ctl);
+    }
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     delete b;
 }

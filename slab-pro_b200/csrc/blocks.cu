@@ -1,13 +1,14 @@
 // The kept blocks of blocks.hpp.
 #include "blocks.hpp"
 
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <mutex>
 #include <string>
 #include <unordered_map>
 
-#include "engine.hpp"
+#include "error.hpp"
 
 namespace slab {
 namespace {
@@ -19,14 +20,13 @@ constexpr int PINNED = -1;  // "device" of the page-locked blocks
 
 struct Kept {
     void* p;
-    uint64_t released;  // release number; in flight until a wait that began later is over
+    uint64_t released;  // release number
 };
 
 struct Pool {
-    std::multimap<size_t, Kept> kept;  // by size
+    std::multimap<size_t, Kept> kept;  // by size; nothing uses them
     size_t bytes = 0;
     size_t bound = 0;                  // of `bytes` while a context lives (0: not yet asked)
-    uint64_t idle_upto = 0;            // blocks released up to this number have no work in flight
 };
 
 struct Live {
@@ -48,6 +48,8 @@ Blocks& blocks() {
     return *b;
 }
 
+thread_local BlockScope* t_scope = nullptr;
+
 // Size classes: four per octave up to 1 MiB, then multiples of 2 MiB (the
 // driver's own granularity).
 size_t size_class(size_t n) {
@@ -57,93 +59,166 @@ size_t size_class(size_t n) {
     return std::max<size_t>(512, (n + step - 1) / step * step);
 }
 
-void driver_free(int dev, void* p) {
+// a block of size `got` serves a request of class `size`: at most a quarter more
+bool serves(size_t got, size_t size) { return got >= size && got <= size + size / 4; }
+
+void driver_free(int dev, void* p) noexcept {
     if (dev == PINNED) cudaFreeHost(p);
     else cudaFree(p);
 }
 
-// oldest first, down to `bound` bytes
-void trim(int dev, Pool& pool, size_t bound) {
-    while (pool.bytes > bound && !pool.kept.empty()) {
-        auto old = pool.kept.begin();
-        for (auto it = pool.kept.begin(); it != pool.kept.end(); ++it)
-            if (it->second.released < old->second.released) old = it;
-        pool.bytes -= old->first;
-        driver_free(dev, old->second.p);
-        pool.kept.erase(old);
+// kept blocks of `dev` back to the driver, oldest first, down to `bound`
+// bytes; true if any went
+bool trim(int dev, size_t bound) noexcept {
+    Blocks& B = blocks();
+    bool any = false;
+    for (;;) {
+        void* p;
+        {
+            std::lock_guard<std::mutex> lk(B.mu);
+            const auto at = B.pools.find(dev);
+            if (at == B.pools.end() || at->second.bytes <= bound || at->second.kept.empty()) return any;
+            Pool& pool = at->second;
+            auto old = pool.kept.begin();
+            for (auto it = pool.kept.begin(); it != pool.kept.end(); ++it)
+                if (it->second.released < old->second.released) old = it;
+            p = old->second.p;
+            pool.bytes -= old->first;
+            pool.kept.erase(old);
+        }
+        driver_free(dev, p);
+        any = true;
     }
+}
+
+// a block that nothing uses, to its kept list
+void keep(const BlockScope::Held& h) noexcept {
+    Blocks& B = blocks();
+    size_t bound = 0;
+    try {
+        {
+            std::lock_guard<std::mutex> lk(B.mu);
+            bound = B.pools[h.dev].bound;
+        }
+        if (!bound) {
+            size_t free_b = 0, total_b = 0;
+            if (h.dev == PINNED) bound = PINNED_BYTES;
+            else if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) bound = std::max<size_t>(total_b / 16, MIB);
+            else bound = MIB;
+        }
+        if (h.size <= bound) {
+            {
+                std::lock_guard<std::mutex> lk(B.mu);
+                Pool& pool = B.pools[h.dev];
+                pool.bound = bound;
+                pool.kept.emplace(h.size, Kept{h.p, ++B.releases});
+                pool.bytes += h.size;
+            }
+            trim(h.dev, bound);
+            return;
+        }
+    } catch (...) {  // no room for the bookkeeping: back to the driver
+    }
+    driver_free(h.dev, h.p);
+}
+
+void* driver_alloc(int dev, size_t size, cudaError_t& e) {
+    void* p = nullptr;
+    e = dev == PINNED ? cudaMallocHost(&p, size) : cudaMalloc(&p, size);
+    if (e != cudaSuccess) cudaGetLastError();
+    return p;
 }
 
 void* take(int dev, size_t bytes, const char* what) {
     Blocks& B = blocks();
     const size_t size = size_class(bytes ? bytes : 1);
-    std::lock_guard<std::mutex> lk(B.mu);
-    Pool& pool = B.pools[dev];
-    // a kept block of at most a quarter more; one without work in flight if there is one
-    auto best = pool.kept.end();
-    int looked = 0;
-    for (auto it = pool.kept.lower_bound(size); it != pool.kept.end() && it->first <= size + size / 4 && looked < 16; ++it, ++looked) {
-        if (best == pool.kept.end()) best = it;
-        if (dev == PINNED || it->second.released <= pool.idle_upto) {
-            best = it;
-            break;
-        }
-    }
-    if (best != pool.kept.end()) {
-        if (dev != PINNED && best->second.released > pool.idle_upto) {
-            SLAB_CUDA(cudaDeviceSynchronize());
-            pool.idle_upto = B.releases;
-        }
-        void* p = best->second.p;
-        const size_t got = best->first;
-        B.live[p] = Live{got, dev};
-        pool.bytes -= got;
-        pool.kept.erase(best);
-        return p;
-    }
     void* p = nullptr;
-    cudaError_t e = dev == PINNED ? cudaMallocHost(&p, size) : cudaMalloc(&p, size);
-    if (e != cudaSuccess && pool.bytes) {
-        cudaGetLastError();
-        trim(dev, pool, 0);
-        e = dev == PINNED ? cudaMallocHost(&p, size) : cudaMalloc(&p, size);
+    size_t got = size;
+    // one that this scope released, the smallest that serves
+    BlockScope* const s = t_scope;
+    if (s) {
+        auto best = s->held.end();
+        for (auto it = s->held.begin(); it != s->held.end(); ++it)
+            if (it->dev == dev && serves(it->size, size) && (best == s->held.end() || it->size < best->size)) best = it;
+        if (best != s->held.end()) {
+            p = best->p;
+            got = best->size;
+            s->held.erase(best);
+        }
     }
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        throw Error{SLAB_E_OOM, std::string(what) + " of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e)};
+    if (!p) {
+        std::lock_guard<std::mutex> lk(B.mu);
+        const auto at = B.pools.find(dev);
+        if (at != B.pools.end()) {
+            const auto it = at->second.kept.lower_bound(size);
+            if (it != at->second.kept.end() && serves(it->first, size)) {
+                p = it->second.p;
+                got = it->first;
+                at->second.bytes -= got;
+                at->second.kept.erase(it);
+            }
+        }
     }
-    B.live[p] = Live{size, dev};
+    if (!p) {
+        cudaError_t e;
+        p = driver_alloc(dev, size, e);
+        if (e != cudaSuccess) {
+            if (s) s->flush();
+            if (trim(dev, 0)) p = driver_alloc(dev, size, e);
+        }
+        if (e != cudaSuccess)
+            throw Error{SLAB_E_OOM, std::string(what) + " of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e)};
+    }
+    try {
+        std::lock_guard<std::mutex> lk(B.mu);
+        B.live[p] = Live{got, dev};
+    } catch (...) {
+        driver_free(dev, p);
+        throw;
+    }
     return p;
 }
 
 void release(void* p) noexcept {
     if (!p) return;
     Blocks& B = blocks();
-    std::lock_guard<std::mutex> lk(B.mu);
-    const auto it = B.live.find(p);
-    if (it == B.live.end()) return;
-    const Live l = it->second;
-    B.live.erase(it);
-    try {
-        Pool& pool = B.pools[l.dev];
-        if (!pool.bound) {
-            size_t free_b = 0, total_b = 0;
-            if (l.dev == PINNED) pool.bound = PINNED_BYTES;
-            else if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) pool.bound = std::max<size_t>(total_b / 16, MIB);
-            else pool.bound = MIB;
-        }
-        if (l.size <= pool.bound) {
-            pool.kept.emplace(l.size, Kept{p, ++B.releases});
-            pool.bytes += l.size;
-            trim(l.dev, pool, pool.bound);
-            return;
-        }
-    } catch (...) {  // no room for the bookkeeping: back to the driver
+    BlockScope::Held h{p, 0, 0};
+    {
+        std::lock_guard<std::mutex> lk(B.mu);
+        const auto it = B.live.find(p);
+        if (it == B.live.end()) return;
+        h.size = it->second.size;
+        h.dev = it->second.dev;
+        B.live.erase(it);
     }
-    driver_free(l.dev, p);
+    if (t_scope && t_scope->stream) {
+        try {
+            t_scope->held.push_back(h);
+            return;
+        } catch (...) {  // no room for the bookkeeping: back to the driver
+        }
+    }
+    driver_free(h.dev, p);
 }
 
 }  // namespace
+
+BlockScope::BlockScope(cudaStream_t st) noexcept : stream(st), outer(t_scope) { t_scope = this; }
+
+BlockScope::~BlockScope() {
+    flush();
+    t_scope = outer;
+}
+
+void BlockScope::flush() noexcept {
+    if (held.empty()) return;
+    const bool idle = cudaStreamSynchronize(stream) == cudaSuccess;
+    for (const Held& h : held) {
+        if (idle) keep(h);
+        else driver_free(h.dev, h.p);
+    }
+    held.clear();
+}
 
 void* take_device(size_t bytes) {
     int dev = 0;
@@ -169,9 +244,17 @@ MemoryUser::MemoryUser() {
 }
 MemoryUser::~MemoryUser() {
     Blocks& B = blocks();
-    std::lock_guard<std::mutex> lk(B.mu);
-    if (--B.users == 0)
-        for (auto& kv : B.pools) trim(kv.first, kv.second, kv.first == PINNED ? IDLE_BYTES / 4 : IDLE_BYTES);
+    int dev = PINNED - 1;
+    for (;;) {  // every pool, in order
+        {
+            std::lock_guard<std::mutex> lk(B.mu);
+            if (dev < PINNED && --B.users != 0) return;
+            const auto next = B.pools.upper_bound(dev);
+            if (next == B.pools.end()) return;
+            dev = next->first;
+        }
+        trim(dev, dev == PINNED ? IDLE_BYTES / 4 : IDLE_BYTES);
+    }
 }
 
 }  // namespace slab

@@ -7,21 +7,29 @@
 // 64 MiB cudaMallocHost 41 ms: more than the steps of a small run.
 //
 // Rules:
-//  - release_device() may be called with work in flight on the block, as
-//    cudaFree may: the block is handed out again only after a
-//    cudaDeviceSynchronize() that began after the release (one such wait
-//    covers every block released before it). cudaFree waits the same way.
-//  - release_pinned() is called when no copy uses the block any more.
+//  - A block may be released with work in flight on it, if that work is on the
+//    stream of the calling thread's BlockScope. The scope holds the block: the
+//    same scope may take it again at once, since what it does with the block
+//    comes later on the same stream; everybody else gets it after the scope
+//    has waited for its stream, at its end. Released outside a scope a block
+//    goes to the driver, which waits by itself. So a kept block has no work in
+//    flight, and no wait is wider than one stream: CUDA refuses to wait for a
+//    device, whatever the capture mode, while any stream of it is being
+//    captured, and other contexts' threads capture their step graphs at any time.
 //  - The blocks kept are bounded per device (1/16 of its memory while a
 //    context lives, IDLE_BYTES after the last one closed; page-locked memory:
 //    PINNED_BYTES, IDLE_BYTES / 4), and all of a device's go back to the
 //    driver when an allocation fails, before it is tried again.
 //  - A block belongs to the device that was current when it was taken.
-//  - One mutex guards the lists: any thread may take and release blocks.
+//  - One mutex guards the lists: any thread may take and release blocks. No
+//    driver call is made while it is held.
 //  - Contents are undefined, as cudaMalloc's are.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstddef>
+#include <vector>
 
 namespace slab {
 
@@ -30,6 +38,31 @@ void release_device(void* p) noexcept;
 void* take_pinned(size_t bytes);
 void release_pinned(void* p) noexcept;
 size_t kept_device_bytes();  // kept on the current device, handed back if an allocation needs them
+
+// One per call into a context, on the calling thread: all that the call does
+// with blocks is on `st`, or over before it releases them. nullptr: the stream
+// is not known, releases go to the driver. Scopes may nest.
+class BlockScope {
+  public:
+    explicit BlockScope(cudaStream_t st) noexcept;
+    ~BlockScope();
+    BlockScope(const BlockScope&) = delete;
+    BlockScope& operator=(const BlockScope&) = delete;
+
+    struct Held {
+        void* p;
+        size_t size;
+        int dev;
+    };
+    // Waits for the stream and puts the held blocks on the kept lists.
+    void flush() noexcept;
+
+    const cudaStream_t stream;
+    std::vector<Held> held;
+
+  private:
+    BlockScope* const outer;
+};
 
 // One per context (slab_ctx, slab_batch, slab_server): the last to go trims
 // the kept blocks to the idle bound. First member of its context, so that it

@@ -66,6 +66,7 @@ __global__ void k_arm(Ctl* c, int64_t steps_left, int32_t stop_at_frame) {
 
 template <typename F> slab_status guard(slab_ctx* ctx, F&& f) {
     try {
+        const BlockScope scope(ctx ? ctx->stream : nullptr);
         f();
         if (ctx) ctx->err.clear();
         return SLAB_OK;
@@ -566,19 +567,22 @@ void slab_destroy(slab_ctx* c) {
         cudaStreamSynchronize(c->copy_stream);
         cudaStreamDestroy(c->copy_stream);
     }
-    for (FrameSlot& F : c->frames) {
-        release_pinned(F.host);
-        if (F.packed) cudaEventDestroy(F.packed);
-        if (F.copied) cudaEventDestroy(F.copied);
-        F.dev.reset();
+    {
+        const BlockScope scope(c->stream);
+        for (FrameSlot& F : c->frames) {
+            release_pinned(F.host);
+            if (F.packed) cudaEventDestroy(F.packed);
+            if (F.copied) cudaEventDestroy(F.copied);
+            F.dev.reset();
+        }
+        c->path.reset();
+        c->terrain.z.reset();
+        c->terrain.grad.reset();
+        c->terrain.cos_t.reset();
+        c->terrain.dem32.reset();
+        release_device(c->d_ctl);
+        release_pinned(c->h_ctl);
     }
-    c->path.reset();
-    c->terrain.z.reset();
-    c->terrain.grad.reset();
-    c->terrain.cos_t.reset();
-    c->terrain.dem32.reset();
-    release_device(c->d_ctl);
-    release_pinned(c->h_ctl);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
 }

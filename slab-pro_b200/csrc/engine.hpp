@@ -15,23 +15,10 @@
 
 #include "blocks.hpp"
 #include "common.cuh"
+#include "error.hpp"
 #include "slab_gpu.h"
 
 namespace slab {
-
-// Thrown inside the library, turned into a slab_status at the C boundary.
-struct Error {
-    slab_status code;
-    std::string msg;
-};
-
-#define SLAB_CUDA(call)                                                                                     \
-    do {                                                                                                    \
-        cudaError_t e_ = (call);                                                                            \
-        if (e_ != cudaSuccess)                                                                              \
-            throw ::slab::Error{e_ == cudaErrorMemoryAllocation ? SLAB_E_OOM : SLAB_E_CUDA,                 \
-                                std::string(#call) + ": " + cudaGetErrorString(e_)};                        \
-    } while (0)
 
 template <typename T> T* dmalloc(size_t n) { return static_cast<T*>(take_device((n ? n : 1) * sizeof(T))); }
 
@@ -50,7 +37,7 @@ struct Scratch {
     size_t cap = 0;
     char* get(size_t bytes) {
         if (bytes > cap) {
-            buf.reset();  // handed out again only once no work uses it (blocks.hpp)
+            buf.reset();  // handed to others only once no work uses it (blocks.hpp)
             buf = dalloc<char>(bytes);
             cap = bytes;
         }

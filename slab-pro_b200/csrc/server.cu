@@ -158,6 +158,7 @@ void finish(slab_server* s, int slot, int state, const std::string& err) {
 
 void worker_loop(slab_server* s) {
     for (;;) {
+        const BlockScope scope(s->stream);
         // ---- admission (requests that fit a free slot and the memory budget)
         std::vector<int64_t> admit;
         {
@@ -584,13 +585,16 @@ void slab_server_destroy(slab_server* s) {
     }
     if (s->worker.joinable()) s->worker.join();
     if (s->stream) cudaStreamSynchronize(s->stream);
-    s->E.reset();
-    s->terrain.z.reset();
-    s->terrain.grad.reset();
-    s->terrain.cos_t.reset();
-    s->terrain.dem32.reset();
-    release_device(s->d_ctl);
-    release_pinned(s->h_ctl);
+    {
+        const BlockScope scope(s->stream);
+        s->E.reset();
+        s->terrain.z.reset();
+        s->terrain.grad.reset();
+        s->terrain.cos_t.reset();
+        s->terrain.dem32.reset();
+        release_device(s->d_ctl);
+        release_pinned(s->h_ctl);
+    }
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
 }
