@@ -16,6 +16,7 @@
 #include "blocks.hpp"
 #include "common.cuh"
 #include "error.hpp"
+#include "graphs.hpp"
 #include "slab_gpu.h"
 
 namespace slab {
@@ -114,32 +115,6 @@ template <typename... P, typename... A> void launch_chained(cudaStream_t st, dim
     c.numAttrs = 1;
     SLAB_CUDA(cudaLaunchKernelEx(&c, k, std::forward<A>(args)...));
 }
-
-// CUDA graphs of `chunk` consecutive steps, one per chunk size and kind of step used.
-struct StepGraphs {
-    std::map<std::pair<int, int>, cudaGraphExec_t> g;
-    ~StepGraphs() { clear(); }
-    void clear() {
-        for (auto& kv : g) cudaGraphExecDestroy(kv.second);
-        g.clear();
-    }
-    void launch(int chunk, cudaStream_t st, const std::function<void()>& one_step, int kind = 0) {
-        const std::pair<int, int> key{chunk, kind};
-        auto it = g.find(key);
-        if (it == g.end()) {
-            cudaGraph_t gr;
-            SLAB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            for (int k = 0; k < chunk; ++k) one_step();
-            SLAB_CUDA(cudaStreamEndCapture(st, &gr));
-            cudaGraphExec_t ex;
-            cudaError_t e = cudaGraphInstantiate(&ex, gr, 0);
-            cudaGraphDestroy(gr);
-            SLAB_CUDA(e);
-            it = g.emplace(key, ex).first;
-        }
-        SLAB_CUDA(cudaGraphLaunch(it->second, st));
-    }
-};
 
 // Per-kernel device times of profiled steps: events between the 4 kernels of
 // each step, read back lazily. Phases: 0 begin/dt, 1 (unused: binning is
