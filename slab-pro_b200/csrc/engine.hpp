@@ -192,7 +192,7 @@ struct Path {
                         const double* z) = 0;
     // whether upload() may be called again on this path: its buffers, step
     // graphs and launch shapes then serve the next run
-    virtual bool reusable() const { return false; }
+    virtual bool reusable() { return false; }
     virtual void initial_pass() = 0;
     // enqueue up to `chunk` steps; the device control block decides which run
     virtual void enqueue_steps(int chunk) = 0;

@@ -69,7 +69,8 @@ class Engine32 {
     long long persist_limit = 4000000000ll;
     int grid_persist = 0;
     dptr<unsigned> d_bar;  // k32::GridBar
-    bool dead = false;     // a persistent launch gave up: no further steps
+    bool dead = false;     // a persistent launch gave up: no further steps (the host has seen it)
+    bool gave_up();        // asks the device, where a persistent launch records it; waits for the stream
     void set_persistent(bool on, long long limit_cycles);
     void launch_persistent(int chunk);
     void arm(int64_t steps_left, int stop_at_frame);

@@ -786,14 +786,19 @@ void Engine32::restart_counts() {
     nlaunch = 0;
 }
 
-void Engine32::set_persistent(bool on, long long limit_cycles) {
-    if (on && grid_persist <= 0) throw Error{SLAB_E_ARG, "this device cannot run a cooperative launch"};
-    if (!on && persist && d_bar) {  // back to separate kernels: only from a complete step state
+bool Engine32::gave_up() {
+    if (!dead && d_bar) {
         k32::GridBar b{};
         d2h(&b, reinterpret_cast<k32::GridBar*>(d_bar.get()), 1, st);
         SLAB_CUDA(cudaStreamSynchronize(st));
         if (b.dead) dead = true;
     }
+    return dead;
+}
+
+void Engine32::set_persistent(bool on, long long limit_cycles) {
+    if (on && grid_persist <= 0) throw Error{SLAB_E_ARG, "this device cannot run a cooperative launch"};
+    if (!on && persist) gave_up();  // back to separate kernels: only from a complete step state
     if (on && acc_mode != k32::ACC_MIXED) throw Error{SLAB_E_ARG, "persistent steps run the default P2G scheme only"};
     persist = on;
     if (limit_cycles > 0) persist_limit = limit_cycles;
@@ -819,12 +824,7 @@ void Engine32::launch_persistent(int chunk) {
 }
 
 void Engine32::enqueue_steps(int chunk) {
-    if (persist && d_bar && timer.on) {  // profiled steps run the separate kernels: only from a complete step state
-        k32::GridBar b{};
-        d2h(&b, reinterpret_cast<k32::GridBar*>(d_bar.get()), 1, st);
-        SLAB_CUDA(cudaStreamSynchronize(st));
-        if (b.dead) dead = true;
-    }
+    if (persist && timer.on) gave_up();  // profiled steps run the separate kernels: only from a complete step state
     if (dead) throw Error{SLAB_E_TIMEOUT, "an earlier persistent launch gave up at a barrier; the step state is incomplete"};
     if (persist && acc_mode == k32::ACC_MIXED && !timer.on) {
         launch_persistent(chunk);
@@ -1174,7 +1174,7 @@ struct Split32 final : Path {
         sid = E.add_scenario(prm, dc, hc, Np, x, v, vz, h, m, z);
         E.tune_key_for(Np);
     }
-    bool reusable() const override { return !E.dead; }
+    bool reusable() override { return !E.gave_up(); }
     void observe(const Ctl& c) override {
         if (!c.active && !c.steps) return;
         E.tiles_seen = c.tiles;

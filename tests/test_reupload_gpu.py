@@ -1,0 +1,59 @@
+"""What a context's next upload takes over from the run before it, in the cases
+where that run did not simply end: a persistent launch that gave up, uploads that
+are never run, sizes that grow."""
+import numpy as np
+import pytest
+
+import slab
+
+pytestmark = pytest.mark.gpu
+
+N, DX = 96, 2.0
+CFG = dict(gravity=9.81, rho=300.0, C_cfl=0.5, dt_max=0.01, flip_ratio=0.95, output_dt=0.25, total_time=5.0, friction="VOELLMY",
+           voellmy_mu=0.2, voellmy_xi=1000.0)
+I = np.arange(N)
+Z = -0.4 * I[:, None] * DX + 0.3 * np.sin(0.3 * I)[None, :]
+
+
+def _release(r):
+    return {"type": "ELLIPSE", "center": (60.0, 96.0), "rx": r, "ry": 0.7 * r, "rotation_deg": 20.0, "h0": 1.5}
+
+
+def _context(prec=slab.FP32_SPLIT):
+    s = slab.Slab(Z, DX)
+    s.set_params(CFG, prec)
+    return s
+
+
+def _run(s, r):
+    s.upload_release(_release(r))
+    s.initial_pass()
+    _, _, steps = s.advance_to_frame()
+    steps += s.advance_steps(40)
+    P = s.particles()
+    return [P[k] for k in ("x", "v", "vz", "h", "mass", "z")] + list(s.max_maps()), steps, s.state()
+
+
+@pytest.mark.parametrize("waited", [True, False])
+@pytest.mark.parametrize("persistent", [True, False])
+def test_upload_after_a_persistent_launch_gave_up(waited, persistent):
+    """The run that gave up ends with the upload: the next one is a new context's."""
+    s = _context()
+    s.set_persistent(True, limit_cycles=64)  # far below one phase: the early CTAs give up
+    s.upload_release(_release(20.0))
+    s.initial_pass()
+    if waited:
+        with pytest.raises(slab.SlabError) as ex:
+            s.advance_steps(64)
+        assert ex.value.code == 6  # SLAB_E_TIMEOUT
+    else:
+        s.advance_steps_async(64)
+    s.set_persistent(persistent, limit_cycles=4_000_000_000)
+    got, steps, state = _run(s, 20.0)
+    s.close()
+    f = _context()
+    want, fsteps, fstate = _run(f, 20.0)
+    f.close()
+    assert (steps, state) == (fsteps, fstate) and steps > 40
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
