@@ -22,6 +22,7 @@ class Engine32 {
         int act_cap = 0;
         int Np_alloc = 0;   // particle buffer length
         int act_alloc = 0;  // tile list length
+        int64_t pending = 0;  // its part of pending_blocks
         Ctl* ctl = nullptr;
         Ctl* h_ctl = nullptr;
         dptr<int32_t> grp[2], act_list[2];
@@ -107,7 +108,7 @@ class Engine32 {
     int nscn = 0;
     int TX = 0, TY = 0, ntiles = 0;
     int blk_cap = 0;
-    int64_t pending_blocks = 0;  // node blocks of scenarios added since the last t=0 pass (an estimate)
+    int64_t pending_blocks = 0;  // node blocks of scenarios added since the last t=0 pass and not retired (an estimate)
     int grid_p2g = 0, grid_p2g_cell = 0, grid_p2g_hilo = 0, grid_p2g_sparse = 0, grid_p2g_fused = 0, grid_g2p = 0, grid_g2p_fused = 0, grid_grid = 0, grid_prep = 0;
 
     // Launch-shape tuner of the step's work kernels (k_prep, k_p2g_tiles --

@@ -422,6 +422,8 @@ void Engine32::retire(int sid, const Ctl& empty_ctl) {
     h2d(d_scn.get() + sid, &D, 1, st);
     host_scn[sid] = D;
     work_cap_total -= S.act_cap;
+    pending_blocks -= S.pending;  // retired before its t=0 pass
+    S.pending = 0;
     SLAB_CUDA(cudaStreamSynchronize(st));
     spare[sid] = std::move(slots[sid]);
     free_slots.push_back(sid);
@@ -564,6 +566,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
         d2h(misc, d_misc.get(), 8, st);
         SLAB_CUDA(cudaStreamSynchronize(st));
         pending_blocks += est;
+        S.pending = est;
         const int64_t need = (int64_t)(misc[0] - misc[4]) + pending_blocks;
         if (2 * need > blk_cap) grow_blocks((int)std::min<int64_t>(std::max<int64_t>(2 * (int64_t)blk_cap, 2 * need), INT32_MAX / NCELL));
     }
@@ -630,6 +633,8 @@ void Engine32::launch_t0() {
     SLAB_CUDA(cudaGetLastError());
     nlaunch += 4;
     pending_blocks = 0;  // later reads of the pool count see these blocks
+    for (auto& S : slots)
+        if (S) S->pending = 0;
 }
 
 void Engine32::launch_p2g(const Shared& sh) {

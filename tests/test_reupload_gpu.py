@@ -57,3 +57,22 @@ def test_upload_after_a_persistent_launch_gave_up(waited, persistent):
     assert (steps, state) == (fsteps, fstate) and steps > 40
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+def test_uploads_without_an_initial_pass_do_not_grow_the_pool():
+    """An upload that replaces one whose t = 0 pass was never run needs no more
+    node blocks than the first. 400 of them: each adding its tiles to the
+    estimate would ask for some 400 x 150 blocks of 2.8 KB, more than 160 MB."""
+    torch = pytest.importorskip("torch")
+    s = _context()
+    want, steps, state = _run(s, 35.0)
+    free0 = torch.cuda.mem_get_info()[0]
+    for _ in range(400):
+        s.upload_release(_release(35.0))
+    grown = free0 - torch.cuda.mem_get_info()[0]
+    got, steps2, state2 = _run(s, 35.0)
+    s.close()
+    assert grown < 32 << 20, grown
+    assert (steps, state) == (steps2, state2)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
