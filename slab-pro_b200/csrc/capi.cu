@@ -281,21 +281,28 @@ void upload_arrays(slab_ctx* c, int32_t Np, const double* x, const double* v, co
     // instantiating them takes 1-2 ms), serves again when it can; the
     // parameters are the same, since slab_set_params drops the path
     if (c->path && !c->path->reusable()) c->path.reset();
-    reset_ctl(c);
-    try {
-        if (!c->path) {
-            if (c->params.precision == SLAB_FP64_PLAIN)
-                c->path = make_plain64(c->terrain, c->params, c->stream, c->d_ctl, c->h_ctl);
-            else
-                c->path = make_split32(c->terrain, c->params, c->stream, c->d_ctl, c->h_ctl);
+    for (bool again = c->path != nullptr;; again = false) {
+        reset_ctl(c);
+        try {
+            if (!c->path) {
+                if (c->params.precision == SLAB_FP64_PLAIN)
+                    c->path = make_plain64(c->terrain, c->params, c->stream, c->d_ctl, c->h_ctl);
+                else
+                    c->path = make_split32(c->terrain, c->params, c->stream, c->d_ctl, c->h_ctl);
+            }
+            if (c->persist >= 0 && c->params.precision != SLAB_FP64_PLAIN) c->path->set_persistent(c->persist != 0, c->persist_limit);
+            c->path->upload(Np, x, v, vz, h, A, m, z);
+            pull_ctl(c);
+            raise_device_errors(c);
+            break;
+        } catch (const Error& e) {
+            c->path.reset();  // nothing of a failed upload is kept
+            // short of memory beside the buffers of the run before: once more without them
+            if (!(again && e.code == SLAB_E_OOM)) throw;
+        } catch (...) {
+            c->path.reset();
+            throw;
         }
-        if (c->persist >= 0 && c->params.precision != SLAB_FP64_PLAIN) c->path->set_persistent(c->persist != 0, c->persist_limit);
-        c->path->upload(Np, x, v, vz, h, A, m, z);
-        pull_ctl(c);
-        raise_device_errors(c);
-    } catch (...) {
-        c->path.reset();  // nothing of a failed upload is kept
-        throw;
     }
     c->Np = Np;
     c->uploaded = true;

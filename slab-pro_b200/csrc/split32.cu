@@ -1005,6 +1005,8 @@ std::vector<float> Engine32::gather_nodes(int sid, int stepid, int i0, int j0, i
     if (total == 0) return host;
     // scratch kept between calls (downloads at every retirement must not allocate)
     if ((size_t)nout * total > gather_cap) {
+        gather_cap = 0;
+        d_gather.reset();
         d_gather = dalloc<float>((size_t)nout * total);
         gather_cap = (size_t)nout * total;
     }

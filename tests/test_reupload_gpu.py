@@ -76,3 +76,32 @@ def test_uploads_without_an_initial_pass_do_not_grow_the_pool():
     assert (steps, state) == (steps2, state2)
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+def _host_particles(n, seed):
+    rng = np.random.default_rng(seed)
+    h, A = rng.uniform(0.5, 3.0, n), np.full(n, 1e-2)
+    return {"x": rng.uniform(40.0, 150.0, (n, 2)), "v": np.zeros((n, 2)), "vz": np.zeros(n), "h": h, "A": A, "mass": 300.0 * h * A,
+            "z": np.zeros(n)}
+
+
+def test_a_larger_upload_fits_where_it_would_on_a_new_context():
+    """FP64 particles are 72 bytes each. After 8 M of them (576 MB), with 312 MB
+    of the device left, 12 M (864 MB) fit in the room of both, and not beside any
+    64 MB array of the run before that is still there when the last new one of
+    96 MB is asked for."""
+    torch = pytest.importorskip("torch")
+    small, large = _host_particles(8 << 20, 1), _host_particles(12 << 20, 2)
+    s = _context(slab.FP64_PLAIN)
+    s.upload(small)
+    s.initial_pass()
+    torch.cuda.synchronize()
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (312 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        s.upload(large)
+        s.initial_pass()
+        assert s.conservation()[0] == pytest.approx(large["mass"].sum(), rel=1e-12)
+    finally:
+        del rest
+        torch.cuda.empty_cache()
+        s.close()
