@@ -22,6 +22,12 @@
  *    message. The C++ wrapper rethrows non-OK codes as std::runtime_error,
  *    matching how the reference reports errors (src/main.cpp:52-55).
  *  - One context per host thread; contexts are not internally locked.
+ *  - Memory that a call or a context gives back is kept for the next one: up to
+ *    1/16 of the device's memory and 4 GiB at most (1 GiB of page-locked host
+ *    memory) while a context, batch or server lives, 1 GiB (256 MiB) after the
+ *    last one is destroyed. It goes back to the driver when an allocation of
+ *    this library fails, and on slab_trim_memory(); a program that shares the
+ *    device with another allocator calls that one before the other needs it.
  */
 #ifndef SLAB_GPU_H
 #define SLAB_GPU_H
@@ -274,6 +280,10 @@ int64_t slab_kernel_launches(const slab_ctx* ctx);
  * of the calling thread's last failed slab_create, which leaves no context. */
 const char* slab_last_error(const slab_ctx* ctx);
 void slab_destroy(slab_ctx* ctx);
+/* Gives the memory that is kept between calls (top of this file) back to the
+ * driver: all devices' and the page-locked host memory. From any thread, also
+ * while other threads use their contexts; the next calls allocate anew. */
+slab_status slab_trim_memory(void);
 
 /* ---- batched ensembles ---------------------------------------------------
  * Many release scenarios of uneven size on one shared terrain, each with its

@@ -14,7 +14,9 @@ namespace slab {
 namespace {
 
 constexpr size_t MIB = (size_t)1 << 20;
+constexpr size_t LIVE_BYTES = 4096 * MIB;  // an upload's release or a context of the 8192 x 8192 terrain; 2 % of a B200
 constexpr size_t IDLE_BYTES = 1024 * MIB;
+constexpr size_t SPARE_BYTES = 16 * MIB;
 constexpr size_t PINNED_BYTES = 1024 * MIB;
 constexpr int PINNED = -1;  // "device" of the page-locked blocks
 
@@ -59,8 +61,8 @@ size_t size_class(size_t n) {
     return std::max<size_t>(512, (n + step - 1) / step * step);
 }
 
-// a block of size `got` serves a request of class `size`: at most a quarter more
-bool serves(size_t got, size_t size) { return got >= size && got <= size + size / 4; }
+// a block of size `got` serves a request of class `size`
+bool serves(size_t got, size_t size) { return got >= size && got <= size + std::min(size / 4, SPARE_BYTES); }
 
 void driver_free(int dev, void* p) noexcept {
     if (dev == PINNED) cudaFreeHost(p);
@@ -91,6 +93,20 @@ bool trim(int dev, size_t bound) noexcept {
     }
 }
 
+// every device's kept blocks down to dev_bound bytes, the page-locked ones to pinned_bound
+void trim_all(size_t dev_bound, size_t pinned_bound) noexcept {
+    Blocks& B = blocks();
+    for (int dev = PINNED - 1;;) {
+        {
+            std::lock_guard<std::mutex> lk(B.mu);
+            const auto next = B.pools.upper_bound(dev);
+            if (next == B.pools.end()) return;
+            dev = next->first;
+        }
+        trim(dev, dev == PINNED ? pinned_bound : dev_bound);
+    }
+}
+
 // a block that nothing uses, to its kept list
 void keep(const BlockScope::Held& h) noexcept {
     Blocks& B = blocks();
@@ -103,7 +119,7 @@ void keep(const BlockScope::Held& h) noexcept {
         if (!bound) {
             size_t free_b = 0, total_b = 0;
             if (h.dev == PINNED) bound = PINNED_BYTES;
-            else if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) bound = std::max<size_t>(total_b / 16, MIB);
+            else if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) bound = std::max(std::min(total_b / 16, LIVE_BYTES), MIB);
             else bound = MIB;
         }
         if (h.size <= bound) {
@@ -229,6 +245,8 @@ void release_device(void* p) noexcept { release(p); }
 void* take_pinned(size_t bytes) { return take(PINNED, bytes, "cudaMallocHost"); }
 void release_pinned(void* p) noexcept { release(p); }
 
+void trim_blocks() noexcept { trim_all(0, 0); }
+
 size_t kept_device_bytes() {
     int dev = 0;
     SLAB_CUDA(cudaGetDevice(&dev));
@@ -244,17 +262,11 @@ MemoryUser::MemoryUser() {
 }
 MemoryUser::~MemoryUser() {
     Blocks& B = blocks();
-    int dev = PINNED - 1;
-    for (;;) {  // every pool, in order
-        {
-            std::lock_guard<std::mutex> lk(B.mu);
-            if (dev < PINNED && --B.users != 0) return;
-            const auto next = B.pools.upper_bound(dev);
-            if (next == B.pools.end()) return;
-            dev = next->first;
-        }
-        trim(dev, dev == PINNED ? IDLE_BYTES / 4 : IDLE_BYTES);
+    {
+        std::lock_guard<std::mutex> lk(B.mu);
+        if (--B.users != 0) return;
     }
+    trim_all(IDLE_BYTES, IDLE_BYTES / 4);
 }
 
 }  // namespace slab

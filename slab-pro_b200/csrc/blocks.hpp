@@ -16,10 +16,13 @@
 //    flight, and no wait is wider than one stream: CUDA refuses to wait for a
 //    device, whatever the capture mode, while any stream of it is being
 //    captured, and other contexts' threads capture their step graphs at any time.
-//  - The blocks kept are bounded per device (1/16 of its memory while a
-//    context lives, IDLE_BYTES after the last one closed; page-locked memory:
-//    PINNED_BYTES, IDLE_BYTES / 4), and all of a device's go back to the
-//    driver when an allocation fails, before it is tried again.
+//  - The blocks kept are bounded per device (LIVE_BYTES, at most 1/16 of its
+//    memory, while a context lives, IDLE_BYTES after the last one closed;
+//    page-locked memory: PINNED_BYTES, IDLE_BYTES / 4). All of a device's go
+//    back to the driver when an allocation fails, before it is tried again,
+//    and all there are on trim_blocks().
+//  - A kept block serves a request of at least 4/5 of its size, and no more
+//    than SPARE_BYTES below it.
 //  - A block belongs to the device that was current when it was taken.
 //  - One mutex guards the lists: any thread may take and release blocks. No
 //    driver call is made while it is held.
@@ -37,6 +40,7 @@ void* take_device(size_t bytes);  // throws Error{SLAB_E_OOM | SLAB_E_CUDA}
 void release_device(void* p) noexcept;
 void* take_pinned(size_t bytes);
 void release_pinned(void* p) noexcept;
+void trim_blocks() noexcept;  // every kept block, of any device, back to the driver
 size_t kept_device_bytes();  // kept on the current device, handed back if an allocation needs them
 
 // One per call into a context, on the calling thread: all that the call does

@@ -253,6 +253,11 @@ slab_status slab_create(const slab_terrain_desc* td, const double* z, slab_ctx**
     return SLAB_OK;
 }
 
+slab_status slab_trim_memory(void) {
+    trim_blocks();
+    return SLAB_OK;
+}
+
 slab_status slab_set_params(slab_ctx* c, const slab_params* p) {
     if (!c || !p) return SLAB_E_ARG;
     return guard(c, [&] {
@@ -280,7 +285,7 @@ void upload_arrays(slab_ctx* c, int32_t Np, const double* x, const double* v, co
     // the path of the run before, with its step graphs (capturing and
     // instantiating them takes 1-2 ms), serves again when it can; the
     // parameters are the same, since slab_set_params drops the path
-    if (c->path && !c->path->reusable()) c->path.reset();
+    if (c->path && !c->path->reusable(Np)) c->path.reset();
     for (bool again = c->path != nullptr;; again = false) {
         reset_ctl(c);
         try {

@@ -190,9 +190,9 @@ struct Path {
     virtual ~Path() = default;
     virtual void upload(int Np, const double* x, const double* v, const double* vz, const double* h, const double* A, const double* m,
                         const double* z) = 0;
-    // whether upload() may be called again on this path: its buffers, step
-    // graphs and launch shapes then serve the next run
-    virtual bool reusable() { return false; }
+    // whether upload() of Np particles may be called again on this path: its
+    // buffers, step graphs and launch shapes then serve the next run
+    virtual bool reusable(int /*Np*/) { return false; }
     virtual void initial_pass() = 0;
     // enqueue up to `chunk` steps; the device control block decides which run
     virtual void enqueue_steps(int chunk) = 0;

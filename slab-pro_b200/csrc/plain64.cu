@@ -466,7 +466,7 @@ struct Plain64 final : Path {
         ++nlaunch;
         SLAB_CUDA(cudaMemcpyAsync(&dc->vmax2_bits, &dc->vmax2_acc, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
     }
-    bool reusable() override { return true; }
+    bool reusable(int) override { return true; }
     bool arm(int64_t steps_left, int stop_at_frame) override {
         k64_control<<<1, 32, 0, st>>>(dc, T.Nx, T.Ny, 1, steps_left, stop_at_frame);
         SLAB_CUDA(cudaGetLastError());

@@ -1181,7 +1181,12 @@ struct Split32 final : Path {
         sid = E.add_scenario(prm, dc, hc, Np, x, v, vz, h, m, z);
         E.tune_key_for(Np);
     }
-    bool reusable() override { return !E.gave_up(); }
+    // buffers for more than 4 times the particles, and 160 MB of them, go back
+    // instead: the run before may have been the only large one
+    bool reusable(int Np) override {
+        const int had = sid >= 0 ? E.slots[sid]->Np_alloc : 0;
+        return !(had > (1 << 21) && had / 4 > Np) && !E.gave_up();
+    }
     void observe(const Ctl& c) override {
         if (!c.active && !c.steps) return;
         E.tiles_seen = c.tiles;

@@ -168,6 +168,13 @@ def make_params(cfg: dict, precision: int = FP64_PLAIN) -> Params:
     return p
 
 
+def trim_memory():
+    """Give the device and page-locked memory that the library keeps between
+    calls (bounded, see slab_gpu.h) back to the driver, for example before
+    another allocator on the same device needs it."""
+    lib().slab_trim_memory()
+
+
 class Slab:
     """One simulation context on the current CUDA device."""
 

@@ -36,7 +36,7 @@ struct Fake {
     std::map<void*, size_t> dev, host;            // what the driver has handed out
     std::map<cudaStream_t, std::set<void*>> busy;  // work in flight
     std::map<cudaStream_t, int> waits;
-    int mallocs = 0, frees = 0;
+    int mallocs = 0, frees = 0, device = 0;
     std::vector<void*> freed;
 } F;
 
@@ -97,7 +97,7 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
     return cudaSuccess;
 }
 cudaError_t cudaGetDevice(int* d) {
-    *d = 0;
+    *d = F.device;
     return cudaSuccess;
 }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
@@ -116,9 +116,17 @@ static void same_scope() {
     CHECK(a == b);
     CHECK(F.waits[stream(1)] == 0);
     release_device(b);
-    void* c = take_device(2 * MIB);  // 4 MiB kept for 2 asked: more than a quarter too large
+    void* c = take_device(2 * MIB);  // 4 MiB held for 2 asked: more than a quarter too large
     CHECK(c != a);
     release_device(c);
+    void* d = take_device(100 * MIB);
+    release_device(d);
+    void* e = take_device(90 * MIB);
+    CHECK(e == d);
+    release_device(e);
+    e = take_device(82 * MIB);  // a quarter, but more than 16 MiB
+    CHECK(e != d);
+    release_device(e);
 }
 
 static void other_scope() {
@@ -179,7 +187,7 @@ static void bounds() {
         for (void* p : v) release_device(p);
         release_device(big);
         s.flush();
-        CHECK(kept_device_bytes() <= F.total / 16 && kept_device_bytes() >= F.total / 16 - 512 * MIB);
+        CHECK(kept_device_bytes() <= 4 * GIB && kept_device_bytes() > 4 * GIB - 512 * MIB);
         CHECK(!F.dev.count(big));
         CHECK(!F.dev.count(v.front()) && F.dev.count(v.back()));  // the oldest went
         void* h[5];
@@ -213,6 +221,41 @@ static void failed_allocation() {
     release_device(b);
     s.flush();
     F.total = 160 * GIB;
+}
+
+static void trimmed() {
+    {
+        const MemoryUser u;
+        BlockScope s(stream(8));
+        void *a = take_device(GIB), *h = take_pinned(64 * MIB), *live = take_device(GIB);
+        release_device(a);
+        release_pinned(h);
+        trim_blocks();
+        CHECK(F.dev.count(a) && F.host.count(h));  // still the scope's
+        s.flush();
+        trim_blocks();
+        CHECK(!F.dev.count(a) && !F.host.count(h) && F.dev.count(live) && kept_device_bytes() == 0);
+        release_device(live);
+    }
+    trim_blocks();
+    CHECK(F.used == 0 && F.pinned == 0);
+    {
+        std::lock_guard<std::recursive_mutex> lk(F.mu);
+        F.total = 32 * GIB;  // a small device: 1/16 of it (the bound is asked for once per device, so of the next one)
+        F.device = 1;
+    }
+    {
+        const MemoryUser u;
+        BlockScope s(stream(9));
+        std::vector<void*> v;
+        for (int k = 0; k < 12; ++k) v.push_back(take_device(256 * MIB));
+        for (void* p : v) release_device(p);
+        s.flush();
+        CHECK(kept_device_bytes() == 2 * GIB);
+    }
+    trim_blocks();
+    F.total = 160 * GIB;
+    F.device = 0;
 }
 
 static void threads() {
@@ -265,6 +308,7 @@ int main() {
     no_scope();
     bounds();
     failed_allocation();
+    trimmed();
     threads();
     CHECK(F.used <= GIB && F.pinned <= GIB / 4);
     for (const auto& kv : F.waits) CHECK(kv.first != nullptr);  // never the default stream

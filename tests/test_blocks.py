@@ -95,3 +95,51 @@ def test_uploads_beside_a_capture_of_another_thread(prec):
     g.replay()
     torch.cuda.synchronize()
     assert float(b.sum()) == 3.0 * 1024
+
+
+def _held(torch, free0):
+    torch.cuda.synchronize()
+    return free0 - torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.gpu
+def test_kept_memory_is_given_back():
+    """4 M particles take 80 bytes each and some 500 MB while they are sorted
+    in. After the last context is closed at most 1 GiB stays, after a trim
+    nothing; while the context lives, a small run and a trim leave what a
+    context that only ever had the small run holds."""
+    torch = pytest.importorskip("torch")
+    n = 4 << 20
+    rng = np.random.default_rng(3)
+    h, A = rng.uniform(0.5, 3.0, n), np.full(n, 1e-2)
+    P = {"x": rng.uniform(40.0, 150.0, (n, 2)), "v": np.zeros((n, 2)), "vz": np.zeros(n), "h": h, "A": A, "mass": 300.0 * h * A, "z": np.zeros(n)}
+    few = {k: v[:1000] for k, v in P.items()}
+
+    def context():
+        s = slab.Slab(Z, DX)
+        s.set_params(CFG, slab.FP32_SPLIT)
+        return s
+
+    s = context()
+    s.upload(P)  # (every kernel is loaded)
+    s.initial_pass()
+    s.close()
+    slab.trim_memory()
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    s = context()
+    s.upload(few)
+    slab.trim_memory()
+    small = _held(torch, free0)
+    s.upload(P)
+    slab.trim_memory()
+    assert _held(torch, free0) > 80 * n
+    s.upload(few)
+    slab.trim_memory()
+    assert _held(torch, free0) <= small + (8 << 20)
+    s.upload(P)
+    s.initial_pass()
+    s.close()
+    assert _held(torch, free0) <= (1 << 30) + (8 << 20)
+    slab.trim_memory()
+    assert _held(torch, free0) <= 8 << 20
