@@ -120,7 +120,9 @@ class Engine32 {
     // runs candidate s mod NC, so a workload that changes during the schedule
     // weighs on all candidates alike), and keeps per kernel the fastest. It
     // tunes on the first steps, again after 4x as many steps as at the last
-    // pick, and when the active tile count has halved or doubled.
+    // pick, and when the active tile count has halved or doubled. The two kinds
+    // of step (fused) run other kernels, so each has picks and a cadence of its
+    // own, and a schedule in which the kind changes is dropped.
     struct Tuner {
         static constexpr int NK = 5, NC = 5, ROUNDS = 3, NSTEP = NC * ROUNDS;
         static constexpr int FACTOR4[NC] = {1, 2, 4, 8, 16};  // grid = occupancy grid * FACTOR4[c] / 4
@@ -128,16 +130,18 @@ class Engine32 {
         int state = 0;         // 0: shapes fixed, 1: measuring, 2: measured, events not read yet
         int done = 0;          // schedule steps launched
         int64_t steps = 0;     // steps enqueued
-        int64_t next = 0;      // step count at which the next schedule starts
         int64_t active = 0;    // active tiles seen by the last capacity check
         int64_t active_at = 0; // active tiles when the last schedule started
         int base[NK] = {};     // occupancy-derived grids
         int base_fused[NK] = {};  // of the kernels of short steps (P2G and G2P have two each, which share a pick)
-        int pick[NK] = {2, 2, 2, 2, 2};
+        struct Kind {
+            int pick[NK] = {2, 2, 2, 2, 2};
+            int64_t next = 0;  // step count at which the next schedule starts
+        } kinds[2];            // by fused()
+        int kind = 0;          // the one whose shapes are in use
         int fixed[NK] = {};    // > 0: grid set by the caller, not tuned
         int tunes = 0;
         std::string key;       // a single scenario's workload size: picks shared by later contexts of the same size
-        bool from_cache = false;
         std::vector<cudaEvent_t> ev;  // NK + 2 per schedule step
         ~Tuner() {
             for (auto e : ev) cudaEventDestroy(e);
@@ -145,13 +149,14 @@ class Engine32 {
     } tune;
     int tuned_grid(int k, int c, int base) const;
     void apply_shapes(const int* c);
+    void tune_kind();           // the shapes of the kind of step that comes next
     void tune_pick();
     void launch_step_timed(const Shared& sh, cudaEvent_t* e);
     // the five work kernels' grid sizes now in use
     void launch_shapes(int out[5]) const;
     // grids[k] > 0 fixes kernel k's grid (NULL: none fixed); tune_on: the tuner runs
     void fix_shapes(const int32_t* grids, bool tune_on);
-    void tune_key_for(int Np);  // single scenario: picks of an earlier context of the same size, if any
+    void tune_key_for(int Np);  // single scenario: picks of an earlier run of the same size, if any, or none yet
     int work_cap = 0;
     int64_t work_cap_total = 0;
     void ensure_work_cap(int64_t need);

@@ -682,12 +682,12 @@ constexpr int Engine32::Tuner::FACTOR4[];
 
 
 namespace {
-// Launch shapes picked for single scenarios, by device, tile count and
-// particle count (half-octave buckets), kept for the process: a later context
+// Launch shapes picked for single scenarios, by device, tile count,
+// particle count (half-octave buckets) and kind of step, kept for the process: a later context
 // of the same size starts from them instead of measuring its first steps
 // again. Shapes never change results, only time.
 std::mutex g_tune_mu;
-std::map<std::string, std::vector<int>> g_tune_cache;
+std::map<std::pair<std::string, int>, std::vector<int>> g_tune_cache;
 }  // namespace
 
 void Engine32::tune_key_for(int Np) {
@@ -697,14 +697,32 @@ void Engine32::tune_key_for(int Np) {
     const std::string key = std::to_string(dev) + ":" + std::to_string(TILE) + ":" + std::to_string(ntiles) + ":" + std::to_string(bucket);
     if (key == tune.key) return;  // another run of the same size: its shapes, graphs and cadence go on
     tune.key = key;
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    const auto it = g_tune_cache.find(tune.key);
-    if (it == g_tune_cache.end() || !tune.enabled) return;
-    std::copy(it->second.begin(), it->second.end(), tune.pick);
-    apply_shapes(tune.pick);
-    graphs.clear();
-    tune.from_cache = true;
-    tune.next = 256;  // no schedule on the first steps; the usual cadence after them
+    tune.state = 0;  // (a schedule of the run before is of another size)
+    tune.active_at = 0;
+    {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        for (int k = 0; k < 2; ++k) {
+            tune.kinds[k] = Tuner::Kind{};
+            tune.kinds[k].next = tune.steps;
+            const auto it = g_tune_cache.find({tune.key, k});
+            if (it == g_tune_cache.end() || !tune.enabled) continue;
+            std::copy(it->second.begin(), it->second.end(), tune.kinds[k].pick);
+            tune.kinds[k].next += 256;  // no schedule on the first steps; the usual cadence after them
+        }
+    }
+    tune.kind = fused();
+    apply_shapes(tune.kinds[tune.kind].pick);
+    graphs.clear();  // the step graphs carry the grid sizes
+}
+
+void Engine32::tune_kind() {
+    if (tune.kind == (int)fused()) return;
+    if (tune.state != 0) {  // its steps are of both kinds; not again at once, the kinds may alternate
+        tune.state = 0;
+        tune.kinds[tune.kind].next = tune.steps + 256;
+    }
+    tune.kind = fused();
+    apply_shapes(tune.kinds[tune.kind].pick);
 }
 
 int Engine32::tuned_grid(int k, int c, int base) const {
@@ -729,7 +747,7 @@ void Engine32::fix_shapes(const int32_t* grids, bool tune_on) {
     for (int k = 0; k < Tuner::NK; ++k) tune.fixed[k] = grids ? std::max<int32_t>(grids[k], 0) : 0;
     tune.enabled = tune_on;
     if (tune.state == 1) tune.state = 0;  // a schedule in flight is dropped (its events are not read)
-    apply_shapes(tune.pick);
+    apply_shapes(tune.kinds[tune.kind].pick);
     graphs.clear();
 }
 
@@ -764,23 +782,24 @@ void Engine32::tune_pick() {
             ms[k][c] += t;
         }
     }
+    Tuner::Kind& t = tune.kinds[tune.kind];
     for (int k = 0; k < Tuner::NK; ++k) {
         int best = 2;
         for (int c = 0; c < Tuner::NC; ++c)
             if (ms[k][c] < 0.97 * ms[k][2] && ms[k][c] < ms[k][best]) best = c;
-        tune.pick[k] = best;
+        t.pick[k] = best;
     }
-    tune.pick[2] = tune.pick[1];
-    if (fused()) tune.pick[3] = 2;  // the kernel did not run: its occupancy grid
-    apply_shapes(tune.pick);
+    t.pick[2] = t.pick[1];
+    if (tune.kind == 1) t.pick[3] = 2;  // the kernel did not run: its occupancy grid
+    apply_shapes(t.pick);
     graphs.clear();  // the step graphs carry the grid sizes
     if (!tune.key.empty()) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tune_cache[tune.key] = std::vector<int>(tune.pick, tune.pick + Tuner::NK);
+        g_tune_cache[{tune.key, tune.kind}] = std::vector<int>(t.pick, t.pick + Tuner::NK);
     }
     tune.state = 0;
     tune.tunes += 1;
-    tune.next = std::max<int64_t>(4 * tune.steps, tune.steps + 256);
+    t.next = std::max<int64_t>(4 * tune.steps, tune.steps + 256);
 }
 
 // launch and profile counts start anew with a new run
@@ -840,11 +859,12 @@ void Engine32::enqueue_steps(int chunk) {
         graphs.clear();
         graph_nscn = nscn;
     }
+    tune_kind();
     int k = 0;
     if (tune.enabled && acc_mode == k32::ACC_MIXED && !timer.on) {
         if (tune.state == 2) tune_pick();
         const bool moved = tune.active > 0 && tune.active_at > 0 && (tune.active > 2 * tune.active_at || 2 * tune.active < tune.active_at);
-        if (tune.state == 0 && nscn > 0 && (tune.steps >= tune.next || moved)) {
+        if (tune.state == 0 && nscn > 0 && (tune.steps >= tune.kinds[tune.kind].next || moved)) {
             constexpr int W = Tuner::NK + 2;
             while ((int)tune.ev.size() < Tuner::NSTEP * W) {
                 cudaEvent_t e;
@@ -863,7 +883,7 @@ void Engine32::enqueue_steps(int chunk) {
                 apply_shapes(c);
                 launch_step_timed(sh, tune.ev.data() + (size_t)tune.done * (Tuner::NK + 2));
             }
-            apply_shapes(tune.pick);
+            apply_shapes(tune.kinds[tune.kind].pick);
             for (; k < chunk; ++k) launch_step();
             SLAB_CUDA(cudaGetLastError());
             if (tune.done == Tuner::NSTEP) tune.state = 2;

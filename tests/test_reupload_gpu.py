@@ -105,3 +105,40 @@ def test_a_larger_upload_fits_where_it_would_on_a_new_context():
         del rest
         torch.cuda.empty_cache()
         s.close()
+
+
+def test_the_tuner_starts_anew_with_another_size():
+    """Launch shapes are measured on a run's first steps (15 of them, read when
+    the next are enqueued), whatever the context ran before; steps of a run of
+    another size are not taken together with them."""
+    i = np.arange(104)
+    z = -0.4 * np.arange(203)[:, None] * DX + 0.3 * np.sin(0.3 * i)[None, :]
+    s = slab.Slab(z, DX)
+    s.set_params({**CFG, "friction": "COULOMB", "coulomb_mu": 0.8, "total_time": 60.0}, slab.FP32_SPLIT)
+
+    def start(r):
+        s.upload_release(_release(r))
+        s.initial_pass()
+
+    def tunes():
+        return s.launch_shapes()[1]
+
+    start(20.0)
+    s.advance_steps(64)
+    assert tunes() == 1
+    s.advance_steps(1200)  # measured again at growing distances
+    n = tunes()
+    assert n > 1
+    start(40.0)
+    s.advance_steps(64)
+    assert tunes() == n + 1
+    start(10.0)
+    s.advance_steps(8)
+    start(28.0)  # 8 steps measured, 7 to go: of another size
+    s.advance_steps(8)
+    s.advance_steps(4)
+    assert tunes() == n + 1
+    s.advance_steps(8)
+    s.advance_steps(4)
+    assert tunes() == n + 2
+    s.close()
