@@ -112,6 +112,16 @@ __device__ __forceinline__ void atomic_max_u64(uint64_t* a, uint64_t v) {
 
 namespace slab {
 
+// The particle box that the last G2P, or the upload, left, for the step that
+// begins. If it was taken before and no G2P has run since -- the launch of the
+// begun step failed, or the host gave up waiting for time to move on -- it stays
+// as it is: the accumulators are clear and hold no particle, and a box made of
+// them reaches far outside the terrain.
+__device__ inline void take_box(Ctl* c) {
+    if (c->pos_acc[0] == 0x7ff0000000000000ull) return;
+    for (int k = 0; k < 4; ++k) c->pos[k] = c->pos_acc[k];
+}
+
 // Start of a step, one thread: the stop conditions of the running advance
 // call, then Simulation::updateDt (src/simulation.cpp:565-582) from the
 // previous G2P's max |v|^2, then the reference's remesh box from the
@@ -139,7 +149,7 @@ __device__ inline void ctl_begin(Ctl* c, int Nx, int Ny) {
     c->new_time = __dadd_rn(c->time, dt);
     c->frame_end = (next_frame_time - c->new_time < 1e-13) ? 1 : 0;
     c->write_outputs = (c->frame_end || c->keep_outputs) ? 1 : 0;
-    for (int k = 0; k < 4; ++k) c->pos[k] = c->pos_acc[k];
+    take_box(c);
     remesh_box(__longlong_as_double((long long)c->pos[0]), __longlong_as_double((long long)c->pos[1]),
                __longlong_as_double((long long)c->pos[2]), __longlong_as_double((long long)c->pos[3]), c->dx, c->one_over_dx, c->box);
     if (c->box[0] < 0 || c->box[2] < 0 || c->box[1] > Nx - 1 || c->box[3] > Ny - 1) {
@@ -187,7 +197,7 @@ __device__ inline void ctl_begin_t0(Ctl* c, int Nx, int Ny) {
     c->new_time = c->time;
     c->frame_end = 0;
     c->write_outputs = 1;
-    for (int k = 0; k < 4; ++k) c->pos[k] = c->pos_acc[k];
+    take_box(c);
     remesh_box(__longlong_as_double((long long)c->pos[0]), __longlong_as_double((long long)c->pos[1]),
                __longlong_as_double((long long)c->pos[2]), __longlong_as_double((long long)c->pos[3]), c->dx, c->one_over_dx, c->box);
     if (c->box[0] < 0 || c->box[2] < 0 || c->box[1] > Nx - 1 || c->box[3] > Ny - 1) {
