@@ -194,6 +194,8 @@ slab_status slab_batch_run(slab_batch* b, int64_t max_steps, int64_t* steps_out)
         b->E->arm(max_steps, 0);
         int64_t done = 0;
         pull_all(b);
+        std::vector<int64_t> before(b->E->nscn);
+        for (int s = 0; s < b->E->nscn; ++s) before[s] = b->h_ctl[s].steps;
         while (done < max_steps) {
             // a chunk, or what the scenario with most steps to go still needs
             int64_t need = 1;
@@ -218,7 +220,11 @@ slab_status slab_batch_run(slab_batch* b, int64_t max_steps, int64_t* steps_out)
         }
         pull_all(b);
         raise_errors(b);
-        if (steps_out) *steps_out = done;
+        // the count reported is in whole chunks, however few of the last one's
+        // steps were enqueued
+        int64_t most = 1;
+        for (int s = 0; s < b->E->nscn; ++s) most = std::max(most, b->h_ctl[s].steps - before[s]);
+        if (steps_out) *steps_out = std::max<int64_t>(0, std::min(max_steps, (most + b->chunk - 1) / b->chunk * b->chunk));
     });
 }
 
