@@ -305,11 +305,12 @@ slab_status slab_batch_set_stream(slab_batch* b, void* cuda_stream);
  * SLAB_FP32_SPLIT. Its t=0 pass runs with the next slab_batch_run. */
 slab_status slab_batch_add(slab_batch* b, const slab_params* params, int32_t Np, const double* x_xy, const double* v_xy,
                            const double* vz, const double* h, const double* A, const double* mass, const double* z, int32_t* scenario_id);
-/* Advance every scenario until each has reached its total_time, or for at
- * most max_steps steps of the batch. */
 /* Add a scenario whose particles are built on the device from a release
  * (as slab_upload_release; the same particles as the reference's setup). */
 slab_status slab_batch_add_release(slab_batch* b, const slab_params* params, const slab_release* release, int32_t* scenario_id);
+/* Advance every scenario until each has reached its total_time, or for at
+ * most max_steps steps of the batch. steps_out (may be NULL): those steps in
+ * whole chunks of 32, at most max_steps. */
 slab_status slab_batch_run(slab_batch* b, int64_t max_steps, int64_t* steps_out);
 slab_status slab_batch_state(slab_batch* b, int32_t scenario_id, double* time, int32_t* frame, int64_t* steps);
 /* The scenario's own outcome: SLAB_OK, or the error that stopped it
@@ -336,8 +337,9 @@ int64_t slab_batch_kernel_launches(const slab_batch* b);
  * slab_get_phase_times (adds event records per step while on). */
 slab_status slab_batch_set_profiling(slab_batch* b, int32_t on);
 slab_status slab_batch_phase_times(slab_batch* b, double out[5]);
-/* Launch shapes (CTA counts) of the step's five work kernels: k_prep, P2G of
- * the dense tiles, P2G of the sparse tiles, grid update, G2P. Any shape gives
+/* Launch shapes (CTA counts) of the step's work kernels: k_prep, P2G of the
+ * dense tiles, P2G of the sparse tiles, grid update, G2P. One P2G kernel runs
+ * the tiles of both kinds, with the larger of its two counts. Any shape gives
  * bitwise the same results. A tuner times five candidates per kernel (1/4,
  * 1/2, 1, 2 and 4 times the occupancy grid) on live, interleaved steps and keeps
  * the fastest; it runs on the first steps, after 4x as many steps as at its

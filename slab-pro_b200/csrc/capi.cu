@@ -55,15 +55,6 @@ struct slab_ctx {
 
 namespace {
 
-__global__ void k_arm(Ctl* c, int64_t steps_left, int32_t stop_at_frame) {
-    if (threadIdx.x == 0) {
-        c->stop = 0;
-        c->frame_hit = 0;
-        c->steps_left = steps_left;
-        c->stop_at_frame = stop_at_frame;
-    }
-}
-
 template <typename F> slab_status guard(slab_ctx* ctx, F&& f) {
     try {
         const BlockScope scope(ctx ? ctx->stream : nullptr);
@@ -130,15 +121,8 @@ void raise_device_errors(slab_ctx* c) {
     if (e & ERR_TIMEOUT) throw Error{SLAB_E_TIMEOUT, "bounded device wait gave up"};  // the engine takes no further steps
 }
 
-void arm(slab_ctx* c, int64_t steps_left, int stop_at_frame) {
-    if (c->path->arm(steps_left, stop_at_frame)) return;
-    k_arm<<<1, 32, 0, c->stream>>>(c->d_ctl, steps_left, stop_at_frame);
-    SLAB_CUDA(cudaGetLastError());
-    ++c->extra_launches;
-}
-
 void enqueue_nsteps(slab_ctx* c, int64_t nsteps) {
-    arm(c, nsteps, 0);
+    c->path->arm(nsteps, 0);
     int64_t k = 0;
     for (; k + c->chunk <= nsteps; k += c->chunk) c->path->enqueue_steps(c->chunk);
     if (k < nsteps) c->path->enqueue_steps((int)(nsteps - k));
@@ -153,7 +137,7 @@ void advance(slab_ctx* c, int64_t nsteps, bool stop_at_frame, int64_t* steps_out
         // the step budget is on the device; enqueue up to 8 chunks, then look
         // at the control block, so a run that stops at total_time long before
         // the budget does not keep the host enqueueing empty steps
-        arm(c, nsteps, 0);
+        c->path->arm(nsteps, 0);
         const int64_t poll = 8 * (int64_t)c->chunk;
         int64_t k = 0;
         while (k < nsteps) {
@@ -167,7 +151,7 @@ void advance(slab_ctx* c, int64_t nsteps, bool stop_at_frame, int64_t* steps_out
             if (c->h_ctl->stop || c->h_ctl->err) break;
         }
     } else {
-        arm(c, nsteps, 1);
+        c->path->arm(nsteps, 1);
         double last_time = c->h_ctl->time;
         int stalled = 0;
         for (;;) {

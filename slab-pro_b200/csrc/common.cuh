@@ -48,7 +48,7 @@ struct Ctl {
     // (src/simulation.cpp:602-612): nodes [box[0], box[1]] x [box[2], box[3]].
     int32_t box[4];
     int32_t tiles;         // FP32: active tiles of the current step
-    int32_t heaviest;      // FP32: particles of its heaviest tile, 0 where nobody counted (steps of many tiles)
+    int32_t heaviest;      // FP32: particles of the heaviest tile of the last step that counted them (at most FUSED_MAX_TILES tiles)
     int32_t keep_outputs;  // write grid output fields every step (tests); else frame steps only
     unsigned long long node_steps;  // grid nodes with mass > 1e-6, summed over all steps so far
 };

@@ -116,9 +116,9 @@ template <typename... P, typename... A> void launch_chained(cudaStream_t st, dim
     SLAB_CUDA(cudaLaunchKernelEx(&c, k, std::forward<A>(args)...));
 }
 
-// Per-kernel device times of profiled steps: events between the 4 kernels of
-// each step, read back lazily. Phases: 0 begin/dt, 1 (unused: binning is
-// fused into G2P), 2 P2G, 3 grid update, 4 G2P.
+// Per-kernel device times of profiled steps: events between the kernels of each
+// step, read back lazily. Phases: 0 step control, 1 tile bookkeeping (FP32's
+// k_prep), 2 P2G, 3 grid update (0 where G2P does it), 4 G2P.
 struct PhaseTimer {
     bool on = false;
     std::vector<cudaEvent_t> pool;
@@ -196,9 +196,8 @@ struct Path {
     virtual void initial_pass() = 0;
     // enqueue up to `chunk` steps; the device control block decides which run
     virtual void enqueue_steps(int chunk) = 0;
-    // start an advance call on the device (budget, frame stop); false: the
-    // caller arms the control block itself
-    virtual bool arm(int64_t, int) { return false; }
+    // start an advance call on the device (budget, frame stop) and its first step
+    virtual void arm(int64_t steps_left, int stop_at_frame) = 0;
     virtual void download_particles(double* x, double* v, double* vz, double* h, double* A, double* m, double* z) = 0;
     virtual void download_grid(slab_grid_view* view) = 0;
     virtual void download_max(double* h_max, double* v_max2) = 0;

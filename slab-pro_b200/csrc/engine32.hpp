@@ -29,7 +29,7 @@ class Engine32 {
         dptr<float4> a[2], b[2];  // PBuf
         dptr<float> vz[2], z[2];
         dptr<int2> act;
-        dptr<int32_t> nxt_off, gt_stamp, blk_of;
+        dptr<int32_t> gt_stamp, blk_of;
         SCnt* cnt = nullptr;  // in the engine's counter array
     };
 
@@ -39,7 +39,6 @@ class Engine32 {
     // want_slot >= 0: use that free slot (or the next unused one)
     int add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, const double* x, const double* v, const double* vz,
                      const double* h, const double* m, const double* z, int want_slot = -1);
-    void launch_begin(int t0);
     void launch_t0();
     void launch_step();
     static constexpr int NKERNELS = 5;  // of a step: k_prep, P2G, grid update, G2P, k_end
@@ -57,7 +56,7 @@ class Engine32 {
     // line is at FUSED_MAX_TILES. Both numbers are what the host saw last.
     static constexpr int64_t FUSED_TILES = 1500, FUSED_TILES_PER_PARTICLE = 3;
     int64_t tiles_seen = 0;
-    int64_t heaviest_seen = 0;  // 0: nobody counted, steps of more than FUSED_MAX_TILES tiles
+    int64_t heaviest_seen = 0;  // 0: not counted yet (steps of more than FUSED_MAX_TILES tiles)
     bool fused() const {
         return tiles_seen <= FUSED_MAX_TILES && (batch || tiles_seen <= FUSED_TILES + FUSED_TILES_PER_PARTICLE * heaviest_seen);
     }
@@ -111,11 +110,12 @@ class Engine32 {
     int64_t pending_blocks = 0;  // node blocks of scenarios added since the last t=0 pass and not retired (an estimate)
     int grid_p2g = 0, grid_p2g_cell = 0, grid_p2g_hilo = 0, grid_p2g_sparse = 0, grid_p2g_fused = 0, grid_g2p = 0, grid_g2p_fused = 0, grid_grid = 0, grid_prep = 0;
 
-    // Launch-shape tuner of the step's work kernels (k_prep, k_p2g_tiles --
-    // shapes 1 and 2, its dense and sparse tiles, go together --, k_grid, k_g2p). Each CTA of these kernels takes a
-    // contiguous slice of a device-built work list and every work item is
-    // computed by one CTA alone, so the grid size changes which CTA computes a
-    // tile, never a value: all candidates give bitwise the same results. The
+    // Launch-shape tuner of the step's work kernels: k_prep, P2G (shapes 1 and 2,
+    // of its dense and sparse tiles, go together: one kernel runs both), k_grid and
+    // G2P. Each CTA of these kernels takes items of a device-built work list (of
+    // several scenarios a contiguous run, of one every n-th or the next in turn)
+    // and every item is computed by one CTA alone, so the grid size changes which
+    // CTA computes a tile, never a value: all candidates give bitwise the same results. The
     // tuner times the candidates on live steps, interleaved (schedule step s
     // runs candidate s mod NC, so a workload that changes during the schedule
     // weighs on all candidates alike), and keeps per kernel the fastest. It

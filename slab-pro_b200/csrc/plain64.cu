@@ -103,8 +103,8 @@ __global__ void k64_begin_t0(Ctl* c, int Nx, int Ny) {
 // The atomics bound it (L2 at 71 % of its peak, 2 M particles 238 us), so the
 // sum of m vz, which only output fields use, is left out of the other steps.
 // (Summing each 8 x 8-cell tile of periodically ordered particles in shared
-// memory first, 3 atomics per particle instead of 63, was bound by FP64
-// issue: 218 us, and 354 instead of 134 us where cells hold 4 to 15 particles.)
+// memory first, 3 atomics per particle instead of 63, took 218 us, and 354
+// instead of 134 us where cells hold 4 to 15 particles.)
 __global__ void __launch_bounds__(256) k64_p2g(const Ctl* c, P64 p, N64 n, const double2* __restrict__ grad,
                                                const double* __restrict__ cos_t, Phys P, int Np) {
     chain_wait<true>();
@@ -467,11 +467,10 @@ struct Plain64 final : Path {
         SLAB_CUDA(cudaMemcpyAsync(&dc->vmax2_bits, &dc->vmax2_acc, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
     }
     bool reusable(int) override { return true; }
-    bool arm(int64_t steps_left, int stop_at_frame) override {
+    void arm(int64_t steps_left, int stop_at_frame) override {
         k64_control<<<1, 32, 0, st>>>(dc, T.Nx, T.Ny, 1, steps_left, stop_at_frame);
         SLAB_CUDA(cudaGetLastError());
         ++nlaunch;
-        return true;
     }
 
     int grid_blocks() const { return 148 * 4; }

@@ -527,7 +527,6 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     else S.act_cap = S.act_alloc;  // a reused list keeps its full length
     if (new_tiles) {
         S.act = dalloc<int2>(ntiles);
-        S.nxt_off = dalloc<int32_t>(ntiles);
         S.gt_stamp = dalloc<int32_t>(ntiles);
         S.blk_of = dalloc<int32_t>(ntiles);
     }
@@ -608,7 +607,6 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
         D.act_list[b] = S.act_list[b].get();
     }
     D.act = S.act.get();
-    D.nxt_off = S.nxt_off.get();
     D.gt_stamp = S.gt_stamp.get();
     D.blk_of = S.blk_of.get();
     D.act_cap = S.act_cap;
@@ -620,15 +618,10 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     return sid;
 }
 
-void Engine32::launch_begin(int t0) {
-    k32::k_begin<<<1, k32::CTL_THREADS, 0, st>>>(shared(), t0);
-    SLAB_CUDA(cudaGetLastError());
-}
-
 void Engine32::launch_t0() {
     Shared sh = shared();
     sh.use_xlist = 1;  // the pass has no G2P to run the grid update in
-    k32::k_begin<<<1, k32::CTL_THREADS, 0, st>>>(sh, 1);
+    k32::k_begin_t0<<<1, k32::CTL_THREADS, 0, st>>>(sh);
     for (int k = 0; k < 3; ++k) launch_kernel(k, sh);
     SLAB_CUDA(cudaGetLastError());
     nlaunch += 4;
@@ -1214,10 +1207,7 @@ struct Split32 final : Path {
     }
     void initial_pass() override { E.launch_t0(); }
     void enqueue_steps(int chunk) override { E.enqueue_steps(chunk); }
-    bool arm(int64_t steps_left, int stop_at_frame) override {
-        E.arm(steps_left, stop_at_frame);
-        return true;
-    }
+    void arm(int64_t steps_left, int stop_at_frame) override { E.arm(steps_left, stop_at_frame); }
     void download_particles(double* x, double* v, double* vz, double* h, double* A, double* m, double* z) override {
         E.download_particles(sid, x, v, vz, h, A, m, z, prm.rho);
     }

@@ -123,7 +123,6 @@ struct alignas(16) Scn {
     int32_t* grp[2];        // [ntiles][GRP_STRIDE] segment records (see GRP_STRIDE)
     int2* act;              // [ntiles] {last seq the tile was put on an active list, its place on that list}
     int32_t* act_list[2];   // active tiles of each parity
-    int32_t* nxt_off;       // [ntiles] start of the tile's segment in the next buffer
     int32_t* gt_stamp;      // [ntiles] stepid at which the tile joined the grid list
     int32_t* blk_of;        // [ntiles] node block of the tile, -1 if none yet
     int32_t act_cap;

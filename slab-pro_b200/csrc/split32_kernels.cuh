@@ -13,9 +13,9 @@
 //   k_end    (1 CTA)   per scenario: end of the step, then the next step's
 //                      dt / stop rules and work-list prefix (k_arm_begin does
 //                      the same at the start of an advance call)
-// The CTAs take contiguous runs of a flat list of work items of all
-// scenarios, so one launch advances every running scenario by one step, each
-// with its own dt and friction law.
+// The CTAs share a flat list of work items of all scenarios (work_items,
+// many_rounds), so one launch advances every running scenario by one step,
+// each with its own dt and friction law.
 //
 // Every result is independent of the timing of the threads: the cell-sorted
 // P2G sorts a tile's particles by cell in a stable, data-determined order and
@@ -140,7 +140,7 @@ __device__ __forceinline__ int tile_of_cell(int32_t cell, int TY) { return (cell
 // read. The control block and counters are read whole in one round and written
 // back once: field by field, each branch waited for its own load (5.3 us for
 // the kernel with one scenario, the time of about 12 dependent loads).
-enum : int { CTL_BEGIN = 0, CTL_T0 = 1, CTL_ARM = 2, CTL_END = 3 };
+enum : int { CTL_T0, CTL_ARM, CTL_END };
 
 __device__ __forceinline__ int step_control(const Shared& sh, int s, int what, int64_t steps_left, int stop_at_frame) {
     Ctl k = sh.ctl[s];
@@ -246,9 +246,10 @@ __device__ __forceinline__ void control_scenarios(const Shared& sh, int what, in
 
 constexpr int CTL_THREADS = 256;  // one thread per scenario; enough registers for the control block
 
-__global__ void __launch_bounds__(CTL_THREADS) k_begin(Shared sh, int t0_pass) {
+// Start of simulate()'s t=0 pass of the scenarios that still need it.
+__global__ void __launch_bounds__(CTL_THREADS) k_begin_t0(Shared sh) {
     chain_wait<true>();
-    control_scenarios(sh, t0_pass ? CTL_T0 : CTL_BEGIN);
+    control_scenarios(sh, CTL_T0);
 }
 
 // Start of an advance call: every scenario gets the step budget and the
