@@ -423,7 +423,9 @@ __device__ __forceinline__ void prep_body(const Shared& sh) {
         const bool live = gst == seq && r < 9 && valid;
         const int rs = live ? (r == 4 ? g.x : g.y) : 0, rl = live ? (r == 4 ? g.y - g.x : g.z - g.y) : 0, c = live ? gc : 0;
         const bool new_gt = was < stamp && valid;
-        const int nb = ast == seq && r < 9 && valid ? (one ? 0 : w - loc) + aslot : -1;  // that tile's partial window
+        // that tile's partial window; one past the work list (ERR_CAPACITY) is not written
+        const int sl = (one ? 0 : w - loc) + aslot;
+        const int nb = ast == seq && sl < nwork && r < 9 && valid ? sl : -1;
         // half-warp shuffles: the tile's particle count and the range prefixes
         int incl = rl;
 #pragma unroll
