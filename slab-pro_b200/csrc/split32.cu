@@ -470,6 +470,10 @@ void Engine32::download_max_box(int sid, const int box[4], double* hmax, double*
 void Engine32::ensure_work_cap(int64_t need) {
     if (need <= work_cap) return;
     const int64_t cap = std::min<int64_t>(std::max<int64_t>(need, (int64_t)work_cap * 3 / 2), INT32_MAX / PART_STRIDE);
+    // at that limit already: the lists' lengths are estimates, and steps with more
+    // tiles report it (an ensemble of 256 reaches it at its 147th scenario, and
+    // every one after it exchanged the 8 GiB of partial sums for as many)
+    if (cap <= work_cap) return;
     SLAB_CUDA(cudaStreamSynchronize(st));
     d_desc = dalloc<TileDesc>(cap);
     d_part = dalloc<float>((size_t)cap * PART_STRIDE);
