@@ -63,11 +63,12 @@ class Engine32 {
     void launch_p2g(const Shared& sh);
     CUtensorMap dem_map;   // the FP32 terrain as [Nx][4 Ny] floats, 9 x 9-node boxes (P2G's terrain window)
     // persistent steps: a chunk of steps as one cooperative launch of k_persist
+    // or k_persist_many
     // (SLAB_PERSIST=1 or set_persistent); its grid waits give up after
     // persist_limit clock cycles (ERR_TIMEOUT)
     bool persist = false;
     long long persist_limit = 4000000000ll;
-    int grid_persist = 0;
+    int grid_persist = 0, grid_persist_many = 0;  // CTAs of k_persist, k_persist_many
     dptr<unsigned> d_bar;  // k32::GridBar
     bool dead = false;     // a persistent launch gave up: no further steps (the host has seen it)
     bool gave_up();        // asks the device, where a persistent launch records it; waits for the stream

@@ -302,13 +302,16 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     const int base[Tuner::NK] = {grid_prep, grid_p2g_cell, grid_p2g_sparse, grid_grid, grid_g2p};
     std::copy(base, base + Tuner::NK, tune.base);
     if (const char* e = std::getenv("SLAB_TUNE")) tune.enabled = std::atoi(e) != 0;
-    // the persistent step kernel: as many CTAs as can be resident at once
+    // the persistent step kernels: as many CTAs as can be resident at once
     // (a cooperative launch needs every CTA on the device together)
-    int coop = 0, occ_ps = 0;
+    int coop = 0, occ_ps = 0, occ_pm = 0;
     SLAB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     SLAB_CUDA(cudaFuncSetAttribute(k32::k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k32::PERSIST_SMEM));
     SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_ps, k32::k_persist, k32::P2G_T, k32::PERSIST_SMEM));
-    grid_persist = coop ? sms * occ_ps : 0;
+    SLAB_CUDA(cudaFuncSetAttribute(k32::k_persist_many, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k32::PERSIST_MANY_SMEM));
+    SLAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_pm, k32::k_persist_many, k32::P2X_T, k32::PERSIST_MANY_SMEM));
+    grid_persist = coop && occ_pm > 0 ? sms * occ_ps : 0;
+    grid_persist_many = sms * occ_pm;
     if (const char* e = std::getenv("SLAB_PERSIST")) persist = std::atoi(e) != 0 && grid_persist > 0;
     timer.nk = NKERNELS;  // k_prep, P2G, grid update (unless G2P does it), G2P, k_end
     const int phase_map[NKERNELS] = {1, 2, 3, 4, 0};
@@ -825,7 +828,7 @@ void Engine32::set_persistent(bool on, long long limit_cycles) {
     if (limit_cycles > 0) persist_limit = limit_cycles;
 }
 
-// One cooperative launch of k_persist for `chunk` steps. The barrier state
+// One cooperative launch of k_persist or k_persist_many for `chunk` steps. The barrier state
 // starts from zero at every launch (a launch whose waits ran out leaves it
 // anywhere).
 void Engine32::launch_persistent(int chunk) {
@@ -840,7 +843,8 @@ void Engine32::launch_persistent(int chunk) {
     long long lim = persist_limit;
     k32::GridBar* bar = reinterpret_cast<k32::GridBar*>(d_bar.get());
     void* args[] = {&sh, &z64, &n, &lim, &bar, &dem_map};
-    SLAB_CUDA(cudaLaunchCooperativeKernel((const void*)k32::k_persist, dim3(grid_persist), dim3(k32::P2G_T), args, k32::PERSIST_SMEM, st));
+    if (fused()) SLAB_CUDA(cudaLaunchCooperativeKernel((const void*)k32::k_persist, dim3(grid_persist), dim3(k32::P2G_T), args, k32::PERSIST_SMEM, st));
+    else SLAB_CUDA(cudaLaunchCooperativeKernel((const void*)k32::k_persist_many, dim3(grid_persist_many), dim3(k32::P2X_T), args, k32::PERSIST_MANY_SMEM, st));
     nlaunch += 1;
 }
 

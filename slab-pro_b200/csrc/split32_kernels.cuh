@@ -1893,8 +1893,7 @@ __device__ __forceinline__ void p2g_cell_tile(P2GCellSmem& sm, const TileDesc& D
     }
 }
 
-__global__ void __launch_bounds__(P2X_T, SLAB_P2X_MIN_BLOCKS) k_p2g_cells(Shared sh, const __grid_constant__ CUtensorMap dem_map) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
+__device__ __forceinline__ void p2g_cells_body(const Shared& sh, unsigned char* smem_raw, const CUtensorMap* dem_map) {
     P2GCellSmem& sm = *reinterpret_cast<P2GCellSmem*>(smem_raw);
     const int tid = threadIdx.x;
     int dn = 0;
@@ -1912,7 +1911,7 @@ __global__ void __launch_bounds__(P2X_T, SLAB_P2X_MIN_BLOCKS) k_p2g_cells(Shared
     if (sh.nscn == 1) load_scn_step(sh, 0, sm.z, tid);
     const int nwork = sh.work_pref[sh.nscn];
     const WorkItems W = work_items(sh, nwork, blockIdx.x, gridDim.x);
-    P2GNext<P2GCellSmem> next{sm, sh, &dem_map, W.w0, W.w1, W.step, 0, W.w1, 0, many_rounds(sh, nwork), false, 0};
+    P2GNext<P2GCellSmem> next{sm, sh, dem_map, W.w0, W.w1, W.step, 0, W.w1, 0, many_rounds(sh, nwork), false, 0};
     if (tid == 0 && next.w < next.w1) next.take();
     if (words && next.w < next.w1 && next.w != (int)blockIdx.x) dn = reinterpret_cast<const int*>(sh.desc + next.w)[tid];
     if (words) reinterpret_cast<int*>(&sm.d[0])[tid] = dn;
@@ -1928,7 +1927,7 @@ __global__ void __launch_bounds__(P2X_T, SLAB_P2X_MIN_BLOCKS) k_p2g_cells(Shared
             load_scn(sh, D.sid, sm.z, tid, P2X_T);
             __syncthreads();
         }
-        if (!next.requested) p2g_request(sm, sh, D, q, cb, &dem_map);
+        if (!next.requested) p2g_request(sm, sh, D, q, cb, dem_map);
         if (D.fresh) p2g_clear_fresh(sh, sm.z.s, D, sm.z.y.outs != 0, tid, P2X_T);
         cpa::wait_all();
         float* part = sh.part + (size_t)D.slot * PART_STRIDE;
@@ -1950,6 +1949,11 @@ __global__ void __launch_bounds__(P2X_T, SLAB_P2X_MIN_BLOCKS) k_p2g_cells(Shared
         tma::mbar_inval(&sm.dem_bar[0]);
         tma::mbar_inval(&sm.dem_bar[1]);
     }
+}
+
+__global__ void __launch_bounds__(P2X_T, SLAB_P2X_MIN_BLOCKS) k_p2g_cells(Shared sh, const __grid_constant__ CUtensorMap dem_map) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    p2g_cells_body(sh, smem_raw, &dem_map);
 }
 
 // ------------------------------------------------------------ grid update
@@ -2075,12 +2079,11 @@ __device__ __forceinline__ float4 window_node(const Shared& sh, const Scn& Z, co
 // of divisions, so what counts is how many warps an SM has in flight. Mass and
 // active nodes (diagnostics) are added up over a warp's run of one scenario.
 constexpr int GRID_T = 128;
-constexpr int GRID_MAX_WARPS = GRID_T / 32;
 
-__device__ __forceinline__ void grid_body(const Shared& sh) {
-    __shared__ ScnSm s_scn[GRID_MAX_WARPS];
+template <int T> __device__ __forceinline__ void grid_body(const Shared& sh) {  // T: threads of a CTA
+    __shared__ ScnSm s_scn[T / 32];
     constexpr int PARTS = NCELL / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = T / 32;
     ScnSm& zs = s_scn[warp];
     const int gw = (int)blockIdx.x * nwarp + warp, gn = (int)gridDim.x * nwarp;
     if (sh.nscn == 1) load_scn_static(sh, 0, zs, lane, 32);
@@ -2151,7 +2154,7 @@ __device__ __forceinline__ void grid_body(const Shared& sh) {
 #ifndef SLAB_GRID_MIN_BLOCKS
 #define SLAB_GRID_MIN_BLOCKS 8
 #endif
-__global__ void __launch_bounds__(GRID_T, SLAB_GRID_MIN_BLOCKS) k_grid(Shared sh) { grid_body(sh); }
+__global__ void __launch_bounds__(GRID_T, SLAB_GRID_MIN_BLOCKS) k_grid(Shared sh) { grid_body<GRID_T>(sh); }
 
 // -------------------------------------------------------------------- G2P
 
@@ -2590,9 +2593,10 @@ __device__ __forceinline__ bool grid_sync(const Shared& sh, GridBar* bar, long l
     return s_ok != 0;
 }
 
-// Shared memory of the persistent kernel: the largest phase's, reused by
+// Shared memory of the persistent kernels: the largest phase's, reused by
 // every phase (each phase initialises what it reads).
 constexpr size_t PERSIST_SMEM = sizeof(P2GTileSmem) > sizeof(G2PSmem<P2G_T>) ? sizeof(P2GTileSmem) : sizeof(G2PSmem<P2G_T>);
+constexpr size_t PERSIST_MANY_SMEM = sizeof(P2GCellSmem) > sizeof(G2PSmem<P2X_T>) ? sizeof(P2GCellSmem) : sizeof(G2PSmem<P2X_T>);
 
 // Up to nsteps whole steps (K1 tile bookkeeping, K2 P2G, K3 grid update and
 // K4 G2P, K5 end of step) in one launch, the phases separated by grid_sync
@@ -2600,8 +2604,17 @@ constexpr size_t PERSIST_SMEM = sizeof(P2GTileSmem) > sizeof(G2PSmem<P2G_T>) ? s
 // over the same work lists and in the same per-tile order, so a step gives
 // the same bits either way. The launch ends early once no scenario has work
 // (every one stopped at its frame, step budget or end).
-__global__ void __launch_bounds__(P2G_T, SLAB_P2G_MIN_BLOCKS) k_persist(Shared sh, const double* __restrict__ z64, int nsteps, long long limit,
-                                                                        GridBar* bar, const __grid_constant__ CUtensorMap dem_map) {
+// Two kernels by the same rule as the separate ones (Engine32::fused), each with
+// the CTAs of its P2G. One register budget serves all phases of a kernel:
+//   k_persist       4 CTAs per SM, 80 registers (100 bytes of spill stores). us per
+//                   step at 878 / 56 k / 198 k particles 25.6 / 28 / 40; 5 CTAs 28 /
+//                   31 / 44, 6 CTAs (484 bytes) 30 / 34 / 50, 3 CTAs 24.5 / 27.5 / 45.
+//   k_persist_many  8 CTAs per SM, 128 registers (52 bytes). 2 M particles 154 us
+//                   per step, 256 scenarios over 6 000 steps 19.8 s; 9 CTAs (268
+//                   bytes) 170 and 22.1; these steps by k_persist 173 and 23.1.
+template <bool MANY>
+__device__ __forceinline__ void persist_steps(const Shared& sh, const double* __restrict__ z64, int nsteps, long long limit, GridBar* bar,
+                                              const CUtensorMap* dem_map) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // after a launch whose waits ran out, the tile bookkeeping of the step it
     // left is half done: no phase may run on it again
@@ -2609,14 +2622,37 @@ __global__ void __launch_bounds__(P2G_T, SLAB_P2G_MIN_BLOCKS) k_persist(Shared s
     for (int s = 0; s < nsteps; ++s) {
         prep_body(sh);
         if (!grid_sync(sh, bar, limit)) return;
-        p2g_tiles_body(sh, smem_raw, &dem_map);
-        if (!grid_sync(sh, bar, limit)) return;
-        g2p_body<P2G_T, true>(sh, z64, *reinterpret_cast<G2PSmem<P2G_T>*>(smem_raw));
+        if constexpr (MANY) {
+            p2g_cells_body(sh, smem_raw, dem_map);
+            if (!grid_sync(sh, bar, limit)) return;
+            grid_body<P2X_T>(sh);
+            if (!grid_sync(sh, bar, limit)) return;
+            g2p_body<P2X_T, false>(sh, z64, *reinterpret_cast<G2PSmem<P2X_T>*>(smem_raw));
+        } else {
+            p2g_tiles_body(sh, smem_raw, dem_map);
+            if (!grid_sync(sh, bar, limit)) return;
+            g2p_body<P2G_T, true>(sh, z64, *reinterpret_cast<G2PSmem<P2G_T>*>(smem_raw));
+        }
         if (!grid_sync(sh, bar, limit)) return;
         if (blockIdx.x == 0) control_scenarios(sh, CTL_END);
         if (!grid_sync(sh, bar, limit)) return;
         if (*reinterpret_cast<volatile const int*>(sh.work_pref + sh.nscn) == 0) break;  // the same value in every CTA
     }
+}
+
+#ifndef SLAB_PERSIST_MIN_BLOCKS
+#define SLAB_PERSIST_MIN_BLOCKS (NCELL == 64 ? 4 : 1)
+#endif
+__global__ void __launch_bounds__(P2G_T, SLAB_PERSIST_MIN_BLOCKS) k_persist(Shared sh, const double* __restrict__ z64, int nsteps, long long limit,
+                                                                            GridBar* bar, const __grid_constant__ CUtensorMap dem_map) {
+    persist_steps<false>(sh, z64, nsteps, limit, bar, &dem_map);
+}
+#ifndef SLAB_PERSIST_MANY_MIN_BLOCKS
+#define SLAB_PERSIST_MANY_MIN_BLOCKS SLAB_P2X_MIN_BLOCKS
+#endif
+__global__ void __launch_bounds__(P2X_T, SLAB_PERSIST_MANY_MIN_BLOCKS)
+    k_persist_many(Shared sh, const double* __restrict__ z64, int nsteps, long long limit, GridBar* bar, const __grid_constant__ CUtensorMap dem_map) {
+    persist_steps<true>(sh, z64, nsteps, limit, bar, &dem_map);
 }
 
 // Particle z and vz at the current positions (for downloads between output
