@@ -122,6 +122,17 @@ __device__ inline void take_box(Ctl* c) {
     for (int k = 0; k < 4; ++k) c->pos[k] = c->pos_acc[k];
 }
 
+// The grid box of the step from its particle box; false if it leaves the terrain.
+// The box of the step before then stays: downloads of the grid go by it.
+__device__ inline bool remesh(Ctl* c, int Nx, int Ny) {
+    int32_t b[4];
+    remesh_box(__longlong_as_double((long long)c->pos[0]), __longlong_as_double((long long)c->pos[1]),
+               __longlong_as_double((long long)c->pos[2]), __longlong_as_double((long long)c->pos[3]), c->dx, c->one_over_dx, b);
+    if (b[0] < 0 || b[2] < 0 || b[1] > Nx - 1 || b[3] > Ny - 1) return false;
+    for (int k = 0; k < 4; ++k) c->box[k] = b[k];
+    return true;
+}
+
 // Start of a step, one thread: the stop conditions of the running advance
 // call, then Simulation::updateDt (src/simulation.cpp:565-582) from the
 // previous G2P's max |v|^2, then the reference's remesh box from the
@@ -150,9 +161,7 @@ __device__ inline void ctl_begin(Ctl* c, int Nx, int Ny) {
     c->frame_end = (next_frame_time - c->new_time < 1e-13) ? 1 : 0;
     c->write_outputs = (c->frame_end || c->keep_outputs) ? 1 : 0;
     take_box(c);
-    remesh_box(__longlong_as_double((long long)c->pos[0]), __longlong_as_double((long long)c->pos[1]),
-               __longlong_as_double((long long)c->pos[2]), __longlong_as_double((long long)c->pos[3]), c->dx, c->one_over_dx, c->box);
-    if (c->box[0] < 0 || c->box[2] < 0 || c->box[1] > Nx - 1 || c->box[3] > Ny - 1) {
+    if (!remesh(c, Nx, Ny)) {
         c->err |= ERR_DOMAIN;
         c->stop = 1;
         return;
@@ -198,9 +207,7 @@ __device__ inline void ctl_begin_t0(Ctl* c, int Nx, int Ny) {
     c->frame_end = 0;
     c->write_outputs = 1;
     take_box(c);
-    remesh_box(__longlong_as_double((long long)c->pos[0]), __longlong_as_double((long long)c->pos[1]),
-               __longlong_as_double((long long)c->pos[2]), __longlong_as_double((long long)c->pos[3]), c->dx, c->one_over_dx, c->box);
-    if (c->box[0] < 0 || c->box[2] < 0 || c->box[1] > Nx - 1 || c->box[3] > Ny - 1) {
+    if (!remesh(c, Nx, Ny)) {
         c->err |= ERR_DOMAIN;
         return;
     }

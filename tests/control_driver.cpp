@@ -99,11 +99,14 @@ int main() {
     arm(c, 1);
     CHECK(c.active && box_is(c, 11, 24, 9, 34));
 
-    // a box outside the terrain still stops the run
+    // a box outside the terrain stops the run, and the grid keeps the box of its last step
     box_to(c, 12.5, 63.5, 10.5, 32.5);
     ctl_end(&c);
     arm(c, 1);
     CHECK(!c.active && c.stop && (c.err & ERR_DOMAIN));
+    CHECK(box_is(c, 11, 24, 9, 34));
+    ctl_begin_t0(&c, NX, NY);
+    CHECK(!c.active && box_is(c, 11, 24, 9, 34));
     std::printf("ok\n");
     return 0;
 }
