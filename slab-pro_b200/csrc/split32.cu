@@ -243,8 +243,9 @@ Engine32::Engine32(const Terrain& t, cudaStream_t s, int max_scn, int64_t blk_ca
     spare.resize(max_scn);
     d_collect = dalloc<int32_t>((size_t)ntiles + 8);
     d_free_blocks = dalloc<int32_t>(this->blk_cap);
-    SLAB_CUDA(cudaMemsetAsync(d_hmax.get(), 0, (size_t)this->blk_cap * NCELL * sizeof(float), st));
-    SLAB_CUDA(cudaMemsetAsync(d_vmax2.get(), 0, (size_t)this->blk_cap * NCELL * sizeof(float), st));
+    // maxima, and the output fields, which steps without output leave alone
+    for (const auto* f : {&d_hmax, &d_vmax2, &d_oh, &d_om, &d_ovz, &d_oFx, &d_oFy})
+        SLAB_CUDA(cudaMemsetAsync(f->get(), 0, (size_t)this->blk_cap * NCELL * sizeof(float), st));
     SLAB_CUDA(cudaMemsetAsync(d_blk_stamp.get(), 0xff, (size_t)this->blk_cap * sizeof(int32_t), st));
     SLAB_CUDA(cudaMemsetAsync(d_misc.get(), 0, 16 * sizeof(int32_t), st));
     SLAB_CUDA(cudaMemsetAsync(d_work_pref.get(), 0, (max_scn + 1) * sizeof(int32_t), st));
@@ -383,15 +384,17 @@ __global__ void k_collect_blocks(const int32_t* __restrict__ blk_of, int ntiles,
     }
 }
 
-__global__ void k_release_blocks(const int32_t* ids, int n, float* hmax, float* vmax2, int32_t* stamp, int32_t* owner) {
+// Node blocks as a new engine has them: nothing of this run shows in the next
+// one's maxima, nor in its output fields between frames.
+__global__ void k_release_blocks(const int32_t* ids, int n, Shared sh) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < (int64_t)n * NCELL; k += (int64_t)gridDim.x * blockDim.x) {
         const int b = ids[k / NCELL];
         const size_t e = (size_t)b * NCELL + (k % NCELL);
-        hmax[e] = 0.f;
-        vmax2[e] = 0.f;
+        sh.hmax[e] = sh.vmax2[e] = 0.f;
+        sh.oh[e] = sh.om[e] = sh.ovz[e] = sh.oFx[e] = sh.oFy[e] = 0.f;
         if (k % NCELL == 0) {
-            stamp[b] = -1;
-            owner[b] = -1;
+            sh.blk_stamp[b] = -1;
+            sh.blk_owner[b] = -1;
         }
     }
 }
@@ -408,7 +411,7 @@ void Engine32::retire(int sid, const Ctl& empty_ctl) {
         SLAB_CUDA(cudaStreamSynchronize(st));
         const int32_t* ids = d_collect.get() + 8;
         const int blocks = (int)std::min<int64_t>(((int64_t)nblk * NCELL + 255) / 256, 148 * 8);
-        k32::k_release_blocks<<<blocks, 256, 0, st>>>(ids, nblk, d_hmax.get(), d_vmax2.get(), d_blk_stamp.get(), d_blk_owner.get());
+        k32::k_release_blocks<<<blocks, 256, 0, st>>>(ids, nblk, shared());
         SLAB_CUDA(cudaGetLastError());
         SLAB_CUDA(cudaMemcpyAsync(d_free_blocks.get() + free_count, ids, (size_t)nblk * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
         const int32_t nf = free_count + nblk;
