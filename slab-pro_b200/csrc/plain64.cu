@@ -66,6 +66,12 @@ __device__ __forceinline__ double dNq(double u) {
     return 0.0;
 }
 
+// First node of a particle's stencil along one axis, from its position u >= 0 in
+// cells: truncated as the reference does it (src/simulation.cpp:741-742), so
+// that within half a cell of the terrain's first node the stencil starts at node
+// 0 (the node before it does not exist; the third node's weight is zero there).
+__device__ __forceinline__ int stencil_base(double u) { return (int)(u - 0.5); }
+
 __device__ __forceinline__ void stencil_weights(const Phys& P, double xp, int base, double w[3], double dw[3]) {
     for (int d = 0; d < 3; ++d) {
         const double u = (xp - (double)(base + d) * P.dx) * P.one_over_dx;
@@ -115,7 +121,7 @@ __global__ void __launch_bounds__(256) k64_p2g(const Ctl* c, P64 p, N64 n, const
     const bool outs = c->write_outputs;
     const double vmx = v.x * m, vmy = v.y * m;
     const double vzm = outs ? p.vz[q] * m : 0.0, hm = h * m, hA = h * A;
-    const int ib = (int)floor(x.x * P.one_over_dx - 0.5), jb = (int)floor(x.y * P.one_over_dx - 0.5);
+    const int ib = stencil_base(x.x * P.one_over_dx), jb = stencil_base(x.y * P.one_over_dx);
     const int cell = (int)floor(x.x * P.one_over_dx) * P.Ny + (int)floor(x.y * P.one_over_dx);
     const double2 gr = grad[cell];
     const double ct = cos_t[cell];
@@ -312,7 +318,7 @@ __global__ void __launch_bounds__(256) k64_g2p(Ctl* c, P64 p, N64 n, const doubl
         const double2 x = p.x[q];
         const int cell = (int)floor(x.x * P.one_over_dx) * P.Ny + (int)floor(x.y * P.one_over_dx);
         const double2 pg = grad[cell];
-        const int ib = (int)floor(x.x * P.one_over_dx - 0.5), jb = (int)floor(x.y * P.one_over_dx - 0.5);
+        const int ib = stencil_base(x.x * P.one_over_dx), jb = stencil_base(x.y * P.one_over_dx);
         double wx[3], wy[3], dwx[3], dwy[3];
         stencil_weights(P, x.x, ib, wx, dwx);
         stencil_weights(P, x.y, jb, wy, dwy);
