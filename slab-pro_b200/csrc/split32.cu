@@ -518,6 +518,21 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     S.Np = Np;
     S.ctl = ctl;
     S.h_ctl = h_ctl;
+    S.pending = 0;
+    // a scenario that is refused below leaves its slot, with its arrays, to the next
+    struct Undo {
+        Engine32* e;
+        int sid;
+        int64_t cap = 0;
+        ~Undo() {
+            if (!e) return;
+            e->work_cap_total -= cap;
+            e->pending_blocks -= e->slots[sid]->pending;
+            e->slots[sid]->pending = 0;
+            e->spare[sid] = std::move(e->slots[sid]);
+            if (sid < e->nscn) e->free_slots.push_back(sid);
+        }
+    } undo{this, sid};
     // a single scenario gets the safe bound; in a batch the lists start at an
     // estimate (>= 4 particles per active tile) and grow between chunks
     S.act_cap = batch ? std::max(1, std::min(ntiles, Np / 4 + 256)) : std::max(1, std::min(ntiles, Np));
@@ -547,7 +562,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
     }
     if (ctl0 + sid != ctl) throw Error{SLAB_E_STATE, "control blocks of a context's scenarios must be consecutive"};
     ensure_work_cap(work_cap_total + S.act_cap);
-    work_cap_total += S.act_cap;
+    work_cap_total += undo.cap = S.act_cap;
 
     // ---- bin the particles into tile segments on the device (stable in upload order)
     const double ood = 1.0 / T.dx;
@@ -625,6 +640,7 @@ int Engine32::add_scenario(const slab_params& p, Ctl* ctl, Ctl* h_ctl, int Np, c
         nscn += 1;
         graphs.clear();  // the step graphs carry the scenario count
     }
+    undo.e = nullptr;
     return sid;
 }
 
