@@ -118,8 +118,8 @@ namespace slab {
 // as it is: the accumulators are clear and hold no particle, and a box made of
 // them reaches far outside the terrain.
 __device__ inline void take_box(Ctl* c) {
-    if (c->pos_acc[0] == 0x7ff0000000000000ull) return;
-    for (int k = 0; k < 4; ++k) c->pos[k] = c->pos_acc[k];
+    const bool left = c->pos_acc[0] != 0x7ff0000000000000ull;
+    for (int k = 0; k < 4; ++k) c->pos[k] = left ? c->pos_acc[k] : c->pos[k];
 }
 
 // The grid box of the step from its particle box; false if it leaves the terrain.
@@ -128,9 +128,9 @@ __device__ inline bool remesh(Ctl* c, int Nx, int Ny) {
     int32_t b[4];
     remesh_box(__longlong_as_double((long long)c->pos[0]), __longlong_as_double((long long)c->pos[1]),
                __longlong_as_double((long long)c->pos[2]), __longlong_as_double((long long)c->pos[3]), c->dx, c->one_over_dx, b);
-    if (b[0] < 0 || b[2] < 0 || b[1] > Nx - 1 || b[3] > Ny - 1) return false;
-    for (int k = 0; k < 4; ++k) c->box[k] = b[k];
-    return true;
+    const bool inside = b[0] >= 0 && b[2] >= 0 && b[1] <= Nx - 1 && b[3] <= Ny - 1;
+    for (int k = 0; k < 4; ++k) c->box[k] = inside ? b[k] : c->box[k];
+    return inside;
 }
 
 // Start of a step, one thread: the stop conditions of the running advance
